@@ -205,6 +205,66 @@ def run(state):
                                           window_size=None if case["window"] < 0 else case["window"])
 
 
+def _exact_heads(q, r, k, v, window, first=0):
+    """The operator in 64 bits for some heads: q, r (heads, lq, d) at the last positions of k, v (heads, lk, d);
+    keys before `first` are padding.  With S1 = q.k / sqrt(d), S2 = r.k and P = softmax(S1) over the visible keys
+    the result is (1 + sum(P S2)) P v - (P S2) v."""
+    lq, lk = q.shape[1], k.shape[1]
+    at = torch.arange(lk - lq, lk, device=q.device).view(-1, 1)
+    key = torch.arange(lk, device=q.device).view(1, -1)
+    hidden = (key > at) | (key < first)
+    if window >= 0:
+        hidden = hidden | (key <= at - window)
+    p = torch.softmax((q @ k.mT * q.shape[2] ** -0.5).masked_fill(hidden, -math.inf), dim=-1)
+    ps2 = p * (r @ k.mT)
+    return (1 + ps2.sum(-1, keepdim=True)) * (p @ v) - ps2 @ v
+
+
+def _exact_sequence(q, r, k, v, window, first=0, grad=None):
+    """`_exact_heads` for one sequence of 16-bit tensors (tokens, heads, d), a few kv heads at a time; with `grad`
+    the gradients of the four inputs too."""
+    hq, hkv = q.shape[1], k.shape[1]
+    rep = hq // hkv
+    step = max(1, 2 ** 26 // (q.shape[0] * k.shape[0] * rep))
+    parts = []
+    for h in range(0, hkv, step):
+        n = min(step, hkv - h)
+        x = [t[:, a:b].transpose(0, 1).double().requires_grad_(grad is not None)
+             for t, a, b in ((q, h * rep, (h + n) * rep), (r, h * rep, (h + n) * rep), (k, h, h + n), (v, h, h + n))]
+        with torch.set_grad_enabled(grad is not None):
+            o = _exact_heads(x[0], x[1], *(t.repeat_interleave(rep, 0) for t in x[2:]), window, first)
+        got = [o.detach()]
+        if grad is not None:
+            got += torch.autograd.grad(o, x, grad[:, h * rep:(h + n) * rep].transpose(0, 1).double())
+        parts.append([t.transpose(0, 1) for t in got])
+    return [torch.cat(t, 1) for t in zip(*parts)]
+
+
+def exact(case, seed):
+    """What `run` returns, in 64 bits and plain torch."""
+    state, kind, window = prepare(case, seed), case["kind"], case["window"] if "window" in case else -1
+    if kind == "train":
+        x = [t.detach().transpose(1, 2) for t in (*state["leaves"], state["grad"])]
+        rows = [_exact_sequence(*(t[i] for t in x[:4]), window, grad=x[4][i]) for i in range(case["b"])]
+        return tuple(torch.stack(t).transpose(1, 2) for t in zip(*rows))
+    if kind == "varlen":
+        x = [t.detach()[0] for t in (*state["leaves"], state["grad"])]
+        parts, at = [], 0
+        for n in _sequence_lengths(case):
+            parts.append(_exact_sequence(*(t[at:at + n] for t in x[:4]), window, grad=x[4][at:at + n]))
+            at += n
+        return tuple(torch.cat(t).unsqueeze(0) for t in zip(*parts))
+    caches = (state["step"].k, state["step"].v) if kind == "graph" else (state["k"], state["v"])
+    rows = []
+    for i, (n, first) in enumerate(zip(_row_lengths(case), _row_starts(case))):
+        if case.get("page"):
+            k, v = (c[state["table"][i].long()].flatten(0, 1)[:n] for c in caches)
+        else:
+            k, v = (c[i, :n] for c in caches)
+        rows.append(_exact_sequence(state["q"][i], state["r"][i], k, v, window, first)[0])
+    return torch.stack(rows)
+
+
 def _causal_pairs(lq, lk, window):
     """Visible (query, key) pairs of one head: the lq queries are the last positions of lk keys."""
     if window < 0 or window >= lk:
