@@ -26,7 +26,7 @@
 extern "C" {
 #endif
 
-#define PLX_ABI_VERSION 2
+#define PLX_ABI_VERSION 3
 
 /* cudaStream_t without pulling in the CUDA headers */
 typedef struct CUstream_st *plx_stream_t;
@@ -91,6 +91,23 @@ int plx_train_workspace_bytes(const plx_train_problem *p, size_t *bytes);
 int plx_train_fwd(const plx_train_problem *p, const void *q, const void *r, const void *k,
                   const void *v, void *o, void *barv, float *d1, float *bart, float *m,
                   plx_stream_t stream);
+
+/* Several query rows per sequence against a KV cache (prefill / extend): the len_q
+ * queries of batch row b are the LAST len_q of its seqused_k[b] active keys (device,
+ * int32; NULL: len_k for every row; values are kept inside [len_q, len_k]).  One launch
+ * for all rows.  Dense cache: page_table NULL, k / v (batch, len_k, ...) by the problem's
+ * strides.  Paged: page_table (device, int32, batch x pages_per_seq), kv_stride_b is
+ * the page stride of a pool of n_pages pages of page_size keys (a power of two) and
+ * len_k <= pages_per_seq * page_size; entries past a row's active length are not read.
+ * Keys past the active length never reach the output.  Writes o only.
+ * PLX_ERR_UNSUPPORTED (nothing enqueued): window_left 0, qk_scale <= 0, a page of fewer
+ * than 8 keys, a zero k / v stride; gather the pages and call plx_train_fwd per row then.
+ * (L_q > 1 and page_table are named but not implemented upstream
+ * [parallax/cute/parallax_decode.py:1578-1580, 1627-1632].) */
+int plx_train_extend(const plx_train_problem *p, const void *q, const void *r, const void *k,
+                     const void *v, void *o, const int32_t *seqused_k, const int32_t *page_table,
+                     int32_t page_size, int32_t pages_per_seq, int32_t n_pages,
+                     plx_stream_t stream);
 
 /* Backward: dq, dr (q-like) and dk, dv (kv-like, already summed over the q heads
  * of a group).  `workspace` must hold plx_train_workspace_bytes() bytes.

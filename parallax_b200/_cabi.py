@@ -15,12 +15,12 @@ PLX_BF16, PLX_FP16 = 0, 1
 PLX_ERR_UNSUPPORTED = -2
 PLX_ERR_STATIC_SCRATCH = -6
 DECODE_STATIC_SCRATCH_BYTES = 4 << 20
-ABI_VERSION = 2
+ABI_VERSION = 3
 
 # every symbol include/plx_abi.h declares
 SYMBOLS = (
     "plx_abi_version", "plx_strerror", "plx_kernel_launch_count", "plx_device_error", "plx_device_error_peek",
-    "plx_train_workspace_bytes", "plx_train_fwd", "plx_train_bwd", "plx_train_bwd_stages",
+    "plx_train_workspace_bytes", "plx_train_fwd", "plx_train_extend", "plx_train_bwd", "plx_train_bwd_stages",
     "plx_decode_choose_splits", "plx_decode_choose_splits_gqa", "plx_decode_workspace_bytes", "plx_decode", "plx_decode_static", "plx_decode_partial",
     "plx_decode_merge", "plx_decode_exchange_bytes", "plx_decode_exchange_merge", "plx_decode_partial_exchange",
 )
@@ -85,6 +85,8 @@ def _declare(lib):
     lib.plx_train_workspace_bytes.argtypes = [C.POINTER(TrainProblem), C.POINTER(sz)]
     lib.plx_train_fwd.restype = C.c_int
     lib.plx_train_fwd.argtypes = [C.POINTER(TrainProblem)] + [vp] * 9 + [vp]
+    lib.plx_train_extend.restype = C.c_int
+    lib.plx_train_extend.argtypes = [C.POINTER(TrainProblem)] + [vp] * 7 + [i32, i32, i32, vp]
     lib.plx_train_bwd.restype = C.c_int
     lib.plx_train_bwd.argtypes = [C.POINTER(TrainProblem)] + [vp] * 14 + [vp, sz, vp]
     lib.plx_train_bwd_stages.restype = C.c_int

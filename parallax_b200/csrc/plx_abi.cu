@@ -241,6 +241,30 @@ int plx_train_fwd(const plx_train_problem *p, const void *q, const void *r, cons
     return launch_train_fwd_mma(a, p->dtype, p->head_dim, reinterpret_cast<cudaStream_t>(stream));
 }
 
+int plx_train_extend(const plx_train_problem *p, const void *q, const void *r, const void *k, const void *v, void *o,
+                     const int32_t *seqused_k, const int32_t *page_table, int32_t page_size, int32_t pages_per_seq,
+                     int32_t n_pages, plx_stream_t stream) {
+    int st = check_train(p);
+    if (st != PLX_OK) return st;
+    if (!q || !r || !k || !v || !o || p->cu_seqlens || p->len_q > p->len_k) return PLX_ERR_BAD_ARG;
+    if (misaligned16(q) || misaligned16(r) || misaligned16(k) || misaligned16(v) || misaligned16(o)) return PLX_ERR_BAD_ARG;
+    TrainArgs a = make_train_args(p);
+    a.q = q; a.r = r; a.k = k; a.v = v; a.o = o;
+    a.seqused = seqused_k;
+    if (page_table) {
+        if (page_size < 1 || (page_size & (page_size - 1)) != 0 || pages_per_seq < 1 || n_pages < 1) return PLX_ERR_BAD_ARG;
+        if (static_cast<int64_t>(pages_per_seq) * page_size < p->len_k) return PLX_ERR_BAD_ARG;
+        a.page_table = page_table;
+        a.pages_per_seq = pages_per_seq;
+        a.n_pages = n_pages;
+        a.page_mask = page_size - 1;
+        while ((1 << a.page_shift) < page_size) ++a.page_shift;
+    }
+    if ((st = check_device()) != PLX_OK) return st;
+    if (!train_extend_sm100_supported(a, p->head_dim)) return PLX_ERR_UNSUPPORTED;
+    return launch_train_extend_sm100(a, p->dtype, p->head_dim, reinterpret_cast<cudaStream_t>(stream));
+}
+
 int plx_train_bwd_stages(const plx_train_problem *p, int32_t stages, const void *q, const void *r, const void *k,
                          const void *v, const void *o, const void *barv, const float *d1, const float *bart,
                          const float *m, const void *grad_o, void *dq, void *dr, void *dk, void *dv, void *workspace,

@@ -129,6 +129,9 @@ struct TrainArgs {
     float *cst;  // compact copy {b, mL, 1 + bart, (b - t) * scale}, 4 floats per (batch, head, token)
     const int32_t *cu;
     int n_seqs;
+    // forward against a KV cache only: active keys per batch row (null: len_k), page table (null: dense)
+    const int32_t *seqused, *page_table;
+    int pages_per_seq, page_shift, page_mask, n_pages;
     int batch, heads_q, heads_kv, n_rep, len_q, len_k, window;
     float scale, c2;  // c2 = scale * log2(e)
     int64_t q_sb, q_sh, q_st, kv_sb, kv_sh, kv_st, st_sb, st_sh, st_st;

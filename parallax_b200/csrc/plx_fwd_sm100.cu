@@ -62,6 +62,7 @@ constexpr uint32_t kQPanel = kBM * 128;       // bytes of one 64-channel panel o
 constexpr uint32_t kKVPanel = kBN * 128;
 constexpr uint32_t kTmemCols = 512;
 constexpr float kRescaleThreshold = 8.f;
+constexpr int kMinPage = 8;                   // smallest page a tile can be copied from: boxes start on 1024-byte boundaries (8 rows)
 
 template <typename T>
 struct Fmt;
@@ -87,7 +88,7 @@ struct Smem {
     // barrier indices (8 bytes each)
     static constexpr int kQFull = 0, kQEmpty = 1, kOFree = 2, kKFull = 3, kKEmpty = kKFull + NS,
                          kVFull = kKEmpty + NS, kVEmpty = kVFull + NS, kSFull = kVEmpty + NS, kSFree = kSFull + 3,
-                         kPFull = kSFree + 1, kPVDone = kPFull + 3, kNumBars = kPVDone + 3;
+                         kPFull = kSFree + 1, kPVDone = kPFull + 3, kTail = kPVDone + 3, kNumBars = kTail + 2;   // kTail: K, V (EXT only)
     static constexpr uint32_t kTmemSlot = kBars + 8 * kNumBars;
     static constexpr uint32_t kBytes = kTmemSlot + 16 + 1024;  // + slack to align the base to 1024
 };
@@ -101,6 +102,7 @@ struct Item {
 // Work item `idx` of the launch.  Items are ordered (batch, head)-major so that CTAs running at the
 // same time share K / V in L2; inside a (batch, head) the row tiles alternate last, first, last - 1,
 // second, ... so that under a causal mask any two neighbours add up to the same work.
+template <bool EXT>
 __device__ __forceinline__ Item get_item(const TrainArgs &a, int idx, int n_rt) {
     Item it;
     const int bh = idx / n_rt, k = idx % n_rt;
@@ -114,6 +116,8 @@ __device__ __forceinline__ Item get_item(const TrainArgs &a, int idx, int n_rt) 
     it.r0 = tis * kBM;
     if (it.valid && it.r0 >= it.nq) it.valid = false;
     it.b = bh / a.heads_q;
+    // a row's own active length, kept inside what the tensor map (or the page table) covers
+    if (EXT && a.seqused) it.nk = min(max(__ldg(a.seqused + it.b), it.nq), a.len_k);
     it.h = bh % a.heads_q;
     it.hk = it.h / a.n_rep;
     it.off = it.nk - it.nq;
@@ -133,7 +137,10 @@ __device__ __forceinline__ int item_index(int n, int chunk_shift) {
 // Persistent kernel: gridDim.x CTAs (at most one per SM) walk the item list, so the loads and first
 // score products of the next item overlap the epilogue of the current one, and the TMEM allocation,
 // barrier set-up and launch latency are paid once per SM.
-template <typename T, int D, int NS>
+//
+// EXT is the same kernel against a KV cache: the key count is the batch row's own (a.seqused), keys may be
+// paged (a tile is then one TMA box per page it touches, 64 keys at most), and only `o` is written.
+template <typename T, int D, int NS, bool EXT>
 __global__ void __launch_bounds__(352, 1)
 fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_r,
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const ErrSink sink, int n_rt,
@@ -193,13 +200,16 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
             const CUtensorMap *map = is_k ? &tm_k : &tm_v;
             const uint32_t ring = is_k ? sK : sV;
             const int full0 = is_k ? L::kKFull : L::kVFull, empty0 = is_k ? L::kKEmpty : L::kVEmpty;
-            int s = 0, n_issued = 0, n_items_done = 0;
+            // paged cache: a tile is kBN >> box_shift boxes of min(page size, 64) keys
+            constexpr int kMaxBoxes = kBN / kMinPage;
+            const int box_shift = EXT ? min(a.page_shift, 6) : 6;
+            int s = 0, n_issued = 0, n_items_done = 0, n_tails = 0;
             uint32_t ph = 0;
             bool ok = true;
             for (int n = 0; ok; ++n) {
                 const int idx = item_index(n, chunk_shift);
                 if (idx >= n_items) break;
-                const Item it = get_item(a, idx, n_rt);
+                const Item it = get_item<EXT>(a, idx, n_rt);
                 if (it.n_tiles == 0) continue;
                 if (is_k) {
                     // the q / r tiles of the previous item are free once its last score product has completed
@@ -214,13 +224,52 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
                 }
                 ++n_items_done;
                 for (int j = 0; j < it.n_tiles; ++j) {
+                    const int key0 = (it.t_lo + j) * kBN;
+                    int page[kMaxBoxes];
+                    if (EXT && a.page_table) {
+                        // the tile's page numbers, read before the wait so that their latency is hidden by it
+#pragma unroll
+                        for (int i = 0; i < kMaxBoxes; ++i) {
+                            const int key = key0 + (i << box_shift);
+                            page[i] = (i << box_shift) < kBN && key < it.nk
+                                          ? __ldg(a.page_table + static_cast<int64_t>(it.b) * a.pages_per_seq + (key >> a.page_shift)) : 0;
+                        }
+                    }
                     ok = mbar_wait(bar(empty0 + s), ph ^ 1, err, is_k ? 2 : 3);
                     if (!ok) break;
-                    mbar_expect_tx(bar(full0 + s), kKVBytes);
+                    const uint32_t dst = ring + s * kKVBytes;
+                    // A tile that reaches past the row's active length inside the cache: what lies there must not
+                    // be seen (0 * NaN), so its rows are zeroed once the copy has landed, before the tile is handed
+                    // over.  (Past the end of a tensor map the copy itself fills zeros.)
+                    const bool tail = EXT && key0 + kBN > it.nk && (a.page_table || it.nk < a.len_k);
+                    const uint32_t full = bar(tail ? L::kTail + (is_k ? 0 : 1) : full0 + s);
+                    if (EXT && a.page_table) {
+                        const int n_boxes = min(kBN >> box_shift, (it.nk - key0 + (1 << box_shift) - 1) >> box_shift);
+                        mbar_expect_tx(full, static_cast<uint32_t>(n_boxes) * (128u * L::kPanels << box_shift));
 #pragma unroll
-                    for (int pn = 0; pn < L::kPanels; ++pn)
-                        tma_load_4d(ring + s * kKVBytes + pn * kKVPanel, map, bar(full0 + s), 64 * pn, it.bos + (it.t_lo + j) * kBN,
-                                    it.hk, it.b);
+                        for (int i = 0; i < kMaxBoxes; ++i)
+                            if (i < n_boxes)
+                                for (int pn = 0; pn < L::kPanels; ++pn)
+                                    tma_load_4d(dst + pn * kKVPanel + (128u * i << box_shift), map, full, 64 * pn,
+                                                (key0 + (i << box_shift)) & a.page_mask, it.hk, page[i]);
+                    } else {
+                        mbar_expect_tx(full, kKVBytes);
+#pragma unroll
+                        for (int pn = 0; pn < L::kPanels; ++pn)
+                            tma_load_4d(dst + pn * kKVPanel, map, full, 64 * pn, it.bos + key0, it.hk, it.b);
+                    }
+                    if (tail) {
+                        ok = mbar_wait(full, n_tails & 1, err, is_k ? 17 : 18);
+                        if (!ok) break;
+                        ++n_tails;
+                        for (int row = it.nk - key0; row < kBN; ++row)
+                            for (int pn = 0; pn < L::kPanels; ++pn)
+#pragma unroll
+                                for (int c = 0; c < 8; ++c)
+                                    asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};\n" ::"r"(dst + pn * kKVPanel + row * 128 + c * 16), "r"(0u) : "memory");
+                        fence_proxy_async();
+                        mbar_arrive(bar(full0 + s));
+                    }
                     ++n_issued;
                     if (++s == NS) {
                         s = 0;
@@ -257,7 +306,7 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
             for (int n = 0; ok; ++n) {
                 const int idx = item_index(n, chunk_shift);
                 if (idx >= n_items) break;
-                const Item it = get_item(a, idx, n_rt);
+                const Item it = get_item<EXT>(a, idx, n_rt);
                 if (it.n_tiles == 0) continue;
                 ok = __all_sync(0xffffffffu, mbar_wait(bar(L::kQFull), n_items_done & 1, err, 4));
                 ++n_items_done;
@@ -313,7 +362,7 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
             for (int n = 0; ok; ++n) {
                 const int idx = item_index(n, chunk_shift);
                 if (idx >= n_items) break;
-                const Item it = get_item(a, idx, n_rt);
+                const Item it = get_item<EXT>(a, idx, n_rt);
                 if (it.n_tiles == 0) continue;
                 for (int j = 0; j < it.n_tiles && ok; ++j, ++g) {
                     const int buf = g % kPBufs;
@@ -368,7 +417,7 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
         for (int n = 0; ok; ++n) {
             const int idx = item_index(n, chunk_shift);
             if (idx >= n_items) break;
-            const Item it = get_item(a, idx, n_rt);
+            const Item it = get_item<EXT>(a, idx, n_rt);
             if (!it.valid) continue;
             if (it.n_tiles == 0) {
                 // no key is visible to any row of the tile: outputs are zero (one thread per row and column half)
@@ -376,15 +425,15 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
                 if (row < it.nq) {
                     const int64_t q_base = it.b * a.q_sb + it.h * a.q_sh + static_cast<int64_t>(it.bos + row) * a.q_st;
                     T *go = static_cast<T *>(a.o) + q_base + (D / 2) * hf;
-                    T *gb = static_cast<T *>(a.barv) + q_base + (D / 2) * hf;
+                    T *gb = EXT ? nullptr : static_cast<T *>(a.barv) + q_base + (D / 2) * hf;
                     const int64_t si = it.b * a.st_sb + it.h * a.st_sh + static_cast<int64_t>(it.bos + row) * a.st_st;
                     const uint4 z = make_uint4(0u, 0u, 0u, 0u);
 #pragma unroll
                     for (int i = 0; i < D / 16; ++i) {
                         *reinterpret_cast<uint4 *>(go + 8 * i) = z;
-                        *reinterpret_cast<uint4 *>(gb + 8 * i) = z;
+                        if (!EXT) *reinterpret_cast<uint4 *>(gb + 8 * i) = z;
                     }
-                    if (hf == 0) {
+                    if (!EXT && hf == 0) {
                         a.d1[si] = 0.f;
                         a.bart[si] = 0.f;
                         a.m[si] = -INFINITY;
@@ -566,7 +615,7 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
                 inv[hh] = r1f > 0.f ? 1.f / r1f : 0.f;                           // normaliser of the output
                 bart_o[hh] = r2f * inv[hh];                                      // bart used for the output
                 const int row = r0 + rl0 + 8 * hh;
-                if (t == 0 && row < it.nq) {
+                if (!EXT && t == 0 && row < it.nq) {
                     const int64_t si = it.b * a.st_sb + it.h * a.st_sh + static_cast<int64_t>(it.bos + row) * a.st_st;
                     // the sums are relative to m_ref; the saved pair is relative to the true row maximum
                     a.d1[si] = (m_true[hh] == -INFINITY) ? 0.f : s1f * fast_exp2(m_ref[hh] - m_true[hh]);
@@ -580,7 +629,7 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
             tc_fence_after();
             const int64_t q_base = it.b * a.q_sb + it.h * a.q_sh + static_cast<int64_t>(it.bos + r0 + rl0) * a.q_st + 8 * t;
             T *go = static_cast<T *>(a.o) + q_base;
-            T *gb = static_cast<T *>(a.barv) + q_base;
+            T *gb = EXT ? nullptr : static_cast<T *>(a.barv) + q_base;
 #pragma unroll
             for (int cc = 0; cc < D / 64; ++cc) {
                 uint32_t o1[32], o2[32];
@@ -607,11 +656,11 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
                             wb[kk] = Elem<T>::pack(b0, b1);
                         }
                         quad_transpose(wo, t);
-                        quad_transpose(wb, t);
+                        if (!EXT) quad_transpose(wb, t);
                         if (r0 + rl0 + 8 * hh < it.nq) {
                             const int64_t at = static_cast<int64_t>(8 * hh) * a.q_st + 64 * cc + 32 * grp;
                             *reinterpret_cast<uint4 *>(go + at) = make_uint4(wo[0], wo[1], wo[2], wo[3]);
-                            *reinterpret_cast<uint4 *>(gb + at) = make_uint4(wb[0], wb[1], wb[2], wb[3]);
+                            if (!EXT) *reinterpret_cast<uint4 *>(gb + at) = make_uint4(wb[0], wb[1], wb[2], wb[3]);
                         }
                     }
             }
@@ -674,21 +723,25 @@ int *mirror_host_view() {
     return w.word ? h : nullptr;
 }
 
-template <typename T, int D>
+template <typename T, int D, bool EXT>
 int launch_t(const TrainArgs &a, cudaStream_t stream) {
     constexpr int NS = 4;
     using L = Smem<D, NS>;
     const ErrorWords ew = error_words();
     if (!ew.word) return PLX_ERR_LAUNCH;
     const ErrSink sink{ew.word, ew.mirror};
+    // keys: (batch, len_k) of a dense cache or of the training op, (page, key of the page) of a paged one
+    const bool paged = EXT && a.page_table;
+    const int kv_rows = paged ? a.page_mask + 1 : a.len_k, kv_batch = paged ? a.n_pages : a.batch;
+    const int kv_box = paged && a.page_mask + 1 < kBN ? a.page_mask + 1 : kBN;
     CUtensorMap tq, tr, tk, tv;
     const CUtensorMapDataType dt = Fmt<T>::kTma;
     if (!make_map(&tq, dt, a.q, D, a.len_q, a.heads_q, a.batch, a.q_st, a.q_sh, a.q_sb, kBM) ||
         !make_map(&tr, dt, a.r, D, a.len_q, a.heads_q, a.batch, a.q_st, a.q_sh, a.q_sb, kBM) ||
-        !make_map(&tk, dt, a.k, D, a.len_k, a.heads_kv, a.batch, a.kv_st, a.kv_sh, a.kv_sb, kBN) ||
-        !make_map(&tv, dt, a.v, D, a.len_k, a.heads_kv, a.batch, a.kv_st, a.kv_sh, a.kv_sb, kBN))
+        !make_map(&tk, dt, a.k, D, kv_rows, a.heads_kv, kv_batch, a.kv_st, a.kv_sh, a.kv_sb, kv_box) ||
+        !make_map(&tv, dt, a.v, D, kv_rows, a.heads_kv, kv_batch, a.kv_st, a.kv_sh, a.kv_sb, kv_box))
         return PLX_ERR_LAUNCH;
-    auto kern = fwd_sm100_kernel<T, D, NS>;
+    auto kern = fwd_sm100_kernel<T, D, NS, EXT>;
     static std::mutex attr_mu;
     static bool attr_done[tma::kMaxDevices] = {};
     if (!tma::opt_in_smem(kern, static_cast<int>(L::kBytes), attr_done, attr_mu)) return PLX_ERR_LAUNCH;
@@ -696,7 +749,8 @@ int launch_t(const TrainArgs &a, cudaStream_t stream) {
     const int n_items = tiles * a.batch * a.heads_q, sms = sm_count();
     if (sms <= 0) return PLX_ERR_LAUNCH;
     // with plenty of items a CTA takes them in neighbouring pairs (a heavy and a light row tile)
-    const int chunk_shift = n_items >= 2 * sms ? 1 : 0;
+    // (EXT: the row tiles of a row see nearly the same keys, so single items balance better)
+    const int chunk_shift = !EXT && n_items >= 2 * sms ? 1 : 0;
     const int units = (n_items + (1 << chunk_shift) - 1) >> chunk_shift;
     kern<<<units < sms ? units : sms, 352, L::kBytes, stream>>>(a, tq, tr, tk, tv, sink, tiles, n_items, chunk_shift);
     count_launch();
@@ -714,8 +768,21 @@ bool train_fwd_sm100_supported(const TrainArgs &a, int head_dim) {
 }
 
 int launch_train_fwd_sm100(const TrainArgs &a, int dtype, int head_dim, cudaStream_t stream) {
-    if (dtype == PLX_BF16) return head_dim == 64 ? launch_t<__nv_bfloat16, 64>(a, stream) : launch_t<__nv_bfloat16, 128>(a, stream);
-    if (dtype == PLX_FP16) return head_dim == 64 ? launch_t<__half, 64>(a, stream) : launch_t<__half, 128>(a, stream);
+    if (dtype == PLX_BF16) return head_dim == 64 ? launch_t<__nv_bfloat16, 64, false>(a, stream) : launch_t<__nv_bfloat16, 128, false>(a, stream);
+    if (dtype == PLX_FP16) return head_dim == 64 ? launch_t<__half, 64, false>(a, stream) : launch_t<__half, 128, false>(a, stream);
+    return PLX_ERR_UNSUPPORTED;
+}
+
+// Against a cache: any key range the forward takes; pages from 8 keys on (below that a box would not start on
+// the 1024-byte swizzle period of its tile), and strides a tensor map can express (no broadcast axes).
+bool train_extend_sm100_supported(const TrainArgs &a, int head_dim) {
+    if (a.kv_sb <= 0 || a.kv_sh <= 0 || a.kv_st <= 0 || (a.page_table && a.page_mask + 1 < kMinPage)) return false;
+    return train_fwd_sm100_supported(a, head_dim);
+}
+
+int launch_train_extend_sm100(const TrainArgs &a, int dtype, int head_dim, cudaStream_t stream) {
+    if (dtype == PLX_BF16) return head_dim == 64 ? launch_t<__nv_bfloat16, 64, true>(a, stream) : launch_t<__nv_bfloat16, 128, true>(a, stream);
+    if (dtype == PLX_FP16) return head_dim == 64 ? launch_t<__half, 64, true>(a, stream) : launch_t<__half, 128, true>(a, stream);
     return PLX_ERR_UNSUPPORTED;
 }
 

@@ -19,6 +19,9 @@ int launch_train_bwd_mma(const TrainArgs &a, int dtype, int head_dim, int stages
 // tcgen05 + TMEM + TMA forward (head_dim 128, no sliding window); `supported` decides per problem
 bool train_fwd_sm100_supported(const TrainArgs &a, int head_dim);
 int launch_train_fwd_sm100(const TrainArgs &a, int dtype, int head_dim, cudaStream_t stream);
+// the same kernel for several query rows per sequence against a dense or paged KV cache (writes `o` only)
+bool train_extend_sm100_supported(const TrainArgs &a, int head_dim);
+int launch_train_extend_sm100(const TrainArgs &a, int dtype, int head_dim, cudaStream_t stream);
 // Error words of the current device (see sm100::ErrSink): `word` in device memory, `mirror` in mapped
 // pinned host memory.  Both null on failure.  The first call on a device allocates the mirror.
 struct ErrorWords {

@@ -15,6 +15,8 @@ from typing import Optional
 import torch
 
 from . import ops
+from ._cabi import PLX_ERR_UNSUPPORTED, PlxError
+from .train import kernel_ready
 
 # split-KV scratch of EAGER calls, one per (device, stream, batch*heads, splits, head_dim): never shared
 # by two streams.  A captured launch must not use it (every capture runs on the same capture stream, so
@@ -193,10 +195,8 @@ def parallax_attn_with_kvcache(q: torch.Tensor, r: torch.Tensor, k_cache: torch.
     * ``q`` / ``r`` with ``L_q > 1`` rows ``(B, L_q, H, D)`` -- prefill / extend: the ``L_q`` queries are
       the LAST ``L_q`` positions of the sequence (row ``i`` sees keys up to ``L - L_q + i``), as in
       ``flash_attn_with_kvcache``.  This runs the training forward kernel (tensor cores), not the decode
-      sweep: one launch for a dense cache whose rows share an active length, one launch per batch row
-      for row-dependent ``seqused_k`` and for a paged cache (whose pages are first gathered into a dense
-      temporary).  Reading ``seqused_k`` synchronises, so only the single-token form can be captured in
-      a CUDA graph.
+      sweep, in one launch for all rows, their own lengths and a paged cache included.  Reading
+      ``seqused_k`` synchronises, so only the single-token form can be captured in a CUDA graph.
     """
     if q.ndim == 4 and q.shape[1] > 1:
         return _extend_core(q, r, k_cache, v_cache, page_table=page_table, seqused_k=seqused_k,
@@ -213,19 +213,47 @@ def parallax_attn_with_kvcache(q: torch.Tensor, r: torch.Tensor, k_cache: torch.
 def _extend_dense(q, r, k, v, scale, window_size_left):
     """One launch of the training forward kernel for `L_q` query rows against the keys of `k` / `v`
     (B, L, H_kv, D): bottom-right aligned causal mask (parallax/reference.py:64-68)."""
-    from .train import kernel_ready
-
     qk = kernel_ready(q)
     kk = k if (k.stride(-1) == 1 and all(s % 8 == 0 for s in k.stride()[:-1]) and k.data_ptr() % 16 == 0) else k.contiguous()
     vv = v if v.stride() == kk.stride() and v.data_ptr() % 16 == 0 else torch.empty_strided(kk.shape, kk.stride(), dtype=v.dtype, device=v.device).copy_(v)
     return ops.train_fwd(qk, kernel_ready(r, qk), kk, vv, float(scale), int(window_size_left), ops.BTHD, None)[0]
 
 
+def _differentiable(*tensors) -> bool:
+    """True if the call may have to be recorded or transformed: a gradient could be asked of it, or
+    forward-mode differentiation or a functorch transform is active."""
+    return (torch.is_grad_enabled() and any(t.requires_grad for t in tensors)) or \
+        torch.autograd.forward_ad._current_level >= 0 or torch._C._functorch.peek_interpreter_stack() is not None
+
+
+def _extend_fused(q, r, k, v, scale, window_size_left, seqused_k, page_table, res) -> bool:
+    """All rows of an L_q > 1 call in one launch, written to `res` (and nothing else done) -- or False where
+    that kernel does not apply: a call that autograd or a transform has to see, cache strides that a tensor
+    map cannot express, and what plx_train_extend refuses."""
+    if _differentiable(q, r, k, v, res) or not _kv_ok(k) or not _kv_ok(v) or k.stride() != v.stride():
+        return False
+    qk = kernel_ready(q)
+    apart = all(res.untyped_storage().data_ptr() != x.untyped_storage().data_ptr() for x in (qk, r, k, v))
+    o = res if res.stride() == qk.stride() and res.data_ptr() % 16 == 0 and apart else torch.empty_like(qk)
+    try:
+        ops.train_extend(qk, kernel_ready(r, qk), k, v, o, float(scale), int(window_size_left),
+                         None if seqused_k is None else seqused_k.contiguous(),
+                         None if page_table is None else page_table.contiguous())
+    except PlxError as e:
+        if e.status != PLX_ERR_UNSUPPORTED:
+            raise
+        return False
+    if o is not res:
+        res.copy_(o)
+    return True
+
+
 def _extend_core(q, r, k_cache, v_cache, *, page_table, seqused_k, window_size_left, scale, out):
-    """L_q > 1 queries against a cache through the training forward kernel.  Rows that share an active
-    length (or all rows, without `seqused_k`) of a dense cache run as one launch; row-dependent lengths and
-    paged caches run one launch per batch row, a paged row's pages being gathered into a dense temporary
-    first.  Reading the lengths synchronises, so this path cannot be captured in a CUDA graph."""
+    """L_q > 1 queries against a cache through the training forward kernel: one launch for all rows
+    (:func:`_extend_fused`).  Where that does not apply, rows that share an active length of a dense cache
+    run as one launch of the training op; row-dependent lengths and paged caches run one launch per batch
+    row, a paged row's pages being gathered into a dense temporary first.  Reading the lengths
+    synchronises, so this path cannot be captured in a CUDA graph."""
     if q.dtype not in (torch.bfloat16, torch.float16):
         raise TypeError(f"parallax_attn_with_kvcache requires bf16 or fp16 input, got {q.dtype}")
     if r.shape != q.shape:
@@ -254,13 +282,19 @@ def _extend_core(q, r, k_cache, v_cache, *, page_table, seqused_k, window_size_l
     if min(lens) < lq:
         raise ValueError(f"a row holds {min(lens)} keys but L_q = {lq}: the queries are the last L_q positions")
 
-    if not paged and len(set(lens)) == 1:
+    uniform = not paged and len(set(lens)) == 1
+    res = out
+    if res is None:      # as the training op lays it out for rows of one length, else contiguous
+        res = torch.empty_like(kernel_ready(q)) if uniform else torch.empty_like(q, memory_format=torch.contiguous_format)
+    ks, vs = (k_cache[:, :lens[0]], v_cache[:, :lens[0]]) if uniform else (k_cache, v_cache)
+    if _extend_fused(q, r, ks, vs, scale, window_size_left, None if uniform else seqused_k, page_table, res):
+        return res
+    if uniform:
         o = _extend_dense(q, r, k_cache[:, :lens[0]], v_cache[:, :lens[0]], scale, window_size_left)
         if out is None:
             return o
         out.copy_(o)
         return out
-    res = out if out is not None else torch.empty_like(q, memory_format=torch.contiguous_format)
     for b, n in enumerate(lens):
         if paged:
             pages = page_table[b, :(n + page - 1) // page].long()

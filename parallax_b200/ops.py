@@ -104,6 +104,28 @@ def _(q, r, k, v, qk_scale, window_left, layout, cu_seqlens):
     return torch.empty_like(q), torch.empty_like(q), stats, torch.empty_like(stats), torch.empty_like(stats)
 
 
+@torch.library.custom_op("plx::train_extend", mutates_args=("out",), device_types="cuda")
+def train_extend(q: Tensor, r: Tensor, k: Tensor, v: Tensor, out: Tensor, qk_scale: float, window_left: int,
+                 seqused_k: Optional[Tensor], page_table: Optional[Tensor]) -> None:
+    """Several query rows per sequence against a cache, all rows in one launch (BTHD; `out` strided like q).
+    Raises PlxError with status PLX_ERR_UNSUPPORTED, having enqueued nothing, where no kernel takes the problem."""
+    p = _train_problem(q, k, q, qk_scale, window_left, BTHD, None)
+    page_size = pages_per_seq = n_pages = 0
+    if page_table is not None:
+        n_pages, page_size, pages_per_seq = k.shape[0], k.shape[1], page_table.shape[1]
+        p.len_k = pages_per_seq * page_size
+    with torch.cuda.device(q.device):
+        _cabi.raise_if_device_error("plx_train_extend")
+        st = _cabi.lib().plx_train_extend(C.byref(p), _ptr(q), _ptr(r), _ptr(k), _ptr(v), _ptr(out), _ptr(seqused_k),
+                                          _ptr(page_table), page_size, pages_per_seq, n_pages, _stream(q.device))
+    _cabi.check(st, "plx_train_extend")
+
+
+@train_extend.register_fake
+def _(q, r, k, v, out, qk_scale, window_left, seqused_k, page_table):
+    return None
+
+
 BWD_STATS, BWD_DQR, BWD_DKV, BWD_ALL = 1, 2, 4, 7
 
 

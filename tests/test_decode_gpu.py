@@ -6,7 +6,7 @@ import torch
 
 import parallax_b200 as plx
 from oracle import parallax_oracle as orc
-from parallax_b200 import ops
+from parallax_b200 import _cabi, ops
 from tests._util import DECODE_MAX_REL, DECODE_REL_L2, assert_close, golden_names, load_golden, seeded_bf16
 
 pytestmark = pytest.mark.gpu
@@ -628,3 +628,55 @@ def test_extend_with_several_query_rows(case):
     paged = plx.parallax_attn_with_kvcache(q.cuda(), r.cuda(), pool_k.cuda(), pool_v.cuda(), page_table=order.int().cuda(),
                                            seqused_k=su, window_size=window)
     assert torch.equal(paged, out)
+
+
+@pytest.mark.parametrize("case", [
+    # hq, hkv, lq, active lengths, head_dim, page size (0: dense), window, dtype
+    (8, 2, 5, (300, 64, 5), 128, 16, None, torch.bfloat16),          # tails inside a page and inside a tile, a row of lq keys
+    (4, 4, 130, (130, 191, 512), 128, 64, None, torch.bfloat16),     # one box per tile, two row tiles
+    (8, 8, 17, (700, 257), 64, 256, 100, torch.float16),             # four tiles per page, sliding window
+    (4, 1, 3, (9, 65, 63), 128, 8, None, torch.bfloat16),            # the smallest page with a box of its own
+    (4, 1, 3, (9, 65, 63), 64, 4, None, torch.bfloat16),             # smaller: pages are gathered, a launch per row
+    (8, 2, 33, (640, 100, 321), 128, 0, None, torch.float16),        # dense, lengths of their own
+    (8, 8, 12, (40, 40), 64, 0, None, torch.bfloat16),               # dense, one length
+    (32, 8, 2, (128, 2), 128, 128, 1, torch.bfloat16),               # window of one key
+])
+def test_extend_in_one_launch_is_the_launch_per_row(case):
+    """One launch over rows of their own lengths and over pages gives the bits of a launch per row (which is
+    what a call that autograd records still runs), whatever lies in the cache past the active lengths."""
+    hq, hkv, lq, lens, d, page, window, dtype = case
+    gen = torch.Generator().manual_seed(17)
+    mk = lambda *s: torch.randn(*s, generator=gen).to(dtype)
+    bsz, ceiling = len(lens), max(lens) + 37
+    q, r = mk(bsz, hq, lq, d).cuda().transpose(1, 2), mk(bsz, lq, hq, d).cuda()          # different strides
+    nan = float("nan")
+    if page:
+        per_row = -(-ceiling // page)
+        pool = bsz * per_row + 2
+        table = torch.full((bsz, per_row + 3), 10 ** 9, dtype=torch.int32)
+        order = torch.randperm(pool, generator=gen)
+        k, v = mk(pool, page, hkv, d), mk(pool, page, hkv, d)
+        live = torch.zeros(pool, page, dtype=torch.bool)
+        for b, n in enumerate(lens):
+            ids = order[b * per_row:b * per_row + -(-n // page)]
+            table[b, :len(ids)] = ids.int()
+            for j in range(n):
+                live[ids[j // page], j % page] = True
+        table = table.cuda()[:, :per_row]                                                # not contiguous
+    else:
+        table = None
+        k, v = mk(bsz, ceiling, hkv, d), mk(bsz, ceiling, hkv, d)
+        live = torch.arange(ceiling)[None] < torch.tensor(lens)[:, None]
+    k[~live], v[~live] = nan, nan
+    k, v = k.cuda(), v.cuda()
+    su = torch.tensor([x for n in lens for x in (n, -1)], dtype=torch.int32, device="cuda")[::2]
+    args = dict(page_table=table, seqused_k=su, window_size=window)
+    before = _cabi.launch_count()
+    got = plx.parallax_attn_with_kvcache(q, r, k, v, **args)
+    assert page == 4 or _cabi.launch_count() - before == 1
+    want = plx.parallax_attn_with_kvcache(q.clone().requires_grad_(True), r, k, v, **args)
+    assert want.requires_grad and torch.equal(got, want.detach())
+    out = torch.empty(bsz, hq, lq, d, dtype=dtype, device="cuda").transpose(1, 2)        # not contiguous
+    assert plx.parallax_attn_with_kvcache(q, r, k, v, out=out, **args) is out and torch.equal(out, got)
+    mine = q.clone()
+    assert torch.equal(plx.parallax_attn_with_kvcache(mine, r, k, v, out=mine, **args), got)   # written over an input
