@@ -248,6 +248,103 @@ __device__ __forceinline__ void exchange_merge_warp(const DecodeArgs &a, int64_t
     }
 }
 
+// Active key range [lo, hi) of a batch row, as indices into this buffer.
+__device__ __forceinline__ void row_range(const DecodeArgs &a, int b, int &lo, int &hi) {
+    int hi_g = a.total_len;
+    if (a.seqused) hi_g = min(max(__ldg(a.seqused + b), 1), a.total_len);
+    int lo_g = a.cache_start ? max(__ldg(a.cache_start + b), 0) : 0;
+    if (a.window >= 0) lo_g = max(lo_g, hi_g - a.window);
+    lo = min(max(lo_g - a.kv_offset, 0), a.cache_len);
+    hi = min(max(hi_g - a.kv_offset, 0), a.cache_len);
+}
+
+// What one of the batch * n_splits slots of a launch (per head) sweeps: part `part` of the `n_parts` into
+// which the keys of row `b` are cut.  The records of (b, head) start at record first + head * n_parts.
+struct SplitPlan {
+    int b, part, n_parts, lo, hi;
+    int64_t first;
+};
+
+// Slot -> plan, computed by a whole warp.  G: keys come in multiples of G.
+// Rows of one length get n_splits parts each.  With lengths of their own (seqused / cache_start) that makes the
+// longest row set the time while the warps of the others idle, so there the slots are dealt out by length: the
+// smallest part size for which the parts of all rows still fit into the slots.  Lane l looks after rows l, l + 32,
+// ..: up to kBalancedRows rows.  A row's parts must fit the merge: 32 records in one level, 32 per group in two.
+template <int G, bool UNIFORM>
+__device__ __forceinline__ SplitPlan plan_slot(const DecodeArgs &a, int slot, int lane) {
+    SplitPlan p;
+    if (UNIFORM || !a.balanced) {
+        p.b = slot / a.n_splits;
+        p.part = slot - p.b * a.n_splits;
+        p.n_parts = a.n_splits;
+        p.first = static_cast<int64_t>(p.b) * a.n_splits * a.heads_q;
+        int lo, hi;
+        row_range(a, p.b, lo, hi);
+        const int n = max(hi - lo, 0);
+        const int chunk = ((n + a.n_splits - 1) / a.n_splits + G - 1) / G * G;
+        p.lo = min(lo + p.part * chunk, hi);
+        p.hi = min(p.lo + chunk, hi);
+        return p;
+    }
+    constexpr int kRows = kBalancedRows / 32;
+    int start[kRows], n[kRows], units[kRows], sum = 0, most = 0;   // units: multiples of G keys
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+        start[i] = n[i] = units[i] = 0;
+        if (lane + 32 * i < a.batch) {
+            int hi;
+            row_range(a, lane + 32 * i, start[i], hi);
+            n[i] = max(hi - start[i], 0);
+            units[i] = (n[i] + G - 1) / G;
+        }
+        sum += units[i];
+        most = max(most, units[i]);
+    }
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    most = __reduce_max_sync(0xffffffffu, most);
+    const int slots = a.batch * a.n_splits, cap = a.n_groups ? 32 * a.n_groups : 32;
+    // part size in units: `good` fits (every row has at most n_splits parts), below `bad` none can
+    int good = max((most + a.n_splits - 1) / a.n_splits, 1);
+    int bad = max(max((sum + slots - 1) / slots, (most + cap - 1) / cap), 1);
+    while (bad < good) {
+        const int mid = (bad + good) >> 1;
+        int parts = 0;
+#pragma unroll
+        for (int i = 0; i < kRows; ++i)
+            if (lane + 32 * i < a.batch) parts += max((units[i] + mid - 1) / mid, 1);
+        if (static_cast<int>(__reduce_add_sync(0xffffffffu, parts)) <= slots) good = mid;
+        else bad = mid + 1;
+    }
+    // the row that owns this slot
+    p.b = -1;
+    int before = 0;       // parts of the rows of earlier i
+#pragma unroll
+    for (int i = 0; i < kRows; ++i) {
+        if (32 * i >= a.batch || p.b >= 0) continue;
+        const int mine = lane + 32 * i < a.batch ? max((units[i] + good - 1) / good, 1) : 0;
+        int incl = mine;
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, incl, off);
+            if (lane >= off) incl += x;
+        }
+        const unsigned owner = __ballot_sync(0xffffffffu, slot >= before + incl - mine && slot < before + incl);
+        if (owner) {
+            const int l = __ffs(owner) - 1;
+            p.b = l + 32 * i;
+            const int head = before + __shfl_sync(0xffffffffu, incl - mine, l);
+            p.n_parts = __shfl_sync(0xffffffffu, mine, l);
+            p.part = slot - head;
+            p.first = static_cast<int64_t>(head) * a.heads_q;
+            const int lo = __shfl_sync(0xffffffffu, start[i], l), hi = lo + __shfl_sync(0xffffffffu, n[i], l);
+            p.lo = min(lo + p.part * good * G, hi);
+            p.hi = min(p.lo + good * G, hi);
+        }
+        before += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    return p;             // p.b < 0: a slot that no row needs
+}
+
 // One WARP per (split, q head, batch row); a CTA is HG warps working on HG adjacent q
 // heads of the same key range, so that together they sweep contiguous memory (all heads
 // of a key are adjacent in the cache layout) and, under grouped-query attention, the q
@@ -267,25 +364,15 @@ __global__ void __launch_bounds__(HG * 32, U > 4 ? 1 : 512 / (HG * 32)) decode_k
     constexpr int REC = 2 * D + 4;  // floats per partial record
     constexpr int CH = D / 32;      // channels per lane in the merge
 
-    const int b = blockIdx.z;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int split = SG ? blockIdx.x * HG + warp : blockIdx.x;
     const int hq = SG ? blockIdx.y : blockIdx.y * HG + warp;
     const int hk = hq / a.n_rep;
     const int sid = lane / LPK, sl = lane % LPK;
 
-    // active key range of this batch row, then of this split (local key indices)
-    int hi_g = a.total_len;
-    if (a.seqused) hi_g = min(max(a.seqused[b], 1), a.total_len);
-    int lo_g = a.cache_start ? max(a.cache_start[b], 0) : 0;
-    if (a.window >= 0) lo_g = max(lo_g, hi_g - a.window);
-    const int lo = min(max(lo_g - a.kv_offset, 0), a.cache_len);
-    const int hi = min(max(hi_g - a.kv_offset, 0), a.cache_len);
-    const int n = max(hi - lo, 0);
-    int chunk = (n + a.n_splits - 1) / a.n_splits;
-    chunk = (chunk + NS - 1) / NS * NS;
-    const int my_lo = min(lo + split * chunk, hi);
-    const int my_hi = min(my_lo + chunk, hi);
+    // the part of a batch row's keys that this warp sweeps
+    const SplitPlan plan = plan_slot<NS, SG>(a, blockIdx.z * a.n_splits + (SG ? blockIdx.x * HG + warp : blockIdx.x), lane);
+    if (!SG && plan.b < 0) return;
+    const int b = plan.b, my_lo = plan.lo, my_hi = plan.hi;
     const int n_iter = (my_hi - my_lo + NS * U - 1) / (NS * U);
 
     // this lane's 8 channels of q and r
@@ -545,13 +632,14 @@ __global__ void __launch_bounds__(HG * 32, U > 4 ? 1 : 512 / (HG * 32)) decode_k
         return;
     }
 
-    if (a.n_splits == 1) {
+    if (plan.n_parts == 1) {
         emit(m, d1, d2, o1, o2);
         return;
     }
 
     // publish this split's state; the last warp of the (batch, head) to arrive merges all splits
-    float *ws = a.ws_parts + (bh * a.n_splits + split) * REC;
+    float *recs = a.ws_parts + (plan.first + static_cast<int64_t>(hq) * plan.n_parts) * REC;   // of this (batch, head)
+    float *ws = recs + static_cast<int64_t>(plan.part) * REC;
     if (writer) {
         if (lane == 0) __stcg(reinterpret_cast<float4 *>(ws), make_float4(m, d1, d2, 0.f));
         __stcg(reinterpret_cast<float4 *>(ws + 4 + sl * 8), make_float4(o1[0], o1[1], o1[2], o1[3]));
@@ -575,15 +663,16 @@ __global__ void __launch_bounds__(HG * 32, U > 4 ? 1 : 512 / (HG * 32)) decode_k
         if (last) __threadfence();
         return last != 0;
     };
-    if (a.n_groups == 0) {
-        if (!arrive_last(a.ws_counters + bh, a.n_splits)) return;
-        warp_merge<D>(a.ws_parts + bh * a.n_splits * REC, a.n_splits, lane, big, D1, D2, O1, O2);
+    if (plan.n_parts <= 32) {
+        if (!arrive_last(a.ws_counters + bh, plan.n_parts)) return;
+        warp_merge<D>(recs, plan.n_parts, lane, big, D1, D2, O1, O2);
     } else {
-        const int group = split / PLX_DECODE_GROUP;
-        const int first = group * PLX_DECODE_GROUP, size = min(PLX_DECODE_GROUP, a.n_splits - first);
+        const int gsize = a.balanced ? 32 : PLX_DECODE_GROUP, n_groups = (plan.n_parts + gsize - 1) / gsize;
+        const int group = plan.part / gsize;
+        const int first = group * gsize, size = min(gsize, plan.n_parts - first);
         int *gc = a.ws_gcounters + bh * a.n_groups + group;
         if (!arrive_last(gc, size)) return;
-        warp_merge<D>(a.ws_parts + (bh * a.n_splits + first) * REC, size, lane, big, D1, D2, O1, O2);
+        warp_merge<D>(recs + static_cast<int64_t>(first) * REC, size, lane, big, D1, D2, O1, O2);
         float *grec = a.ws_gparts + (bh * a.n_groups + group) * REC;
         if (lane == 0) {
             __stcg(reinterpret_cast<float4 *>(grec), make_float4(big, D1, D2, 0.f));
@@ -596,8 +685,8 @@ __global__ void __launch_bounds__(HG * 32, U > 4 ? 1 : 512 / (HG * 32)) decode_k
         }
         __threadfence();
         __syncwarp();
-        if (!arrive_last(a.ws_counters + bh, a.n_groups)) return;
-        warp_merge<D>(a.ws_gparts + bh * a.n_groups * REC, a.n_groups, lane, big, D1, D2, O1, O2);
+        if (!arrive_last(a.ws_counters + bh, n_groups)) return;
+        warp_merge<D>(a.ws_gparts + bh * a.n_groups * REC, n_groups, lane, big, D1, D2, O1, O2);
     }
     if (a.xch.world > 0) {
         exchange_merge_warp<T, D>(a, bh, lane, big, D1, D2, O1, O2);
@@ -764,32 +853,30 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
     extern __shared__ __align__(16) unsigned char gqa_smem[];
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    // warps are dealt out split-fastest over (batch, kv head, head group, split), so a CTA is full whatever the split count
+    // warps are dealt out over (batch, kv head, head group, split), so a CTA is full whatever the split count:
+    // split-fastest for rows of one length; with the slots dealt out by length, head-fastest within a slot
     const int64_t wid = static_cast<int64_t>(blockIdx.x) * kGqaWarps + warp;
-    const int64_t n_units = static_cast<int64_t>(a.batch) * a.heads_kv * n_hgroups;
-    if (wid >= n_units * a.n_splits) return;
-    const int split = static_cast<int>(wid % a.n_splits);
-    const int unit = static_cast<int>(wid / a.n_splits);
-    const int b = unit / (a.heads_kv * n_hgroups), hk = (unit / n_hgroups) % a.heads_kv, hgrp = unit % n_hgroups;
+    const int n_hunits = a.heads_kv * n_hgroups, n_slots = a.batch * a.n_splits;
+    if (wid >= static_cast<int64_t>(n_slots) * n_hunits) return;
+    int slot, hunit;
+    if (a.balanced) {
+        slot = static_cast<int>(wid / n_hunits);
+        hunit = static_cast<int>(wid - static_cast<int64_t>(slot) * n_hunits);
+    } else {
+        const int unit = static_cast<int>(wid / a.n_splits);
+        hunit = unit % n_hunits;
+        slot = unit / n_hunits * a.n_splits + static_cast<int>(wid % a.n_splits);
+    }
+    const int hk = hunit / n_hgroups, hgrp = hunit % n_hgroups;
+    const SplitPlan plan = plan_slot<kGqaTile, false>(a, slot, lane);
+    if (plan.b < 0) return;
+    const int b = plan.b, my_lo = plan.lo, my_hi = plan.hi;
+    const int n_tiles = (my_hi - my_lo + kGqaTile - 1) / kGqaTile;
     const int hq0 = hk * a.n_rep + hgrp * 16;       // first q head of this warp's rows
     const int n_rows = min(16, a.n_rep - hgrp * 16);
     const uint32_t sbase = smem_u32(gqa_smem) + warp * GqaSmem<D>::kPerWarp;
     auto sK = [&](int st) -> uint32_t { return sbase + st * 2 * kTileBytes; };
     auto sV = [&](int st) -> uint32_t { return sbase + st * 2 * kTileBytes + kTileBytes; };
-
-    // active key range of this batch row, then of this split (local key indices)
-    int hi_g = a.total_len;
-    if (a.seqused) hi_g = min(max(a.seqused[b], 1), a.total_len);
-    int lo_g = a.cache_start ? max(a.cache_start[b], 0) : 0;
-    if (a.window >= 0) lo_g = max(lo_g, hi_g - a.window);
-    const int lo = min(max(lo_g - a.kv_offset, 0), a.cache_len);
-    const int hi = min(max(hi_g - a.kv_offset, 0), a.cache_len);
-    const int n = max(hi - lo, 0);
-    int chunk = (n + a.n_splits - 1) / a.n_splits;
-    chunk = (chunk + kGqaTile - 1) / kGqaTile * kGqaTile;
-    const int my_lo = min(lo + split * chunk, hi);
-    const int my_hi = min(my_lo + chunk, hi);
-    const int n_tiles = (my_hi - my_lo + kGqaTile - 1) / kGqaTile;
 
     // ---- q and r of the group -> A fragments (staged through the first two tile buffers)
     uint32_t qa[KS][4], ra[KS][4];
@@ -958,7 +1045,7 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
     const bool row_ok[2] = {g < n_rows, g + 8 < n_rows};
     auto bh_of = [&](int row) -> int64_t { return static_cast<int64_t>(b) * a.heads_q + hq0 + row; };
 
-    if (a.n_splits == 1) {
+    if (plan.n_parts == 1) {
 #pragma unroll
         for (int hh = 0; hh < 2; ++hh) {
             if (!row_ok[hh]) continue;
@@ -984,10 +1071,11 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
     }
 
     // publish this split's state of every row
+    auto recs_of = [&](int row) -> float * { return a.ws_parts + (plan.first + static_cast<int64_t>(hq0 + row) * plan.n_parts) * REC; };
 #pragma unroll
     for (int hh = 0; hh < 2; ++hh) {
         if (!row_ok[hh]) continue;
-        float *ws = a.ws_parts + (bh_of(g + 8 * hh) * a.n_splits + split) * REC;
+        float *ws = recs_of(g + 8 * hh) + static_cast<int64_t>(plan.part) * REC;
         if (t == 0) __stcg(reinterpret_cast<float4 *>(ws), make_float4(m[hh], d1[hh], d2[hh], 0.f));
 #pragma unroll
         for (int i = 0; i < D / 8; ++i) {
@@ -1084,12 +1172,13 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
             sink(r);
         }
     };
-    const int group = split / PLX_DECODE_GROUP;
-    const int first = group * PLX_DECODE_GROUP, gsize = min(PLX_DECODE_GROUP, a.n_splits - first);
+    const bool one_level = plan.n_parts <= 32;
+    const int gmax = a.balanced ? 32 : PLX_DECODE_GROUP, n_groups = (plan.n_parts + gmax - 1) / gmax;
+    const int group = plan.part / gmax, first = group * gmax, gsize = min(gmax, plan.n_parts - first);
     unsigned mine = 0;
     if (lane < n_rows) {
-        int *counter = a.n_groups == 0 ? a.ws_counters + bh_of(lane) : a.ws_gcounters + bh_of(lane) * a.n_groups + group;
-        if (atomicAdd(counter, 1) == (a.n_groups == 0 ? a.n_splits : gsize) - 1) mine = 1u << lane;
+        int *counter = one_level ? a.ws_counters + bh_of(lane) : a.ws_gcounters + bh_of(lane) * a.n_groups + group;
+        if (atomicAdd(counter, 1) == (one_level ? plan.n_parts : gsize) - 1) mine = 1u << lane;
     }
     unsigned todo = __reduce_or_sync(0xffffffffu, mine);
     if (todo == 0) return;
@@ -1099,12 +1188,12 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
         emit(bh);
         if (lane == 0) a.ws_counters[bh] = 0;   // ready for the next launch on this workspace
     };
-    if (a.n_groups == 0) {
-        merge_rows(todo, [&](int row) { return a.ws_parts + bh_of(row) * a.n_splits * REC; }, a.n_splits, finish);
+    if (one_level) {
+        merge_rows(todo, recs_of, plan.n_parts, finish);
         return;
     }
     // two levels: merge this group's records of the rows in `todo`, then arrive for those rows at the second level
-    merge_rows(todo, [&](int row) { return a.ws_parts + (bh_of(row) * a.n_splits + first) * REC; }, gsize, [&](int row) {
+    merge_rows(todo, [&](int row) { return recs_of(row) + static_cast<int64_t>(first) * REC; }, gsize, [&](int row) {
         const int64_t bh = bh_of(row);
         float *grec = a.ws_gparts + (bh * a.n_groups + group) * REC;
         if (lane == 0) {
@@ -1120,11 +1209,11 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
     __threadfence();
     __syncwarp();
     mine = 0;
-    if (lane < n_rows && ((todo >> lane) & 1) && atomicAdd(a.ws_counters + bh_of(lane), 1) == a.n_groups - 1) mine = 1u << lane;
+    if (lane < n_rows && ((todo >> lane) & 1) && atomicAdd(a.ws_counters + bh_of(lane), 1) == n_groups - 1) mine = 1u << lane;
     todo = __reduce_or_sync(0xffffffffu, mine);
     if (todo == 0) return;
     __threadfence();
-    merge_rows(todo, [&](int row) { return a.ws_gparts + bh_of(row) * a.n_groups * REC; }, a.n_groups, finish);
+    merge_rows(todo, [&](int row) { return a.ws_gparts + bh_of(row) * a.n_groups * REC; }, n_groups, finish);
 }
 
 template <typename T, int D>
@@ -1255,7 +1344,12 @@ bool decode_fused_exchange_supported(const DecodeArgs &a) {
     return a.n_rep == 1 && a.n_splits >= 2 && !decode_split_groups(a);
 }
 
-int launch_decode(const DecodeArgs &a, int dtype, int head_dim, cudaStream_t stream) {
+int launch_decode(const DecodeArgs &problem, int dtype, int head_dim, cudaStream_t stream) {
+    DecodeArgs a = problem;
+    // Rows with lengths of their own: deal the splits out by length.  Not split groups, whose CTAs belong to one
+    // row, and not a key-sharded launch, whose fused and two-launch forms have to cut the keys alike.
+    a.balanced = (a.seqused || a.cache_start) && a.batch > 1 && a.batch <= kBalancedRows && a.n_splits > 1 && !a.part_out &&
+                 a.xch.world == 0 && !decode_split_groups(a);
     if (dtype == PLX_BF16) {
         if (head_dim == 128) return launch_decode_t<__nv_bfloat16, 128>(a, stream);
         if (head_dim == 64) return launch_decode_t<__nv_bfloat16, 64>(a, stream);

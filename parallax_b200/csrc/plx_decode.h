@@ -15,6 +15,8 @@ struct ExchangeArgs {
     int *err_word, *err_mirror;   // error words of this device (see sm100::ErrSink), used by the fused sweep + exchange
 };
 
+constexpr int kBalancedRows = 128;   // most batch rows whose splits are dealt out by length
+
 struct DecodeArgs {
     const void *q, *r, *k, *v;
     void *out;         // (batch, heads_q, D) or nullptr
@@ -25,6 +27,7 @@ struct DecodeArgs {
     float *ws_gparts;  // (batch * heads_q, n_groups) records of the first merge level (n_groups > 0)
     int *ws_gcounters; // (batch * heads_q, n_groups) arrival counters of the groups
     int n_groups;      // 0: single-level merge
+    bool balanced;     // splits dealt out to the batch rows by length (see plan_slot)
     int batch, heads_q, heads_kv, n_rep, cache_len, window, n_splits, kv_offset, total_len;
     float c2;  // qk_scale * log2(e)
     int64_t kv_sb, kv_st, kv_sh;   // paged: kv_sb is the stride between pages

@@ -680,3 +680,37 @@ def test_extend_in_one_launch_is_the_launch_per_row(case):
     assert plx.parallax_attn_with_kvcache(q, r, k, v, out=out, **args) is out and torch.equal(out, got)
     mine = q.clone()
     assert torch.equal(plx.parallax_attn_with_kvcache(mine, r, k, v, out=mine, **args), got)   # written over an input
+
+
+@pytest.mark.parametrize("case", [
+    # batch, hq, hkv, cache, head_dim, window, dtype: the splits are dealt out by row length from 2 to 128 rows
+    (2, 32, 8, 12000, 128, -1, torch.bfloat16),      # two-level merge, one long and one short row
+    (16, 32, 8, 3000, 128, -1, torch.bfloat16),
+    (33, 16, 2, 700, 64, 300, torch.float16),        # more rows than lanes, a window
+    (24, 8, 8, 2500, 128, -1, torch.bfloat16),       # one q head per kv head, outside the split groups
+    (5, 16, 16, 9000, 64, -1, torch.float16),        # ... with a two-level merge
+    (128, 8, 8, 400, 64, -1, torch.bfloat16),        # the most rows
+    (129, 4, 2, 400, 128, -1, torch.bfloat16),       # one more: every row gets the same number of splits
+])
+def test_rows_of_very_different_lengths(case):
+    """Each row of a ragged batch is what the oracle gives for its own keys, a row without keys is zero, and a
+    second launch on the same workspace (whose counters the first one reset) gives the same bits."""
+    bsz, hq, hkv, kv_len, d, window, dtype = case
+    gen = torch.Generator().manual_seed(5)
+    mk = lambda *s: torch.randn(*s, generator=gen).to(dtype).cuda()
+    q, r, k, v = mk(bsz, 1, hq, d), mk(bsz, 1, hq, d), mk(bsz, kv_len, hkv, d), mk(bsz, kv_len, hkv, d)
+    used = [kv_len if b == 1 else 1 + (b * 7919) % (kv_len // (1 + b % 5)) for b in range(bsz)]
+    start = [n // 3 if b % 3 == 2 else 0 for b, n in enumerate(used)]
+    if bsz > 2:
+        start[-1] = used[-1]                                                     # no key left
+    t32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    args = dict(window_size_left=window, cache_start=t32(start), seqused_k=t32(used))
+    out = plx.parallax_decode(q, r, k, v, **args)
+    assert torch.equal(out, plx.parallax_decode(q, r, k, v, **args))
+    for b in list(range(min(bsz, 6))) + [bsz - 1]:
+        lo = max(start[b], used[b] - window if window >= 0 else 0)
+        if lo >= used[b]:
+            assert not out[b].any()
+            continue
+        ref = orc.decode(q[b:b + 1].cpu(), r[b:b + 1].cpu(), k[b:b + 1, lo:used[b]].cpu(), v[b:b + 1, lo:used[b]].cpu())
+        assert_close(out[b:b + 1].float().cpu(), ref, DECODE_REL_L2, DECODE_MAX_REL, f"{case} row {b}")
