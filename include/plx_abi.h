@@ -177,6 +177,7 @@ typedef struct plx_decode_problem {
     const int32_t *page_table;   /* device, int32 */
     int32_t page_size;
     int32_t pages_per_seq;
+    int32_t n_pages;      /* pages in the pool; > 0: page numbers are kept below it, 0: taken as they are */
 } plx_decode_problem;
 
 #define PLX_DECODE_MAX_SPLITS 256   /* upper bound of plx_decode_problem.n_splits */

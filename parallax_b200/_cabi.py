@@ -6,10 +6,11 @@ is raised.  Nothing here computes on the CPU.
 from __future__ import annotations
 
 import ctypes as C
+import importlib.util
 import os
 import threading
 
-from ._paths import LIB_PATH
+from ._paths import HOST_PATH, LIB_PATH
 
 PLX_BF16, PLX_FP16 = 0, 1
 PLX_ERR_UNSUPPORTED = -2
@@ -45,7 +46,7 @@ class DecodeProblem(C.Structure):
         ("cache_len", C.c_int32), ("head_dim", C.c_int32), ("window_left", C.c_int32), ("n_splits", C.c_int32),
         ("qk_scale", C.c_float), ("kv_offset", C.c_int32), ("total_len", C.c_int32),
         ("kv_stride_b", C.c_int64), ("kv_stride_t", C.c_int64), ("kv_stride_h", C.c_int64),
-        ("page_table", C.c_void_p), ("page_size", C.c_int32), ("pages_per_seq", C.c_int32),
+        ("page_table", C.c_void_p), ("page_size", C.c_int32), ("pages_per_seq", C.c_int32), ("n_pages", C.c_int32),
     ]
 
 
@@ -130,6 +131,26 @@ def lib():
                     raise RuntimeError(f"libplx_sm100.so has ABI version {got}, expected {ABI_VERSION}")
                 _lib = handle
     return _lib
+
+
+_host = None
+
+
+def host():
+    """The C++ host side of eager calls (csrc/plx_host.cpp), bound to the loaded library."""
+    global _host
+    if _host is None:
+        handle = lib()
+        with _lock:
+            if _host is None:
+                if not os.path.exists(HOST_PATH):
+                    raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m parallax_b200.build`")
+                spec = importlib.util.spec_from_file_location("_plx_host", HOST_PATH)
+                module = importlib.util.module_from_spec(spec)
+                spec.loader.exec_module(module)
+                module.bind({name: C.cast(getattr(handle, name), C.c_void_p).value for name in SYMBOLS})
+                _host = module
+    return _host
 
 
 def check(status: int, what: str) -> None:

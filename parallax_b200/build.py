@@ -1,9 +1,9 @@
-"""Build recipe for libplx_sm100.so (hand-written CUDA for sm_100a + the C ABI).
+"""Build recipe for libplx_sm100.so (hand-written CUDA for sm_100a + the C ABI) and _plx_host.so (the host side
+of eager calls in C++, against the headers of the installed PyTorch).
 
     python -m parallax_b200.build [--force]
 
-The library is built in-tree (``parallax_b200/lib/libplx_sm100.so``) with nvcc;
-nvcc cross-compiles for sm_100a, so no GPU is needed to build.
+Both are built in-tree (``parallax_b200/lib``); nvcc cross-compiles for sm_100a, so no GPU is needed to build.
 """
 from __future__ import annotations
 
@@ -12,7 +12,7 @@ import shutil
 import subprocess
 import sys
 
-from ._paths import CSRC, INCLUDE, LIB_DIR, LIB_PATH
+from ._paths import CSRC, HOST_PATH, INCLUDE, LIB_DIR, LIB_PATH
 
 SOURCES = ["plx_abi.cu", "plx_decode.cu", "plx_train_mma.cu", "plx_fwd_sm100.cu", "plx_bwd_sm100.cu"]
 NVCC_FLAGS = [
@@ -35,17 +35,34 @@ def _inputs():
 
 
 def is_stale() -> bool:
-    if not os.path.exists(LIB_PATH):
-        return True
-    built = os.path.getmtime(LIB_PATH)
-    return any(os.path.getmtime(f) > built for f in _inputs())
+    return any(not os.path.exists(built) or any(os.path.getmtime(f) > os.path.getmtime(built) for f in _inputs())
+               for built in (LIB_PATH, HOST_PATH))
+
+
+def _build_host() -> None:
+    import sysconfig
+
+    import torch
+
+    inc = os.path.join(os.path.dirname(torch.__file__), "include")
+    libs = os.path.join(os.path.dirname(torch.__file__), "lib")
+    cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
+    dirs = [inc, os.path.join(inc, "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f for d in dirs for f in ("-isystem", d)],
+           "-o", HOST_PATH, os.path.join(CSRC, "plx_host.cpp"), f"-L{libs}", f"-L{os.path.join(cuda, 'lib64')}",
+           "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-lcudart", "-Wl,-z,now"]
+    res = subprocess.run(cmd, capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError("g++ failed:\n" + res.stdout + res.stderr)
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile the library if it is missing or older than its sources; returns its path."""
+    """Compile both if one is missing or older than its sources; returns the path of libplx_sm100.so."""
     if not force and not is_stale():
         return LIB_PATH
     os.makedirs(LIB_DIR, exist_ok=True)
+    _build_host()
     cmd = [_nvcc(), *NVCC_FLAGS, *(["-Xptxas", "-v"] if verbose else []), "-o", LIB_PATH,
            *[os.path.join(CSRC, s) for s in SOURCES]]
     res = subprocess.run(cmd, capture_output=True, text=True)

@@ -170,6 +170,7 @@ static int run_decode(const plx_decode_problem *p, const void *q, const void *r,
     a.page_table = p->page_table;
     if (p->page_table) {
         a.pages_per_seq = p->pages_per_seq;
+        a.last_page = p->n_pages > 0 ? static_cast<uint32_t>(p->n_pages) - 1u : INT32_MAX;
         a.page_mask = p->page_size - 1;
         a.page_shift = 0;
         while ((1 << a.page_shift) < p->page_size) ++a.page_shift;

@@ -89,8 +89,9 @@ __device__ __forceinline__ void cluster_sync() {
 // Paged cache: element offset of key kj of batch row b inside k / v (head and channel offsets not
 // included).  Dense caches are addressed by strides directly at the call sites.
 __device__ __forceinline__ int64_t paged_key_offset(const DecodeArgs &a, int b, int kj) {
-    const int page = __ldg(a.page_table + static_cast<int64_t>(b) * a.pages_per_seq + (kj >> a.page_shift));
-    return page * a.kv_sb + static_cast<int64_t>(kj & a.page_mask) * a.kv_st;
+    // page numbers are kept inside the pool: a row length that the caller is yet to find out of range may lead here
+    const uint32_t page = min(static_cast<uint32_t>(__ldg(a.page_table + static_cast<int64_t>(b) * a.pages_per_seq + (kj >> a.page_shift))), a.last_page);
+    return static_cast<int64_t>(page) * a.kv_sb + static_cast<int64_t>(kj & a.page_mask) * a.kv_st;
 }
 
 __device__ __forceinline__ float finalize(float d1, float d2, float o1, float o2) {

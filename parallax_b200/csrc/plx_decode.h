@@ -35,6 +35,7 @@ struct DecodeArgs {
     // page_table[b * pages_per_seq + (j >> page_shift)] at row j & page_mask
     const int32_t *page_table;
     int page_shift, page_mask, pages_per_seq;
+    uint32_t last_page;   // page numbers above it are read as it
     // Fused sweep + exchange (xch.world >= 1): the warp that holds the merged state of a (batch, head) does
     // not write a partial record but pushes it to every rank's inbox, waits for the peers' and merges.
     ExchangeArgs xch;

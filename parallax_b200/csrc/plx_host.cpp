@@ -1,0 +1,449 @@
+// The host side of an ordinary eager call, in C++: argument checks, output allocation, workspace, the autograd
+// node and the call into libplx_sm100.so.
+//
+// Everything here is a SHORT CUT of the Python path (train.py / decode.py over the torch custom ops of ops.py),
+// which stays the definition of the API: each function returns None, having enqueued nothing that shows, for any
+// call that is not plainly an eager one on well-formed CUDA tensors -- a tensor subclass, a torch function or
+// dispatch mode, functorch or forward-mode differentiation, tracing, a stream that is being captured, shapes,
+// strides or types that need a copy or an error message, a device error waiting to be reported -- and the caller
+// then takes the Python path, which handles it or raises.
+#include <ATen/PythonTorchFunctionTLS.h>
+#include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <torch/csrc/autograd/custom_function.h>
+#include <torch/csrc/autograd/python_variable.h>
+#include <torch/extension.h>
+
+#include <array>
+#include <cmath>
+#include <cstdlib>
+#include <list>
+#include <mutex>
+#include <optional>
+
+#include "../../include/plx_abi.h"
+
+namespace {
+
+using at::Tensor;
+using OptTensor = std::optional<Tensor>;
+using Tensors = std::initializer_list<const Tensor *>;
+
+enum Layout { kBHLD = 0, kBTHD = 1 };
+
+// entry points of the loaded libplx_sm100.so (the one ops.py calls; set once by bind())
+struct Api {
+    decltype(&plx_device_error_peek) device_error_peek;
+    decltype(&plx_train_workspace_bytes) train_workspace_bytes;
+    decltype(&plx_train_fwd) train_fwd;
+    decltype(&plx_train_bwd) train_bwd;
+    decltype(&plx_train_extend) train_extend;
+    decltype(&plx_decode_choose_splits_gqa) decode_choose_splits_gqa;
+    decltype(&plx_decode_workspace_bytes) decode_workspace_bytes;
+    decltype(&plx_decode) decode;
+};
+Api api;
+
+template <typename F>
+void bind_one(F &slot, const py::dict &addresses, const char *name) {
+    slot = reinterpret_cast<F>(addresses[name].cast<uintptr_t>());
+}
+void bind(const py::dict &addresses) {
+    bind_one(api.device_error_peek, addresses, "plx_device_error_peek");
+    bind_one(api.train_workspace_bytes, addresses, "plx_train_workspace_bytes");
+    bind_one(api.train_fwd, addresses, "plx_train_fwd");
+    bind_one(api.train_bwd, addresses, "plx_train_bwd");
+    bind_one(api.train_extend, addresses, "plx_train_extend");
+    bind_one(api.decode_choose_splits_gqa, addresses, "plx_decode_choose_splits_gqa");
+    bind_one(api.decode_workspace_bytes, addresses, "plx_decode_workspace_bytes");
+    bind_one(api.decode, addresses, "plx_decode");
+}
+
+// ------------------------------------------------------------------------- //
+// what counts as a plain call
+// ------------------------------------------------------------------------- //
+// exactly a Tensor or a Parameter, and no torch function mode
+bool plain_object(PyObject *o) {
+    return (reinterpret_cast<PyObject *>(Py_TYPE(o)) == THPVariableClass || reinterpret_cast<PyObject *>(Py_TYPE(o)) == ParameterClass) &&
+           !at::impl::torch_function_mode_enabled();
+}
+
+// The tensor of a plain Python object; `ok` is cleared for anything else.
+Tensor take(const py::object &o, bool &ok) {
+    if (!plain_object(o.ptr())) {
+        ok = false;
+        return Tensor();
+    }
+    return THPVariable_Unpack(o.ptr());
+}
+OptTensor take_optional(const py::object &o, bool &ok) {
+    if (o.is_none()) return std::nullopt;
+    return take(o, ok);
+}
+// qk_scale (None: head_dim ** -0.5) and the window as plain Python numbers
+bool take_scale(const py::object &o, int64_t head_dim, double &scale) {
+    if (o.is_none()) scale = 1.0 / std::sqrt(static_cast<double>(head_dim));
+    else if (PyFloat_CheckExact(o.ptr())) scale = PyFloat_AS_DOUBLE(o.ptr());
+    else return false;
+    return true;
+}
+bool take_window(const py::object &o, int64_t &window) {
+    if (!PyLong_CheckExact(o.ptr())) return false;
+    int overflow = 0;
+    window = PyLong_AsLongLongAndOverflow(o.ptr(), &overflow);
+    return overflow == 0 && window >= -1 && window <= INT32_MAX;
+}
+
+// No dispatch key beyond those of an ordinary dense CUDA tensor and its autograd, and no forward-mode tangent.
+bool plain_tensor(const Tensor &t) {
+    static const c10::DispatchKeySet usual =
+        c10::DispatchKeySet({c10::DispatchKey::CUDA, c10::DispatchKey::AutogradCUDA, c10::DispatchKey::ADInplaceOrView,
+                             c10::DispatchKey::AutocastCUDA});
+    return t.is_cuda() && (t.key_set().raw_repr() & ~usual.raw_repr()) == 0 && !t._fw_grad(0).defined();
+}
+bool plain_thread() {
+    static const c10::DispatchKeySet usual =
+        c10::DispatchKeySet({c10::DispatchKey::BackendSelect, c10::DispatchKey::ADInplaceOrView}) | c10::autocast_dispatch_keyset;
+    return (c10::impl::tls_local_dispatch_key_set().included_.raw_repr() & ~usual.raw_repr()) == 0;
+}
+
+bool capturing() { return at::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None; }
+
+bool device_error_waiting() {
+    int32_t v = 0;
+    return api.device_error_peek(&v, 0) != PLX_OK || v != 0;
+}
+
+int dtype_code(const Tensor &t) {
+    return t.scalar_type() == at::kBFloat16 ? PLX_BF16 : t.scalar_type() == at::kHalf ? PLX_FP16 : -1;
+}
+bool aligned16(const Tensor &t) { return (reinterpret_cast<uintptr_t>(t.data_ptr()) & 15u) == 0; }
+
+// train.kernel_ready without the copy: last axis contiguous, the other strides multiples of 8 elements, the base
+// 16-byte aligned, no gaps or overlap in some axis order.
+bool kernel_ready(const Tensor &t) {
+    if (t.stride(3) != 1 || !aligned16(t)) return false;
+    for (int i = 0; i < 3; ++i)
+        if (t.stride(i) % 8 != 0) return false;
+    return t.is_non_overlapping_and_dense();
+}
+
+const int32_t *int_ptr(const OptTensor &t) { return t ? static_cast<const int32_t *>(t->data_ptr()) : nullptr; }
+
+bool recorded(Tensors tensors) {
+    if (!at::GradMode::is_enabled()) return false;
+    for (const Tensor *t : tensors)
+        if (t->requires_grad()) return true;
+    return false;
+}
+
+// ------------------------------------------------------------------------- //
+// training
+// ------------------------------------------------------------------------- //
+plx_train_problem train_problem(const Tensor &q, const Tensor &k, const Tensor &stats, double scale, int64_t window, int64_t layout,
+                                const OptTensor &cu) {
+    const int h = layout == kBHLD ? 1 : 2, l = layout == kBHLD ? 2 : 1;
+    plx_train_problem p{};
+    p.dtype = dtype_code(q);
+    p.batch = static_cast<int32_t>(q.size(0));
+    p.heads_q = static_cast<int32_t>(q.size(h));
+    p.heads_kv = static_cast<int32_t>(k.size(h));
+    p.len_q = static_cast<int32_t>(q.size(l));
+    p.len_k = static_cast<int32_t>(k.size(l));
+    p.head_dim = static_cast<int32_t>(q.size(3));
+    p.window_left = static_cast<int32_t>(window);
+    p.qk_scale = static_cast<float>(scale);
+    p.q_stride_b = q.stride(0); p.q_stride_h = q.stride(h); p.q_stride_t = q.stride(l);
+    p.kv_stride_b = k.stride(0); p.kv_stride_h = k.stride(h); p.kv_stride_t = k.stride(l);
+    if (stats.defined()) {
+        p.st_stride_b = stats.stride(0); p.st_stride_h = stats.stride(h); p.st_stride_t = stats.stride(l);
+    }
+    if (cu) {
+        p.cu_seqlens = int_ptr(cu);
+        p.n_seqs = static_cast<int32_t>(cu->numel() - 1);
+    }
+    return p;
+}
+
+struct Refused {};   // a status of the library that the Python path has to report
+
+// One node for forward and backward, as the custom op plx::train_fwd registers it.
+struct Train : torch::autograd::Function<Train> {
+    static Tensor forward(torch::autograd::AutogradContext *ctx, const Tensor &q, const Tensor &r, const Tensor &k, const Tensor &v,
+                          double scale, int64_t window, int64_t layout, const OptTensor &cu) {
+        at::AutoDispatchBelowADInplaceOrView below;
+        const c10::cuda::CUDAGuard device(q.device());
+        Tensor o = at::empty_like(q), barv = at::empty_like(q);
+        const Tensor stats = at::empty({3, q.size(0), q.size(1), q.size(2)}, q.options().dtype(at::kFloat));   // d1, bart, m
+        const Tensor d1 = stats[0];
+        float *st = stats.data_ptr<float>();
+        const int64_t n = d1.numel();
+        const plx_train_problem p = train_problem(q, k, d1, scale, window, layout, cu);
+        if (api.train_fwd(&p, q.data_ptr(), r.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), barv.data_ptr(), st, st + n, st + 2 * n,
+                          c10::cuda::getCurrentCUDAStream().stream()) != PLX_OK)
+            throw Refused();
+        ctx->save_for_backward({q, r, k, v, o, barv, stats, cu ? *cu : Tensor()});
+        ctx->saved_data["scale"] = scale;
+        ctx->saved_data["window"] = window;
+        ctx->saved_data["layout"] = layout;
+        return o;
+    }
+
+    static torch::autograd::variable_list backward(torch::autograd::AutogradContext *ctx, torch::autograd::variable_list grads) {
+        const auto saved = ctx->get_saved_variables();
+        const Tensor &q = saved[0], &r = saved[1], &k = saved[2], &v = saved[3], &o = saved[4], &barv = saved[5], &stats = saved[6];
+        const OptTensor cu = saved[7].defined() ? OptTensor(saved[7]) : std::nullopt;
+        const double scale = ctx->saved_data["scale"].toDouble();
+        const int64_t window = ctx->saved_data["window"].toInt(), layout = ctx->saved_data["layout"].toInt();
+        Tensor go = grads[0];
+        if (go.strides() != q.strides()) go = at::empty_like(q).copy_(go);   // one stride set for all q-like tensors
+        Tensor dq, dr, dk, dv;
+        bool done = false;
+        // A backward that is itself recorded, traced or transformed goes through the dispatcher, and so does one on
+        // saved tensors that a hook has brought back in another form.
+        bool plain = !at::GradMode::is_enabled() && plain_thread() && !at::impl::torch_function_mode_enabled() && stats.is_contiguous();
+        for (const Tensor *t : Tensors{&go, &q, &r, &k, &v, &o, &barv, &stats}) plain = plain && plain_tensor(*t);
+        for (const Tensor *t : Tensors{&go, &r, &o, &barv}) plain = plain && t->strides() == q.strides() && t->scalar_type() == q.scalar_type();
+        plain = plain && v.strides() == k.strides();
+        if (plain) {
+            at::AutoDispatchBelowADInplaceOrView below;
+            const c10::cuda::CUDAGuard device(q.device());
+            const Tensor d1 = stats[0];
+            const plx_train_problem p = train_problem(q, k, d1, scale, window, layout, cu);
+            size_t need = 0;
+            if (!device_error_waiting() && api.train_workspace_bytes(&p, &need) == PLX_OK) {
+                dq = at::empty_like(q);
+                dr = at::empty_like(q);
+                dk = at::empty_like(k);
+                dv = at::empty_like(k);
+                const Tensor ws = at::empty({static_cast<int64_t>(need)}, q.options().dtype(at::kByte));
+                const float *st = stats.data_ptr<float>();
+                const int64_t n = d1.numel();
+                done = api.train_bwd(&p, q.data_ptr(), r.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), barv.data_ptr(), st, st + n,
+                                     st + 2 * n, go.data_ptr(), dq.data_ptr(), dr.data_ptr(), dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), need,
+                                     c10::cuda::getCurrentCUDAStream().stream()) == PLX_OK;
+            }
+        }
+        if (!done) {
+            static const auto op = c10::Dispatcher::singleton().findSchemaOrThrow("plx::train_bwd", "")
+                .typed<std::tuple<Tensor, Tensor, Tensor, Tensor>(const Tensor &, const Tensor &, const Tensor &, const Tensor &,
+                    const Tensor &, const Tensor &, const Tensor &, const Tensor &, const Tensor &, const Tensor &, double, int64_t, int64_t,
+                    const OptTensor &)>();
+            std::tie(dq, dr, dk, dv) = op.call(q, r, k, v, o, barv, stats[0], stats[1], stats[2], go, scale, window, layout, cu);
+        }
+        return {dq, dr, dk, dv, Tensor(), Tensor(), Tensor(), Tensor()};
+    }
+};
+
+py::object train(const py::object &q_, const py::object &r_, const py::object &k_, const py::object &v_, const py::object &scale_,
+                 const py::object &window_, int64_t layout, const py::object &cu_) {
+    bool ok = true;
+    const Tensor q = take(q_, ok), r = take(r_, ok), k = take(k_, ok), v = take(v_, ok);
+    const OptTensor cu = take_optional(cu_, ok);
+    if (!ok || !plain_thread()) return py::none();
+    for (const Tensor *t : Tensors{&q, &r, &k, &v})
+        if (!plain_tensor(*t) || t->dim() != 4 || t->scalar_type() != q.scalar_type() || t->device() != q.device() || t->numel() == 0 ||
+            !kernel_ready(*t))
+            return py::none();
+    const int h = layout == kBHLD ? 1 : 2;
+    if (dtype_code(q) < 0 || r.sizes() != q.sizes() || r.strides() != q.strides() || v.sizes() != k.sizes() || v.strides() != k.strides() ||
+        k.size(0) != q.size(0) || k.size(3) != q.size(3) || q.size(h) % k.size(h) != 0)
+        return py::none();
+    if (cu && (!plain_tensor(*cu) || cu->scalar_type() != at::kInt || cu->dim() != 1 || !cu->is_contiguous() || cu->device() != q.device() ||
+               q.size(0) != 1 || cu->numel() < 2))
+        return py::none();
+    double scale;
+    int64_t window;
+    if (!take_scale(scale_, q.size(3), scale) || !take_window(window_, window)) return py::none();
+    const c10::cuda::CUDAGuard device(q.device());
+    if (device_error_waiting()) return py::none();
+    Tensor o;
+    try {
+        py::gil_scoped_release nogil;
+        o = Train::apply(q, r, k, v, scale, window, static_cast<int64_t>(layout), cu);
+    } catch (const Refused &) {
+        return py::none();
+    }
+    return py::reinterpret_steal<py::object>(THPVariable_Wrap(o));
+}
+
+// ------------------------------------------------------------------------- //
+// decode
+// ------------------------------------------------------------------------- //
+// Split-KV scratch of eager calls: one per (device, stream, problem shape), zero-filled when made; a launch leaves
+// its arrival counters at zero.  At most kMax are kept, the least recently used going back to the allocator: a
+// workspace is only ever used on the stream it was allocated on, so the allocator reuses its memory in stream order.
+class Workspaces {
+public:
+    Tensor get(const c10::cuda::CUDAStream &stream, const Tensor &q, int n_splits, int64_t floats) {
+        const Key key{q.get_device(), static_cast<int64_t>(reinterpret_cast<uintptr_t>(stream.stream())), q.size(0), q.size(2), q.size(3), n_splits};
+        std::lock_guard<std::mutex> lock(mu_);
+        for (auto it = list_.begin(); it != list_.end(); ++it)
+            if (it->first == key) {
+                list_.splice(list_.begin(), list_, it);
+                return it->second;
+            }
+        list_.emplace_front(key, at::zeros({floats}, q.options().dtype(at::kFloat)));
+        if (list_.size() > kMax) list_.pop_back();
+        return list_.front().second;
+    }
+
+private:
+    using Key = std::array<int64_t, 6>;
+    static constexpr size_t kMax = 32;
+    std::mutex mu_;
+    std::list<std::pair<Key, Tensor>> list_;
+};
+Workspaces &workspaces() {
+    static Workspaces *w = new Workspaces;   // not destroyed at exit, when the CUDA context may be gone
+    return *w;
+}
+
+// The lengths of the rows on their way to the host.  The copy is queued BEFORE the launch they belong to and
+// waited for after it, so reading them does not leave the GPU idle.  Launching on lengths that turn out to be out
+// of range is harmless: the kernels clamp them (and page numbers) to the buffers, and the result is dropped.
+class LengthCheck {
+public:
+    LengthCheck(const OptTensor &lens, const c10::cuda::CUDAStream &stream) {
+        if (!lens) return;
+        host_ = at::empty({lens->numel()}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+        C10_CUDA_CHECK(cudaMemcpyAsync(host_.data_ptr(), lens->data_ptr(), sizeof(int32_t) * lens->numel(), cudaMemcpyDeviceToHost, stream.stream()));
+        copied_.record(stream);
+    }
+    ~LengthCheck() {
+        if (host_.defined() && !waited_) cudaEventSynchronize(copied_.event());   // the copy still writes to host_
+    }
+    bool within(int64_t lo, int64_t hi) {
+        if (!host_.defined()) return true;
+        {
+            py::gil_scoped_release nogil;
+            copied_.synchronize();
+        }
+        waited_ = true;
+        const int32_t *n = host_.data_ptr<int32_t>();
+        for (int64_t i = 0; i < host_.numel(); ++i)
+            if (n[i] < lo || n[i] > hi) return false;
+        return true;
+    }
+
+private:
+    Tensor host_;
+    at::cuda::CUDAEvent copied_{cudaEventDisableTiming};
+    bool waited_ = false;
+};
+
+bool int32_vector(const OptTensor &t, int64_t n, const at::Device &device) {
+    return !t || (plain_tensor(*t) && t->scalar_type() == at::kInt && t->dim() == 1 && t->size(0) == n && t->is_contiguous() && t->device() == device);
+}
+bool page_table_ok(const OptTensor &t, int64_t batch, int64_t page, const at::Device &device) {
+    return !t || (plain_tensor(*t) && t->scalar_type() == at::kInt && t->dim() == 2 && t->size(0) == batch && t->size(1) > 0 && t->is_contiguous() &&
+                  t->device() == device && page > 0 && (page & (page - 1)) == 0);
+}
+bool kv_ok(const Tensor &k, const Tensor &v) {
+    for (int i = 0; i < 3; ++i)
+        if (k.stride(i) % 8 != 0) return false;
+    return k.stride(3) == 1 && aligned16(k) && aligned16(v) && v.strides() == k.strides();
+}
+// what decode and extend ask of their tensors alike: q, r (B, L_q, H, D) contiguous, k, v in the cache layout
+bool cache_call_ok(const Tensor &q, const Tensor &r, const Tensor &k, const Tensor &v, const OptTensor &lens, const OptTensor &table) {
+    for (const Tensor *t : Tensors{&q, &r, &k, &v})
+        if (!plain_tensor(*t) || t->dim() != 4 || t->scalar_type() != q.scalar_type() || t->device() != q.device() || t->numel() == 0)
+            return false;
+    if (dtype_code(q) < 0 || r.sizes() != q.sizes() || !q.is_contiguous() || !r.is_contiguous() || !aligned16(q) || !aligned16(r)) return false;
+    if (v.sizes() != k.sizes() || k.size(3) != q.size(3) || (!table && k.size(0) != q.size(0)) || q.size(2) % k.size(2) != 0 || !kv_ok(k, v)) return false;
+    if (q.size(3) != 64 && q.size(3) != 128) return false;
+    return int32_vector(lens, q.size(0), q.device()) && page_table_ok(table, q.size(0), k.size(1), q.device()) && !recorded({&q, &r, &k, &v});
+}
+
+py::object decode(const py::object &q_, const py::object &r_, const py::object &k_, const py::object &v_, const py::object &scale_,
+                  const py::object &window_, const py::object &lens_, const py::object &start_, const py::object &table_) {
+    bool ok = true;
+    const Tensor q = take(q_, ok), r = take(r_, ok), k = take(k_, ok), v = take(v_, ok);
+    const OptTensor lens = take_optional(lens_, ok), start = take_optional(start_, ok), table = take_optional(table_, ok);
+    if (!ok || !plain_thread() || !cache_call_ok(q, r, k, v, lens, table) || q.size(1) != 1 || !int32_vector(start, q.size(0), q.device()) ||
+        std::getenv("PLX_DECODE_SPLITS"))
+        return py::none();
+    double scale;
+    int64_t window;
+    const int64_t ceiling = table ? table->size(1) * k.size(1) : k.size(1);
+    if (!take_scale(scale_, q.size(3), scale) || !take_window(window_, window) || ceiling > INT32_MAX) return py::none();
+    at::AutoDispatchBelowADInplaceOrView below;
+    const c10::cuda::CUDAGuard device(q.device());
+    if (capturing()) return py::none();
+    const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream();
+    plx_decode_problem p{};
+    p.dtype = dtype_code(q);
+    p.batch = static_cast<int32_t>(q.size(0));
+    p.heads_q = static_cast<int32_t>(q.size(2));
+    p.heads_kv = static_cast<int32_t>(k.size(2));
+    p.head_dim = static_cast<int32_t>(q.size(3));
+    p.cache_len = static_cast<int32_t>(ceiling);
+    p.window_left = static_cast<int32_t>(window);
+    p.qk_scale = static_cast<float>(scale);
+    p.kv_stride_b = k.stride(0);
+    p.kv_stride_t = k.stride(1);
+    p.kv_stride_h = k.stride(2);
+    if (table) {
+        p.page_table = int_ptr(table);
+        p.page_size = static_cast<int32_t>(k.size(1));
+        p.pages_per_seq = static_cast<int32_t>(table->size(1));
+        p.n_pages = static_cast<int32_t>(k.size(0));
+    }
+    const int32_t n_keys = window < 0 ? p.cache_len : std::max(1, std::min(p.cache_len, p.window_left));
+    p.n_splits = api.decode_choose_splits_gqa(p.batch, p.heads_q, p.heads_kv, n_keys, at::cuda::getDeviceProperties(q.get_device())->multiProcessorCount);
+    size_t need = 0;
+    if (api.decode_workspace_bytes(&p, &need) != PLX_OK) return py::none();
+    const Tensor ws = workspaces().get(stream, q, p.n_splits, static_cast<int64_t>(need / sizeof(float)));
+    Tensor out = at::empty(q.sizes(), q.options());
+    LengthCheck check(lens, stream);
+    if (api.decode(&p, q.data_ptr(), r.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), int_ptr(lens), int_ptr(start), ws.data_ptr(), need,
+                   stream.stream()) != PLX_OK ||
+        !check.within(1, ceiling))
+        return py::none();
+    return py::reinterpret_steal<py::object>(THPVariable_Wrap(out));
+}
+
+// L_q > 1: one launch of the training forward kernel against the cache.
+py::object extend(const py::object &q_, const py::object &r_, const py::object &k_, const py::object &v_, const py::object &scale_,
+                  const py::object &window_, const py::object &lens_, const py::object &table_) {
+    bool ok = true;
+    const Tensor q = take(q_, ok), r = take(r_, ok), k = take(k_, ok), v = take(v_, ok);
+    const OptTensor lens = take_optional(lens_, ok), table = take_optional(table_, ok);
+    if (!ok || !plain_thread() || !cache_call_ok(q, r, k, v, lens, table)) return py::none();
+    double scale;
+    int64_t window;
+    const int64_t ceiling = table ? table->size(1) * k.size(1) : k.size(1);
+    if (!take_scale(scale_, q.size(3), scale) || !take_window(window_, window) || ceiling > INT32_MAX || q.size(1) > ceiling) return py::none();
+    at::AutoDispatchBelowADInplaceOrView below;
+    const c10::cuda::CUDAGuard device(q.device());
+    if (capturing() || device_error_waiting()) return py::none();
+    const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream();
+    plx_train_problem p = train_problem(q, k, Tensor(), scale, window, kBTHD, std::nullopt);
+    p.len_k = static_cast<int32_t>(ceiling);
+    Tensor out = at::empty(q.sizes(), q.options());
+    LengthCheck check(lens, stream);
+    if (api.train_extend(&p, q.data_ptr(), r.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), int_ptr(lens), int_ptr(table),
+                         table ? static_cast<int32_t>(k.size(1)) : 0, table ? static_cast<int32_t>(table->size(1)) : 0,
+                         table ? static_cast<int32_t>(k.size(0)) : 0, stream.stream()) != PLX_OK ||
+        !check.within(q.size(1), ceiling))
+        return py::none();
+    return py::reinterpret_steal<py::object>(THPVariable_Wrap(out));
+}
+
+py::object attend(const py::object &q, const py::object &r, const py::object &k, const py::object &v, const py::object &scale,
+                  const py::object &window, const py::object &lens, const py::object &table) {
+    if (!plain_object(q.ptr())) return py::none();
+    const Tensor &t = THPVariable_Unpack(q.ptr());
+    return t.dim() == 4 && t.size(1) == 1 ? decode(q, r, k, v, scale, window, lens, py::none(), table) : extend(q, r, k, v, scale, window, lens, table);
+}
+
+}  // namespace
+
+PYBIND11_MODULE(_plx_host, m) {
+    m.def("bind", &bind);
+    m.def("train", &train);
+    m.def("decode", &decode);
+    m.def("attend", &attend);
+}

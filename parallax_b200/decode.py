@@ -130,6 +130,11 @@ def parallax_decode(q: torch.Tensor, r: torch.Tensor, k: torch.Tensor, v: torch.
     ``seqused_k`` ``(B,)`` int32 the active length per row (clamped to
     ``[1, L]`` in the kernel); ``out`` an optional caller-owned output.
     """
+    host = ops.eager_host() if out is None else None
+    if host is not None:
+        res = host.decode(q, r, k, v, qk_scale, window_size_left, seqused_k, cache_start, None)
+        if res is not None:
+            return res
     if q.ndim == 4 and q.shape[1] != 1:
         raise ValueError(f"parallax_decode requires a single query (Sq=1), got Sq={q.shape[1]}.")
     if qk_scale is None:
@@ -198,6 +203,11 @@ def parallax_attn_with_kvcache(q: torch.Tensor, r: torch.Tensor, k_cache: torch.
       sweep, in one launch for all rows, their own lengths and a paged cache included.  Reading
       ``seqused_k`` synchronises, so only the single-token form can be captured in a CUDA graph.
     """
+    host = ops.eager_host() if out is None and (window_size is None or type(window_size) is int) else None
+    if host is not None:
+        res = host.attend(q, r, k_cache, v_cache, scale, -1 if window_size is None else window_size, seqused_k, page_table)
+        if res is not None:
+            return res
     if q.ndim == 4 and q.shape[1] > 1:
         return _extend_core(q, r, k_cache, v_cache, page_table=page_table, seqused_k=seqused_k,
                             window_size_left=_window_size_to_left(window_size), scale=scale, out=out)

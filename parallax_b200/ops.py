@@ -23,6 +23,11 @@ from . import _cabi
 BHLD, BTHD = 0, 1
 
 
+def eager_host():
+    """The C++ short cut of eager calls, or None while a compiler records the call (it has to see the ops)."""
+    return None if torch.compiler.is_compiling() else _cabi.host()
+
+
 def dtype_code(dtype: torch.dtype) -> int:
     if dtype == torch.bfloat16:
         return _cabi.PLX_BF16
@@ -211,6 +216,7 @@ def _decode_problem(q: Tensor, k: Tensor, qk_scale: float, window_left: int, n_s
     p.cache_len, p.heads_kv = k.shape[1], k.shape[2]
     if page_table is not None:        # k: (num_pages, page_size, heads_kv, head_dim); stride(0) is the page stride
         p.page_table, p.page_size, p.pages_per_seq = page_table.data_ptr(), k.shape[1], page_table.shape[1]
+        p.n_pages = k.shape[0]
         p.cache_len = page_table.shape[1] * k.shape[1]
     p.window_left, p.n_splits, p.qk_scale = int(window_left), int(n_splits), float(qk_scale)
     p.kv_offset, p.total_len = int(kv_offset), int(total_len)

@@ -65,6 +65,11 @@ def parallax_func(q: torch.Tensor, r: torch.Tensor, k: torch.Tensor, v: torch.Te
     For ``L_q != L_kv`` the causal diagonal is aligned to the END of the keys,
     as in ``parallax/reference.py:64-68``.  Returns ``(B, H_q, L_q, D)``.
     """
+    host = ops.eager_host()
+    if host is not None:
+        o = host.train(q, r, k, v, qk_scale, window_size_left, ops.BHLD, None)
+        if o is not None:
+            return o
     _check_dtype("parallax_func", q)
     bsz, hq, lq, d = q.shape
     hkv = k.shape[1]

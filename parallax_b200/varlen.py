@@ -26,6 +26,11 @@ def parallax_varlen_func(q: torch.Tensor, r: torch.Tensor, k: torch.Tensor, v: t
     independent causal sequences along T and requires ``B == 1``; ``None`` runs
     every batch row as one dense causal sequence.  Returns ``(B, T, H_q, D)``.
     """
+    host = ops.eager_host()
+    if host is not None:
+        o = host.train(q, r, k, v, qk_scale, window_size_left, ops.BTHD, cu_seqlens)
+        if o is not None:
+            return o
     if q.dtype not in (torch.bfloat16, torch.float16):
         raise TypeError(f"parallax_varlen_func requires bf16 or fp16 inputs, got q.dtype={q.dtype}")
     if q.shape[2] % k.shape[2] != 0:
