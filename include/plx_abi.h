@@ -208,6 +208,14 @@ int plx_decode_choose_splits_gqa(int32_t batch, int32_t heads_q, int32_t heads_k
 
 int plx_decode_workspace_bytes(const plx_decode_problem *p, size_t *bytes);
 
+/* The inputs of one step into the stable buffers that a captured decode launch reads, in one launch: `bytes`
+ * (a multiple of 16) of q and of r, and n (at most PLX_DECODE_STAGE_LENS) active lengths from HOST memory.  A null
+ * source leaves its buffer alone.  Plays the role of the copies of GraphedDecode.__call__
+ * [parallax/cute/parallax_decode.py:1665-1815]. */
+#define PLX_DECODE_STAGE_LENS 512
+int plx_decode_stage(void *q, const void *q_src, void *r, const void *r_src, size_t bytes,
+                     int32_t *seqused_k, const int32_t *seqused_src, int32_t n, plx_stream_t stream);
+
 /* out = Parallax decode.  seqused_k and cache_start are device int32 (batch,)
  * arrays or NULL.  Replaces parallax.triton.parallax_decode + its kernel
  * [parallax/triton/parallax_decode.py:100-148, 20-97] and the CuTeDSL path

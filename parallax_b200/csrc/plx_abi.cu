@@ -392,6 +392,16 @@ int plx_decode_check_args(const plx_decode_problem *p, const void *q, const void
     return check_decode_args(p, q, r, k, v, out, nullptr);
 }
 
+int plx_decode_stage(void *q, const void *q_src, void *r, const void *r_src, size_t bytes, int32_t *seqused_k,
+                     const int32_t *seqused_src, int32_t n, plx_stream_t stream) {
+    if ((q_src && !q) || (r_src && !r) || (seqused_src && !seqused_k) || n < 0 || n > PLX_DECODE_STAGE_LENS || (bytes & 15u) != 0)
+        return PLX_ERR_BAD_ARG;
+    if (misaligned16(q) || misaligned16(q_src) || misaligned16(r) || misaligned16(r_src)) return PLX_ERR_BAD_ARG;
+    int st = check_device();
+    if (st != PLX_OK) return st;
+    return launch_decode_stage(q, q_src, r, r_src, bytes, seqused_k, seqused_src, n, reinterpret_cast<cudaStream_t>(stream));
+}
+
 int plx_decode(const plx_decode_problem *p, const void *q, const void *r, const void *k, const void *v, void *out,
                const int32_t *seqused_k, const int32_t *cache_start, void *workspace, size_t workspace_bytes,
                plx_stream_t stream) {

@@ -1361,6 +1361,35 @@ int launch_decode(const DecodeArgs &problem, int dtype, int head_dim, cudaStream
     return PLX_ERR_UNSUPPORTED;
 }
 
+// The inputs of a captured step into its buffers: q and r by 16-byte copies, the lengths out of the launch
+// parameters.  One launch in place of two device copies, a host tensor and its synchronising copy.
+struct StageLens {
+    int32_t n[PLX_DECODE_STAGE_LENS];
+};
+__global__ void __launch_bounds__(256) decode_stage_kernel(uint4 *q, const uint4 *q_src, uint4 *r, const uint4 *r_src, int64_t n16, int32_t *lens,
+                                                           const __grid_constant__ StageLens src, int n) {
+    const int64_t i0 = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x, step = static_cast<int64_t>(gridDim.x) * 256;
+    for (int64_t i = i0; i < n16; i += step) {
+        if (q_src) q[i] = q_src[i];
+        if (r_src) r[i] = r_src[i];
+    }
+    for (int64_t i = i0; i < n; i += step) lens[i] = src.n[i];
+}
+
+int launch_decode_stage(void *q, const void *q_src, void *r, const void *r_src, size_t bytes, int32_t *lens, const int32_t *lens_src, int n,
+                        cudaStream_t stream) {
+    StageLens src{};
+    if (!lens_src) n = 0;
+    for (int i = 0; i < n; ++i) src.n[i] = lens_src[i];
+    const int64_t n16 = q_src || r_src ? static_cast<int64_t>(bytes / 16) : 0, items = n16 > n ? n16 : n;
+    if (items == 0) return PLX_OK;
+    const int64_t blocks = (items + 255) / 256;
+    decode_stage_kernel<<<static_cast<unsigned>(blocks < 1024 ? blocks : 1024), 256, 0, stream>>>(
+        static_cast<uint4 *>(q), static_cast<const uint4 *>(q_src), static_cast<uint4 *>(r), static_cast<const uint4 *>(r_src), n16, lens, src, n);
+    count_launch();
+    return cudaGetLastError() == cudaSuccess ? PLX_OK : PLX_ERR_LAUNCH;
+}
+
 template <typename T, int D>
 static int launch_merge_t(const float *parts, int n_parts, int n_records, void *out, cudaStream_t stream) {
     decode_merge_kernel<T, D><<<n_records, D, 0, stream>>>(parts, n_parts, n_records, out);

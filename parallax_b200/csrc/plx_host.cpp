@@ -43,6 +43,7 @@ struct Api {
     decltype(&plx_decode_choose_splits_gqa) decode_choose_splits_gqa;
     decltype(&plx_decode_workspace_bytes) decode_workspace_bytes;
     decltype(&plx_decode) decode;
+    decltype(&plx_decode_stage) decode_stage;
 };
 Api api;
 
@@ -59,6 +60,7 @@ void bind(const py::dict &addresses) {
     bind_one(api.decode_choose_splits_gqa, addresses, "plx_decode_choose_splits_gqa");
     bind_one(api.decode_workspace_bytes, addresses, "plx_decode_workspace_bytes");
     bind_one(api.decode, addresses, "plx_decode");
+    bind_one(api.decode_stage, addresses, "plx_decode_stage");
 }
 
 // ------------------------------------------------------------------------- //
@@ -439,6 +441,42 @@ py::object attend(const py::object &q, const py::object &r, const py::object &k,
     return t.dim() == 4 && t.size(1) == 1 ? decode(q, r, k, v, scale, window, lens, py::none(), table) : extend(q, r, k, v, scale, window, lens, table);
 }
 
+// q, r and the lengths of a GraphedDecode step into its buffers; False, having done nothing, for anything but
+// tensors like the buffers and lengths given as Python integers in [1, most].
+bool stage(const py::object &q_, const py::object &q_src_, const py::object &r_, const py::object &r_src_, const py::object &lens_,
+           const py::object &lens_src, int64_t most) {
+    bool ok = true;
+    const Tensor q = take(q_, ok), r = take(r_, ok);
+    const OptTensor q_src = take_optional(q_src_, ok), r_src = take_optional(r_src_, ok), lens = take_optional(lens_, ok);
+    if (!ok || !plain_thread() || !plain_tensor(q) || !plain_tensor(r) || !q.is_contiguous() || !r.is_contiguous() || q.numel() != r.numel() ||
+        !aligned16(q) || !aligned16(r) || recorded({&q, &r}))
+        return false;
+    for (const OptTensor *src : {&q_src, &r_src})
+        if (*src && (!plain_tensor(**src) || (*src)->sizes() != q.sizes() || (*src)->scalar_type() != q.scalar_type() ||
+                     (*src)->device() != q.device() || !(*src)->is_contiguous() || !aligned16(**src) || recorded({&**src})))
+            return false;
+    int32_t values[PLX_DECODE_STAGE_LENS];
+    int64_t n = 0;
+    if (!lens_src.is_none()) {
+        if (!lens || !int32_vector(lens, q.size(0), q.device()) || lens->numel() > PLX_DECODE_STAGE_LENS) return false;
+        n = lens->numel();
+        const bool list = PyList_CheckExact(lens_src.ptr());
+        if (list ? PyList_GET_SIZE(lens_src.ptr()) != n : !PyLong_CheckExact(lens_src.ptr())) return false;
+        for (int64_t i = 0; i < n; ++i) {
+            PyObject *x = list ? PyList_GET_ITEM(lens_src.ptr(), i) : lens_src.ptr();
+            int overflow = 0;
+            const long long len = PyLong_CheckExact(x) ? PyLong_AsLongLongAndOverflow(x, &overflow) : 0;
+            if (overflow || len < 1 || len > most) return false;
+            values[i] = static_cast<int32_t>(len);
+        }
+    }
+    const c10::cuda::CUDAGuard device(q.device());
+    if (capturing()) return false;
+    return api.decode_stage(q.data_ptr(), q_src ? q_src->data_ptr() : nullptr, r.data_ptr(), r_src ? r_src->data_ptr() : nullptr, q.nbytes(),
+                            lens ? static_cast<int32_t *>(lens->data_ptr()) : nullptr, n ? values : nullptr, static_cast<int32_t>(n),
+                            c10::cuda::getCurrentCUDAStream().stream()) == PLX_OK;
+}
+
 }  // namespace
 
 PYBIND11_MODULE(_plx_host, m) {
@@ -446,4 +484,5 @@ PYBIND11_MODULE(_plx_host, m) {
     m.def("train", &train);
     m.def("decode", &decode);
     m.def("attend", &attend);
+    m.def("stage", &stage);
 }

@@ -39,6 +39,8 @@ int launch_decode(const DecodeArgs &a, int dtype, int head_dim, cudaStream_t str
 bool decode_fused_exchange_supported(const DecodeArgs &a);   // see exchange_merge_warp in plx_decode.cu
 int launch_decode_exchange_merge(const ExchangeArgs &x, const float *part, int head_dim, int dtype, void *out,
                                  const ErrorWords &err, cudaStream_t stream);
+int launch_decode_stage(void *q, const void *q_src, void *r, const void *r_src, size_t bytes, int32_t *lens, const int32_t *lens_src, int n,
+                        cudaStream_t stream);
 int launch_decode_merge(const float *parts, int n_parts, int n_records, int head_dim, int dtype, void *out,
                         cudaStream_t stream);
 

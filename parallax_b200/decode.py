@@ -372,6 +372,10 @@ class GraphedDecode:
         return self.out
 
     def __call__(self, *, q=None, r=None, k=None, v=None, cache_seqlens=None) -> torch.Tensor:
+        host = ops.eager_host()
+        lens = cache_seqlens if self.cache_seqlens is not None else None
+        if host is not None and host.stage(self.q, q, self.r, r, self.cache_seqlens, lens, self.max_kv_len):
+            q = r = cache_seqlens = None                   # done, in one launch
         for dst, src in ((self.q, q), (self.r, r), (self.k, k), (self.v, v)):
             if src is not None:
                 dst.copy_(src)

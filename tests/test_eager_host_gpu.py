@@ -142,3 +142,31 @@ def test_two_streams_at_once():
                 got[i].append(plx.parallax_decode(q * (i + 1), r, k, v))
     torch.cuda.synchronize()
     assert all(torch.equal(x, want[i]) for i in range(2) for x in got[i])
+
+
+@pytest.mark.parametrize("bsz,h,d", [(1, 1, 64), (4, 8, 128), (512, 1, 64), (513, 1, 64)])
+def test_staging_of_a_captured_step(bsz, h, d):
+    """q, r and the lengths of a step reach the buffers of the captured launch: in one launch (up to 512 rows, host
+    lengths), and by the copies where that does not apply."""
+    gd = plx.GraphedDecode(bsz, h, max_kv_len=96, head_dim=d)
+    gd.k.copy_(randn(bsz, 96, h, d, seed=1))
+    gd.v.copy_(randn(bsz, 96, h, d, seed=2))
+    q, r = randn(bsz, 1, h, d, seed=3), randn(bsz, 1, h, d, seed=4)
+    lens = [1 + (i * 31) % 96 for i in range(bsz)]
+    for given in (lens, tuple(lens), torch.tensor(lens, dtype=torch.int32, device="cuda")):
+        gd.q.zero_(), gd.r.zero_(), gd.cache_seqlens.fill_(1)
+        before = _cabi.launch_count()
+        out = gd(q=q, r=r, cache_seqlens=given).clone()
+        assert _cabi.launch_count() - before == (1 if given is lens and bsz <= 512 else 0)
+        assert torch.equal(gd.q, q) and torch.equal(gd.r, r) and gd.cache_seqlens.tolist() == lens
+        assert torch.equal(out, plx.parallax_decode(q, r, gd.k, gd.v, seqused_k=gd.cache_seqlens))
+    gd(q=r)                                                    # the others stay
+    assert torch.equal(gd.q, r) and torch.equal(gd.r, r) and gd.cache_seqlens.tolist() == lens
+    gd(q=q.transpose(0, 1).contiguous().transpose(0, 1), cache_seqlens=96)
+    assert torch.equal(gd.q, q) and gd.cache_seqlens.tolist() == [96] * bsz
+    gd(r=q.float())                                            # converted, as copy_ does
+    assert torch.equal(gd.r, q)
+    for bad in ([0] * bsz, [97] * bsz, 0, 97):
+        with pytest.raises(ValueError, match="out of range"):
+            gd(cache_seqlens=bad)
+    assert gd.cache_seqlens.tolist() == [96] * bsz
