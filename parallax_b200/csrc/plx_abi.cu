@@ -288,11 +288,16 @@ int plx_train_bwd_stages(const plx_train_problem *p, int32_t stages, const void 
     a.cst = a.bst + train_stat_rows(p) * 8;
     cudaStream_t cs = reinterpret_cast<cudaStream_t>(stream);
     const bool tc = train_bwd_sm100_supported(a, p->head_dim);
-    for (int stage : {PLX_BWD_STATS, PLX_BWD_DQR, PLX_BWD_DKV}) {
+    // dk/dv before dq/dr: the two are independent, and the CTAs of the second start as those of the first, longer
+    // one leave their SMs
+    int before = 0;
+    for (int stage : {PLX_BWD_STATS, PLX_BWD_DKV, PLX_BWD_DQR}) {
         if (!(stages & stage)) continue;
-        st = (tc && stage != PLX_BWD_STATS) ? launch_train_bwd_sm100(a, p->dtype, p->head_dim, stage, cs)
+        const bool overlap = before == (stage == PLX_BWD_DKV ? PLX_BWD_STATS : PLX_BWD_DKV);
+        st = (tc && stage != PLX_BWD_STATS) ? launch_train_bwd_sm100(a, p->dtype, p->head_dim, stage, overlap, cs)
                                             : launch_train_bwd_mma(a, p->dtype, p->head_dim, stage, cs);
         if (st != PLX_OK) return st;
+        before = stage;
     }
     return PLX_OK;
 }

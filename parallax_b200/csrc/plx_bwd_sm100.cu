@@ -119,11 +119,18 @@ struct Item {
 // Work item `idx` of the launch.  Items are (batch, head)-major, so that CTAs running at the same time
 // share their streamed tiles in L2; inside a (batch, head) the 128-wide tiles alternate last, first,
 // last - 1, second, ...: under the causal mask any two neighbours add up to the same work.
+// With one item per CTA (n_bh > 0: the number of (batch, head) pairs) the longest items come first instead: the
+// CTAs of dq/dr take over the SMs that dk/dv leaves one by one.
 template <bool DQR>
-__device__ __forceinline__ Item get_item(const TrainArgs &a, int idx, int n_mt) {
+__device__ __forceinline__ Item get_item(const TrainArgs &a, int idx, int n_mt, int n_bh) {
     Item it;
-    const int bh = idx / n_mt, k = idx % n_mt;
-    const int tile_id = (k & 1) ? (k >> 1) : n_mt - 1 - (k >> 1);
+    int bh = idx / n_mt, k = idx % n_mt;
+    int tile_id = (k & 1) ? (k >> 1) : n_mt - 1 - (k >> 1);
+    if (n_bh > 0) {
+        bh = idx % n_bh;
+        k = idx / n_bh;
+        tile_id = DQR ? n_mt - 1 - k : k;
+    }
     Seq s;
     int tis = 0;
     it.valid = locate_tile(a, tile_id, kBM, s, tis);
@@ -172,7 +179,7 @@ __global__ void __launch_bounds__((4 + EW) * 32, 1)
 bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorMap tm_q,
                  const __grid_constant__ CUtensorMap tm_r, const __grid_constant__ CUtensorMap tm_go,
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const ErrSink sink,
-                 int n_mt, int n_items, int chunk_shift) {
+                 int n_mt, int n_items, int chunk_shift, int n_bh) {
     using L = Smem<D, MODE, NS>;
     constexpr bool DQR = MODE == kModeDQR;
     constexpr uint32_t kResBytes = L::kResBytes, kStrBytes = L::kStrBytes;
@@ -219,6 +226,13 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
     const uint32_t tAcc0 = tmem_base, tAcc1 = tmem_base + 128, tS = tmem_base + 256;  // S1, S2, A at tS + 0 / 64 / 128
     const uint32_t tK = tmem_base + 448;                                              // the M-side tile as an A operand
     const bool misaligned = cta_aborted(err);
+    // Set-up may run under the end of the kernel before.  dk/dv waits here for the row statistics, then lets dq/dr
+    // start, for which they are therefore complete too; dq/dr waits for dk/dv at its end, so that whatever follows
+    // on the stream follows both.
+    if (!DQR) {
+        grid_wait();
+        launch_dependents();
+    }
 
     if (misaligned) {
         // nothing was started: fall through to the common exit
@@ -232,7 +246,7 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
             for (int i = 0; ok; ++i) {
                 const int idx = item_index(i, chunk_shift);
                 if (idx >= n_items) break;
-                const Item it = get_item<DQR>(a, idx, n_mt);
+                const Item it = get_item<DQR>(a, idx, n_mt, n_bh);
                 if (it.n_iter == 0) continue;
                 // the resident tiles of the previous item are free once its last score product has completed
                 if (n > 0) {
@@ -369,7 +383,7 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
         for (int i = 0; ok; ++i) {
             const int idx = item_index(i, chunk_shift);
             if (idx >= n_items) break;
-            const Item it = get_item<DQR>(a, idx, n_mt);
+            const Item it = get_item<DQR>(a, idx, n_mt, n_bh);
             if (it.n_iter == 0) continue;
             if (warp == 1) {
                 ok = mbar_wait(bar(L::kXFull), n & 1, err, 4) && mbar_wait(bar(L::kKReady), n & 1, err, 14);
@@ -461,7 +475,7 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
             for (;;) {
                 const int idx = item_index(i_next++, chunk_shift);
                 if (idx >= n_items) return false;
-                cur = get_item<DQR>(a, idx, n_mt);
+                cur = get_item<DQR>(a, idx, n_mt, n_bh);
                 if (!cur.valid) continue;
                 if (cur.n_iter > 0) return true;
                 const int row = cur.m0 + ml;
@@ -697,13 +711,14 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
     tc_fence_before();
     __syncthreads();
     if (warp == 1) tmem_dealloc(tmem_base, kTmemCols);
+    if (DQR) grid_wait();
 }
 
 // ------------------------------------------------------------------------- //
 // host side
 // ------------------------------------------------------------------------- //
 template <typename T, int D, int MODE>
-int launch_mode(const TrainArgs &a, int n_tok, const ErrSink &sink, cudaStream_t stream) {
+int launch_mode(const TrainArgs &a, int n_tok, const ErrSink &sink, bool overlap, cudaStream_t stream) {
     // Ring depth: as many stages as the 227 KB of shared memory allow at head_dim 128 (dk/dv 3, dq/dr 4); six at
     // head_dim 64 (measured against four: dq/dr 0.883 vs 0.919 ms, dk/dv 1.337 vs 1.352 ms; two stages cost 20 %).
     constexpr int NS = D == 64 ? 6 : (MODE == kModeDKV ? 3 : 4);
@@ -734,9 +749,20 @@ int launch_mode(const TrainArgs &a, int n_tok, const ErrSink &sink, cudaStream_t
     // with plenty of items a CTA takes them in neighbouring pairs (a heavy and a light tile)
     const int chunk_shift = n_items >= 2 * sms ? 1 : 0;
     const int units = (n_items + (1 << chunk_shift) - 1) >> chunk_shift;
-    kern<<<units < sms ? units : sms, (4 + EW) * 32, L::kBytes, stream>>>(a, n_tok, tq, tr, tg, tk, tv, sink, tiles, n_items, chunk_shift);
+    const int n_bh = n_items <= sms ? a.batch * (DQR ? a.heads_q : a.heads_kv) : 0;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(units < sms ? units : sms);
+    cfg.blockDim = dim3((4 + EW) * 32);
+    cfg.dynamicSmemBytes = L::kBytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap ? 1 : 0;
+    const cudaError_t st = cudaLaunchKernelEx(&cfg, kern, a, n_tok, tq, tr, tg, tk, tv, sink, tiles, n_items, chunk_shift, n_bh);
     count_launch();
-    return cudaGetLastError() == cudaSuccess ? PLX_OK : PLX_ERR_LAUNCH;
+    return st == cudaSuccess && cudaGetLastError() == cudaSuccess ? PLX_OK : PLX_ERR_LAUNCH;
 }
 
 }  // namespace
@@ -748,7 +774,7 @@ bool train_bwd_sm100_supported(const TrainArgs &a, int head_dim) {
     return tma::encode_fn() != nullptr;
 }
 
-int launch_train_bwd_sm100(const TrainArgs &a, int dtype, int head_dim, int stage, cudaStream_t stream) {
+int launch_train_bwd_sm100(const TrainArgs &a, int dtype, int head_dim, int stage, bool overlap, cudaStream_t stream) {
     const ErrorWords ew = sm100_error_words();
     if (!ew.word) return PLX_ERR_LAUNCH;
     const ErrSink err{ew.word, ew.mirror};
@@ -756,17 +782,17 @@ int launch_train_bwd_sm100(const TrainArgs &a, int dtype, int head_dim, int stag
     const bool dqr = stage == PLX_BWD_DQR;
     if (dtype == PLX_BF16) {
         if (head_dim == 64)
-            return dqr ? launch_mode<__nv_bfloat16, 64, kModeDQR>(a, n_tok, err, stream)
-                       : launch_mode<__nv_bfloat16, 64, kModeDKV>(a, n_tok, err, stream);
-        return dqr ? launch_mode<__nv_bfloat16, 128, kModeDQR>(a, n_tok, err, stream)
-                   : launch_mode<__nv_bfloat16, 128, kModeDKV>(a, n_tok, err, stream);
+            return dqr ? launch_mode<__nv_bfloat16, 64, kModeDQR>(a, n_tok, err, overlap, stream)
+                       : launch_mode<__nv_bfloat16, 64, kModeDKV>(a, n_tok, err, overlap, stream);
+        return dqr ? launch_mode<__nv_bfloat16, 128, kModeDQR>(a, n_tok, err, overlap, stream)
+                   : launch_mode<__nv_bfloat16, 128, kModeDKV>(a, n_tok, err, overlap, stream);
     }
     if (dtype == PLX_FP16) {
         if (head_dim == 64)
-            return dqr ? launch_mode<__half, 64, kModeDQR>(a, n_tok, err, stream)
-                       : launch_mode<__half, 64, kModeDKV>(a, n_tok, err, stream);
-        return dqr ? launch_mode<__half, 128, kModeDQR>(a, n_tok, err, stream)
-                   : launch_mode<__half, 128, kModeDKV>(a, n_tok, err, stream);
+            return dqr ? launch_mode<__half, 64, kModeDQR>(a, n_tok, err, overlap, stream)
+                       : launch_mode<__half, 64, kModeDKV>(a, n_tok, err, overlap, stream);
+        return dqr ? launch_mode<__half, 128, kModeDQR>(a, n_tok, err, overlap, stream)
+                   : launch_mode<__half, 128, kModeDKV>(a, n_tok, err, overlap, stream);
     }
     return PLX_ERR_UNSUPPORTED;
 }

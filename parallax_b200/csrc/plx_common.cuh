@@ -73,6 +73,11 @@ __device__ __forceinline__ float fast_exp2(float x) {
     return y;
 }
 
+// Programmatic dependent launch.  launch_dependents: this CTA no longer holds back the next kernel of the stream
+// (if that one was launched for it).  grid_wait: wait for the kernels this one may overlap, and see their writes.
+__device__ __forceinline__ void launch_dependents() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+
 // 16-byte asynchronous copy global -> shared; bytes == 0 zero-fills the destination.
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void *src, int bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(bytes));

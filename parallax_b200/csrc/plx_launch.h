@@ -32,7 +32,9 @@ int sm100_error_word(int *value, bool clear);   // synchronises the device
 int sm100_error_peek(int *value, bool clear);   // reads (and optionally clears) the host mirror only: no synchronisation
 // tcgen05 backward: stage is PLX_BWD_DQR or PLX_BWD_DKV (the row statistics must already be in a.bst)
 bool train_bwd_sm100_supported(const TrainArgs &a, int head_dim);
-int launch_train_bwd_sm100(const TrainArgs &a, int dtype, int head_dim, int stage, cudaStream_t stream);
+// `overlap`: the kernel launched just before on this stream is the row statistics (dk/dv) or dk/dv (dq/dr) of the
+// same call, and this one may start under its end
+int launch_train_bwd_sm100(const TrainArgs &a, int dtype, int head_dim, int stage, bool overlap, cudaStream_t stream);
 
 constexpr int kDecodeGqaWarps = 8;   // warps (independent splits) per CTA of the grouped-query decode kernel
 int launch_decode(const DecodeArgs &a, int dtype, int head_dim, cudaStream_t stream);

@@ -379,6 +379,7 @@ __global__ void __launch_bounds__(256, 4) bwd_stats_kernel(const TrainArgs a, in
     const int lane = threadIdx.x & 31;
     const int64_t total = static_cast<int64_t>(a.batch) * a.heads_q * n_tok;
     const int64_t first = (static_cast<int64_t>(blockIdx.x) * 8 + (threadIdx.x >> 5)) * R;
+    launch_dependents();   // the kernel behind sets itself up under the last wave of this one
     if (first >= total) return;
     // Row `gid` = first + off, off < R: the 64-bit division happens once per warp (for `first`), the rows
     // of the warp follow by stepping -- with a division per row the kernel was bound by integer
