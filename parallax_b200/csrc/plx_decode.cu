@@ -273,7 +273,7 @@ struct SplitPlan {
 // ..: up to kBalancedRows rows.  A row's parts must fit the merge: 32 records in one level, 32 per group in two.
 template <int G, bool UNIFORM>
 __device__ __forceinline__ SplitPlan plan_slot(const DecodeArgs &a, int slot, int lane) {
-    SplitPlan p;
+    SplitPlan p{-1, 0, 1, 0, 0, 0};
     if (UNIFORM || !a.balanced) {
         p.b = slot / a.n_splits;
         p.part = slot - p.b * a.n_splits;
@@ -317,7 +317,6 @@ __device__ __forceinline__ SplitPlan plan_slot(const DecodeArgs &a, int slot, in
         else bad = mid + 1;
     }
     // the row that owns this slot
-    p.b = -1;
     int before = 0;       // parts of the rows of earlier i
 #pragma unroll
     for (int i = 0; i < kRows; ++i) {
@@ -832,9 +831,25 @@ int launch_decode_exchange_merge(const ExchangeArgs &x, const float *part, int h
 // K and V in its own shared memory (16-byte cp.async, kGqaStages deep, rows padded to D + 8
 // elements; one bulk copy per row measured 1.6x slower: 32 small copies per tile queue up),
 // forms S1 = Q_g K^T and S2 = R_g K^T, runs the online softmax per row in the accumulator
-// fragments, and accumulates O1 += P1 V, O2 += P2 V with the P fragments as the A operand.  Warps
-// never synchronise with each other; splits are merged as above.
+// fragments, and accumulates O1 += P1 V, O2 += P2 V with the P fragments as the A operand.  The eight
+// warps of a CTA are adjacent splits of one kv head; they meet in shared memory at the end.
 // ========================================================================= //
+// a lane's channels of a record, 16 or 8 bytes
+__device__ __forceinline__ void load_channels(const float *p, float (&x)[4]) {
+    const float4 v = *reinterpret_cast<const float4 *>(p);
+    x[0] = v.x; x[1] = v.y; x[2] = v.z; x[3] = v.w;
+}
+__device__ __forceinline__ void load_channels(const float *p, float (&x)[2]) {
+    const float2 v = *reinterpret_cast<const float2 *>(p);
+    x[0] = v.x; x[1] = v.y;
+}
+__device__ __forceinline__ void store_channels(float *p, const float (&x)[4]) {
+    __stcg(reinterpret_cast<float4 *>(p), make_float4(x[0], x[1], x[2], x[3]));
+}
+__device__ __forceinline__ void store_channels(float *p, const float (&x)[2]) {
+    __stcg(reinterpret_cast<float2 *>(p), make_float2(x[0], x[1]));
+}
+
 constexpr int kGqaTile = 16;     // keys per staged tile
 constexpr int kGqaStages = 3;
 constexpr int kGqaWarps = kDecodeGqaWarps;   // warps (independent splits) per CTA
@@ -851,36 +866,28 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
     constexpr int KS = D / 16;                      // k-steps of the score products
     constexpr uint32_t kTileBytes = kGqaTile * LD * 2;
     constexpr int CPR = D / 8;                      // 16-byte chunks per row
+    static_assert(16 * REC * 4 <= GqaSmem<D>::kPerWarp, "a warp's records fit where its tiles were");
     extern __shared__ __align__(16) unsigned char gqa_smem[];
+    __shared__ int s_row[kGqaWarps], s_arrived[kGqaWarps];   // batch row of each warp (-1: none); arrival order of its segment
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    // warps are dealt out over (batch, kv head, head group, split), so a CTA is full whatever the split count:
-    // split-fastest for rows of one length; with the slots dealt out by length, head-fastest within a slot
-    const int64_t wid = static_cast<int64_t>(blockIdx.x) * kGqaWarps + warp;
+    // A CTA is eight adjacent slots of one (kv head, head group); heads are fastest over the grid, so CTAs that run
+    // together read neighbouring memory.
     const int n_hunits = a.heads_kv * n_hgroups, n_slots = a.batch * a.n_splits;
-    if (wid >= static_cast<int64_t>(n_slots) * n_hunits) return;
-    int slot, hunit;
-    if (a.balanced) {
-        slot = static_cast<int>(wid / n_hunits);
-        hunit = static_cast<int>(wid - static_cast<int64_t>(slot) * n_hunits);
-    } else {
-        const int unit = static_cast<int>(wid / a.n_splits);
-        hunit = unit % n_hunits;
-        slot = unit / n_hunits * a.n_splits + static_cast<int>(wid % a.n_splits);
-    }
+    const int hunit = blockIdx.x % n_hunits, cta = blockIdx.x / n_hunits, slot = cta * kGqaWarps + warp;
     const int hk = hunit / n_hgroups, hgrp = hunit % n_hgroups;
-    const SplitPlan plan = plan_slot<kGqaTile, false>(a, slot, lane);
-    if (plan.b < 0) return;
-    const int b = plan.b, my_lo = plan.lo, my_hi = plan.hi;
+    SplitPlan plan{-1, 0, 0, 0, 0, 0};
+    if (slot < n_slots) plan = plan_slot<kGqaTile, false>(a, slot, lane);
+    const int b = max(plan.b, 0), my_lo = plan.lo, my_hi = plan.b < 0 ? plan.lo : plan.hi;
     const int n_tiles = (my_hi - my_lo + kGqaTile - 1) / kGqaTile;
-    const int hq0 = hk * a.n_rep + hgrp * 16;       // first q head of this warp's rows
+    const int hq0 = hk * a.n_rep + hgrp * 16;       // first q head of this CTA's rows
     const int n_rows = min(16, a.n_rep - hgrp * 16);
     const uint32_t sbase = smem_u32(gqa_smem) + warp * GqaSmem<D>::kPerWarp;
     auto sK = [&](int st) -> uint32_t { return sbase + st * 2 * kTileBytes; };
     auto sV = [&](int st) -> uint32_t { return sbase + st * 2 * kTileBytes + kTileBytes; };
+    if (lane == 0) s_row[warp] = plan.b;
 
-    // ---- q and r of the group -> A fragments (staged through the first two tile buffers)
-    uint32_t qa[KS][4], ra[KS][4];
+    // ---- q and r of the group -> the buffers of the last stage; the first tiles follow at once
     {
         const T *qg = static_cast<const T *>(a.q) + (static_cast<int64_t>(b) * a.heads_q + hq0) * D;
         const T *rg = static_cast<const T *>(a.r) + (static_cast<int64_t>(b) * a.heads_q + hq0) * D;
@@ -889,36 +896,34 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
             const int row = c / CPR, col = c % CPR;
             const int bytes = row < n_rows ? 16 : 0;                      // rows past the group: zeros
             const int64_t at = static_cast<int64_t>(row < n_rows ? row : 0) * D + col * 8;
-            cp_async16(sK(0) + (row * LD + col * 8) * 2, qg + at, bytes);
-            cp_async16(sV(0) + (row * LD + col * 8) * 2, rg + at, bytes);
+            cp_async16(sK(kGqaStages - 1) + (row * LD + col * 8) * 2, qg + at, bytes);
+            cp_async16(sV(kGqaStages - 1) + (row * LD + col * 8) * 2, rg + at, bytes);
         }
         cp_async_commit();
-        cp_async_wait<0>();
-        __syncwarp();
-#pragma unroll
-        for (int ks = 0; ks < KS; ++ks) {
-            ldsm_x4(qa[ks], a_addr<LD>(sK(0), 0, ks * 16, lane));
-            ldsm_x4(ra[ks], a_addr<LD>(sV(0), 0, ks * 16, lane));
-        }
-        __syncwarp();
     }
 
     // Tile i of this warp -> stage i % kGqaStages.  A lane copies the same 16-byte column of every
     // (32 / CPR)-th row, so its source and destination advance by constants; rows past my_hi (last tile
-    // only) are zero-filled.
+    // only) are zero-filled.  In a paged cache a tile lies in one page when pages hold at least a tile and the
+    // range starts on a tile boundary (it does but for windows and cache_start): one page number per tile then,
+    // read a tile ahead.
     constexpr int RPI = 32 / CPR;                                  // rows covered by one instruction of the warp
     const int my_row = lane / CPR, my_col = lane % CPR;
     const bool paged = a.page_table != nullptr;      // uniform over the launch
+    const bool page_per_tile = paged && a.page_mask + 1 >= kGqaTile && my_lo % kGqaTile == 0;
     const T *kp = static_cast<const T *>(a.k) + (paged ? 0 : b * a.kv_sb) + hk * a.kv_sh + my_col * 8;
     const T *vp = static_cast<const T *>(a.v) + (paged ? 0 : b * a.kv_sb) + hk * a.kv_sh + my_col * 8;
     const uint32_t my_dst = (my_row * LD + my_col * 8) * 2;
+    int64_t next_tile = page_per_tile && n_tiles > 0 ? paged_key_offset(a, b, my_lo) : 0;   // of the next tile's first row
     auto load_tile = [&](int i) {
         if (i < n_tiles) {
-            const int st = i % kGqaStages, key0 = my_lo + i * kGqaTile + my_row;
+            const int st = i % kGqaStages, tile0 = my_lo + i * kGqaTile, key0 = tile0 + my_row;
             const uint32_t dk = sK(st) + my_dst, dv = sV(st) + my_dst;
-            const bool whole = key0 - my_row + kGqaTile <= my_hi;
-            if (!paged) {
-                const int64_t at = static_cast<int64_t>(key0) * a.kv_st, step = static_cast<int64_t>(RPI) * a.kv_st;
+            const bool whole = tile0 + kGqaTile <= my_hi;
+            if (!paged || page_per_tile) {
+                const int64_t step = static_cast<int64_t>(RPI) * a.kv_st;
+                const int64_t at = page_per_tile ? next_tile + my_row * a.kv_st : static_cast<int64_t>(key0) * a.kv_st;
+                if (page_per_tile && i + 1 < n_tiles) next_tile = paged_key_offset(a, b, tile0 + kGqaTile);
                 if (whole) {
 #pragma unroll
                     for (int j = 0; j < kGqaTile / RPI; ++j) {
@@ -945,6 +950,17 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
         }
         cp_async_commit();             // always: keeps the group count uniform
     };
+#pragma unroll
+    for (int i = 0; i < kGqaStages - 1; ++i) load_tile(i);
+
+    uint32_t qa[KS][4], ra[KS][4];     // q and r as A fragments
+    cp_async_wait<kGqaStages - 1>();
+    __syncwarp();
+#pragma unroll
+    for (int ks = 0; ks < KS; ++ks) {
+        ldsm_x4(qa[ks], a_addr<LD>(sK(kGqaStages - 1), 0, ks * 16, lane));
+        ldsm_x4(ra[ks], a_addr<LD>(sV(kGqaStages - 1), 0, ks * 16, lane));
+    }
 
     // per-row state (rows g and g + 8 of the group); d1 / d2 are this thread's share until the end
     float m[2] = {-INFINITY, -INFINITY}, d1[2] = {0.f, 0.f}, d2[2] = {0.f, 0.f};
@@ -954,13 +970,10 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
 #pragma unroll
         for (int e = 0; e < 4; ++e) o1[i][e] = o2[i][e] = 0.f;
 
-#pragma unroll
-    for (int i = 0; i < kGqaStages - 1; ++i) load_tile(i);
-
     for (int i = 0; i < n_tiles; ++i) {
         const int st = i % kGqaStages, key0 = my_lo + i * kGqaTile;
         cp_async_wait<kGqaStages - 2>();
-        __syncwarp();                    // tile i has landed for every lane, and every lane has left tile i - 1
+        __syncwarp();                    // tile i has landed for every lane, and every lane has left tile i - 1 (i = 0: q and r)
         load_tile(i + kGqaStages - 1);   // into the stage that tile i - 1 has just left
 
         // S1, S2: 16 rows x 16 keys (two 8-key blocks)
@@ -1042,54 +1055,37 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
         d2[hh] += __shfl_xor_sync(0xffffffffu, d2[hh], 2);
     }
 
-    // Row g + 8 hh of the group is q head hq0 + g + 8 hh; this thread holds its channels 8 i + 2 t, + 1.
-    const bool row_ok[2] = {g < n_rows, g + 8 < n_rows};
-    auto bh_of = [&](int row) -> int64_t { return static_cast<int64_t>(b) * a.heads_q + hq0 + row; };
-
-    if (plan.n_parts == 1) {
-#pragma unroll
-        for (int hh = 0; hh < 2; ++hh) {
-            if (!row_ok[hh]) continue;
-            const int64_t bh = bh_of(g + 8 * hh);
-            if (a.part_out) {
-                float *rec = a.part_out + bh * REC;
-                if (t == 0) *reinterpret_cast<float4 *>(rec) = make_float4(m[hh], d1[hh], d2[hh], 0.f);
-#pragma unroll
-                for (int i = 0; i < D / 8; ++i) {
-                    *reinterpret_cast<float2 *>(rec + 4 + 8 * i + 2 * t) = make_float2(o1[i][2 * hh], o1[i][2 * hh + 1]);
-                    *reinterpret_cast<float2 *>(rec + 4 + D + 8 * i + 2 * t) = make_float2(o2[i][2 * hh], o2[i][2 * hh + 1]);
-                }
-            } else {
-                T *dst = static_cast<T *>(a.out) + bh * D;
-#pragma unroll
-                for (int i = 0; i < D / 8; ++i)
-                    *reinterpret_cast<uint32_t *>(dst + 8 * i + 2 * t) =
-                        Elem<T>::pack(finalize(d1[hh], d2[hh], o1[i][2 * hh], o2[i][2 * hh]),
-                                      finalize(d1[hh], d2[hh], o1[i][2 * hh + 1], o2[i][2 * hh + 1]));
-            }
-        }
-        return;
-    }
-
-    // publish this split's state of every row
-    auto recs_of = [&](int row) -> float * { return a.ws_parts + (plan.first + static_cast<int64_t>(hq0 + row) * plan.n_parts) * REC; };
+    // ---- merge.  Every warp leaves its state in its own shared memory, where its tiles were: one record per row of
+    // the group.  The warps of a batch row are neighbours (a segment).  The rows of all segments are dealt out to the
+    // warps; a segment that is all of its (batch row, head) writes the result, any other one record per row to
+    // global memory, and the CTA whose segment arrives last there merges those.
+    // (Through global memory warp by warp, in two levels beyond 32 splits, the merge was most of a short launch.)
+    float *own = reinterpret_cast<float *>(gqa_smem + warp * GqaSmem<D>::kPerWarp);
+    __syncwarp();                        // every lane has left the last tile (and q, r, where there was none)
 #pragma unroll
     for (int hh = 0; hh < 2; ++hh) {
-        if (!row_ok[hh]) continue;
-        float *ws = recs_of(g + 8 * hh) + static_cast<int64_t>(plan.part) * REC;
-        if (t == 0) __stcg(reinterpret_cast<float4 *>(ws), make_float4(m[hh], d1[hh], d2[hh], 0.f));
+        const int row = g + 8 * hh;
+        if (row >= n_rows) continue;
+        float *rec = own + row * REC;    // this thread holds channels 8 i + 2 t, + 1
+        if (t == 0) *reinterpret_cast<float4 *>(rec) = make_float4(m[hh], d1[hh], d2[hh], 0.f);
 #pragma unroll
         for (int i = 0; i < D / 8; ++i) {
-            __stcg(reinterpret_cast<float2 *>(ws + 4 + 8 * i + 2 * t), make_float2(o1[i][2 * hh], o1[i][2 * hh + 1]));
-            __stcg(reinterpret_cast<float2 *>(ws + 4 + D + 8 * i + 2 * t), make_float2(o2[i][2 * hh], o2[i][2 * hh + 1]));
+            *reinterpret_cast<float2 *>(rec + 4 + 8 * i + 2 * t) = make_float2(o1[i][2 * hh], o1[i][2 * hh + 1]);
+            *reinterpret_cast<float2 *>(rec + 4 + D + 8 * i + 2 * t) = make_float2(o2[i][2 * hh], o2[i][2 * hh + 1]);
         }
     }
-    __threadfence();
-    __syncwarp();
+    // segment of this warp: warps w0 .. w0 + n_seg - 1; where its (batch row, head) begins among the slots
+    __syncthreads();
+    int w0 = warp, n_seg = 0;
+    while (w0 > 0 && s_row[w0 - 1] == plan.b) --w0;
+    while (w0 + n_seg < kGqaWarps && s_row[w0 + n_seg] == plan.b) ++n_seg;
+    const int head_slot = slot - plan.part, first_cta = head_slot / kGqaWarps;
+    const int n_ctas = plan.b < 0 ? 0 : (head_slot + plan.n_parts - 1) / kGqaWarps - first_cta + 1;
+    const bool alone = n_ctas == 1;
+    auto bh_of = [&](int row) -> int64_t { return static_cast<int64_t>(b) * a.heads_q + hq0 + row; };
+    auto recs_of = [&](int row) -> float * { return a.ws_parts + (plan.first + static_cast<int64_t>(hq0 + row) * plan.n_parts) * REC; };
 
-    // Arrival: lane r < n_rows counts for row r (all rows at once, one round trip); the warp then merges
-    // the rows for which it arrived last.
-    float big, D1, D2, O1[CH], O2[CH];
+    float big = -INFINITY, D1 = 0.f, D2 = 0.f, O1[CH], O2[CH];
     auto emit = [&](int64_t bh) {
         if (a.part_out) {
             float *rec = a.part_out + bh * REC;
@@ -1110,111 +1106,68 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
             }
         }
     };
-    // Merge, for every row in `rows`, its n <= 32 records (the first one of row r at first_rec(r)), and hand
-    // each result to sink(r).  Record by record and row by row this is a chain of L2 round trips (three per
-    // row); here the header loads of all rows are in flight together (parked in this warp's shared memory,
-    // which the tiles no longer need) and every row then takes one round of 16 record loads.
-    float *hpark = reinterpret_cast<float *>(gqa_smem + warp * GqaSmem<D>::kPerWarp);
-    auto merge_rows = [&](unsigned rows, auto first_rec, int n, auto sink) {
-#pragma unroll
-        for (int r = 0; r < 16; ++r) {
-            float4 h = make_float4(-INFINITY, 0.f, 0.f, 0.f);
-            if (((rows >> r) & 1) && lane < n) h = __ldcg(reinterpret_cast<const float4 *>(first_rec(r) + static_cast<int64_t>(lane) * REC));
-            hpark[r * 32 + lane] = h.x;
-            hpark[512 + r * 32 + lane] = h.y;
-            hpark[1024 + r * 32 + lane] = h.z;
-        }
-#pragma unroll 1
-        for (int r = 0; r < n_rows; ++r) {
-            if (!((rows >> r) & 1)) continue;
-            const float hm = hpark[r * 32 + lane];
-            big = hm;
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, off));
+    // the warps of a segment share its rows
+    if (plan.b >= 0) {
+        for (int row = warp - w0; row < n_rows; row += n_seg) {
+            const float *rec0 = reinterpret_cast<const float *>(gqa_smem + w0 * GqaSmem<D>::kPerWarp) + row * REC;
+            constexpr int kStride = GqaSmem<D>::kPerWarp / 4;
+            big = -INFINITY;
+            for (int w = 0; w < n_seg; ++w) big = fmaxf(big, rec0[w * kStride]);
             const float safe = big == -INFINITY ? 0.f : big;
-            const float wl = fast_exp2(hm - safe);   // weight of record `lane` (0 beyond n: m = -inf there)
-            D1 = wl * hpark[512 + r * 32 + lane];
-            D2 = wl * hpark[1024 + r * 32 + lane];
-#pragma unroll
-            for (int off = 16; off > 0; off >>= 1) {
-                D1 += __shfl_xor_sync(0xffffffffu, D1, off);
-                D2 += __shfl_xor_sync(0xffffffffu, D2, off);
-            }
+            D1 = D2 = 0.f;
 #pragma unroll
             for (int e = 0; e < CH; ++e) O1[e] = O2[e] = 0.f;
-            const float *col = first_rec(r) + 4 + lane * CH;
+            for (int w = 0; w < n_seg; ++w) {
+                const float *rec = rec0 + w * kStride;
+                const float wt = fast_exp2(rec[0] - safe);
+                D1 = fmaf(wt, rec[1], D1);
+                D2 = fmaf(wt, rec[2], D2);
+                float x[CH], y[CH];
+                load_channels(rec + 4 + lane * CH, x);
+                load_channels(rec + 4 + D + lane * CH, y);
 #pragma unroll
-            for (int j0 = 0; j0 < 32; j0 += 16) {
-                if (j0 >= n) break;
-                float x[16][CH], y[16][CH];
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const float *pr = col + static_cast<int64_t>(min(j0 + j, n - 1)) * REC;   // weight 0 past the end
-                    if (CH == 4) {
-                        const float4 u = __ldcg(reinterpret_cast<const float4 *>(pr)), v = __ldcg(reinterpret_cast<const float4 *>(pr + D));
-                        x[j][0] = u.x; x[j][1] = u.y; x[j][CH - 2] = u.z; x[j][CH - 1] = u.w;
-                        y[j][0] = v.x; y[j][1] = v.y; y[j][CH - 2] = v.z; y[j][CH - 1] = v.w;
-                    } else {
-                        const float2 u = __ldcg(reinterpret_cast<const float2 *>(pr)), v = __ldcg(reinterpret_cast<const float2 *>(pr + D));
-                        x[j][0] = u.x; x[j][1] = u.y;
-                        y[j][0] = v.x; y[j][1] = v.y;
-                    }
-                }
-#pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const float w = __shfl_sync(0xffffffffu, wl, j0 + j);
-#pragma unroll
-                    for (int e = 0; e < CH; ++e) {
-                        O1[e] = fmaf(w, x[j][e], O1[e]);
-                        O2[e] = fmaf(w, y[j][e], O2[e]);
-                    }
+                for (int e = 0; e < CH; ++e) {
+                    O1[e] = fmaf(wt, x[e], O1[e]);
+                    O2[e] = fmaf(wt, y[e], O2[e]);
                 }
             }
-            sink(r);
+            if (alone) {
+                emit(bh_of(row));
+            } else {
+                float *dst = recs_of(row) + static_cast<int64_t>(cta - first_cta) * REC;
+                if (lane == 0) __stcg(reinterpret_cast<float4 *>(dst), make_float4(big, D1, D2, 0.f));
+                store_channels(dst + 4 + lane * CH, O1);
+                store_channels(dst + 4 + D + lane * CH, O2);
+            }
         }
-    };
-    const bool one_level = plan.n_parts <= 32;
-    const int gmax = a.balanced ? 32 : PLX_DECODE_GROUP, n_groups = (plan.n_parts + gmax - 1) / gmax;
-    const int group = plan.part / gmax, first = group * gmax, gsize = min(gmax, plan.n_parts - first);
-    unsigned mine = 0;
-    if (lane < n_rows) {
-        int *counter = one_level ? a.ws_counters + bh_of(lane) : a.ws_gcounters + bh_of(lane) * a.n_groups + group;
-        if (atomicAdd(counter, 1) == (one_level ? plan.n_parts : gsize) - 1) mine = 1u << lane;
     }
-    unsigned todo = __reduce_or_sync(0xffffffffu, mine);
-    if (todo == 0) return;
     __threadfence();
-    auto finish = [&](int row) {
-        const int64_t bh = bh_of(row);
-        emit(bh);
-        if (lane == 0) a.ws_counters[bh] = 0;   // ready for the next launch on this workspace
-    };
-    if (one_level) {
-        merge_rows(todo, recs_of, plan.n_parts, finish);
-        return;
-    }
-    // two levels: merge this group's records of the rows in `todo`, then arrive for those rows at the second level
-    merge_rows(todo, [&](int row) { return recs_of(row) + static_cast<int64_t>(first) * REC; }, gsize, [&](int row) {
-        const int64_t bh = bh_of(row);
-        float *grec = a.ws_gparts + (bh * a.n_groups + group) * REC;
-        if (lane == 0) {
-            __stcg(reinterpret_cast<float4 *>(grec), make_float4(big, D1, D2, 0.f));
-            a.ws_gcounters[bh * a.n_groups + group] = 0;
-        }
+    __syncthreads();
+    if (plan.b >= 0 && !alone && warp == w0 && lane == 0) s_arrived[warp] = atomicAdd(a.ws_counters + bh_of(0), 1);
+    __syncthreads();
+    if (plan.b < 0 || alone || s_arrived[w0] != n_ctas - 1) return;
+    __threadfence();
+    // last: merge the n_ctas records of every row, 32 at a time
+    for (int row = warp - w0; row < n_rows; row += n_seg) {
+        const float *recs = recs_of(row);
+        warp_merge<D>(recs, min(n_ctas, 32), lane, big, D1, D2, O1, O2);
+        for (int j = 32; j < n_ctas; j += 32) {
+            float big2, E1, E2, P1[CH], P2[CH];
+            warp_merge<D>(recs + static_cast<int64_t>(j) * REC, min(n_ctas - j, 32), lane, big2, E1, E2, P1, P2);
+            const float top = fmaxf(big, big2), safe = top == -INFINITY ? 0.f : top;
+            const float wa = fast_exp2(big - safe), wb = fast_exp2(big2 - safe);
+            big = top;
+            D1 = wa * D1 + wb * E1;
+            D2 = wa * D2 + wb * E2;
 #pragma unroll
-        for (int e = 0; e < CH; ++e) {
-            __stcg(grec + 4 + lane * CH + e, O1[e]);
-            __stcg(grec + 4 + D + lane * CH + e, O2[e]);
+            for (int e = 0; e < CH; ++e) {
+                O1[e] = wa * O1[e] + wb * P1[e];
+                O2[e] = wa * O2[e] + wb * P2[e];
+            }
         }
-    });
-    __threadfence();
-    __syncwarp();
-    mine = 0;
-    if (lane < n_rows && ((todo >> lane) & 1) && atomicAdd(a.ws_counters + bh_of(lane), 1) == n_groups - 1) mine = 1u << lane;
-    todo = __reduce_or_sync(0xffffffffu, mine);
-    if (todo == 0) return;
-    __threadfence();
-    merge_rows(todo, [&](int row) { return a.ws_gparts + bh_of(row) * a.n_groups * REC; }, n_groups, finish);
+        emit(bh_of(row));
+    }
+    if (warp == w0 && lane == 0) a.ws_counters[bh_of(0)] = 0;   // ready for the next launch on this workspace
 }
 
 template <typename T, int D>
@@ -1237,8 +1190,8 @@ static int launch_decode_gqa(const DecodeArgs &a, cudaStream_t stream) {
             done[dev] = true;
         }
     }
-    const int64_t n_warps = static_cast<int64_t>(a.batch) * a.heads_kv * n_hgroups * a.n_splits;
-    kern<<<static_cast<unsigned>((n_warps + kGqaWarps - 1) / kGqaWarps), kGqaWarps * 32, kSmem, stream>>>(a, n_hgroups);
+    const int64_t ctas = (static_cast<int64_t>(a.batch) * a.n_splits + kGqaWarps - 1) / kGqaWarps * a.heads_kv * n_hgroups;
+    kern<<<static_cast<unsigned>(ctas), kGqaWarps * 32, kSmem, stream>>>(a, n_hgroups);
     count_launch();
     return cudaGetLastError() == cudaSuccess ? PLX_OK : PLX_ERR_LAUNCH;
 }

@@ -714,3 +714,40 @@ def test_rows_of_very_different_lengths(case):
             continue
         ref = orc.decode(q[b:b + 1].cpu(), r[b:b + 1].cpu(), k[b:b + 1, lo:used[b]].cpu(), v[b:b + 1, lo:used[b]].cpu())
         assert_close(out[b:b + 1].float().cpu(), ref, DECODE_REL_L2, DECODE_MAX_REL, f"{case} row {b}")
+
+
+@pytest.mark.parametrize("case", [
+    # batch, hq, hkv, cache, head_dim, page (0: dense), ragged, splits
+    (1, 8, 2, 4111, 128, 0, False, 61),      # one row over eight CTAs
+    (3, 8, 1, 5000, 64, 64, False, 255),     # a row over 33 CTAs, its first and last shared with other rows
+    (3, 32, 1, 700, 128, 16, True, 5),       # 32 q heads: two head groups; three rows in two CTAs
+    (5, 16, 2, 650, 64, 8, True, 3),         # pages smaller than a tile
+    (9, 24, 2, 333, 128, 32, True, 1),       # 12 q heads; every warp a row of its own
+    (2, 8, 2, 16384, 64, 0, True, 256),      # ragged: more than 256 parts of one row
+])
+def test_grouped_decode_merges_inside_and_between_ctas(case, monkeypatch):
+    """The warps of a CTA are neighbouring splits, of one row or of several; a row may end in the middle of a CTA."""
+    bsz, hq, hkv, kv_len, d, page, ragged, splits = case
+    monkeypatch.setenv("PLX_DECODE_SPLITS", str(splits))
+    q, r, k, v = make(bsz, hq, kv_len, d, hkv, seed=71)
+    used = [max(1, kv_len // (1 + 40 * (b % 2)) - 3 * b) for b in range(bsz)] if ragged else None
+    args, pk, pv = {}, k, v
+    if page:
+        per_row = -(-kv_len // page)
+        order = torch.randperm(bsz * per_row, generator=torch.Generator().manual_seed(3)).view(bsz, per_row)
+        pk, pv = (torch.zeros(bsz * per_row, page, hkv, d, dtype=k.dtype) for _ in range(2))
+        for b in range(bsz):
+            for pool, x in ((pk, k), (pv, v)):
+                flat = torch.zeros(per_row * page, hkv, d, dtype=k.dtype)
+                flat[:kv_len] = x[b]
+                pool[order[b]] = flat.view(per_row, page, hkv, d)
+        args["page_table"] = order.int().cuda()
+        used = used or [kv_len] * bsz
+    if used:
+        args["seqused_k"] = torch.tensor(used, dtype=torch.int32, device="cuda")
+    for window in (None, 77):
+        call = lambda: plx.parallax_attn_with_kvcache(*cuda(q, r, pk, pv), window_size=window, **args)
+        out = call()
+        ref = orc.decode(q, r, k, v, window_size_left=-1 if window is None else window, seqused_k=used)
+        assert_close(out.float().cpu(), ref, DECODE_REL_L2, DECODE_MAX_REL, f"{case} {window}")
+        assert torch.equal(out, call())
