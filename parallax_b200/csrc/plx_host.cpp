@@ -173,46 +173,46 @@ struct Refused {};   // a status of the library that the Python path has to repo
 
 // One node for forward and backward, as the custom op plx::train_fwd registers it.
 struct Train : torch::autograd::Function<Train> {
-    static Tensor forward(torch::autograd::AutogradContext *ctx, const Tensor &q, const Tensor &r, const Tensor &k, const Tensor &v,
+    static torch::autograd::variable_list forward(torch::autograd::AutogradContext *ctx, const Tensor &q, const Tensor &r, const Tensor &k, const Tensor &v,
                           double scale, int64_t window, int64_t layout, const OptTensor &cu) {
         at::AutoDispatchBelowADInplaceOrView below;
         const c10::cuda::CUDAGuard device(q.device());
         Tensor o = at::empty_like(q), barv = at::empty_like(q);
-        const Tensor stats = at::empty({3, q.size(0), q.size(1), q.size(2)}, q.options().dtype(at::kFloat));   // d1, bart, m
-        const Tensor d1 = stats[0];
-        float *st = stats.data_ptr<float>();
-        const int64_t n = d1.numel();
+        const auto stat = [&] { return at::empty({q.size(0), q.size(1), q.size(2)}, q.options().dtype(at::kFloat)); };
+        Tensor d1 = stat(), bart = stat(), m = stat();
         const plx_train_problem p = train_problem(q, k, d1, scale, window, layout, cu);
-        if (api.train_fwd(&p, q.data_ptr(), r.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), barv.data_ptr(), st, st + n, st + 2 * n,
-                          c10::cuda::getCurrentCUDAStream().stream()) != PLX_OK)
+        if (api.train_fwd(&p, q.data_ptr(), r.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), barv.data_ptr(),
+                          d1.data_ptr<float>(), bart.data_ptr<float>(), m.data_ptr<float>(), c10::cuda::getCurrentCUDAStream().stream()) != PLX_OK)
             throw Refused();
-        ctx->save_for_backward({q, r, k, v, o, barv, stats, cu ? *cu : Tensor()});
+        ctx->save_for_backward({q, r, k, v, o, barv, d1, bart, m, cu ? *cu : Tensor()});
+        ctx->set_materialize_grads(false);   // gradients of barv and the statistics are not looked at
         ctx->saved_data["scale"] = scale;
         ctx->saved_data["window"] = window;
         ctx->saved_data["layout"] = layout;
-        return o;
+        return {o, barv, d1, bart, m};
     }
 
     static torch::autograd::variable_list backward(torch::autograd::AutogradContext *ctx, torch::autograd::variable_list grads) {
         const auto saved = ctx->get_saved_variables();
-        const Tensor &q = saved[0], &r = saved[1], &k = saved[2], &v = saved[3], &o = saved[4], &barv = saved[5], &stats = saved[6];
-        const OptTensor cu = saved[7].defined() ? OptTensor(saved[7]) : std::nullopt;
+        const Tensor &q = saved[0], &r = saved[1], &k = saved[2], &v = saved[3], &o = saved[4], &barv = saved[5], &d1 = saved[6],
+                     &bart = saved[7], &m = saved[8];
+        const OptTensor cu = saved[9].defined() ? OptTensor(saved[9]) : std::nullopt;
         const double scale = ctx->saved_data["scale"].toDouble();
         const int64_t window = ctx->saved_data["window"].toInt(), layout = ctx->saved_data["layout"].toInt();
-        Tensor go = grads[0];
+        Tensor go = grads[0].defined() ? grads[0] : at::zeros_like(o);
         if (go.strides() != q.strides()) go = at::empty_like(q).copy_(go);   // one stride set for all q-like tensors
         Tensor dq, dr, dk, dv;
         bool done = false;
         // A backward that is itself recorded, traced or transformed goes through the dispatcher, and so does one on
         // saved tensors that a hook has brought back in another form.
-        bool plain = !at::GradMode::is_enabled() && plain_thread() && !at::impl::torch_function_mode_enabled() && stats.is_contiguous();
-        for (const Tensor *t : Tensors{&go, &q, &r, &k, &v, &o, &barv, &stats}) plain = plain && plain_tensor(*t);
+        bool plain = !at::GradMode::is_enabled() && plain_thread() && !at::impl::torch_function_mode_enabled();
+        for (const Tensor *t : Tensors{&go, &q, &r, &k, &v, &o, &barv, &d1, &bart, &m}) plain = plain && plain_tensor(*t);
+        for (const Tensor *t : Tensors{&d1, &bart, &m}) plain = plain && t->is_contiguous();
         for (const Tensor *t : Tensors{&go, &r, &o, &barv}) plain = plain && t->strides() == q.strides() && t->scalar_type() == q.scalar_type();
         plain = plain && v.strides() == k.strides();
         if (plain) {
             at::AutoDispatchBelowADInplaceOrView below;
             const c10::cuda::CUDAGuard device(q.device());
-            const Tensor d1 = stats[0];
             const plx_train_problem p = train_problem(q, k, d1, scale, window, layout, cu);
             size_t need = 0;
             if (!device_error_waiting() && api.train_workspace_bytes(&p, &need) == PLX_OK) {
@@ -221,10 +221,8 @@ struct Train : torch::autograd::Function<Train> {
                 dk = at::empty_like(k);
                 dv = at::empty_like(k);
                 const Tensor ws = at::empty({static_cast<int64_t>(need)}, q.options().dtype(at::kByte));
-                const float *st = stats.data_ptr<float>();
-                const int64_t n = d1.numel();
-                done = api.train_bwd(&p, q.data_ptr(), r.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), barv.data_ptr(), st, st + n,
-                                     st + 2 * n, go.data_ptr(), dq.data_ptr(), dr.data_ptr(), dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), need,
+                done = api.train_bwd(&p, q.data_ptr(), r.data_ptr(), k.data_ptr(), v.data_ptr(), o.data_ptr(), barv.data_ptr(),
+                                     d1.data_ptr<float>(), bart.data_ptr<float>(), m.data_ptr<float>(), go.data_ptr(), dq.data_ptr(), dr.data_ptr(), dk.data_ptr(), dv.data_ptr(), ws.data_ptr(), need,
                                      c10::cuda::getCurrentCUDAStream().stream()) == PLX_OK;
             }
         }
@@ -233,26 +231,36 @@ struct Train : torch::autograd::Function<Train> {
                 .typed<std::tuple<Tensor, Tensor, Tensor, Tensor>(const Tensor &, const Tensor &, const Tensor &, const Tensor &,
                     const Tensor &, const Tensor &, const Tensor &, const Tensor &, const Tensor &, const Tensor &, double, int64_t, int64_t,
                     const OptTensor &)>();
-            std::tie(dq, dr, dk, dv) = op.call(q, r, k, v, o, barv, stats[0], stats[1], stats[2], go, scale, window, layout, cu);
+            std::tie(dq, dr, dk, dv) = op.call(q, r, k, v, o, barv, d1, bart, m, go, scale, window, layout, cu);
         }
         return {dq, dr, dk, dv, Tensor(), Tensor(), Tensor(), Tensor()};
     }
 };
 
+// four tensors that the kernels can address as they are, and whose shapes fit together
+bool train_tensors_ok(const Tensor &q, const Tensor &r, const Tensor &k, const Tensor &v, int64_t layout) {
+    for (const Tensor *t : Tensors{&q, &r, &k, &v})
+        if (!plain_tensor(*t) || t->dim() != 4 || t->scalar_type() != q.scalar_type() || t->device() != q.device() || t->numel() == 0 ||
+            !kernel_ready(*t))
+            return false;
+    const int h = layout == kBHLD ? 1 : 2;
+    return dtype_code(q) >= 0 && r.sizes() == q.sizes() && r.strides() == q.strides() && v.sizes() == k.sizes() && v.strides() == k.strides() &&
+           k.size(0) == q.size(0) && k.size(3) == q.size(3) && q.size(h) % k.size(h) == 0;
+}
+
+bool train_ready(const py::object &q_, const py::object &r_, const py::object &k_, const py::object &v_, int64_t layout) {
+    bool ok = true;
+    const Tensor q = take(q_, ok), r = take(r_, ok), k = take(k_, ok), v = take(v_, ok);
+    return ok && train_tensors_ok(q, r, k, v, layout);
+}
+
+// o, barv, d1, bart, m
 py::object train(const py::object &q_, const py::object &r_, const py::object &k_, const py::object &v_, const py::object &scale_,
                  const py::object &window_, int64_t layout, const py::object &cu_) {
     bool ok = true;
     const Tensor q = take(q_, ok), r = take(r_, ok), k = take(k_, ok), v = take(v_, ok);
     const OptTensor cu = take_optional(cu_, ok);
-    if (!ok || !plain_thread()) return py::none();
-    for (const Tensor *t : Tensors{&q, &r, &k, &v})
-        if (!plain_tensor(*t) || t->dim() != 4 || t->scalar_type() != q.scalar_type() || t->device() != q.device() || t->numel() == 0 ||
-            !kernel_ready(*t))
-            return py::none();
-    const int h = layout == kBHLD ? 1 : 2;
-    if (dtype_code(q) < 0 || r.sizes() != q.sizes() || r.strides() != q.strides() || v.sizes() != k.sizes() || v.strides() != k.strides() ||
-        k.size(0) != q.size(0) || k.size(3) != q.size(3) || q.size(h) % k.size(h) != 0)
-        return py::none();
+    if (!ok || !plain_thread() || !train_tensors_ok(q, r, k, v, layout)) return py::none();
     if (cu && (!plain_tensor(*cu) || cu->scalar_type() != at::kInt || cu->dim() != 1 || !cu->is_contiguous() || cu->device() != q.device() ||
                q.size(0) != 1 || cu->numel() < 2))
         return py::none();
@@ -261,14 +269,16 @@ py::object train(const py::object &q_, const py::object &r_, const py::object &k
     if (!take_scale(scale_, q.size(3), scale) || !take_window(window_, window)) return py::none();
     const c10::cuda::CUDAGuard device(q.device());
     if (device_error_waiting()) return py::none();
-    Tensor o;
+    torch::autograd::variable_list res;
     try {
         py::gil_scoped_release nogil;
-        o = Train::apply(q, r, k, v, scale, window, static_cast<int64_t>(layout), cu);
+        res = Train::apply(q, r, k, v, scale, window, static_cast<int64_t>(layout), cu);
     } catch (const Refused &) {
         return py::none();
     }
-    return py::reinterpret_steal<py::object>(THPVariable_Wrap(o));
+    py::tuple t(res.size());
+    for (size_t i = 0; i < res.size(); ++i) t[i] = py::reinterpret_steal<py::object>(THPVariable_Wrap(res[i]));
+    return t;
 }
 
 // ------------------------------------------------------------------------- //
@@ -481,6 +491,7 @@ bool stage(const py::object &q_, const py::object &q_src_, const py::object &r_,
 
 PYBIND11_MODULE(_plx_host, m) {
     m.def("bind", &bind);
+    m.def("train_ready", &train_ready);
     m.def("train", &train);
     m.def("decode", &decode);
     m.def("attend", &attend);

@@ -87,8 +87,8 @@ def _stats_shape(q: Tensor, layout: int):
 # training
 # --------------------------------------------------------------------------- #
 @torch.library.custom_op("plx::train_fwd", mutates_args=(), device_types="cuda")
-def train_fwd(q: Tensor, r: Tensor, k: Tensor, v: Tensor, qk_scale: float, window_left: int, layout: int,
-              cu_seqlens: Optional[Tensor]) -> Tuple[Tensor, Tensor, Tensor, Tensor, Tensor]:
+def train_fwd_op(q: Tensor, r: Tensor, k: Tensor, v: Tensor, qk_scale: float, window_left: int, layout: int,
+                 cu_seqlens: Optional[Tensor]) -> Tuple[Tensor, Tensor, Tensor, Tensor, Tensor]:
     o = torch.empty_like(q)
     barv = torch.empty_like(q)
     d1 = torch.empty(_stats_shape(q, layout), device=q.device, dtype=torch.float32)
@@ -103,7 +103,7 @@ def train_fwd(q: Tensor, r: Tensor, k: Tensor, v: Tensor, qk_scale: float, windo
     return o, barv, d1, bart, m
 
 
-@train_fwd.register_fake
+@train_fwd_op.register_fake
 def _(q, r, k, v, qk_scale, window_left, layout, cu_seqlens):
     stats = q.new_empty(q.shape[:3], dtype=torch.float32)
     return torch.empty_like(q), torch.empty_like(q), stats, torch.empty_like(stats), torch.empty_like(stats)
@@ -188,7 +188,15 @@ def _backward(ctx, grad_o, *_unused):
     return dq, dr, dk, dv, None, None, None, None
 
 
-train_fwd.register_autograd(_backward, setup_context=_setup_ctx)
+train_fwd_op.register_autograd(_backward, setup_context=_setup_ctx)
+
+
+def train_fwd(q: Tensor, r: Tensor, k: Tensor, v: Tensor, qk_scale: float, window_left: int, layout: int,
+              cu_seqlens: Optional[Tensor]) -> Tuple[Tensor, Tensor, Tensor, Tensor, Tensor]:
+    """(o, barv, d1, bart, m): plx::train_fwd, a plainly eager call through the C++ host side."""
+    host = eager_host()
+    res = None if host is None else host.train(q, r, k, v, qk_scale, window_left, layout, cu_seqlens)
+    return train_fwd_op(q, r, k, v, qk_scale, window_left, layout, cu_seqlens) if res is None else res
 
 
 # --------------------------------------------------------------------------- #

@@ -66,21 +66,18 @@ def parallax_func(q: torch.Tensor, r: torch.Tensor, k: torch.Tensor, v: torch.Te
     as in ``parallax/reference.py:64-68``.  Returns ``(B, H_q, L_q, D)``.
     """
     host = ops.eager_host()
-    if host is not None:
-        o = host.train(q, r, k, v, qk_scale, window_size_left, ops.BHLD, None)
-        if o is not None:
-            return o
-    _check_dtype("parallax_func", q)
-    bsz, hq, lq, d = q.shape
-    hkv = k.shape[1]
-    if hq % hkv != 0:
-        raise ValueError(f"H_q ({hq}) must be divisible by H_kv ({hkv}) for GQA")
-    _check_cuda("parallax_func", q, r, k, v)
+    if host is None or not host.train_ready(q, r, k, v, ops.BHLD):
+        _check_dtype("parallax_func", q)
+        bsz, hq, lq, d = q.shape
+        hkv = k.shape[1]
+        if hq % hkv != 0:
+            raise ValueError(f"H_q ({hq}) must be divisible by H_kv ({hkv}) for GQA")
+        _check_cuda("parallax_func", q, r, k, v)
+        q, k = kernel_ready(q), kernel_ready(k)
+        r, v = kernel_ready(r, q), kernel_ready(v, k)
     if qk_scale is None:
-        qk_scale = d ** -0.5
-    q, k = kernel_ready(q), kernel_ready(k)
-    o, _, _, _, _ = ops.train_fwd(q, kernel_ready(r, q), k, kernel_ready(v, k),
-                                  float(qk_scale), int(window_size_left), ops.BHLD, None)
+        qk_scale = q.shape[-1] ** -0.5
+    o, _, _, _, _ = ops.train_fwd(q, r, k, v, float(qk_scale), int(window_size_left), ops.BHLD, None)
     return o
 
 

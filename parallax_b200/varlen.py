@@ -26,11 +26,6 @@ def parallax_varlen_func(q: torch.Tensor, r: torch.Tensor, k: torch.Tensor, v: t
     independent causal sequences along T and requires ``B == 1``; ``None`` runs
     every batch row as one dense causal sequence.  Returns ``(B, T, H_q, D)``.
     """
-    host = ops.eager_host()
-    if host is not None:
-        o = host.train(q, r, k, v, qk_scale, window_size_left, ops.BTHD, cu_seqlens)
-        if o is not None:
-            return o
     if q.dtype not in (torch.bfloat16, torch.float16):
         raise TypeError(f"parallax_varlen_func requires bf16 or fp16 inputs, got q.dtype={q.dtype}")
     if q.shape[2] % k.shape[2] != 0:
@@ -43,10 +38,12 @@ def parallax_varlen_func(q: torch.Tensor, r: torch.Tensor, k: torch.Tensor, v: t
         if cu_seqlens.dtype not in (torch.int32, torch.int64):
             raise TypeError(f"cu_seqlens must be int32 or int64, got {cu_seqlens.dtype}")
         cu_seqlens = cu_seqlens.to(device=q.device, dtype=torch.int32).contiguous()
-    _check_cuda("parallax_varlen_func", q, r, k, v)
     if qk_scale is None:
         qk_scale = q.shape[-1] ** -0.5
-    q, k = kernel_ready(q), kernel_ready(k)
-    o, _, _, _, _ = ops.train_fwd(q, kernel_ready(r, q), k, kernel_ready(v, k),
-                                  float(qk_scale), int(window_size_left), ops.BTHD, cu_seqlens)
+    host = ops.eager_host()
+    if host is None or not host.train_ready(q, r, k, v, ops.BTHD):
+        _check_cuda("parallax_varlen_func", q, r, k, v)
+        q, k = kernel_ready(q), kernel_ready(k)
+        r, v = kernel_ready(r, q), kernel_ready(v, k)
+    o, _, _, _, _ = ops.train_fwd(q, r, k, v, float(qk_scale), int(window_size_left), ops.BTHD, cu_seqlens)
     return o

@@ -100,14 +100,14 @@ def test_decode_and_prefill(hq, hkv, page):
 def test_what_is_left_to_the_python_path():
     host = _cabi.host()
     q = randn(1, 4, 64, 64)
-    scalars = (None, -1, ops.BHLD, None)
+    scalars = (0.125, -1, ops.BHLD, None)
     assert host.train(q, q, q, q, *scalars) is not None
     assert host.train(q.cpu(), q, q, q, *scalars) is None
     assert host.train(q.float(), q, q, q, *scalars) is None
     assert host.train(q.as_subclass(type("Sub", (torch.Tensor,), {})), q, q, q, *scalars) is None
     assert host.train(q[..., 1:], q, q, q, *scalars) is None
     assert host.train(q, q, q, randn(1, 4, 64, 64).transpose(1, 2).contiguous().transpose(1, 2), *scalars) is None
-    assert host.train(q, q, q, q, None, -2, ops.BHLD, None) is None
+    assert host.train(q, q, q, q, 0.125, -2, ops.BHLD, None) is None
     assert host.train(q, q, q, q, 1, -1, ops.BHLD, None) is None
     with PythonPath():
         assert host.train(q, q, q, q, *scalars) is None
