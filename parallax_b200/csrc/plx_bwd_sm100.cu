@@ -98,8 +98,11 @@ struct Smem {
     // per work item: XFull / XEmpty (resident tiles), KReady (M-side tile in tensor memory), AccDone / AccFree
     static constexpr int kXFull = 0, kXEmpty = 1, kNFull = 2, kNEmpty = 2 + NS, kSFull = 2 + 2 * NS, kSFree = kSFull + 1,
                          kGFull = kSFull + 2, kGFree = kSFull + 3, kAccDone = kSFull + 4, kAccFree = kSFull + 5,
-                         kKReady = kSFull + 6, kStatFull = kSFull + 7, kNumBars = kStatFull + kStatStages;
-    static constexpr uint32_t kTmemSlot = kBars + 8 * kNumBars;
+                         kKReady = kSFull + 6, kStatFull = kSFull + 7, kItemFull = kStatFull + kStatStages,
+                         kItemEmpty = kItemFull + kItemSlots, kClcFull = kItemEmpty + kItemSlots, kNumBars = kClcFull + 1;
+    static constexpr uint32_t kItems = (kBars + 8 * kNumBars + 15u) & ~15u;      // item ring, then the launch-control answer
+    static constexpr uint32_t kClc = kItems + 4 * kItemWords * kItemSlots;
+    static constexpr uint32_t kTmemSlot = kClc + 16;
     static constexpr uint32_t kAbort = kTmemSlot + 8;
     static constexpr uint32_t kBytes = kTmemSlot + 16;   // the dynamic shared memory must start 1024-byte aligned
     static constexpr uint32_t kStageTx = kStage;
@@ -113,7 +116,7 @@ __device__ __forceinline__ void st_shared_v4(uint32_t addr, uint32_t x, uint32_t
 // and the range of 64-wide tiles of the other side that it streams.
 struct Item {
     int bos, nq, nk, m0, b, hy, hk, off, t_lo, n_t, n_iter;   // streamed tiles t_lo .. t_lo + n_t - 1, per q head
-    bool valid;
+    int valid;
 };
 
 // Work item `idx` of the launch.  Items are (batch, head)-major, so that CTAs running at the same time
@@ -163,7 +166,8 @@ __device__ __forceinline__ Item get_item(const TrainArgs &a, int idx, int n_mt, 
     return it;
 }
 
-// n-th item of this CTA: CTAs take chunks of 2^chunk_shift neighbouring items, round robin.
+// n-th item of this CTA: CTAs take chunks of 2^chunk_shift neighbouring items, round robin.  (chunk_shift < 0: the
+// hardware hands the items out one by one.)
 __device__ __forceinline__ int item_index(int n, int chunk_shift) {
     return ((blockIdx.x + gridDim.x * (n >> chunk_shift)) << chunk_shift) + (n & ((1 << chunk_shift) - 1));
 }
@@ -204,7 +208,9 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
             // arrivals from all element-wise threads
             const bool all_ew = i == L::kSFree || i == L::kGFull || i == L::kKReady || i == L::kAccFree;
             const bool stat = i >= L::kStatFull && i < L::kStatFull + kStatStages;
-            mbar_init(bar(i), all_ew ? kEwThreads : stat ? kStatWriters : 1);
+            // every role that reads the items: two MMA issuers and the element-wise warps
+            const bool item_empty = i >= L::kItemEmpty && i < L::kItemEmpty + kItemSlots;
+            mbar_init(bar(i), all_ew ? kEwThreads : stat ? kStatWriters : item_empty ? 2 + EW : 1);
         }
         fence_barrier_init();
         prefetch_tensormap(&tm_q);
@@ -234,6 +240,41 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
         launch_dependents();
     }
 
+    // Items: the producer finds them (`valid` = 0: no more) ...
+    const ItemRing ring{base + L::kItems, bar(L::kItemFull), bar(L::kItemEmpty)};
+    struct Source {
+        int taken, asked;
+    };
+    auto find_item = [&](Source &src, Item &it) -> bool {
+        for (;;) {
+            int idx = -1;
+            if (chunk_shift >= 0) {
+                idx = item_index(src.taken, chunk_shift);
+                if (idx >= n_items) idx = -1;
+            } else if (src.taken == 0) {
+                idx = blockIdx.x;
+            } else {
+                if (!mbar_wait(bar(L::kClcFull), (src.taken - 1) & 1, err, 19)) return false;
+                idx = clc_answer(base + L::kClc);
+            }
+            ++src.taken;
+            if (idx < 0) {
+                it.valid = 0;
+                return true;
+            }
+            if (chunk_shift < 0) {
+                clc_ask(base + L::kClc, bar(L::kClcFull));
+                src.asked = src.taken;
+            }
+            it = get_item<DQR>(a, idx, n_mt, n_bh);
+            if (it.valid) return true;
+        }
+    };
+    // ... and lets no answer of the hardware arrive in shared memory that is no longer its own
+    auto leave_source = [&](const Source &src) {
+        if (src.asked == src.taken && src.asked > 0) mbar_wait_quiet(bar(L::kClcFull), (src.asked - 1) & 1);
+    };
+
     if (misaligned) {
         // nothing was started: fall through to the common exit
     } else if (warp == 0) {
@@ -243,11 +284,25 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
             uint32_t ph = 0;              // phase of the ring
             bool ok = true;
             int x_issued = 0;             // resident-tile loads started
+            Source src{0, 0};
             for (int i = 0; ok; ++i) {
-                const int idx = item_index(i, chunk_shift);
-                if (idx >= n_items) break;
-                const Item it = get_item<DQR>(a, idx, n_mt, n_bh);
+                Item it;
+                ok = find_item(src, it) && ring.publish(i, it, err, 20);
+                if (!ok || !it.valid) break;
                 if (it.n_iter == 0) continue;
+                // short items: what they wait for is the first touch of their own tiles, so have those on the way into
+                // L2 while the tiles of the item before still occupy the shared (and tensor) memory
+                if (chunk_shift < 0 && n > 0)
+                    for (int pn = 0; pn < L::kPanels; ++pn) {
+                        if (DQR) {
+                            tma_prefetch_4d(&tm_q, 64 * pn, it.bos + it.m0, it.hy, it.b);
+                            tma_prefetch_4d(&tm_r, 64 * pn, it.bos + it.m0, it.hy, it.b);
+                            tma_prefetch_4d(&tm_go, 64 * pn, it.bos + it.m0, it.hy, it.b);
+                        } else {
+                            tma_prefetch_4d(&tm_k, 64 * pn, it.bos + it.m0, it.hk, it.b);
+                            tma_prefetch_4d(&tm_v, 64 * pn, it.bos + it.m0, it.hk, it.b);
+                        }
+                    }
                 // the resident tiles of the previous item are free once its last score product has completed
                 if (n > 0) {
                     ok = mbar_wait(bar(L::kXEmpty), (n - 1) & 1, err, 1);
@@ -305,6 +360,7 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
                     mbar_wait_quiet(bar(L::kNFull + s), ph);
                 }
                 if (x_issued > 0) mbar_wait_quiet(bar(L::kXFull), (x_issued - 1) & 1);
+                leave_source(src);
             }
         }
     } else if (warp == 1 || warp == 2) {
@@ -381,9 +437,9 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
         uint32_t ph = 0;
         bool ok = true;
         for (int i = 0; ok; ++i) {
-            const int idx = item_index(i, chunk_shift);
-            if (idx >= n_items) break;
-            const Item it = get_item<DQR>(a, idx, n_mt, n_bh);
+            Item it;
+            ok = ring.read(i, it, true, err, 21);
+            if (!ok || !it.valid) break;
             if (it.n_iter == 0) continue;
             if (warp == 1) {
                 ok = mbar_wait(bar(L::kXFull), n & 1, err, 4) && mbar_wait(bar(L::kKReady), n & 1, err, 14);
@@ -473,10 +529,8 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
         // that sees the keys) get their zero outputs here
         auto next_item = [&]() -> bool {
             for (;;) {
-                const int idx = item_index(i_next++, chunk_shift);
-                if (idx >= n_items) return false;
-                cur = get_item<DQR>(a, idx, n_mt, n_bh);
-                if (!cur.valid) continue;
+                ok = ring.read(i_next++, cur, true, err, 21);
+                if (!ok || !cur.valid) return false;
                 if (cur.n_iter > 0) return true;
                 const int row = cur.m0 + ml;
                 if (row < (DQR ? cur.nq : cur.nk)) {
@@ -534,7 +588,7 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
         };
 
         bool have = next_item();
-        if (have) ok = prologue(0);
+        if (have && ok) ok = prologue(0);
         while (have && ok) {
             const int m0 = cur.m0, nq = cur.nq, nk = cur.nk, off = cur.off, mg = m0 + ml;
             for (int it = 0; it < cur.n_iter; ++it, ++g) {
@@ -659,10 +713,8 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
                 row_stride = a.kv_st;
             }
             have = next_item();
-            if (have) {
-                ok = prologue(n + 1);
-                if (!ok) break;
-            }
+            if (have) ok = prologue(n + 1);
+            if (!ok) break;
 
             // epilogue: half of the element-wise warps write acc0 (dQ | dK), the other half acc1 (dR | dV); an
             // accumulator is 2 x D / 64 units of 16 rows x 64 columns per lane quarter, dealt out to the CG / 2
@@ -747,11 +799,13 @@ int launch_mode(const TrainArgs &a, int n_tok, const ErrSink &sink, bool overlap
     const int n_items = tiles * a.batch * (DQR ? a.heads_q : a.heads_kv), sms = tma::sm_count();
     if (sms <= 0) return PLX_ERR_LAUNCH;
     // with plenty of items a CTA takes them in neighbouring pairs (a heavy and a light tile)
-    const int chunk_shift = n_items >= 2 * sms ? 1 : 0;
-    const int units = (n_items + (1 << chunk_shift) - 1) >> chunk_shift;
+    // packed sequences: the work of an item is as uneven as the lengths, so the items are handed out as they are done
+    const bool dynamic = a.cu && n_items > sms;
+    const int chunk_shift = dynamic ? -1 : n_items >= 2 * sms ? 1 : 0;
+    const int units = dynamic ? n_items : (n_items + (1 << chunk_shift) - 1) >> chunk_shift;
     const int n_bh = n_items <= sms ? a.batch * (DQR ? a.heads_q : a.heads_kv) : 0;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(units < sms ? units : sms);
+    cfg.gridDim = dim3(dynamic || units < sms ? units : sms);
     cfg.blockDim = dim3((4 + EW) * 32);
     cfg.dynamicSmemBytes = L::kBytes;
     cfg.stream = stream;

@@ -88,25 +88,30 @@ struct Smem {
     // barrier indices (8 bytes each)
     static constexpr int kQFull = 0, kQEmpty = 1, kOFree = 2, kKFull = 3, kKEmpty = kKFull + NS,
                          kVFull = kKEmpty + NS, kVEmpty = kVFull + NS, kSFull = kVEmpty + NS, kSFree = kSFull + 3,
-                         kPFull = kSFree + 1, kPVDone = kPFull + 3, kTail = kPVDone + 3, kNumBars = kTail + 2;   // kTail: K, V (EXT only)
-    static constexpr uint32_t kTmemSlot = kBars + 8 * kNumBars;
+                         kPFull = kSFree + 1, kPVDone = kPFull + 3, kTail = kPVDone + 3, kItemFull = kTail + 2, kItemEmpty = kItemFull + kItemSlots,
+                         kClcFull = kItemEmpty + kItemSlots, kNumBars = kClcFull + 1;   // kTail: K, V (EXT only)
+    static constexpr uint32_t kItems = (kBars + 8 * kNumBars + 15u) & ~15u;      // item ring, then the launch-control answer
+    static constexpr uint32_t kClc = kItems + 4 * kItemWords * kItemSlots;
+    static constexpr uint32_t kTmemSlot = kClc + 16;
     static constexpr uint32_t kBytes = kTmemSlot + 16 + 1024;  // + slack to align the base to 1024
 };
 
 // One unit of work: a 128-row query tile of one (batch, q head).
 struct Item {
     int bos, nq, nk, r0, b, h, hk, off, t_lo, n_tiles;   // key tiles t_lo .. t_lo + n_tiles - 1
-    bool valid;
+    int valid, pad;
 };
 
 // Work item `idx` of the launch.  Items are ordered (batch, head)-major so that CTAs running at the
 // same time share K / V in L2; inside a (batch, head) the row tiles alternate last, first, last - 1,
 // second, ... so that under a causal mask any two neighbours add up to the same work.
+// (Handed out one by one, they simply go from last to first.)
 template <bool EXT>
-__device__ __forceinline__ Item get_item(const TrainArgs &a, int idx, int n_rt) {
+__device__ __forceinline__ Item get_item(const TrainArgs &a, int idx, int n_rt, int chunk_shift) {
     Item it;
     const int bh = idx / n_rt, k = idx % n_rt;
-    const int tile_id = (k & 1) ? (k >> 1) : n_rt - 1 - (k >> 1);
+    const int tile_id = chunk_shift < 0 ? n_rt - 1 - k : (k & 1) ? (k >> 1) : n_rt - 1 - (k >> 1);
+    it.pad = 0;
     Seq s;
     int tis = 0;
     it.valid = locate_tile(a, tile_id, kBM, s, tis);
@@ -129,7 +134,8 @@ __device__ __forceinline__ Item get_item(const TrainArgs &a, int idx, int n_rt) 
     return it;
 }
 
-// n-th item of this CTA: CTAs take chunks of 2^chunk_shift neighbouring items, round robin.
+// n-th item of this CTA: CTAs take chunks of 2^chunk_shift neighbouring items, round robin.  (chunk_shift < 0: the
+// hardware hands the items out one by one.)
 __device__ __forceinline__ int item_index(int n, int chunk_shift) {
     return ((blockIdx.x + gridDim.x * (n >> chunk_shift)) << chunk_shift) + (n & ((1 << chunk_shift) - 1));
 }
@@ -161,7 +167,10 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
         for (int i = 0; i < L::kNumBars; ++i) {
             const bool all_softmax =
                 (i >= L::kPFull && i < L::kPFull + 3) || i == L::kOFree || i == L::kSFree;
-            mbar_init(bar(i), all_softmax ? 256 : 1);   // arrivals from all 256 softmax threads, else one
+            const bool item_empty = i >= L::kItemEmpty && i < L::kItemEmpty + kItemSlots;
+            // arrivals from all 256 softmax threads; from every role that reads the items (V loads, two MMA issuers,
+            // eight softmax warps); else one
+            mbar_init(bar(i), all_softmax ? 256 : item_empty ? 11 : 1);
         }
         fence_barrier_init();
         prefetch_tensormap(&tm_q);
@@ -191,6 +200,41 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
     auto tP1 = [&](int pb) -> uint32_t { return kInPlace ? tS1(pb) : tmem_base + 384 + 64 * pb; };
     auto tP2 = [&](int pb) -> uint32_t { return kInPlace ? tS2(pb) : tmem_base + 384 + 64 * pb + 32; };
 
+    // Items: the producer finds them (`valid` = 0: no more) ...
+    const ItemRing ring{base + L::kItems, bar(L::kItemFull), bar(L::kItemEmpty)};
+    struct Source {
+        int taken, asked;
+    };
+    auto find_item = [&](Source &src, Item &it) -> bool {
+        for (;;) {
+            int idx = -1;
+            if (chunk_shift >= 0) {
+                idx = item_index(src.taken, chunk_shift);
+                if (idx >= n_items) idx = -1;
+            } else if (src.taken == 0) {
+                idx = blockIdx.x;
+            } else {
+                if (!mbar_wait(bar(L::kClcFull), (src.taken - 1) & 1, err, 19)) return false;
+                idx = clc_answer(base + L::kClc);
+            }
+            ++src.taken;
+            if (idx < 0) {
+                it.valid = 0;
+                return true;
+            }
+            if (chunk_shift < 0) {
+                clc_ask(base + L::kClc, bar(L::kClcFull));
+                src.asked = src.taken;
+            }
+            it = get_item<EXT>(a, idx, n_rt, chunk_shift);
+            if (it.valid) return true;
+        }
+    };
+    // ... and lets no answer of the hardware arrive in shared memory that is no longer its own
+    auto leave_source = [&](const Source &src) {
+        if (src.asked == src.taken && src.asked > 0) mbar_wait_quiet(bar(L::kClcFull), (src.asked - 1) & 1);
+    };
+
     if (warp == 0) {
         // ------------------------------------------------------------------ TMA producer
         // lane 0: Q, R of every item and the K ring; lane 1: the V ring (a V stage is released a tile
@@ -198,7 +242,7 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
         if (lane < 2) {
             const bool is_k = lane == 0;
             const CUtensorMap *map = is_k ? &tm_k : &tm_v;
-            const uint32_t ring = is_k ? sK : sV;
+            const uint32_t tiles = is_k ? sK : sV;
             const int full0 = is_k ? L::kKFull : L::kVFull, empty0 = is_k ? L::kKEmpty : L::kVEmpty;
             // paged cache: a tile is kBN >> box_shift boxes of min(page size, 64) keys
             constexpr int kMaxBoxes = kBN / kMinPage;
@@ -206,12 +250,21 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
             int s = 0, n_issued = 0, n_items_done = 0, n_tails = 0;
             uint32_t ph = 0;
             bool ok = true;
+            Source src{0, 0};
             for (int n = 0; ok; ++n) {
-                const int idx = item_index(n, chunk_shift);
-                if (idx >= n_items) break;
-                const Item it = get_item<EXT>(a, idx, n_rt);
+                Item it;
+                ok = is_k ? find_item(src, it) && ring.publish(n, it, err, 20) : ring.read(n, it, false, err, 21);
+                if (!ok || !it.valid) break;
                 if (it.n_tiles == 0) continue;
                 if (is_k) {
+                    // short items: what they wait for is the first touch of q and r, so have them on the way into L2
+                    // while the tiles of the item before still occupy the shared memory
+                    if (chunk_shift < 0 && n_items_done > 0)
+#pragma unroll
+                        for (int pn = 0; pn < L::kPanels; ++pn) {
+                            tma_prefetch_4d(&tm_q, 64 * pn, it.bos + it.r0, it.h, it.b);
+                            tma_prefetch_4d(&tm_r, 64 * pn, it.bos + it.r0, it.h, it.b);
+                        }
                     // the q / r tiles of the previous item are free once its last score product has completed
                     ok = mbar_wait(bar(L::kQEmpty), (n_items_done & 1) ^ 1, err, 1);
                     if (!ok) break;
@@ -237,7 +290,7 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
                     }
                     ok = mbar_wait(bar(empty0 + s), ph ^ 1, err, is_k ? 2 : 3);
                     if (!ok) break;
-                    const uint32_t dst = ring + s * kKVBytes;
+                    const uint32_t dst = tiles + s * kKVBytes;
                     // A tile that reaches past the row's active length inside the cache: what lies there must not
                     // be seen (0 * NaN), so its rows are zeroed once the copy has landed, before the tile is handed
                     // over.  (Past the end of a tensor map the copy itself fills zeros.)
@@ -287,6 +340,7 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
                     mbar_wait_quiet(bar(full0 + s), ph);
                 }
                 if (is_k && n_items_done > 0) mbar_wait_quiet(bar(L::kQFull), (n_items_done - 1) & 1);
+                leave_source(src);
             }
         }
     } else if (warp == 1) {
@@ -304,9 +358,9 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
             int s = 0, g = 0, n_items_done = 0;                           // K ring stage, key tiles and items so far
             uint32_t ph = 0;                                              // phase of the K ring
             for (int n = 0; ok; ++n) {
-                const int idx = item_index(n, chunk_shift);
-                if (idx >= n_items) break;
-                const Item it = get_item<EXT>(a, idx, n_rt);
+                Item it;
+                ok = ring.read(n, it, true, err, 21);
+                if (!ok || !it.valid) break;
                 if (it.n_tiles == 0) continue;
                 ok = __all_sync(0xffffffffu, mbar_wait(bar(L::kQFull), n_items_done & 1, err, 4));
                 ++n_items_done;
@@ -360,9 +414,9 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
             int s = 0, g = 0, n_items_done = 0;
             uint32_t ph = 0;
             for (int n = 0; ok; ++n) {
-                const int idx = item_index(n, chunk_shift);
-                if (idx >= n_items) break;
-                const Item it = get_item<EXT>(a, idx, n_rt);
+                Item it;
+                ok = ring.read(n, it, true, err, 21);
+                if (!ok || !it.valid) break;
                 if (it.n_tiles == 0) continue;
                 for (int j = 0; j < it.n_tiles && ok; ++j, ++g) {
                     const int buf = g % kPBufs;
@@ -415,10 +469,9 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
         int g = 0, n_items_done = 0;                       // key tiles and items (with keys) so far
 
         for (int n = 0; ok; ++n) {
-            const int idx = item_index(n, chunk_shift);
-            if (idx >= n_items) break;
-            const Item it = get_item<EXT>(a, idx, n_rt);
-            if (!it.valid) continue;
+            Item it;
+            ok = ring.read(n, it, true, err, 21);
+            if (!ok || !it.valid) break;
             if (it.n_tiles == 0) {
                 // no key is visible to any row of the tile: outputs are zero (one thread per row and column half)
                 const int row = it.r0 + quarter * 32 + lane;
@@ -750,9 +803,12 @@ int launch_t(const TrainArgs &a, cudaStream_t stream) {
     if (sms <= 0) return PLX_ERR_LAUNCH;
     // with plenty of items a CTA takes them in neighbouring pairs (a heavy and a light row tile)
     // (EXT: the row tiles of a row see nearly the same keys, so single items balance better)
-    const int chunk_shift = !EXT && n_items >= 2 * sms ? 1 : 0;
-    const int units = (n_items + (1 << chunk_shift) - 1) >> chunk_shift;
-    kern<<<units < sms ? units : sms, 352, L::kBytes, stream>>>(a, tq, tr, tk, tv, sink, tiles, n_items, chunk_shift);
+    // packed sequences, rows of a cache: the work of an item is as uneven as the lengths, so the items are handed out
+    // as they are done
+    const bool dynamic = (a.cu || (EXT && a.seqused)) && n_items > sms;
+    const int chunk_shift = dynamic ? -1 : !EXT && n_items >= 2 * sms ? 1 : 0;
+    const int units = dynamic ? n_items : (n_items + (1 << chunk_shift) - 1) >> chunk_shift;
+    kern<<<dynamic || units < sms ? units : sms, 352, L::kBytes, stream>>>(a, tq, tr, tk, tv, sink, tiles, n_items, chunk_shift);
     count_launch();
     return cudaGetLastError() == cudaSuccess ? PLX_OK : PLX_ERR_LAUNCH;
 }

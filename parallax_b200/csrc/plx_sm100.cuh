@@ -112,8 +112,84 @@ __device__ __forceinline__ void tma_load_4d(uint32_t dst, const CUtensorMap *map
         ::"r"(dst), "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
         : "memory");
 }
+// the same box into L2 only
+__device__ __forceinline__ void tma_prefetch_4d(const CUtensorMap *map, int c0, int c1, int c2, int c3) {
+    asm volatile("cp.async.bulk.prefetch.tensor.4d.L2.global.tile [%0, {%1, %2, %3, %4}];\n" ::"l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3)
+                 : "memory");
+}
 __device__ __forceinline__ void prefetch_tensormap(const CUtensorMap *map) {
     asm volatile("prefetch.tensormap [%0];\n" ::"l"(map) : "memory");
+}
+
+// ------------------------------------------------------------------------- //
+// Work items.  One thread of a CTA (the TMA producer) finds the next item and passes it to the other roles through a
+// ring in shared memory, so that finding it (a search in cu_seqlens for packed sequences) happens once and ahead of
+// time.  Where the work per item is uneven the hardware hands the items out (cluster launch control): the grid has
+// one CTA per item, and a running CTA asks for one that has not started ("try_cancel") and does its work.
+// ------------------------------------------------------------------------- //
+constexpr int kItemSlots = 4, kItemWords = 12;
+struct ItemRing {
+    uint32_t slots, full, empty;   // shared-memory addresses: kItemSlots records of 48 bytes, and as many barriers each
+    // item n, by one thread; false if the ring did not drain in time
+    template <typename Item>
+    __device__ __forceinline__ bool publish(int n, const Item &it, const WaitCtx &w, int where) const {
+        static_assert(sizeof(Item) == 4 * kItemWords, "an item is twelve words");
+        const int s = n % kItemSlots;
+        if (n >= kItemSlots && !mbar_wait(empty + 8u * s, (n / kItemSlots - 1) & 1, w, where)) return false;
+        const uint32_t *x = reinterpret_cast<const uint32_t *>(&it);
+#pragma unroll
+        for (int i = 0; i < kItemWords; i += 4)
+            asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};\n" ::"r"(slots + 48u * s + 4u * i), "r"(x[i]), "r"(x[i + 1]), "r"(x[i + 2]),
+                         "r"(x[i + 3])
+                         : "memory");
+        mbar_arrive(full + 8u * s);
+        return true;
+    }
+    // item n, by every lane of a warp (whole) or one thread; each reading role arrives once on the slot's `empty`
+    template <typename Item>
+    __device__ __forceinline__ bool read(int n, Item &it, bool whole, const WaitCtx &w, int where) const {
+        const int s = n % kItemSlots;
+        bool ok = mbar_wait(full + 8u * s, (n / kItemSlots) & 1, w, where);
+        if (whole) ok = __all_sync(0xffffffffu, ok);
+        if (!ok) return false;
+        uint32_t *x = reinterpret_cast<uint32_t *>(&it);
+#pragma unroll
+        for (int i = 0; i < kItemWords; i += 4)
+            asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];\n"
+                         : "=r"(x[i]), "=r"(x[i + 1]), "=r"(x[i + 2]), "=r"(x[i + 3])
+                         : "r"(slots + 48u * s + 4u * i)
+                         : "memory");
+        if (whole) __syncwarp();
+        if (!whole || (threadIdx.x & 31) == 0) mbar_arrive(empty + 8u * s);
+        return true;
+    }
+};
+
+// Asks for another item; the answer (16 bytes) is there when `bar` has completed its next phase.  One thread, one
+// question at a time.
+__device__ __forceinline__ void clc_ask(uint32_t answer, uint32_t bar) {
+    mbar_expect_tx(bar, 16);
+    asm volatile("clusterlaunchcontrol.try_cancel.async.shared::cta.mbarrier::complete_tx::bytes.b128 [%0], [%1];\n" ::"r"(answer), "r"(bar)
+                 : "memory");
+}
+// The block index of the item, or -1 when no more are to be had.
+__device__ __forceinline__ int clc_answer(uint32_t answer) {
+    uint32_t got, x;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        ".reg .b128 r;\n"
+        "mov.u32 %1, 0;\n"
+        "ld.shared.b128 r, [%2];\n"
+        "clusterlaunchcontrol.query_cancel.is_canceled.pred.b128 p, r;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "@p clusterlaunchcontrol.query_cancel.get_first_ctaid::x.b32.b128 %1, r;\n"
+        "}\n"
+        : "=r"(got), "=&r"(x)
+        : "r"(answer)
+        : "memory");
+    fence_proxy_async();           // the next answer is written by the async proxy
+    return got ? static_cast<int>(x) : -1;
 }
 
 // ------------------------------------------------------------------------- //

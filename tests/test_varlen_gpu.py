@@ -185,3 +185,17 @@ def test_one_sequence_of_65536_tokens():
         x.grad = None
     plx.parallax_varlen_func(*leaves, cu_seqlens=cu).backward(go)
     assert all(torch.equal(a, x.grad) for a, x in zip(first, leaves))
+
+
+@pytest.mark.parametrize("hq,hkv,d", [(24, 24, 64), (25, 25, 64), (25, 5, 128), (60, 4, 128)])
+def test_items_handed_out_by_the_hardware(hq, hkv, d):
+    """144 items fit the SMs one by one, 150 and 360 do not and are handed out as the CTAs get through them (of dk/dv:
+    as many as 25 and 150 of 6 tiles each): every sequence, the empty one included, is what it gives alone."""
+    lens = [130, 0, 1, 253]
+    q, r, k, v, go, cu = make(lens, hq, hkv, d, 5)
+    got = run_gpu(q, r, k, v, go, cu)
+    for a, b in zip(cu[:-1], cu[1:]):
+        if b > a:
+            alone = run_gpu(*(x[:, a:b].contiguous() for x in (q, r, k, v, go)), None)
+            for name, x, y in zip(NAMES, got, alone):
+                assert torch.equal(x[:, a:b], y), f"{name} of [{a}, {b})"
