@@ -379,6 +379,13 @@ int plx_decode_choose_splits_gqa(int32_t batch, int32_t heads_q, int32_t heads_k
         }
         if (fill >= 0.85) break;
     }
+    // A warp sweeps whole tiles of 16 keys, so a part of 65 keys costs as much as one of 80 and leaves the last warps
+    // without any: cut at a tile boundary instead where the warps still fit into as many waves.
+    const int64_t waves = (units * best + resident - 1) / resident, part = n_keys / best / 16 * 16;
+    if (part >= 64) {
+        const int64_t even = (n_keys + part - 1) / part;
+        if (even <= cap && units * even <= waves * resident) best = even;
+    }
     return static_cast<int>(best);
 }
 
