@@ -345,7 +345,6 @@ int plx_decode_choose_splits(int32_t batch, int32_t heads_q, int32_t n_keys, int
         g -= g % 8;
         if (g >= 8) return static_cast<int>(g);
     }
-    if (decode_one_cta_per_head(bh, n_keys, sm_count)) return 8;
     int64_t s = resident / bh;
     if (s < 1) s = 1;
     if (n_keys / s > 1024) s = (n_keys + 1023) / 1024;

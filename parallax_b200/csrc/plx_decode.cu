@@ -1230,11 +1230,6 @@ static int tma_free_sm_count() {
 static bool decode_split_groups(const DecodeArgs &a) {
     const int64_t bh = static_cast<int64_t>(a.batch) * a.heads_q;
     const int64_t n_keys = a.window >= 0 && a.window < a.cache_len ? a.window : a.cache_len;
-    // (rows with lengths of their own go to the kernel that deals the splits out by length; a key-sharded launch to
-    // the one that can exchange)
-    if (a.n_rep == 1 && a.n_splits == 8 && !a.seqused && !a.cache_start && !a.part_out && a.xch.world == 0 &&
-        decode_one_cta_per_head(bh, n_keys, tma_free_sm_count()))
-        return true;
     return a.n_rep == 1 && a.n_splits >= 8 && a.n_splits % 8 == 0 && a.n_splits <= 256 &&
            bh <= PLX_DECODE_SPLIT_GROUP_MAX_BH && bh * n_keys <= (static_cast<int64_t>(1) << 19);
 }

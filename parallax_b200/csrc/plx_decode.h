@@ -17,13 +17,6 @@ struct ExchangeArgs {
 
 constexpr int kBalancedRows = 128;   // most batch rows whose splits are dealt out by length
 
-// A split group per (batch, head) and no more: eight warps whose states meet in shared memory, nothing of the merge in
-// global memory.  Pays where these CTAs, two per SM, fill the chip once (85 % or more) and a warp sweeps no more than
-// 1024 keys; below that some SMs would have two CTAs and others one.
-inline bool decode_one_cta_per_head(int64_t bh, int64_t n_keys, int sm_count) {
-    return bh <= 2 * static_cast<int64_t>(sm_count) && 100 * bh >= 170 * static_cast<int64_t>(sm_count) && n_keys >= 128 && n_keys <= 8192;
-}
-
 struct DecodeArgs {
     const void *q, *r, *k, *v;
     void *out;         // (batch, heads_q, D) or nullptr
