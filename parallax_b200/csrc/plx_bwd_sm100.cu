@@ -123,12 +123,14 @@ struct Item {
 // share their streamed tiles in L2; inside a (batch, head) the 128-wide tiles alternate last, first,
 // last - 1, second, ...: under the causal mask any two neighbours add up to the same work.
 // With one item per CTA (n_bh > 0: the number of (batch, head) pairs) the longest items come first instead: the
-// CTAs of dq/dr take over the SMs that dk/dv leaves one by one.
+// CTAs of dq/dr take over the SMs that dk/dv leaves one by one.  Handed out by the hardware (n_bh < 0) the items of a
+// (batch, head) go from the longest to the shortest.
 template <bool DQR>
 __device__ __forceinline__ Item get_item(const TrainArgs &a, int idx, int n_mt, int n_bh) {
     Item it;
     int bh = idx / n_mt, k = idx % n_mt;
     int tile_id = (k & 1) ? (k >> 1) : n_mt - 1 - (k >> 1);
+    if (n_bh < 0) tile_id = DQR ? n_mt - 1 - k : k;
     if (n_bh > 0) {
         bh = idx % n_bh;
         k = idx / n_bh;
@@ -799,11 +801,10 @@ int launch_mode(const TrainArgs &a, int n_tok, const ErrSink &sink, bool overlap
     const int n_items = tiles * a.batch * (DQR ? a.heads_q : a.heads_kv), sms = tma::sm_count();
     if (sms <= 0) return PLX_ERR_LAUNCH;
     // with plenty of items a CTA takes them in neighbouring pairs (a heavy and a light tile)
-    // packed sequences: the work of an item is as uneven as the lengths, so the items are handed out as they are done
-    const bool dynamic = a.cu && n_items > sms;
+    const bool dynamic = items_by_hardware(n_items, sms, a.cu != nullptr);
     const int chunk_shift = dynamic ? -1 : n_items >= 2 * sms ? 1 : 0;
     const int units = dynamic ? n_items : (n_items + (1 << chunk_shift) - 1) >> chunk_shift;
-    const int n_bh = n_items <= sms ? a.batch * (DQR ? a.heads_q : a.heads_kv) : 0;
+    const int n_bh = dynamic ? -1 : n_items <= sms ? a.batch * (DQR ? a.heads_q : a.heads_kv) : 0;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(dynamic || units < sms ? units : sms);
     cfg.blockDim = dim3((4 + EW) * 32);

@@ -802,11 +802,8 @@ int launch_t(const TrainArgs &a, cudaStream_t stream) {
     const int n_items = tiles * a.batch * a.heads_q, sms = sm_count();
     if (sms <= 0) return PLX_ERR_LAUNCH;
     // with plenty of items a CTA takes them in neighbouring pairs (a heavy and a light row tile)
-    // (EXT: the row tiles of a row see nearly the same keys, so single items balance better)
-    // packed sequences, rows of a cache: the work of an item is as uneven as the lengths, so the items are handed out
-    // as they are done
-    const bool dynamic = (a.cu || (EXT && a.seqused)) && n_items > sms;
-    const int chunk_shift = dynamic ? -1 : !EXT && n_items >= 2 * sms ? 1 : 0;
+    const bool dynamic = items_by_hardware(n_items, sms, a.cu || EXT);
+    const int chunk_shift = dynamic ? -1 : n_items >= 2 * sms ? 1 : 0;
     const int units = dynamic ? n_items : (n_items + (1 << chunk_shift) - 1) >> chunk_shift;
     kern<<<dynamic || units < sms ? units : sms, 352, L::kBytes, stream>>>(a, tq, tr, tk, tv, sink, tiles, n_items, chunk_shift);
     count_launch();
