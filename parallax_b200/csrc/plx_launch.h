@@ -11,7 +11,8 @@ struct ExchangeArgs;
 
 // Are the items of a tcgen05 kernel handed out by the hardware (see ItemRing in plx_sm100.cuh) or dealt out in advance,
 // in pairs of a heavy and a light one?  `uneven`: packed sequences and rows of a cache, whose items take as long as the
-// lengths say, always by the hardware.  Dense problems, where every pair is the same work, only when the last round of
+// lengths say, always by the hardware: 32768 tokens in 255 sequences, fwd 334 -> 269, dk/dv 320 -> 250, dq/dr 390 -> 293 us
+// (the fullest CTA of dk/dv had 1.48 times the average work), 65536 tokens in 14 sequences 12.93 -> 12.13 ms.  Dense problems, where every pair is the same work, only when the last round of
 // pairs is so empty that it costs more than 4 %: 720 items (360 pairs, 3 rounds for 2.4) 245 -> 203 us forward and
 // backward at B = 9, H = 16, L = 548; 4096 items (2048 pairs, 14 rounds for 13.8) are 2.7 % faster dealt out.
 inline bool items_by_hardware(int64_t n_items, int sms, bool uneven) {
