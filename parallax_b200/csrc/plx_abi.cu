@@ -289,7 +289,8 @@ int plx_train_bwd_stages(const plx_train_problem *p, int32_t stages, const void 
     cudaStream_t cs = reinterpret_cast<cudaStream_t>(stream);
     const bool tc = train_bwd_sm100_supported(a, p->head_dim);
     // dk/dv before dq/dr: the two are independent, and the CTAs of the second start as those of the first, longer
-    // one leave their SMs
+    // one leave their SMs.  (The three kernels, B = 2, H = 8, L = 1024: 62.9 us one after the other, 43.5 so; at B = 4,
+    // H = 16 174 against 145, at B = 8, H = 16, L = 4096 the same.)
     int before = 0;
     for (int stage : {PLX_BWD_STATS, PLX_BWD_DKV, PLX_BWD_DQR}) {
         if (!(stages & stage)) continue;
