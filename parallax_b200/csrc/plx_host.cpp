@@ -213,6 +213,8 @@ struct Train : torch::autograd::Function<Train> {
         for (const Tensor *t : Tensors{&d1, &bart, &m}) plain = plain && t->is_contiguous();
         for (const Tensor *t : Tensors{&go, &r, &o, &barv}) plain = plain && t->strides() == q.strides() && t->scalar_type() == q.scalar_type();
         plain = plain && v.strides() == k.strides();
+        // gradients are written by the strides of q and k, which empty_like reproduces for tensors without gaps only
+        plain = plain && q.is_non_overlapping_and_dense() && k.is_non_overlapping_and_dense();
         if (plain) {
             at::AutoDispatchBelowADInplaceOrView below;
             const c10::cuda::CUDAGuard device(q.device());

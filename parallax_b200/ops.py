@@ -83,6 +83,13 @@ def _stats_shape(q: Tensor, layout: int):
     return q.shape[:3]
 
 
+def _with_strides_of(like: Tensor, *tensors: Tensor):
+    """The tensors in the layout of `like`, copied where theirs differs.  The kernels write an output by the strides
+    of the input it belongs to, and ``empty_like`` reproduces those of a tensor without gaps only: an input with gaps (a
+    slice of a longer cache) has to be brought to the layout of its output, or it is written past its end."""
+    return tuple(x if x.stride() == like.stride() else torch.empty_like(like).copy_(x) for x in tensors)
+
+
 # --------------------------------------------------------------------------- #
 # training
 # --------------------------------------------------------------------------- #
@@ -91,6 +98,7 @@ def train_fwd_op(q: Tensor, r: Tensor, k: Tensor, v: Tensor, qk_scale: float, wi
                  cu_seqlens: Optional[Tensor]) -> Tuple[Tensor, Tensor, Tensor, Tensor, Tensor]:
     o = torch.empty_like(q)
     barv = torch.empty_like(q)
+    q, r = _with_strides_of(o, q, r)
     d1 = torch.empty(_stats_shape(q, layout), device=q.device, dtype=torch.float32)
     bart = torch.empty_like(d1)
     m = torch.empty_like(d1)
@@ -161,6 +169,9 @@ def train_bwd(q: Tensor, r: Tensor, k: Tensor, v: Tensor, o: Tensor, barv: Tenso
               cu_seqlens: Optional[Tensor]) -> Tuple[Tensor, Tensor, Tensor, Tensor]:
     dq, dr = torch.empty_like(q), torch.empty_like(q)
     dk, dv = torch.empty_like(k), torch.empty_like(k)
+    q, r, o, barv, grad_o = _with_strides_of(dq, q, r, o, barv, grad_o)
+    k, v = _with_strides_of(dk, k, v)
+    d1, bart, m = d1.contiguous(), bart.contiguous(), m.contiguous()
     ws = train_bwd_workspace(q, k, d1, layout, cu_seqlens)
     train_bwd_stages(BWD_ALL, q, r, k, v, o, barv, d1, bart, m, grad_o, dq, dr, dk, dv, ws, qk_scale, window_left,
                      layout, cu_seqlens)

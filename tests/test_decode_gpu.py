@@ -683,6 +683,31 @@ def test_extend_in_one_launch_is_the_launch_per_row(case):
 
 
 @pytest.mark.parametrize("case", [
+    # hq, hkv, lq, active lengths, cache, head_dim
+    (4, 2, 70, (150, 150), 230, 128),        # one launch on a slice of the cache
+    (4, 4, 33, (64, 64, 64), 65, 64),
+    (8, 2, 20, (90, 33), 130, 128),          # a launch per row
+])
+def test_gradients_of_prefill_stay_inside_the_active_keys(case):
+    """A prefill call that autograd records: gradients of q and r, and of k and v at the active keys, are the
+    oracle's; those of the rest of the cache are zero."""
+    hq, hkv, lq, lens, cache, d = case
+    bsz = len(lens)
+    mk = lambda n, h, s: seeded_bf16((bsz, n, h, d), s)
+    q, r, k, v, go = mk(lq, hq, 80), mk(lq, hq, 81), mk(cache, hkv, 82), mk(cache, hkv, 83), mk(lq, hq, 84)
+    leaves = [x.cuda().requires_grad_(True) for x in (q, r, k, v)]
+    out = plx.parallax_attn_with_kvcache(*leaves, seqused_k=torch.tensor(lens, dtype=torch.int32, device="cuda"))
+    grads = [g.float().cpu() for g in torch.autograd.grad(out, leaves, go.cuda())]
+    bhld = lambda x: x.permute(0, 2, 1, 3).contiguous()
+    for b, n in enumerate(lens):
+        ref = orc.train_backward(*(bhld(x[b:b + 1]) for x in (q, r, k[:, :n], v[:, :n])), bhld(go[b:b + 1]).float())
+        for name, got, want in zip(("dq", "dr", "dk", "dv"), grads, ref):
+            want = want.permute(0, 2, 1, 3)
+            assert_close(got[b:b + 1, :want.shape[1]], want, 1e-2, 2e-2, f"{case} row {b} {name}")
+            assert not got[b, want.shape[1]:].any()
+
+
+@pytest.mark.parametrize("case", [
     # batch, hq, hkv, cache, head_dim, window, dtype: the splits are dealt out by row length from 2 to 128 rows
     (2, 32, 8, 12000, 128, -1, torch.bfloat16),      # two-level merge, one long and one short row
     (16, 32, 8, 3000, 128, -1, torch.bfloat16),
