@@ -235,11 +235,17 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
     const uint32_t tK = tmem_base + 448;                                              // the M-side tile as an A operand
     const bool misaligned = cta_aborted(err);
     // Set-up may run under the end of the kernel before.  dk/dv waits here for the row statistics, then lets dq/dr
-    // start, for which they are therefore complete too; dq/dr waits for dk/dv at its end, so that whatever follows
-    // on the stream follows both.
+    // start; dq/dr waits for dk/dv at its end, so that whatever follows on the stream follows both.
+    // What dq/dr reads of the statistics it reads without a wait of its own: they were complete and visible to dk/dv
+    // (its wait), dk/dv passes them on (fence) before any CTA of dq/dr can exist, and dq/dr takes them up (fence).  For
+    // both kernels the statistics are written while the kernel may already be resident, so they are read at the
+    // L2 (ld.global.cg), never by the non-coherent path or from a line of L1.
     if (!DQR) {
         grid_wait();
+        __threadfence();
         launch_dependents();
+    } else {
+        __threadfence();
     }
 
     // Items: the producer finds them (`valid` = 0: no more) ...
@@ -515,7 +521,7 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
             if (t >= it.n_iter) return make_float4(0.f, 0.f, 0.f, 0.f);
             const int hq = it.hk * a.n_rep + t / it.n_t;
             const int row0 = it.bos + (it.t_lo + t % it.n_t) * kBN;
-            return __ldg(reinterpret_cast<const float4 *>(a.cst + ((static_cast<int64_t>(it.b) * a.heads_q + hq) * n_tok + row0 + wid) * 4));
+            return __ldcg(reinterpret_cast<const float4 *>(a.cst + ((static_cast<int64_t>(it.b) * a.heads_q + hq) * n_tok + row0 + wid) * 4));
         };
         auto stat_publish = [&](int gg, const float4 &v) {
             float *dst = reinterpret_cast<float *>(smem_raw + L::kStats + (gg % kStatStages) * kStatBytes);
@@ -563,8 +569,8 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
                 r_ml = INFINITY;
                 r_c1 = r_ct = r_b = 0.f;
                 if (mg < cur.nq) {
-                    const float4 hi4 = *reinterpret_cast<const float4 *>(
-                        a.cst + ((static_cast<int64_t>(cur.b) * a.heads_q + cur.hy) * n_tok + cur.bos + mg) * 4);   // b, mL, 1 + bart, (b - t) * scale
+                    const float4 hi4 = __ldcg(reinterpret_cast<const float4 *>(
+                        a.cst + ((static_cast<int64_t>(cur.b) * a.heads_q + cur.hy) * n_tok + cur.bos + mg) * 4));   // b, mL, 1 + bart, (b - t) * scale
                     r_b = hi4.x;
                     r_ml = hi4.y;
                     r_c1 = hi4.z;
