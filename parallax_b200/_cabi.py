@@ -9,8 +9,9 @@ import ctypes as C
 import importlib.util
 import os
 import threading
+import warnings
 
-from ._paths import HOST_PATH, LIB_PATH
+from ._paths import LIB_PATH, host_path
 
 PLX_BF16, PLX_FP16 = 0, 1
 PLX_ERR_UNSUPPORTED = -2
@@ -135,24 +136,38 @@ def lib():
     return _lib
 
 
-_host = None
+_host = None          # the module once loaded, False once it is known not to load
+
+
+def _load_host(handle):
+    path = host_path()
+    if not os.path.exists(path):
+        raise ImportError(f"{path} is missing")
+    spec = importlib.util.spec_from_file_location("_plx_host", path)
+    module = importlib.util.module_from_spec(spec)
+    spec.loader.exec_module(module)
+    if module.abi_version != ABI_VERSION:
+        raise ImportError(f"{path} has ABI version {module.abi_version}, expected {ABI_VERSION}")
+    module.bind({name: C.cast(getattr(handle, name), C.c_void_p).value for name in SYMBOLS})
+    return module
 
 
 def host():
-    """The C++ host side of eager calls (csrc/plx_host.cpp), bound to the loaded library."""
+    """The C++ host side of eager calls (csrc/plx_host.cpp), bound to the loaded library.  None if there is none for
+    this PyTorch (said once): every call then takes the Python path, which does the same with more host time."""
     global _host
     if _host is None:
         handle = lib()
         with _lock:
             if _host is None:
-                if not os.path.exists(HOST_PATH):
-                    raise RuntimeError(f"{HOST_PATH} is missing: build it with `python -m parallax_b200.build`")
-                spec = importlib.util.spec_from_file_location("_plx_host", HOST_PATH)
-                module = importlib.util.module_from_spec(spec)
-                spec.loader.exec_module(module)
-                module.bind({name: C.cast(getattr(handle, name), C.c_void_p).value for name in SYMBOLS})
-                _host = module
-    return _host
+                try:
+                    _host = _load_host(handle)
+                except ImportError as e:
+                    _host = False
+                    warnings.warn(f"parallax_b200: the C++ host side of eager calls is not in use ({e}); build it with "
+                                  "`python -m parallax_b200.build`. Calls take the Python path, which needs more host time.",
+                                  RuntimeWarning, stacklevel=3)
+    return _host or None
 
 
 def check(status: int, what: str) -> None:

@@ -1,5 +1,5 @@
-"""Build recipe for libplx_sm100.so (hand-written CUDA for sm_100a + the C ABI) and _plx_host.so (the host side
-of eager calls in C++, against the headers of the installed PyTorch).
+"""Build recipe for libplx_sm100.so (hand-written CUDA for sm_100a + the C ABI) and the host side of eager calls in C++
+(_plx_host.*.so, against the headers of the installed PyTorch; without it those calls take the slower Python path).
 
     python -m parallax_b200.build [--force]
 
@@ -12,7 +12,7 @@ import shutil
 import subprocess
 import sys
 
-from ._paths import CSRC, HOST_PATH, INCLUDE, LIB_DIR, LIB_PATH
+from ._paths import CSRC, INCLUDE, LIB_DIR, LIB_PATH, host_path
 
 SOURCES = ["plx_abi.cu", "plx_decode.cu", "plx_train_mma.cu", "plx_fwd_sm100.cu", "plx_bwd_sm100.cu"]
 NVCC_FLAGS = [
@@ -34,9 +34,12 @@ def _inputs():
     return files
 
 
+def _stale(built: str) -> bool:
+    return not os.path.exists(built) or any(os.path.getmtime(f) > os.path.getmtime(built) for f in _inputs())
+
+
 def is_stale() -> bool:
-    return any(not os.path.exists(built) or any(os.path.getmtime(f) > os.path.getmtime(built) for f in _inputs())
-               for built in (LIB_PATH, HOST_PATH))
+    return _stale(LIB_PATH) or _stale(host_path())
 
 
 def _build_host() -> None:
@@ -50,19 +53,14 @@ def _build_host() -> None:
     dirs = [inc, os.path.join(inc, "torch", "csrc", "api", "include"), sysconfig.get_paths()["include"], os.path.join(cuda, "include")]
     cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-Wall",
            f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *[f for d in dirs for f in ("-isystem", d)],
-           "-o", HOST_PATH, os.path.join(CSRC, "plx_host.cpp"), f"-L{libs}", f"-L{os.path.join(cuda, 'lib64')}",
+           "-o", host_path(), os.path.join(CSRC, "plx_host.cpp"), f"-L{libs}", f"-L{os.path.join(cuda, 'lib64')}",
            "-ltorch_python", "-ltorch", "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-lcudart", "-Wl,-z,now"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError("g++ failed:\n" + res.stdout + res.stderr)
 
 
-def build(force: bool = False, verbose: bool = False) -> str:
-    """Compile both if one is missing or older than its sources; returns the path of libplx_sm100.so."""
-    if not force and not is_stale():
-        return LIB_PATH
-    os.makedirs(LIB_DIR, exist_ok=True)
-    _build_host()
+def _build_library(verbose: bool) -> None:
     cmd = [_nvcc(), *NVCC_FLAGS, *(["-Xptxas", "-v"] if verbose else []), "-o", LIB_PATH,
            *[os.path.join(CSRC, s) for s in SOURCES]]
     res = subprocess.run(cmd, capture_output=True, text=True)
@@ -70,6 +68,15 @@ def build(force: bool = False, verbose: bool = False) -> str:
         raise RuntimeError("nvcc failed:\n" + res.stdout + res.stderr)
     if verbose:
         print(res.stderr)
+
+
+def build(force: bool = False, verbose: bool = False) -> str:
+    """Compile what is missing or older than the sources, the kernels first; returns the path of libplx_sm100.so."""
+    os.makedirs(LIB_DIR, exist_ok=True)
+    if force or _stale(LIB_PATH):
+        _build_library(verbose)
+    if force or _stale(host_path()):
+        _build_host()
     return LIB_PATH
 
 

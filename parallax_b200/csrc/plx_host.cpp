@@ -495,6 +495,7 @@ bool stage(const py::object &q_, const py::object &q_src_, const py::object &r_,
 }  // namespace
 
 PYBIND11_MODULE(_plx_host, m) {
+    m.attr("abi_version") = PLX_ABI_VERSION;
     m.def("bind", &bind);
     m.def("train_ready", &train_ready);
     m.def("train", &train);
