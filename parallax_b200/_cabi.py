@@ -157,7 +157,10 @@ def host():
     this PyTorch (said once): every call then takes the Python path, which does the same with more host time."""
     global _host
     if _host is None:
-        handle = lib()
+        try:
+            handle = lib()
+        except (RuntimeError, OSError):
+            return None              # without the kernel library: the launch says so, after the argument checks
         with _lock:
             if _host is None:
                 try:

@@ -56,3 +56,20 @@ def test_the_kernels_are_built_before_the_host_side(fresh):
     fresh.setattr(build, "_build_host", lambda: done.append("host"))
     build.build(force=True)
     assert done == ["library", "host"]
+
+
+def test_argument_errors_come_before_a_missing_library(monkeypatch):
+    import parallax_b200 as plx
+
+    monkeypatch.setattr(_cabi, "_lib", None)
+    monkeypatch.setattr(_cabi, "_host", None)
+    monkeypatch.setattr(_cabi, "LIB_PATH", "/nonexistent/libplx_sm100.so")
+    x = torch.zeros(1, 1, 8, 64)
+    with pytest.raises(TypeError, match="bf16 or fp16"):
+        plx.parallax_func(x, x, x, x)
+    with pytest.raises(TypeError, match="bf16 or fp16"):
+        plx.parallax_decode(x, x, x, x)
+    with pytest.raises(ValueError, match="single query"):
+        plx.parallax_decode(*[torch.zeros(1, 2, 8, 64, dtype=torch.bfloat16)] * 4)
+    with pytest.raises(RuntimeError, match="is missing"):
+        _cabi.lib()
