@@ -13,6 +13,7 @@
 #include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
+#include <ATen/record_function.h>
 #include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/csrc/autograd/custom_function.h>
@@ -33,6 +34,7 @@ namespace {
 using at::Tensor;
 using OptTensor = std::optional<Tensor>;
 using Tensors = std::initializer_list<const Tensor *>;
+using Values = std::vector<c10::IValue>;   // what a profiler is shown of a call, under the name of the op it stands for
 
 enum Layout { kBHLD = 0, kBTHD = 1 };
 
@@ -216,6 +218,7 @@ struct Train : torch::autograd::Function<Train> {
         // gradients are written by the strides of q and k, which empty_like reproduces for tensors without gaps only
         plain = plain && q.is_non_overlapping_and_dense() && k.is_non_overlapping_and_dense();
         if (plain) {
+            RECORD_FUNCTION("plx::train_bwd", Values({q, r, k, v, o, barv, d1, bart, m, go}));
             at::AutoDispatchBelowADInplaceOrView below;
             const c10::cuda::CUDAGuard device(q.device());
             const plx_train_problem p = train_problem(q, k, d1, scale, window, layout, cu);
@@ -275,6 +278,7 @@ py::object train(const py::object &q_, const py::object &r_, const py::object &k
     const c10::cuda::CUDAGuard device(q.device());
     if (device_error_waiting()) return py::none();
     torch::autograd::variable_list res;
+    RECORD_FUNCTION("plx::train_fwd", Values({q, r, k, v}));
     try {
         py::gil_scoped_release nogil;
         res = Train::apply(q, r, k, v, scale, window, static_cast<int64_t>(layout), cu);
@@ -389,6 +393,7 @@ py::object decode(const py::object &q_, const py::object &r_, const py::object &
     at::AutoDispatchBelowADInplaceOrView below;
     const c10::cuda::CUDAGuard device(q.device());
     if (capturing()) return py::none();
+    RECORD_FUNCTION("plx::decode_out", Values({q, r, k, v}));
     const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream();
     plx_decode_problem p{};
     p.dtype = dtype_code(q);
@@ -436,6 +441,7 @@ py::object extend(const py::object &q_, const py::object &r_, const py::object &
     at::AutoDispatchBelowADInplaceOrView below;
     const c10::cuda::CUDAGuard device(q.device());
     if (capturing() || device_error_waiting()) return py::none();
+    RECORD_FUNCTION("plx::train_extend", Values({q, r, k, v}));
     const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream();
     plx_train_problem p = train_problem(q, k, Tensor(), scale, window, kBTHD, std::nullopt);
     p.len_k = static_cast<int32_t>(ceiling);

@@ -170,3 +170,21 @@ def test_staging_of_a_captured_step(bsz, h, d):
         with pytest.raises(ValueError, match="out of range"):
             gd(cache_seqlens=bad)
     assert gd.cache_seqlens.tolist() == [96] * bsz
+
+
+def test_a_profiler_sees_the_ops():
+    """A call by the short cut shows up in a profile under the name of the op it stands for, with its input shapes."""
+    from torch.profiler import ProfilerActivity, profile
+
+    leaves = [randn(1, 2, 128, 64, seed=s).requires_grad_(True) for s in range(4)]
+    q, kv = randn(2, 1, 4, 64), randn(2, 128, 4, 64)
+    chunk = randn(2, 3, 4, 64)
+    with profile(activities=[ProfilerActivity.CPU], record_shapes=True) as prof:
+        plx.parallax_func(*leaves).sum().backward()
+        plx.parallax_decode(q, q, kv, kv)
+        plx.parallax_attn_with_kvcache(chunk, chunk, kv, kv)
+    shapes = {e.name: e.input_shapes for e in prof.events() if e.name.startswith("plx::")}
+    assert shapes["plx::train_fwd"][:4] == [[1, 2, 128, 64]] * 4
+    assert shapes["plx::train_bwd"][0] == [1, 2, 128, 64]
+    assert shapes["plx::decode_out"][:3] == [[2, 1, 4, 64], [2, 1, 4, 64], [2, 128, 4, 64]]
+    assert shapes["plx::train_extend"][0] == [2, 3, 4, 64]
