@@ -122,18 +122,15 @@ struct Item {
 // Work item `idx` of the launch.  Items are (batch, head)-major, so that CTAs running at the same time
 // share their streamed tiles in L2; inside a (batch, head) the 128-wide tiles alternate last, first,
 // last - 1, second, ...: under the causal mask any two neighbours add up to the same work.
-// With one item per CTA (n_bh > 0: the number of (batch, head) pairs) the longest items come first instead: the
-// CTAs of dq/dr take over the SMs that dk/dv leaves one by one.  Handed out by the hardware (n_bh < 0) the items of a
-// (batch, head) go from the longest to the shortest.
+// With one item per CTA, and handed out by the hardware (group > 0), the longest items come first instead (see
+// longest_first): the CTAs of dq/dr take over the SMs that dk/dv leaves one by one.
 template <bool DQR>
-__device__ __forceinline__ Item get_item(const TrainArgs &a, int idx, int n_mt, int n_bh) {
+__device__ __forceinline__ Item get_item(const TrainArgs &a, int idx, int n_mt, int group) {
     Item it;
     int bh = idx / n_mt, k = idx % n_mt;
     int tile_id = (k & 1) ? (k >> 1) : n_mt - 1 - (k >> 1);
-    if (n_bh < 0) tile_id = DQR ? n_mt - 1 - k : k;
-    if (n_bh > 0) {
-        bh = idx % n_bh;
-        k = idx / n_bh;
+    if (group > 0) {
+        longest_first(idx, n_mt, a.batch * (DQR ? a.heads_q : a.heads_kv), group, bh, k);
         tile_id = DQR ? n_mt - 1 - k : k;
     }
     Seq s;
@@ -185,7 +182,7 @@ __global__ void __launch_bounds__((4 + EW) * 32, 1)
 bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorMap tm_q,
                  const __grid_constant__ CUtensorMap tm_r, const __grid_constant__ CUtensorMap tm_go,
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const ErrSink sink,
-                 int n_mt, int n_items, int chunk_shift, int n_bh) {
+                 int n_mt, int n_items, int chunk_shift, int group) {
     using L = Smem<D, MODE, NS>;
     constexpr bool DQR = MODE == kModeDQR;
     constexpr uint32_t kResBytes = L::kResBytes, kStrBytes = L::kStrBytes;
@@ -274,7 +271,7 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
                 clc_ask(base + L::kClc, bar(L::kClcFull));
                 src.asked = src.taken;
             }
-            it = get_item<DQR>(a, idx, n_mt, n_bh);
+            it = get_item<DQR>(a, idx, n_mt, group);
             if (it.valid) return true;
         }
     };
@@ -810,7 +807,7 @@ int launch_mode(const TrainArgs &a, int n_tok, const ErrSink &sink, bool overlap
     const bool dynamic = items_by_hardware(n_items, sms, a.cu != nullptr);
     const int chunk_shift = dynamic ? -1 : n_items >= 2 * sms ? 1 : 0;
     const int units = dynamic ? n_items : (n_items + (1 << chunk_shift) - 1) >> chunk_shift;
-    const int n_bh = dynamic ? -1 : n_items <= sms ? a.batch * (DQR ? a.heads_q : a.heads_kv) : 0;
+    const int group = !dynamic && n_items > sms ? 0 : dynamic && a.cu ? 1 : item_group(a.batch * (DQR ? a.heads_q : a.heads_kv), tiles, sms);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(dynamic || units < sms ? units : sms);
     cfg.blockDim = dim3((4 + EW) * 32);
@@ -821,7 +818,7 @@ int launch_mode(const TrainArgs &a, int n_tok, const ErrSink &sink, bool overlap
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = overlap ? 1 : 0;
-    const cudaError_t st = cudaLaunchKernelEx(&cfg, kern, a, n_tok, tq, tr, tg, tk, tv, sink, tiles, n_items, chunk_shift, n_bh);
+    const cudaError_t st = cudaLaunchKernelEx(&cfg, kern, a, n_tok, tq, tr, tg, tk, tv, sink, tiles, n_items, chunk_shift, group);
     count_launch();
     return st == cudaSuccess && cudaGetLastError() == cudaSuccess ? PLX_OK : PLX_ERR_LAUNCH;
 }

@@ -105,12 +105,13 @@ struct Item {
 // Work item `idx` of the launch.  Items are ordered (batch, head)-major so that CTAs running at the
 // same time share K / V in L2; inside a (batch, head) the row tiles alternate last, first, last - 1,
 // second, ... so that under a causal mask any two neighbours add up to the same work.
-// (Handed out one by one, they simply go from last to first.)
+// (Handed out by the hardware, group > 0, they go from last to first: see longest_first.)
 template <bool EXT>
-__device__ __forceinline__ Item get_item(const TrainArgs &a, int idx, int n_rt, int chunk_shift) {
+__device__ __forceinline__ Item get_item(const TrainArgs &a, int idx, int n_rt, int group) {
     Item it;
-    const int bh = idx / n_rt, k = idx % n_rt;
-    const int tile_id = chunk_shift < 0 ? n_rt - 1 - k : (k & 1) ? (k >> 1) : n_rt - 1 - (k >> 1);
+    int bh = idx / n_rt, k = idx % n_rt;
+    if (group > 0) longest_first(idx, n_rt, a.batch * a.heads_q, group, bh, k);
+    const int tile_id = group > 0 ? n_rt - 1 - k : (k & 1) ? (k >> 1) : n_rt - 1 - (k >> 1);
     it.pad = 0;
     Seq s;
     int tis = 0;
@@ -152,7 +153,7 @@ template <typename T, int D, int NS, bool EXT>
 __global__ void __launch_bounds__(352, 1)
 fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_r,
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const ErrSink sink, int n_rt,
-                 int n_items, int chunk_shift) {
+                 int n_items, int chunk_shift, int group) {
     using L = Smem<D, NS>;
     constexpr uint32_t kQBytes = L::kQBytes, kKVBytes = L::kKVBytes;
     extern __shared__ unsigned char smem_raw[];
@@ -228,7 +229,7 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
                 clc_ask(base + L::kClc, bar(L::kClcFull));
                 src.asked = src.taken;
             }
-            it = get_item<EXT>(a, idx, n_rt, chunk_shift);
+            it = get_item<EXT>(a, idx, n_rt, group);
             if (it.valid) return true;
         }
     };
@@ -807,7 +808,8 @@ int launch_t(const TrainArgs &a, cudaStream_t stream) {
     const bool dynamic = items_by_hardware(n_items, sms, a.cu || EXT);
     const int chunk_shift = dynamic ? -1 : n_items >= 2 * sms ? 1 : 0;
     const int units = dynamic ? n_items : (n_items + (1 << chunk_shift) - 1) >> chunk_shift;
-    kern<<<dynamic || units < sms ? units : sms, 352, L::kBytes, stream>>>(a, tq, tr, tk, tv, sink, tiles, n_items, chunk_shift);
+    const int group = !dynamic ? 0 : a.cu || EXT ? 1 : item_group(a.batch * a.heads_q, tiles, sms);
+    kern<<<dynamic || units < sms ? units : sms, 352, L::kBytes, stream>>>(a, tq, tr, tk, tv, sink, tiles, n_items, chunk_shift, group);
     count_launch();
     return cudaGetLastError() == cudaSuccess ? PLX_OK : PLX_ERR_LAUNCH;
 }

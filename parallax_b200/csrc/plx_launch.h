@@ -11,15 +11,25 @@ struct ExchangeArgs;
 
 // Are the items of a tcgen05 kernel handed out by the hardware (see ItemRing in plx_sm100.cuh) or dealt out in advance,
 // in pairs of a heavy and a light one?  `uneven`: packed sequences and rows of a cache, whose items take as long as the
-// lengths say, always by the hardware: 32768 tokens in 255 sequences, fwd 334 -> 269, dk/dv 320 -> 250, dq/dr 390 -> 293 us
-// (the fullest CTA of dk/dv had 1.48 times the average work), 65536 tokens in 14 sequences 12.93 -> 12.13 ms.  Dense problems, where every pair is the same work, only when the last round of
-// pairs is so empty that it costs more than 4 %: 720 items (360 pairs, 3 rounds for 2.4) 245 -> 203 us forward and
-// backward at B = 9, H = 16, L = 548; 4096 items (2048 pairs, 14 rounds for 13.8) are 2.7 % faster dealt out.
+// lengths say, always by the hardware (32768 tokens in 270 sequences of 1 to 256: fwd 334 -> 269, dk/dv 320 -> 250, dq/dr
+// 390 -> 293 us; the fullest CTA of dk/dv had 1.48 times the average work).  Dense problems, where every pair is the same
+// work, when the last round of pairs is so empty that it costs more than 4 %.  Measured, dealt out against by hardware:
+// waste 23 % (720 items, B = 9, H = 16, L = 548) fwd 63 -> 50, bwd 171 -> 134 us; 16 % (512 items, B = 1, H = 16, L = 4096)
+// fwd 142 -> 130, bwd 390 -> 356; 6 % (1536 items, B = 4, H = 16, L = 3000) fwd 316 -> 281, bwd 891 -> 786; at 1.2 % (4096
+// items, L = 4096) pairs were 2.7 % faster.
 inline bool items_by_hardware(int64_t n_items, int sms, bool uneven) {
     if (n_items <= sms) return false;                      // one item per CTA
     if (uneven) return true;
     const int64_t units = n_items >= 2 * sms ? (n_items + 1) / 2 : n_items, rounds = (units + sms - 1) / sms;
     return 100 * rounds * sms > 104 * units;
+}
+
+// Pairs of (batch, head) whose items are interleaved, the longest first (see longest_first): groups of about equal size
+// with at least four items per SM, which is enough for the items that end a group to be short.  (One pair at a time left
+// the longest items of the last pairs to the end: forward at B = 1, H = 16, L = 4096 145 us dealt out in pairs, 176 so.)
+inline int item_group(int n_bh, int n_tiles, int sms) {
+    const int64_t groups = static_cast<int64_t>(n_bh) * n_tiles / (4 * static_cast<int64_t>(sms));
+    return groups <= 1 ? n_bh : static_cast<int>((n_bh + groups - 1) / groups);
 }
 
 // Every kernel launch of this library goes through count_launch() so that

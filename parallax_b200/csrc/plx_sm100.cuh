@@ -165,6 +165,15 @@ struct ItemRing {
     }
 };
 
+// Place of item `idx` among n_bh (batch, head) pairs of n_tiles items each, the k-th longest of its pair: inside groups
+// of `group` pairs the longest items of all of them come first, so that the last ones to start are short, while the
+// CTAs that run together still share a few heads in L2.
+__device__ __forceinline__ void longest_first(int idx, int n_tiles, int n_bh, int group, int &bh, int &k) {
+    const int first = idx / (group * n_tiles) * group, in = idx - first * n_tiles, n = min(group, n_bh - first);
+    bh = first + in % n;
+    k = in / n;
+}
+
 // Asks for another item; the answer (16 bytes) is there when `bar` has completed its next phase.  One thread, one
 // question at a time.
 __device__ __forceinline__ void clc_ask(uint32_t answer, uint32_t bar) {

@@ -56,6 +56,35 @@ def test_config1_loss_gradients():
         assert_close(leaf.grad.float().cpu(), e, TRAIN_REL_L2, TRAIN_MAX_REL, name)
 
 
+# (B, Hq, Hkv, L, D, window): more 128-row items than SMs, a last round that is mostly empty -- the items are handed out by
+# the hardware, the longest first in groups of (batch, head) pairs
+@pytest.mark.parametrize("case", [
+    (1, 54, 54, 300, 64, -1),       # 162 items: one more round than one item per CTA
+    (1, 103, 103, 260, 128, -1),    # 309: an odd number above two per SM
+    (1, 80, 20, 270, 128, 100),     # grouped heads: 240 items of dq/dr, 60 of dk/dv; a window
+    (2, 200, 200, 290, 64, -1),     # 1200: two groups of 200 pairs
+    (1, 1201, 1201, 120, 64, -1),   # one item per pair, groups of unequal size
+])
+def test_items_handed_out_by_the_hardware(case):
+    """A sample of heads (first, last, either side of a group) against the oracle; the others against the same
+    head computed in a launch of a few heads, whose items are dealt out, bit for bit."""
+    bsz, hq, hkv, length, d, window = case
+    q, r, k, v, go = make(bsz, hq, hkv, length, length, d, 900 + hq)
+    got = run_gpu(q, r, k, v, go, window)
+    rep, step = hq // hkv, 8
+    for h in range(0, hkv, step):
+        cut = lambda x, n: x[-1:, h * n:(h + step) * n]
+        few = run_gpu(*(cut(x, n) for x, n in ((q, rep), (r, rep), (k, 1), (v, 1), (go, rep))), window)
+        for name, x, y, n in zip(NAMES, got, few, (rep, rep, rep, 1, 1)):
+            assert torch.equal(cut(x, n), y), f"{case} {name} heads {h}.."
+    for h in (0, hkv // 2, hkv - 1):
+        cut = lambda x, n: x[:1, h * n:(h + 1) * n]
+        q1, r1, k1, v1, go1 = (cut(x, n) for x, n in ((q, rep), (r, rep), (k, 1), (v, 1), (go, rep)))
+        ref = (orc.train_forward(q1, r1, k1, v1, None, window)["o"], *orc.train_backward(q1, r1, k1, v1, go1.float(), None, window))
+        for name, x, e, n in zip(NAMES, got, ref, (rep, rep, rep, 1, 1)):
+            assert_close(cut(x, n), e, TRAIN_REL_L2, TRAIN_MAX_REL, f"{case} {name} head {h}")
+
+
 @pytest.mark.parametrize("length", [1, 2, 15, 16, 17, 63, 64, 65, 127, 128, 129, 255, 257, 1000])
 @pytest.mark.parametrize("d", [64, 128])
 def test_edge_lengths(length, d):
