@@ -307,9 +307,11 @@ __device__ __forceinline__ SplitPlan plan_slot(const DecodeArgs &a, int slot, in
     most = __reduce_max_sync(0xffffffffu, most);
     const int slots = a.batch * a.n_splits, cap = a.n_groups ? 32 * a.n_groups : 32;
     // part size in units: `good` fits (every row has at most n_splits parts), below `bad` none can
-    int good = max((most + a.n_splits - 1) / a.n_splits, 1);
+    // (A row of u units has fewer than u / m + 1 parts of m units, so m = sum / (slots - batch) fits as well.)  Four steps
+    // between the two come within a sixteenth of the best; a step is a division per row and a reduction, in series.
     int bad = max(max((sum + slots - 1) / slots, (most + cap - 1) / cap), 1);
-    while (bad < good) {
+    int good = max(min((most + a.n_splits - 1) / a.n_splits, (sum + slots - a.batch - 1) / (slots - a.batch)), bad);
+    for (int step = 0; step < 4 && bad < good; ++step) {
         const int mid = (bad + good) >> 1;
         int parts = 0;
 #pragma unroll
@@ -372,8 +374,20 @@ __global__ void __launch_bounds__(HG * 32, U > 4 ? 1 : 512 / (HG * 32)) decode_k
     const int sid = lane / LPK, sl = lane % LPK;
 
     // the part of a batch row's keys that this warp sweeps
-    const SplitPlan plan = plan_slot<NS, SG>(a, blockIdx.z * a.n_splits + (SG ? blockIdx.x * HG + warp : blockIdx.x), lane);
-    if (!SG && plan.b < 0) return;
+    SplitPlan plan;
+    if (SG || !a.balanced) {
+        plan = plan_slot<NS, true>(a, blockIdx.z * a.n_splits + (SG ? blockIdx.x * HG + warp : blockIdx.x), lane);
+    } else {
+        // the warps of a CTA have one slot: one of them plans (all eight, they queued for the divisions)
+        __shared__ SplitPlan s_plan;
+        if (warp == 0) {
+            plan = plan_slot<NS, false>(a, blockIdx.z * a.n_splits + blockIdx.x, lane);
+            if (lane == 0) s_plan = plan;
+        }
+        __syncthreads();
+        plan = s_plan;
+        if (plan.b < 0) return;
+    }
     const int b = plan.b, my_lo = plan.lo, my_hi = plan.hi;
     const int n_iter = (my_hi - my_lo + NS * U - 1) / (NS * U);
 
@@ -669,7 +683,7 @@ __global__ void __launch_bounds__(HG * 32, U > 4 ? 1 : 512 / (HG * 32)) decode_k
         if (!arrive_last(a.ws_counters + bh, plan.n_parts)) return;
         warp_merge<D>(recs, plan.n_parts, lane, big, D1, D2, O1, O2);
     } else {
-        const int gsize = a.balanced ? 32 : PLX_DECODE_GROUP, n_groups = (plan.n_parts + gsize - 1) / gsize;
+        const int gsize = max(PLX_DECODE_GROUP, (plan.n_parts + a.n_groups - 1) / a.n_groups), n_groups = (plan.n_parts + gsize - 1) / gsize;
         const int group = plan.part / gsize;
         const int first = group * gsize, size = min(gsize, plan.n_parts - first);
         int *gc = a.ws_gcounters + bh * a.n_groups + group;

@@ -105,13 +105,13 @@ struct Item {
 // Work item `idx` of the launch.  Items are ordered (batch, head)-major so that CTAs running at the
 // same time share K / V in L2; inside a (batch, head) the row tiles alternate last, first, last - 1,
 // second, ... so that under a causal mask any two neighbours add up to the same work.
-// (Handed out by the hardware, group > 0, they go from last to first: see longest_first.)
-template <bool EXT>
+// (Handed out by the hardware, DYN, they go from last to first: see longest_first.)
+template <bool EXT, bool DYN>
 __device__ __forceinline__ Item get_item(const TrainArgs &a, int idx, int n_rt, int group) {
     Item it;
     int bh = idx / n_rt, k = idx % n_rt;
-    if (group > 0) longest_first(idx, n_rt, a.batch * a.heads_q, group, bh, k);
-    const int tile_id = group > 0 ? n_rt - 1 - k : (k & 1) ? (k >> 1) : n_rt - 1 - (k >> 1);
+    if (DYN) longest_first(idx, n_rt, a.batch * a.heads_q, group, bh, k);
+    const int tile_id = DYN ? n_rt - 1 - k : (k & 1) ? (k >> 1) : n_rt - 1 - (k >> 1);
     it.pad = 0;
     Seq s;
     int tis = 0;
@@ -135,8 +135,7 @@ __device__ __forceinline__ Item get_item(const TrainArgs &a, int idx, int n_rt, 
     return it;
 }
 
-// n-th item of this CTA: CTAs take chunks of 2^chunk_shift neighbouring items, round robin.  (chunk_shift < 0: the
-// hardware hands the items out one by one.)
+// n-th item of this CTA where they are dealt out: CTAs take chunks of 2^chunk_shift neighbouring items, round robin.
 __device__ __forceinline__ int item_index(int n, int chunk_shift) {
     return ((blockIdx.x + gridDim.x * (n >> chunk_shift)) << chunk_shift) + (n & ((1 << chunk_shift) - 1));
 }
@@ -149,7 +148,12 @@ __device__ __forceinline__ int item_index(int n, int chunk_shift) {
 // paged (a tile is then one TMA box per page it touches, 64 keys at most), and only `o` is written.  Bound like the
 // forward.  4 rows of 512 tokens against 2048 to 4096 paged keys, 32 q / 8 kv heads: 202 us (0.19 TFLOP, 930 TFLOP/s);
 // the call, which gathered the pages and launched row by row, 590 -> 212 us.
-template <typename T, int D, int NS, bool EXT>
+//
+// DYN: the hardware hands the items out, the producer passes them on through the item ring (see items_by_hardware).
+// Dealt out in advance every role finds its items by itself, in a kernel of its own without ring and launch control: a
+// launch of one small item per CTA is bound by latency, and through the ring it was slower (B = 16, H = 8, L = 100, D = 64:
+// 8.9 -> 9.5 us).
+template <typename T, int D, int NS, bool EXT, bool DYN>
 __global__ void __launch_bounds__(352, 1)
 fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_r,
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const ErrSink sink, int n_rt,
@@ -167,7 +171,7 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
 
     if (threadIdx.x == 0) {
         asm volatile("st.shared.u32 [%0], %1;\n" ::"r"(err.abort_flag), "r"(0u) : "memory");
-        for (int i = 0; i < L::kNumBars; ++i) {
+        for (int i = 0; i < (DYN ? L::kNumBars : L::kItemFull); ++i) {
             const bool all_softmax =
                 (i >= L::kPFull && i < L::kPFull + 3) || i == L::kOFree || i == L::kSFree;
             const bool item_empty = i >= L::kItemEmpty && i < L::kItemEmpty + kItemSlots;
@@ -203,20 +207,15 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
     auto tP1 = [&](int pb) -> uint32_t { return kInPlace ? tS1(pb) : tmem_base + 384 + 64 * pb; };
     auto tP2 = [&](int pb) -> uint32_t { return kInPlace ? tS2(pb) : tmem_base + 384 + 64 * pb + 32; };
 
-    // Items: the producer finds them (`valid` = 0: no more) ...
+    // Items (`valid` = 0: no more).  DYN: the producer finds them ...
     const ItemRing ring{base + L::kItems, bar(L::kItemFull), bar(L::kItemEmpty)};
     struct Source {
         int taken, asked;
     };
     auto find_item = [&](Source &src, Item &it) -> bool {
         for (;;) {
-            int idx = -1;
-            if (chunk_shift >= 0) {
-                idx = item_index(src.taken, chunk_shift);
-                if (idx >= n_items) idx = -1;
-            } else if (src.taken == 0) {
-                idx = blockIdx.x;
-            } else {
+            int idx = blockIdx.x;
+            if (src.taken > 0) {
                 if (!mbar_wait(bar(L::kClcFull), (src.taken - 1) & 1, err, 19)) return false;
                 idx = clc_answer(base + L::kClc);
             }
@@ -225,17 +224,29 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
                 it.valid = 0;
                 return true;
             }
-            if (chunk_shift < 0) {
-                clc_ask(base + L::kClc, bar(L::kClcFull));
-                src.asked = src.taken;
-            }
-            it = get_item<EXT>(a, idx, n_rt, group);
+            clc_ask(base + L::kClc, bar(L::kClcFull));
+            src.asked = src.taken;
+            it = get_item<EXT, DYN>(a, idx, n_rt, group);
             if (it.valid) return true;
         }
     };
     // ... and lets no answer of the hardware arrive in shared memory that is no longer its own
     auto leave_source = [&](const Source &src) {
         if (src.asked == src.taken && src.asked > 0) mbar_wait_quiet(bar(L::kClcFull), (src.asked - 1) & 1);
+    };
+    // The n-th item as a role sees it (whole: by all lanes of its warp), `taken` counting the items it has looked at.
+    auto next_item = [&](int n, int &taken, Item &it, bool whole) -> bool {
+        if constexpr (DYN) {
+            return ring.read(n, it, whole, err, 21);
+        } else {
+            for (;;) {
+                const int idx = item_index(taken++, chunk_shift);
+                it.valid = 0;
+                if (idx >= n_items) return true;
+                it = get_item<EXT, DYN>(a, idx, n_rt, group);
+                if (it.valid) return true;
+            }
+        }
     };
 
     if (warp == 0) {
@@ -256,13 +267,13 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
             Source src{0, 0};
             for (int n = 0; ok; ++n) {
                 Item it;
-                ok = is_k ? find_item(src, it) && ring.publish(n, it, err, 20) : ring.read(n, it, false, err, 21);
+                ok = DYN && is_k ? find_item(src, it) && ring.publish(n, it, err, 20) : next_item(n, src.taken, it, false);
                 if (!ok || !it.valid) break;
                 if (it.n_tiles == 0) continue;
                 if (is_k) {
                     // short items: what they wait for is the first touch of q and r, so have them on the way into L2
                     // while the tiles of the item before still occupy the shared memory
-                    if (chunk_shift < 0 && n_items_done > 0)
+                    if (DYN && n_items_done > 0)
 #pragma unroll
                         for (int pn = 0; pn < L::kPanels; ++pn) {
                             tma_prefetch_4d(&tm_q, 64 * pn, it.bos + it.r0, it.h, it.b);
@@ -343,7 +354,7 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
                     mbar_wait_quiet(bar(full0 + s), ph);
                 }
                 if (is_k && n_items_done > 0) mbar_wait_quiet(bar(L::kQFull), (n_items_done - 1) & 1);
-                leave_source(src);
+                if (DYN) leave_source(src);
             }
         }
     } else if (warp == 1) {
@@ -360,9 +371,10 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
             bool ok = true;
             int s = 0, g = 0, n_items_done = 0;                           // K ring stage, key tiles and items so far
             uint32_t ph = 0;                                              // phase of the K ring
+            int taken = 0;
             for (int n = 0; ok; ++n) {
                 Item it;
-                ok = ring.read(n, it, true, err, 21);
+                ok = next_item(n, taken, it, true);
                 if (!ok || !it.valid) break;
                 if (it.n_tiles == 0) continue;
                 ok = __all_sync(0xffffffffu, mbar_wait(bar(L::kQFull), n_items_done & 1, err, 4));
@@ -416,9 +428,10 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
             bool ok = true;
             int s = 0, g = 0, n_items_done = 0;
             uint32_t ph = 0;
+            int taken = 0;
             for (int n = 0; ok; ++n) {
                 Item it;
-                ok = ring.read(n, it, true, err, 21);
+                ok = next_item(n, taken, it, true);
                 if (!ok || !it.valid) break;
                 if (it.n_tiles == 0) continue;
                 for (int j = 0; j < it.n_tiles && ok; ++j, ++g) {
@@ -471,9 +484,10 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
         bool ok = true;
         int g = 0, n_items_done = 0;                       // key tiles and items (with keys) so far
 
+        int taken = 0;
         for (int n = 0; ok; ++n) {
             Item it;
-            ok = ring.read(n, it, true, err, 21);
+            ok = next_item(n, taken, it, true);
             if (!ok || !it.valid) break;
             if (it.n_tiles == 0) {
                 // no key is visible to any row of the tile: outputs are zero (one thread per row and column half)
@@ -797,19 +811,23 @@ int launch_t(const TrainArgs &a, cudaStream_t stream) {
         !make_map(&tk, dt, a.k, D, kv_rows, a.heads_kv, kv_batch, a.kv_st, a.kv_sh, a.kv_sb, kv_box) ||
         !make_map(&tv, dt, a.v, D, kv_rows, a.heads_kv, kv_batch, a.kv_st, a.kv_sh, a.kv_sb, kv_box))
         return PLX_ERR_LAUNCH;
-    auto kern = fwd_sm100_kernel<T, D, NS, EXT>;
-    static std::mutex attr_mu;
-    static bool attr_done[tma::kMaxDevices] = {};
-    if (!tma::opt_in_smem(kern, static_cast<int>(L::kBytes), attr_done, attr_mu)) return PLX_ERR_LAUNCH;
     const int tiles = a.cu ? (a.len_q + kBM - 1) / kBM + a.n_seqs : (a.len_q + kBM - 1) / kBM;
     const int n_items = tiles * a.batch * a.heads_q, sms = sm_count();
     if (sms <= 0) return PLX_ERR_LAUNCH;
-    // with plenty of items a CTA takes them in neighbouring pairs (a heavy and a light row tile)
-    const bool dynamic = items_by_hardware(n_items, sms, a.cu || EXT);
-    const int chunk_shift = dynamic ? -1 : n_items >= 2 * sms ? 1 : 0;
-    const int units = dynamic ? n_items : (n_items + (1 << chunk_shift) - 1) >> chunk_shift;
-    const int group = !dynamic ? 0 : a.cu || EXT ? 1 : item_group(a.batch * a.heads_q, tiles, sms);
-    kern<<<dynamic || units < sms ? units : sms, 352, L::kBytes, stream>>>(a, tq, tr, tk, tv, sink, tiles, n_items, chunk_shift, group);
+    static std::mutex attr_mu;
+    static bool attr_done[2][tma::kMaxDevices] = {};
+    if (items_by_hardware(n_items, sms, a.cu || EXT)) {
+        auto kern = fwd_sm100_kernel<T, D, NS, EXT, true>;
+        if (!tma::opt_in_smem(kern, static_cast<int>(L::kBytes), attr_done[1], attr_mu)) return PLX_ERR_LAUNCH;
+        const int group = a.cu || EXT ? 1 : item_group(a.batch * a.heads_q, tiles, sms);
+        kern<<<n_items, 352, L::kBytes, stream>>>(a, tq, tr, tk, tv, sink, tiles, n_items, 0, group);
+    } else {
+        auto kern = fwd_sm100_kernel<T, D, NS, EXT, false>;
+        if (!tma::opt_in_smem(kern, static_cast<int>(L::kBytes), attr_done[0], attr_mu)) return PLX_ERR_LAUNCH;
+        // with plenty of items a CTA takes them in neighbouring pairs (a heavy and a light row tile)
+        const int chunk_shift = n_items >= 2 * sms ? 1 : 0, units = (n_items + (1 << chunk_shift) - 1) >> chunk_shift;
+        kern<<<units < sms ? units : sms, 352, L::kBytes, stream>>>(a, tq, tr, tk, tv, sink, tiles, n_items, chunk_shift, 0);
+    }
     count_launch();
     return cudaGetLastError() == cudaSuccess ? PLX_OK : PLX_ERR_LAUNCH;
 }
