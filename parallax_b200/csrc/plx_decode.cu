@@ -266,29 +266,27 @@ struct SplitPlan {
     int64_t first;
 };
 
-// Slot -> plan, computed by a whole warp.  G: keys come in multiples of G.
+// Part `part` of n_splits equal ones of the keys of row b.  G: keys come in multiples of G.
+template <int G>
+__device__ __forceinline__ SplitPlan plan_even(const DecodeArgs &a, int b, int part) {
+    int lo, hi;
+    row_range(a, b, lo, hi);
+    int chunk = (max(hi - lo, 0) + a.n_splits - 1) / a.n_splits;
+    chunk = (chunk + G - 1) / G * G;
+    const int my_lo = min(lo + part * chunk, hi);
+    return SplitPlan{b, part, a.n_splits, my_lo, min(my_lo + chunk, hi), static_cast<int64_t>(b) * a.n_splits * a.heads_q};
+}
+
+// Slot -> plan, computed by a whole warp.
 // Rows of one length get n_splits parts each.  With lengths of their own (seqused / cache_start) that makes the
 // longest row set the time while the warps of the others idle, so there the slots are dealt out by length: the
 // smallest part size for which the parts of all rows still fit into the slots.  Lane l looks after rows l, l + 32,
 // ..: up to kBalancedRows rows.  A row's parts must fit the merge: 32 records in one level, 32 per group in two.
 // Measured with 16 paged rows of 8192 down to 3072 keys, 32 q / 8 kv heads, bound by HBM: the longest row's parts go from
 // 1024 to 752 keys; together with the one page number per tile the kernel went from 127 to 78 us (370 MB, 4.7 TB/s).
-template <int G, bool UNIFORM>
+template <int G>
 __device__ __forceinline__ SplitPlan plan_slot(const DecodeArgs &a, int slot, int lane) {
     SplitPlan p{-1, 0, 1, 0, 0, 0};
-    if (UNIFORM || !a.balanced) {
-        p.b = slot / a.n_splits;
-        p.part = slot - p.b * a.n_splits;
-        p.n_parts = a.n_splits;
-        p.first = static_cast<int64_t>(p.b) * a.n_splits * a.heads_q;
-        int lo, hi;
-        row_range(a, p.b, lo, hi);
-        const int n = max(hi - lo, 0);
-        const int chunk = ((n + a.n_splits - 1) / a.n_splits + G - 1) / G * G;
-        p.lo = min(lo + p.part * chunk, hi);
-        p.hi = min(p.lo + chunk, hi);
-        return p;
-    }
     constexpr int kRows = kBalancedRows / 32;
     int start[kRows], n[kRows], units[kRows], sum = 0, most = 0;   // units: multiples of G keys
 #pragma unroll
@@ -376,12 +374,12 @@ __global__ void __launch_bounds__(HG * 32, U > 4 ? 1 : 512 / (HG * 32)) decode_k
     // the part of a batch row's keys that this warp sweeps
     SplitPlan plan;
     if (SG || !a.balanced) {
-        plan = plan_slot<NS, true>(a, blockIdx.z * a.n_splits + (SG ? blockIdx.x * HG + warp : blockIdx.x), lane);
+        plan = plan_even<NS>(a, blockIdx.z, SG ? blockIdx.x * HG + warp : blockIdx.x);
     } else {
         // the warps of a CTA have one slot: one of them plans (all eight, they queued for the divisions)
         __shared__ SplitPlan s_plan;
         if (warp == 0) {
-            plan = plan_slot<NS, false>(a, blockIdx.z * a.n_splits + blockIdx.x, lane);
+            plan = plan_slot<NS>(a, blockIdx.z * a.n_splits + blockIdx.x, lane);
             if (lane == 0) s_plan = plan;
         }
         __syncthreads();
@@ -893,7 +891,7 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
     const int hunit = blockIdx.x % n_hunits, cta = blockIdx.x / n_hunits, slot = cta * kGqaWarps + warp;
     const int hk = hunit / n_hgroups, hgrp = hunit % n_hgroups;
     SplitPlan plan{-1, 0, 0, 0, 0, 0};
-    if (slot < n_slots) plan = plan_slot<kGqaTile, false>(a, slot, lane);
+    if (slot < n_slots) plan = a.balanced ? plan_slot<kGqaTile>(a, slot, lane) : plan_even<kGqaTile>(a, slot / a.n_splits, slot % a.n_splits);
     const int b = max(plan.b, 0), my_lo = plan.lo, my_hi = plan.b < 0 ? plan.lo : plan.hi;
     const int n_tiles = (my_hi - my_lo + kGqaTile - 1) / kGqaTile;
     const int hq0 = hk * a.n_rep + hgrp * 16;       // first q head of this CTA's rows
