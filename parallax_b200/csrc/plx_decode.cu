@@ -266,26 +266,30 @@ struct SplitPlan {
     int64_t first;
 };
 
-// Part `part` of n_splits equal ones of the keys of row b.  G: keys come in multiples of G.
+// Part `part` of n_splits equal ones of the keys [lo, hi) of row b.  G: keys come in multiples of G.
 template <int G>
-__device__ __forceinline__ SplitPlan plan_even(const DecodeArgs &a, int b, int part) {
-    int lo, hi;
-    row_range(a, b, lo, hi);
+__device__ __forceinline__ SplitPlan even_part(const DecodeArgs &a, int b, int part, int lo, int hi) {
     int chunk = (max(hi - lo, 0) + a.n_splits - 1) / a.n_splits;
     chunk = (chunk + G - 1) / G * G;
     const int my_lo = min(lo + part * chunk, hi);
     return SplitPlan{b, part, a.n_splits, my_lo, min(my_lo + chunk, hi), static_cast<int64_t>(b) * a.n_splits * a.heads_q};
 }
+template <int G>
+__device__ __forceinline__ SplitPlan plan_even(const DecodeArgs &a, int b, int part) {
+    int lo, hi;
+    row_range(a, b, lo, hi);
+    return even_part<G>(a, b, part, lo, hi);
+}
 
 // Slot -> plan, computed by a whole warp.
 // Rows of one length get n_splits parts each.  With lengths of their own (seqused / cache_start) that makes the
-// longest row set the time while the warps of the others idle, so there the slots are dealt out by length: the
+// longest row set the time while the warps of the others idle.  There the slots are dealt out by length: the
 // smallest part size for which the parts of all rows still fit into the slots.  Lane l looks after rows l, l + 32,
-// ..: up to kBalancedRows rows.  A row's parts must fit the merge: 32 records in one level, 32 per group in two.
-// Measured with 16 paged rows of 8192 down to 3072 keys, 32 q / 8 kv heads, bound by HBM: the longest row's parts go from
-// 1024 to 752 keys; together with the one page number per tile the kernel went from 127 to 78 us (370 MB, 4.7 TB/s).
+// ..: up to kBalancedRows rows.  `cap`: the most parts of a row that the merge takes.
+// Not so where the longest row is within a.balanced quarters of the mean (see balance_from): dealing out costs the
+// search and leaves parts and rows that no longer fall together with CTAs.
 template <int G>
-__device__ __forceinline__ SplitPlan plan_slot(const DecodeArgs &a, int slot, int lane) {
+__device__ __forceinline__ SplitPlan plan_slot(const DecodeArgs &a, int slot, int lane, int cap) {
     SplitPlan p{-1, 0, 1, 0, 0, 0};
     constexpr int kRows = kBalancedRows / 32;
     int start[kRows], n[kRows], units[kRows], sum = 0, most = 0;   // units: multiples of G keys
@@ -303,7 +307,18 @@ __device__ __forceinline__ SplitPlan plan_slot(const DecodeArgs &a, int slot, in
     }
     sum = __reduce_add_sync(0xffffffffu, sum);
     most = __reduce_max_sync(0xffffffffu, most);
-    const int slots = a.batch * a.n_splits, cap = a.n_groups ? 32 * a.n_groups : 32;
+    if (4 * static_cast<int64_t>(most) * a.batch <= static_cast<int64_t>(a.balanced) * sum) {
+        p.b = slot / a.n_splits;
+        int lo = 0, len = 0;
+#pragma unroll
+        for (int i = 0; i < kRows; ++i)
+            if (p.b >> 5 == i) {
+                lo = __shfl_sync(0xffffffffu, start[i], p.b & 31);
+                len = __shfl_sync(0xffffffffu, n[i], p.b & 31);
+            }
+        return even_part<G>(a, p.b, slot - p.b * a.n_splits, lo, lo + len);
+    }
+    const int slots = a.batch * a.n_splits;
     // part size in units: `good` fits (every row has at most n_splits parts), below `bad` none can
     // (A row of u units has fewer than u / m + 1 parts of m units, so m = sum / (slots - batch) fits as well.)  Four steps
     // between the two come within a sixteenth of the best; a step is a division per row and a reduction, in series.
@@ -379,7 +394,7 @@ __global__ void __launch_bounds__(HG * 32, U > 4 ? 1 : 512 / (HG * 32)) decode_k
         // the warps of a CTA have one slot: one of them plans (all eight, they queued for the divisions)
         __shared__ SplitPlan s_plan;
         if (warp == 0) {
-            plan = plan_slot<NS>(a, blockIdx.z * a.n_splits + blockIdx.x, lane);
+            plan = plan_slot<NS>(a, blockIdx.z * a.n_splits + blockIdx.x, lane, a.n_groups ? 32 * a.n_groups : 32);
             if (lane == 0) s_plan = plan;
         }
         __syncthreads();
@@ -893,7 +908,7 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
     const int hunit = blockIdx.x % n_hunits, cta = blockIdx.x / n_hunits, slot = cta * kGqaWarps + warp;
     const int hk = hunit / n_hgroups, hgrp = hunit % n_hgroups;
     SplitPlan plan{-1, 0, 0, 0, 0, 0};
-    if (slot < n_slots) plan = a.balanced ? plan_slot<kGqaTile>(a, slot, lane) : plan_even<kGqaTile>(a, slot / a.n_splits, slot % a.n_splits);
+    if (slot < n_slots) plan = a.balanced ? plan_slot<kGqaTile>(a, slot, lane, n_slots) : plan_even<kGqaTile>(a, slot / a.n_splits, slot % a.n_splits);
     const int b = max(plan.b, 0), my_lo = plan.lo, my_hi = plan.b < 0 ? plan.lo : plan.hi;
     const int n_tiles = (my_hi - my_lo + kGqaTile - 1) / kGqaTile;
     const int hq0 = hk * a.n_rep + hgrp * 16;       // first q head of this CTA's rows
@@ -1315,12 +1330,35 @@ bool decode_fused_exchange_supported(const DecodeArgs &a) {
     return a.n_rep == 1 && a.n_splits >= 2 && !decode_split_groups(a);
 }
 
+// From which ratio of the longest row to the mean, in quarters, the splits are dealt out by length; 0: never.
+// Not for split groups, whose CTAs belong to one row, and not for a key-sharded launch, whose fused and two-launch forms
+// have to cut the keys alike.
+// Where the parts are large and the launch is bound by HBM, dealing out pays from a small skew on (5): rows from T down
+// to T / 3 keys (a skew of 1.5), even parts against dealt out: 32 rows of 4000, 8 : 8 heads, 76 -> 70 us; 16 rows of 8192,
+// 32 : 8 heads, 94 -> 76.  Elsewhere only from a skew of 2 on (8), since it costs the plan and, with grouped heads, the
+// merge inside a CTA: 64 rows of 512, 16 : 2 heads, 11.6 -> 21.0 us; 128 rows of 1000, 8 : 8 heads, 80 -> 87; but where one
+// row is ten times the others, those 128 rows took 71 us in even parts against 27.
+// `part`, the keys of an even part times head_dim: the lines lie between 250 and 512 keys at head_dim 128 (512 and 1024 at
+// 64) with grouped heads, else between 75 and 111; below 64 the wait for the plan is all there is to see (12 rows of 900, 13.5 ->
+// 14.7 us).  Also against an even cut of grouped heads: rows that end inside a CTA of another row (3 rows of 1000 keys in 15
+// parts, 16 : 2 heads, 20.0 us even, 15.0 dealt out).
+static int balance_from(const DecodeArgs &a, int head_dim) {
+    if ((!a.seqused && !a.cache_start) || a.batch < 2 || a.batch > kBalancedRows || a.n_splits < 2 || a.part_out || a.xch.world != 0 ||
+        decode_split_groups(a))
+        return 0;
+    const int64_t n_keys = a.window >= 0 && a.window < a.cache_len ? a.window : a.cache_len, part = n_keys / a.n_splits * head_dim;
+    if (a.n_rep > 1) {
+        const bool rows_end_with_ctas = a.n_splits % kGqaWarps == 0 || kGqaWarps % a.n_splits == 0;
+        return part < 384 * 128 && rows_end_with_ctas ? 8 : 5;
+    }
+    if (part < 64 * 128) return 0;
+    const bool one_wave = static_cast<int64_t>(a.batch) * a.heads_q * a.n_splits <= 16 * static_cast<int64_t>(tma_free_sm_count());
+    return part < 100 * 128 || a.n_splits < 4 || !one_wave ? 8 : 5;
+}
+
 int launch_decode(const DecodeArgs &problem, int dtype, int head_dim, cudaStream_t stream) {
     DecodeArgs a = problem;
-    // Rows with lengths of their own: deal the splits out by length.  Not split groups, whose CTAs belong to one
-    // row, and not a key-sharded launch, whose fused and two-launch forms have to cut the keys alike.
-    a.balanced = (a.seqused || a.cache_start) && a.batch > 1 && a.batch <= kBalancedRows && a.n_splits > 1 && !a.part_out &&
-                 a.xch.world == 0 && !decode_split_groups(a);
+    a.balanced = balance_from(a, head_dim);
     if (dtype == PLX_BF16) {
         if (head_dim == 128) return launch_decode_t<__nv_bfloat16, 128>(a, stream);
         if (head_dim == 64) return launch_decode_t<__nv_bfloat16, 64>(a, stream);

@@ -27,7 +27,7 @@ struct DecodeArgs {
     float *ws_gparts;  // (batch * heads_q, n_groups) records of the first merge level (n_groups > 0)
     int *ws_gcounters; // (batch * heads_q, n_groups) arrival counters of the groups
     int n_groups;      // 0: single-level merge
-    bool balanced;     // splits dealt out to the batch rows by length (see plan_slot)
+    int balanced;      // splits dealt out to the batch rows by length, from this skew on; 0: never (see plan_slot)
     int batch, heads_q, heads_kv, n_rep, cache_len, window, n_splits, kv_offset, total_len;
     float c2;  // qk_scale * log2(e)
     int64_t kv_sb, kv_st, kv_sh;   // paged: kv_sb is the stride between pages

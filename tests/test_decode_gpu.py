@@ -775,6 +775,26 @@ def test_rows_of_very_different_lengths(case):
 
 
 @pytest.mark.parametrize("case", [
+    # batch, hq, hkv, cache, head_dim: either side of the lines between even parts and parts by length
+    (4, 8, 8, 17000, 64), (16, 8, 8, 1300, 128), (40, 8, 8, 230, 128), (128, 8, 8, 600, 64), (12, 16, 16, 4000, 64),
+    (16, 8, 2, 7000, 128), (64, 8, 2, 500, 64), (3, 16, 2, 1000, 128), (9, 16, 4, 3300, 64), (2, 8, 4, 40000, 128),
+])
+def test_rows_of_little_and_much_different_lengths(case):
+    """Equal lengths give the bits of a call without lengths; rows down to a third of the longest, and one long row among
+    short ones, give what each row gives against the oracle."""
+    bsz, hq, hkv, kv_len, d = case
+    q, r, k, v = cuda(*make(bsz, hq, kv_len, d, hkv, seed=73))
+    t32 = lambda x: torch.tensor(x, dtype=torch.int32, device="cuda")
+    assert torch.equal(plx.parallax_decode(q, r, k, v), plx.parallax_decode(q, r, k, v, seqused_k=t32([kv_len] * bsz)))
+    for used in ([kv_len - 2 * kv_len * b // (3 * bsz) for b in range(bsz)], [kv_len if b == bsz // 2 else 1 + kv_len // 12 for b in range(bsz)]):
+        out = plx.parallax_decode(q, r, k, v, seqused_k=t32(used))
+        assert torch.equal(out, plx.parallax_decode(q, r, k, v, seqused_k=t32(used)))
+        for b in sorted({0, bsz // 2, bsz - 1}):
+            ref = orc.decode(*(x[b:b + 1].cpu() for x in (q, r)), *(x[b:b + 1, :used[b]].cpu() for x in (k, v)))
+            assert_close(out[b:b + 1].float().cpu(), ref, DECODE_REL_L2, DECODE_MAX_REL, f"{case} row {b} of {used[b]}")
+
+
+@pytest.mark.parametrize("case", [
     # batch, hq, hkv, cache, head_dim, page (0: dense), ragged, splits
     (1, 8, 2, 4111, 128, 0, False, 61),      # one row over eight CTAs
     (3, 8, 1, 5000, 64, 64, False, 255),     # a row over 33 CTAs, its first and last shared with other rows
