@@ -364,9 +364,8 @@ __device__ __forceinline__ SplitPlan plan_slot(const DecodeArgs &a, int slot, in
 
 // One WARP per (split, q head, batch row); a CTA is HG warps working on HG adjacent q
 // heads of the same key range, so that together they sweep contiguous memory (all heads
-// of a key are adjacent in the cache layout) and, under grouped-query attention, the q
-// heads of a group find the shared K / V rows in L1.  Warps never synchronise with each
-// other: streams are merged by shuffles, splits by the last warp to arrive.
+// of a key are adjacent in the cache layout).  One q head per kv head.  Streams are merged by
+// shuffles, splits by the last warp to arrive.
 //
 // SG ("split group") is the arrangement for launches with few (batch, head) pairs, which are bound by
 // latency, not bandwidth: a CTA is the HG = 8 warps of eight ADJACENT SPLITS of one q head.  Every
@@ -374,7 +373,7 @@ __device__ __forceinline__ SplitPlan plan_slot(const DecodeArgs &a, int slot, in
 // record per CTA goes through global memory, and the CTA that arrives last merges the (at most 32) CTA
 // records with all 256 threads at once -- one round trip to L2 where a single merging warp needs one
 // per eight records.  That allows splits of ~16 keys, whose loads are all in flight together.
-template <typename T, int D, int HG, int U, bool GQA, bool SG>
+template <typename T, int D, int HG, int U, bool SG>
 __global__ void __launch_bounds__(HG * 32, U > 4 ? 1 : 512 / (HG * 32)) decode_kernel(const DecodeArgs a) {
     constexpr int LPK = D / 8;      // lanes per key row
     constexpr int NS = 32 / LPK;    // streams per warp
@@ -383,7 +382,6 @@ __global__ void __launch_bounds__(HG * 32, U > 4 ? 1 : 512 / (HG * 32)) decode_k
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int hq = SG ? blockIdx.y : blockIdx.y * HG + warp;
-    const int hk = hq / a.n_rep;
     const int sid = lane / LPK, sl = lane % LPK;
 
     // the part of a batch row's keys that this warp sweeps
@@ -412,7 +410,7 @@ __global__ void __launch_bounds__(HG * 32, U > 4 ? 1 : 512 / (HG * 32)) decode_k
         unpack8<T>(*reinterpret_cast<const uint4 *>(static_cast<const T *>(a.r) + qi), rf);
     }
     const bool paged = a.page_table != nullptr;      // uniform over the launch
-    const int64_t row0 = (paged ? 0 : b * a.kv_sb) + hk * a.kv_sh + sl * 8;
+    const int64_t row0 = (paged ? 0 : b * a.kv_sb) + hq * a.kv_sh + sl * 8;
     const T *kp = static_cast<const T *>(a.k) + row0;
     const T *vp = static_cast<const T *>(a.v) + row0;
 
@@ -431,8 +429,8 @@ __global__ void __launch_bounds__(HG * 32, U > 4 ? 1 : 512 / (HG * 32)) decode_k
             if (kj < my_hi) {
                 const int64_t at = decltype(paged_tag)::value ? paged_key_offset(a, b, kj) : static_cast<int64_t>(kj) * a.kv_st;
                 const T *pk = kp + at, *pv = vp + at;
-                kr[u] = GQA ? __ldg(reinterpret_cast<const uint4 *>(pk)) : ld_stream16(pk);
-                vr[u] = GQA ? __ldg(reinterpret_cast<const uint4 *>(pv)) : ld_stream16(pv);
+                kr[u] = ld_stream16(pk);
+                vr[u] = ld_stream16(pv);
             } else {
                 kr[u] = make_uint4(0u, 0u, 0u, 0u);
                 vr[u] = make_uint4(0u, 0u, 0u, 0u);
@@ -1231,10 +1229,7 @@ template <typename T, int D, int HG>
 static int launch_decode_hg(const DecodeArgs &a, cudaStream_t stream) {
     constexpr int U = 4;  // key rows per stream and register buffer (two buffers: 8 rows of K and of V in flight)
     dim3 grid(a.n_splits, a.heads_q / HG, a.batch);
-    if (a.n_rep > 1)
-        decode_kernel<T, D, HG, U, true, false><<<grid, HG * 32, 0, stream>>>(a);
-    else
-        decode_kernel<T, D, HG, U, false, false><<<grid, HG * 32, 0, stream>>>(a);
+    decode_kernel<T, D, HG, U, false><<<grid, HG * 32, 0, stream>>>(a);
     count_launch();
     return cudaGetLastError() == cudaSuccess ? PLX_OK : PLX_ERR_LAUNCH;
 }
@@ -1298,7 +1293,7 @@ static int launch_decode_sg(const DecodeArgs &a, cudaStream_t stream) {
         int n = resident[dev][slot].load(std::memory_order_acquire);
         if (n == 0) {
             cfg.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&n, decode_kernel<T, D, 8, 8, false, true>, &cfg) != cudaSuccess || n < 1) {
+            if (cudaOccupancyMaxActiveClusters(&n, decode_kernel<T, D, 8, 8, true>, &cfg) != cudaSuccess || n < 1) {
                 (void)cudaGetLastError();
                 n = -1;
             }
@@ -1306,7 +1301,7 @@ static int launch_decode_sg(const DecodeArgs &a, cudaStream_t stream) {
         }
         roomy = roomy && units <= n;
     }
-    auto kern = roomy ? decode_kernel<T, D, 8, 8, false, true> : decode_kernel<T, D, 8, 4, false, true>;
+    auto kern = roomy ? decode_kernel<T, D, 8, 8, true> : decode_kernel<T, D, 8, 4, true>;
     cfg.numAttrs = cluster ? 1 : 0;
     cudaError_t st = cudaLaunchKernelEx(&cfg, kern, a);
     count_launch();
