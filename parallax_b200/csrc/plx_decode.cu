@@ -373,7 +373,10 @@ __device__ __forceinline__ SplitPlan plan_slot(const DecodeArgs &a, int slot, in
 // record per CTA goes through global memory, and the CTA that arrives last merges the (at most 32) CTA
 // records with all 256 threads at once -- one round trip to L2 where a single merging warp needs one
 // per eight records.  That allows splits of ~16 keys, whose loads are all in flight together.
-template <typename T, int D, int HG, int U, bool SG>
+//
+// DEAL: the slots may be dealt out by length (a.balanced > 0).  A kernel of its own: with the plan of either kind in one,
+// launches without lengths were 0.3 to 0.6 us longer (32 rows of 300 down to 100 keys, 8 : 8 heads, 12.4 -> 13.0).
+template <typename T, int D, int HG, int U, bool SG, bool DEAL>
 __global__ void __launch_bounds__(HG * 32, U > 4 ? 1 : 512 / (HG * 32)) decode_kernel(const DecodeArgs a) {
     constexpr int LPK = D / 8;      // lanes per key row
     constexpr int NS = 32 / LPK;    // streams per warp
@@ -386,7 +389,7 @@ __global__ void __launch_bounds__(HG * 32, U > 4 ? 1 : 512 / (HG * 32)) decode_k
 
     // the part of a batch row's keys that this warp sweeps
     SplitPlan plan;
-    if (SG || !a.balanced) {
+    if constexpr (!DEAL) {
         plan = plan_even<NS>(a, blockIdx.z, SG ? blockIdx.x * HG + warp : blockIdx.x);
     } else {
         // the warps of a CTA have one slot: one of them plans (all eight, they queued for the divisions)
@@ -1229,7 +1232,10 @@ template <typename T, int D, int HG>
 static int launch_decode_hg(const DecodeArgs &a, cudaStream_t stream) {
     constexpr int U = 4;  // key rows per stream and register buffer (two buffers: 8 rows of K and of V in flight)
     dim3 grid(a.n_splits, a.heads_q / HG, a.batch);
-    decode_kernel<T, D, HG, U, false><<<grid, HG * 32, 0, stream>>>(a);
+    if (a.balanced)
+        decode_kernel<T, D, HG, U, false, true><<<grid, HG * 32, 0, stream>>>(a);
+    else
+        decode_kernel<T, D, HG, U, false, false><<<grid, HG * 32, 0, stream>>>(a);
     count_launch();
     return cudaGetLastError() == cudaSuccess ? PLX_OK : PLX_ERR_LAUNCH;
 }
@@ -1293,7 +1299,7 @@ static int launch_decode_sg(const DecodeArgs &a, cudaStream_t stream) {
         int n = resident[dev][slot].load(std::memory_order_acquire);
         if (n == 0) {
             cfg.numAttrs = 1;
-            if (cudaOccupancyMaxActiveClusters(&n, decode_kernel<T, D, 8, 8, true>, &cfg) != cudaSuccess || n < 1) {
+            if (cudaOccupancyMaxActiveClusters(&n, decode_kernel<T, D, 8, 8, true, false>, &cfg) != cudaSuccess || n < 1) {
                 (void)cudaGetLastError();
                 n = -1;
             }
@@ -1301,7 +1307,7 @@ static int launch_decode_sg(const DecodeArgs &a, cudaStream_t stream) {
         }
         roomy = roomy && units <= n;
     }
-    auto kern = roomy ? decode_kernel<T, D, 8, 8, true> : decode_kernel<T, D, 8, 4, true>;
+    auto kern = roomy ? decode_kernel<T, D, 8, 8, true, false> : decode_kernel<T, D, 8, 4, true, false>;
     cfg.numAttrs = cluster ? 1 : 0;
     cudaError_t st = cudaLaunchKernelEx(&cfg, kern, a);
     count_launch();
