@@ -19,8 +19,29 @@ def randn(*shape, dtype=torch.bfloat16, seed=0):
     return torch.randn(*shape, generator=torch.Generator().manual_seed(seed + sum(shape))).to(dtype).cuda()
 
 
-def both(call):
-    fast = call()
+class Recorder:
+    """The C++ host side, with a note of which of its entry points answered."""
+
+    def __init__(self, host):
+        self.host, self.answered = host, set()
+
+    def __getattr__(self, name):
+        def entry(*args):
+            res = getattr(self.host, name)(*args)
+            if res is not None and res is not False:
+                self.answered.add(name)
+            return res
+
+        return entry
+
+
+def both(call, by):
+    """`call` by the short cut -- the entry points `by` answer, and no others -- and by the Python path."""
+    recorder = Recorder(_cabi.host())
+    with pytest.MonkeyPatch.context() as patch:
+        patch.setattr(_cabi, "_host", recorder)
+        fast = call()
+    assert recorder.answered == by
     with PythonPath():
         slow = call()
     for a, b in zip(fast, slow):
@@ -48,10 +69,14 @@ def test_training(layout, window, dtype, d):
         o = call(*leaves)
         return (o.detach(), *torch.autograd.grad(o, leaves, go))
 
-    both(step)
-    both(lambda: (call(*leaves[:3], leaves[3].detach()).detach(),))
+    by = {"train", "train_ready"}
+    both(step, by)
+    both(lambda: (call(*leaves[:3], leaves[3].detach()).detach(),), by)
     with torch.no_grad():
-        both(lambda: (call(*leaves),))
+        both(lambda: (call(*leaves),), by)
+    with torch.inference_mode():
+        both(lambda: (call(*leaves),), by)
+        both(lambda: (call(*[x.clone() for x in leaves]),), by)
     # a gradient in another layout, saved-tensor hooks, and a recorded backward
     o = call(*leaves)
     want = torch.autograd.grad(o, leaves, go, retain_graph=True)
@@ -83,8 +108,12 @@ def test_decode_and_prefill(hq, hkv, page):
     t32 = lambda *x: torch.tensor(x, dtype=torch.int32, device="cuda")
     for lq in (1, 7):
         q, r = randn(bsz, lq, hq, d, seed=3), randn(bsz, lq, hq, d, seed=4)
-        for args in (dict(), dict(seqused_k=t32(300, 7, 320)), dict(window_size=40, scale=0.2), dict(window_size=(40, 0))):
-            both(lambda: (plx.parallax_attn_with_kvcache(q, r, k, v, page_table=table, **args),))
+        call = lambda **args: (plx.parallax_attn_with_kvcache(q, r, k, v, page_table=table, **args),)
+        for args in (dict(), dict(seqused_k=t32(300, 7, 320)), dict(window_size=40, scale=0.2)):
+            both(lambda: call(**args), {"attend"})
+        both(lambda: call(window_size=(40, 0)), set())
+        with torch.inference_mode():
+            both(lambda: call(seqused_k=t32(300, 7, 320)), {"attend"})
         for bad in (t32(0, 7, 320), t32(1, 321, 7), t32(-5, 10 ** 9, 9)):
             with pytest.raises(ValueError, match="seqused_k"):
                 plx.parallax_attn_with_kvcache(q, r, k, v, page_table=table, seqused_k=bad)
@@ -94,7 +123,9 @@ def test_decode_and_prefill(hq, hkv, page):
     if not page:
         q, r = randn(bsz, 1, hq, d, seed=3), randn(bsz, 1, hq, d, seed=4)
         for args in (dict(), dict(cache_start=t32(0, 5, 320)), dict(seqused_k=t32(300, 7, 320), window_size_left=33), dict(qk_scale=0.3)):
-            both(lambda: (plx.parallax_decode(q, r, k, v, **args),))
+            both(lambda: (plx.parallax_decode(q, r, k, v, **args),), {"decode"})
+        with torch.inference_mode():
+            both(lambda: (plx.parallax_decode(q, r, k, v),), {"decode"})
 
 
 def test_what_is_left_to_the_python_path():
