@@ -286,7 +286,7 @@ __device__ __forceinline__ SplitPlan plan_even(const DecodeArgs &a, int b, int p
 // longest row set the time while the warps of the others idle.  There the slots are dealt out by length: the
 // smallest part size for which the parts of all rows still fit into the slots.  Lane l looks after rows l, l + 32,
 // ..: up to kBalancedRows rows.  `cap`: the most parts of a row that the merge takes.
-// Not so where the longest row is within a.balanced quarters of the mean (see balance_from): dealing out costs the
+// Not so where the longest row is within a.balanced sixteenths of the mean (see balance_from): dealing out costs the
 // search and leaves parts and rows that no longer fall together with CTAs.
 template <int G>
 __device__ __forceinline__ SplitPlan plan_slot(const DecodeArgs &a, int slot, int lane, int cap) {
@@ -307,7 +307,7 @@ __device__ __forceinline__ SplitPlan plan_slot(const DecodeArgs &a, int slot, in
     }
     sum = __reduce_add_sync(0xffffffffu, sum);
     most = __reduce_max_sync(0xffffffffu, most);
-    if (4 * static_cast<int64_t>(most) * a.batch <= static_cast<int64_t>(a.balanced) * sum) {
+    if (16 * static_cast<int64_t>(most) * a.batch <= static_cast<int64_t>(a.balanced) * sum) {
         p.b = slot / a.n_splits;
         int lo = 0, len = 0;
 #pragma unroll
@@ -1331,12 +1331,12 @@ bool decode_fused_exchange_supported(const DecodeArgs &a) {
     return a.n_rep == 1 && a.n_splits >= 2 && !decode_split_groups(a);
 }
 
-// From which ratio of the longest row to the mean, in quarters, the splits are dealt out by length; 0: never.
+// From which ratio of the longest row to the mean, in sixteenths, the splits are dealt out by length; 0: never.
 // Not for split groups, whose CTAs belong to one row, and not for a key-sharded launch, whose fused and two-launch forms
 // have to cut the keys alike.
-// Where the parts are large and the launch is bound by HBM, dealing out pays from a small skew on (5): rows from T down
+// Where the parts are large and the launch is bound by HBM, dealing out pays from a small skew on (17): rows from T down
 // to T / 3 keys (a skew of 1.5), even parts against dealt out: 32 rows of 4000, 8 : 8 heads, 76 -> 70 us; 16 rows of 8192,
-// 32 : 8 heads, 94 -> 76.  Elsewhere only from a skew of 2 on (8), since it costs the plan and, with grouped heads, the
+// 32 : 8 heads, 94 -> 76; two rows of 29184 and 19456 (1.2), 64 -> 55.  Elsewhere only from a skew of 2 on (32), since it costs the plan and, with grouped heads, the
 // merge inside a CTA: 64 rows of 512, 16 : 2 heads, 11.6 -> 21.0 us; 128 rows of 1000, 8 : 8 heads, 80 -> 87; but where one
 // row is ten times the others, those 128 rows took 71 us in even parts against 27.
 // `part`, the keys of an even part times head_dim: the lines lie between 250 and 512 keys at head_dim 128 (512 and 1024 at
@@ -1350,11 +1350,11 @@ static int balance_from(const DecodeArgs &a, int head_dim) {
     const int64_t n_keys = a.window >= 0 && a.window < a.cache_len ? a.window : a.cache_len, part = n_keys / a.n_splits * head_dim;
     if (a.n_rep > 1) {
         const bool rows_end_with_ctas = a.n_splits % kGqaWarps == 0 || kGqaWarps % a.n_splits == 0;
-        return part < 384 * 128 && rows_end_with_ctas ? 8 : 5;
+        return part < 384 * 128 && rows_end_with_ctas ? 32 : 17;
     }
     if (part < 64 * 128) return 0;
     const bool one_wave = static_cast<int64_t>(a.batch) * a.heads_q * a.n_splits <= 16 * static_cast<int64_t>(tma_free_sm_count());
-    return part < 100 * 128 || a.n_splits < 4 || !one_wave ? 8 : 5;
+    return part < 100 * 128 || a.n_splits < 4 || !one_wave ? 32 : 17;
 }
 
 int launch_decode(const DecodeArgs &problem, int dtype, int head_dim, cudaStream_t stream) {
