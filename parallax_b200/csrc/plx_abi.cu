@@ -382,13 +382,15 @@ int plx_decode_choose_splits_gqa(int32_t batch, int32_t heads_q, int32_t heads_k
     }
     // A warp sweeps whole tiles of 16 keys, so a part of 65 keys costs as much as one of 80 and leaves the last warps
     // without any: where that wastes more than 8 %, cut at a tile boundary instead if the warps still fit into as many
-    // waves.  (B = 1, 8192 keys, 32 : 8 heads, 128 parts of 64 keys for 126 of 65: 16.45 -> 16.01 us; a waste of 2 %
-    // is not worth more parts, 3 rows of 17104 keys in 90 parts took 35.6 us against 34.0 in 84.)
+    // waves and the parts of a row into whole CTAs.  (B = 1, 8192 keys, 32 : 8 heads: 126 parts would be swept as 103 of 80
+    // keys and 23 of none, waste 23 %; 128 parts of 64 keys, 16.4 -> 16.0 us.  Where rows then end inside a CTA it does not
+    // pay: B = 2, 5200 keys, 16 %, 65 parts for 63 17.0 -> 20.8 us; B = 8, 1300 keys, 18 %, 17 for 16 16.4 -> 18.6.  Nor for a
+    // waste of 2 %: 3 rows of 17104 keys in 90 parts took 35.6 us against 34.0 in 84.)
     const int64_t waves = (units * best + resident - 1) / resident, part = n_keys / best / 16 * 16;
     const int64_t swept = ((n_keys + best - 1) / best + 15) / 16 * 16;
     if (part >= 64 && 100 * swept * best > 108 * static_cast<int64_t>(n_keys)) {
         const int64_t even = (n_keys + part - 1) / part;
-        if (even <= cap && units * even <= waves * resident) best = even;
+        if (even <= cap && even % kDecodeGqaWarps == 0 && units * even <= waves * resident) best = even;
     }
     return static_cast<int>(best);
 }

@@ -121,3 +121,12 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_cabi, "LIB_PATH", str(tmp_path / "nope.so"))
     with pytest.raises(RuntimeError, match="no CPU or PyTorch fallback"):
         _cabi.lib()
+
+
+def test_grouped_splits_move_to_a_tile_boundary_where_rows_end_with_ctas():
+    """Parts of 65 keys are swept as 80: one row gets 128 parts of 64 keys in place of 126.  Two rows of 65 parts, or eight of
+    17, would end inside a CTA of another row; those keep the parts that fill the wave."""
+    splits = _cabi.lib().plx_decode_choose_splits_gqa
+    assert splits(1, 32, 8, 8192, 148) == 128
+    assert splits(2, 32, 8, 5200, 148) == 63 and splits(2, 32, 8, 5400, 148) == 63
+    assert splits(8, 32, 8, 1300, 148) == 16 and splits(3, 32, 8, 6200, 148) == 42
