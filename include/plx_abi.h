@@ -151,8 +151,9 @@ int plx_train_bwd_stages(const plx_train_problem *p, int32_t stages, const void 
  * more than PLX_DECODE_GROUP_MIN splits the merge has two levels: the last warp
  * of every group of PLX_DECODE_GROUP splits merges its group, the last group the
  * group results.  Grouped-query shapes merge the eight splits of a CTA in shared memory
- * first.  With seqused_k or cache_start the batch * n_splits splits of a head are dealt
- * out to the rows by their lengths (up to 128 rows).
+ * first.  With seqused_k or cache_start, where the lengths differ by enough, the
+ * batch * n_splits splits of a head are dealt out to the rows by their lengths (up to
+ * 128 rows).
  *
  * Workspace: plx_decode_workspace_bytes() bytes, ZERO-FILLED ONCE by the caller
  * before its first use (it holds arrival counters that the kernel resets itself).

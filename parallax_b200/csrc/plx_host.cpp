@@ -2,11 +2,13 @@
 // node and the call into libplx_sm100.so.
 //
 // Everything here is a SHORT CUT of the Python path (train.py / decode.py over the torch custom ops of ops.py),
-// which stays the definition of the API: each function returns None, having enqueued nothing that shows, for any
+// which stays the definition of the API: each function returns None, with nothing enqueued that shows, for any
 // call that is not plainly an eager one on well-formed CUDA tensors -- a tensor subclass, a torch function or
-// dispatch mode, functorch or forward-mode differentiation, tracing, a stream that is being captured, shapes,
-// strides or types that need a copy or an error message, a device error waiting to be reported -- and the caller
-// then takes the Python path, which handles it or raises.
+// dispatch mode, functorch or forward-mode differentiation, tracing, shapes, strides or types that need a copy or an
+// error message -- and the caller then takes the Python path, which handles it or raises.  decode, extend and stage also
+// leave a stream that is being captured to it; train and extend a device error waiting to be reported (the ops
+// of a single-token step do not look at it either).  decode and extend find a length out of range after their launch,
+// whose result is then dropped.
 //
 // Measured per call, Python path -> here: decode at B = 1, H = 8, 1024 keys 52 -> 6.4 us; training forward and backward
 // at B = 2, H = 8, L = 1024 303 -> 100 us (24 us of host time forward; 70 us backward, 28 of them in Train::backward).

@@ -39,7 +39,7 @@ void count_launch();
 int launch_train_fwd_mma(const TrainArgs &a, int dtype, int head_dim, cudaStream_t stream);
 int launch_train_bwd_mma(const TrainArgs &a, int dtype, int head_dim, int stages, cudaStream_t stream);
 
-// tcgen05 + TMEM + TMA forward (head_dim 128, no sliding window); `supported` decides per problem
+// tcgen05 + TMEM + TMA forward; `supported` decides per problem
 bool train_fwd_sm100_supported(const TrainArgs &a, int head_dim);
 int launch_train_fwd_sm100(const TrainArgs &a, int dtype, int head_dim, cudaStream_t stream);
 // the same kernel for several query rows per sequence against a dense or paged KV cache (writes `o` only)
