@@ -100,8 +100,7 @@ int plx_train_fwd(const plx_train_problem *p, const void *q, const void *r, cons
  * the page stride of a pool of n_pages pages of page_size keys (a power of two) and
  * len_k <= pages_per_seq * page_size; entries past a row's active length are not read.
  * Keys past the active length never reach the output.  Writes o only.
- * A page number outside the pool below a row's active length is reported through
- * plx_device_error (site 30) and gives NaN in the rows that see its keys.
+ * The keys of a page number outside the pool below a row's active length read as zeros.
  * PLX_ERR_UNSUPPORTED (nothing enqueued): window_left 0, qk_scale <= 0, a page of fewer
  * than 8 keys, a zero k / v stride; gather the pages and call plx_train_fwd per row then.
  * (L_q > 1 and page_table are named but not implemented upstream

@@ -189,8 +189,6 @@ def describe_error(word: int) -> str:
     site = word >> 8
     if 40 <= site < 40 + EXCHANGE_MAX_RANKS:
         return f"the peer-memory exchange gave up waiting for the records of rank {site - 40}"
-    if site == 30:
-        return "a page_table of a prefill call holds a page number outside the pool"
     return f"a pipelined kernel gave up a bounded wait at site {site}"
 
 

@@ -62,7 +62,6 @@ constexpr uint32_t kQPanel = kBM * 128;       // bytes of one 64-channel panel o
 constexpr uint32_t kKVPanel = kBN * 128;
 constexpr uint32_t kTmemCols = 512;
 constexpr float kRescaleThreshold = 8.f;
-constexpr int kStrayPage = (30 << 8) | 1;     // error report: a page number outside the pool
 constexpr int kMinPage = 8;                   // smallest page a tile can be copied from: boxes start on 1024-byte boundaries (8 rows)
 
 template <typename T>
@@ -100,7 +99,7 @@ struct Smem {
 // One unit of work: a 128-row query tile of one (batch, q head).
 struct Item {
     int bos, nq, nk, r0, b, h, hk, off, t_lo, n_tiles;   // key tiles t_lo .. t_lo + n_tiles - 1
-    int valid, clamped;   // clamped (EXT): the row's active length was out of range
+    int valid, pad;
 };
 
 // Work item `idx` of the launch.  Items are ordered (batch, head)-major so that CTAs running at the
@@ -113,7 +112,7 @@ __device__ __forceinline__ Item get_item(const TrainArgs &a, int idx, int n_rt, 
     int bh = idx / n_rt, k = idx % n_rt;
     if (DYN) longest_first(idx, n_rt, a.batch * a.heads_q, group, bh, k);
     const int tile_id = DYN ? n_rt - 1 - k : (k & 1) ? (k >> 1) : n_rt - 1 - (k >> 1);
-    it.clamped = 0;
+    it.pad = 0;
     Seq s;
     int tis = 0;
     it.valid = locate_tile(a, tile_id, kBM, s, tis);
@@ -124,11 +123,7 @@ __device__ __forceinline__ Item get_item(const TrainArgs &a, int idx, int n_rt, 
     if (it.valid && it.r0 >= it.nq) it.valid = false;
     it.b = bh / a.heads_q;
     // a row's own active length, kept inside what the tensor map (or the page table) covers
-    if (EXT && a.seqused) {
-        const int used = __ldg(a.seqused + it.b);
-        it.nk = min(max(used, it.nq), a.len_k);
-        it.clamped = used != it.nk;
-    }
+    if (EXT && a.seqused) it.nk = min(max(__ldg(a.seqused + it.b), it.nq), a.len_k);
     it.h = bh % a.heads_q;
     it.hk = it.h / a.n_rep;
     it.off = it.nk - it.nq;
@@ -309,25 +304,11 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
                     }
                     ok = mbar_wait(bar(empty0 + s), ph ^ 1, err, is_k ? 2 : 3);
                     if (!ok) break;
-                    // (checked only here: in front of the wait the check would wait for the loads; 213 -> 265 us for 4 rows of
-                    // 512 tokens against 2048 to 4096 keys in pages of 64)
-                    uint32_t strays = 0;   // boxes whose page lies outside the pool
-                    if (EXT && a.page_table) {
-#pragma unroll
-                        for (int i = 0; i < kMaxBoxes; ++i)
-                            if (static_cast<uint32_t>(page[i]) >= static_cast<uint32_t>(a.n_pages)) {
-                                strays |= 1u << i;
-                                page[i] = 0;
-                            }
-                        // (a length that the caller is yet to find out of range may lead past a row's pages: no report)
-                        if (strays != 0 && is_k && !it.clamped) report_error(sink, kStrayPage);
-                    }
                     const uint32_t dst = tiles + s * kKVBytes;
                     // A tile that reaches past the row's active length inside the cache: what lies there must not
                     // be seen (0 * NaN), so its rows are zeroed once the copy has landed, before the tile is handed
-                    // over.  (Past the end of a tensor map the copy itself fills zeros.)  So are the values of a page
-                    // outside the pool replaced by NaN: no row that sees them gets a result that looks valid.
-                    const bool tail = EXT && ((key0 + kBN > it.nk && (a.page_table || it.nk < a.len_k)) || strays != 0);
+                    // over.  (Past the end of a tensor map the copy itself fills zeros.)
+                    const bool tail = EXT && key0 + kBN > it.nk && (a.page_table || it.nk < a.len_k);
                     const uint32_t full = bar(tail ? L::kTail + (is_k ? 0 : 1) : full0 + s);
                     if (EXT && a.page_table) {
                         const int n_boxes = min(kBN >> box_shift, (it.nk - key0 + (1 << box_shift) - 1) >> box_shift);
@@ -348,16 +329,11 @@ fwd_sm100_kernel(const TrainArgs a, const __grid_constant__ CUtensorMap tm_q, co
                         ok = mbar_wait(full, n_tails & 1, err, is_k ? 17 : 18);
                         if (!ok) break;
                         ++n_tails;
-                        auto fill = [&](int row, uint32_t x) {
+                        for (int row = it.nk - key0; row < kBN; ++row)
                             for (int pn = 0; pn < L::kPanels; ++pn)
 #pragma unroll
                                 for (int c = 0; c < 8; ++c)
-                                    asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};\n" ::"r"(dst + pn * kKVPanel + row * 128 + c * 16), "r"(x) : "memory");
-                        };
-                        if (!is_k && strays != 0)
-                            for (int row = 0; row < min(kBN, it.nk - key0); ++row)
-                                if ((strays >> (row >> box_shift)) & 1u) fill(row, 0x7fff7fffu);   // NaN in both types
-                        for (int row = it.nk - key0; row < kBN; ++row) fill(row, 0u);
+                                    asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};\n" ::"r"(dst + pn * kKVPanel + row * 128 + c * 16), "r"(0u) : "memory");
                         fence_proxy_async();
                         mbar_arrive(bar(full0 + s));
                     }

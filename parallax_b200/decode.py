@@ -197,9 +197,9 @@ def parallax_attn_with_kvcache(q: torch.Tensor, r: torch.Tensor, k_cache: torch.
       ``j % page_size`` of block ``page_table[b, j // page_size]``.  The logical cache length is
       ``max_num_blocks * page_size``; pass ``seqused_k`` for the active lengths -- only table entries
       below a row's active length are read, so the rest of the row may hold anything.  A page number below that
-      length but outside the pool cannot be seen by the host without waiting for the device: with ``L_q > 1``
-      the queries of the row that see its keys (at least) become NaN and the next training or prefill call on the
-      device raises :class:`PlxError`; the single-token sweep reads the last page of the pool in its place.
+      length but outside the pool is not noticed (the host cannot see it without waiting for the device) and
+      the row's result means nothing: with ``L_q > 1`` its keys read as zeros, the single-token sweep reads the last
+      page of the pool in its place.
     * ``q`` / ``r`` with ``L_q > 1`` rows ``(B, L_q, H, D)`` -- prefill / extend: the ``L_q`` queries are
       the LAST ``L_q`` positions of the sequence (row ``i`` sees keys up to ``L - L_q + i``), as in
       ``flash_attn_with_kvcache``.  This runs the training forward kernel (tensor cores), not the decode

@@ -682,39 +682,6 @@ def test_extend_in_one_launch_is_the_launch_per_row(case):
     assert torch.equal(plx.parallax_attn_with_kvcache(mine, r, k, v, out=mine, **args), got)   # written over an input
 
 
-@pytest.mark.parametrize("page", [8, 16, 64, 256])
-def test_prefill_reports_a_page_outside_the_pool(page):
-    """Such a row gets NaN and the next call raises; the other rows are what they are without it, and table entries past
-    a row's active length, or behind a length that is refused, are nobody's business."""
-    hq, hkv, lq, d, lens, bad_row = 4, 2, 20, 64, (700, 600, 530), 1
-    mk = lambda *s, seed: seeded_bf16(s, seed).cuda()
-    per_row = 1024 // page
-    pool = 3 * per_row
-    q, r, k, v = mk(3, lq, hq, d, seed=1), mk(3, lq, hq, d, seed=2), mk(pool, page, hkv, d, seed=3), mk(pool, page, hkv, d, seed=4)
-    table = torch.randperm(pool, generator=torch.Generator().manual_seed(5)).int().view(3, per_row).cuda()
-    su = torch.tensor(lens, dtype=torch.int32, device="cuda")
-    call = lambda t, n=su: plx.parallax_attn_with_kvcache(q, r, k, v, page_table=t, seqused_k=n)
-    want = call(table)
-    for at, number in ((0, -1), ((lens[bad_row] - 1) // page, pool), (300 // page, 10 ** 9)):
-        broken = table.clone()
-        broken[bad_row, at] = number
-        got = call(broken)
-        torch.cuda.synchronize()
-        assert torch.isnan(got[bad_row].float()).all()
-        assert all(torch.equal(got[b], want[b]) for b in range(3) if b != bad_row)
-        with pytest.raises(_cabi.PlxError, match="page"):
-            call(table)
-        assert _cabi.device_error(clear=True) == (30 << 8) | 1
-        assert torch.equal(call(table), want)
-    unused = table.clone()
-    for b, n in enumerate(lens):
-        unused[b, -(-n // page):] = -7
-    assert torch.equal(call(unused), want)
-    with pytest.raises(ValueError, match="seqused_k"):
-        call(unused, torch.tensor([700, 1025, 530], dtype=torch.int32, device="cuda"))
-    assert torch.equal(call(unused), want) and _cabi.device_error() == 0
-
-
 @pytest.mark.parametrize("case", [
     # hq, hkv, lq, active lengths, cache, head_dim
     (4, 2, 70, (150, 150), 230, 128),        # one launch on a slice of the cache
