@@ -17,20 +17,21 @@
 // Pipeline per CTA (12 warps):
 //   warp 0      TMA producer (resident tiles once per item, streamed tiles through an NS-deep ring)
 //   warp 1      TMEM allocation + the lane that issues the score products
-//   warp 2      the lane that issues the output products          (warp 3 idles)
-//   warps 4-11  element-wise: warp 4 + w works on TMEM lane quarter w % 4 (128 rows of the M tile, one
-//               per thread) and column group w / 4 (32 of the 64 streamed columns; with sixteen such
-//               warps, a build option, 16).  A thread reads its columns of the three score tiles from
-//               TMEM, releases them at once (so the next tile's scores are computed while it works),
+//   warp 2      the lane that issues the output products
+//   warp 3      dk/dv: the row statistics of the streamed tiles
+//   warps 4-11  element-wise: warp 4 + w works on TMEM lane quarter w % 4.  At head_dim 128 on column
+//               group w / 4 (32 of the 64 streamed columns, one row per thread): a thread reads its columns of the three
+//               score tiles from TMEM, releases them at once (so the next tile's scores are computed while it works),
 //               writes gl / gu / -W as 16-bit values into shared memory in the 128-byte-swizzled K-major
-//               layout, and the MMA lane consumes them as the A operand of the output products.
+//               layout, and the MMA lane consumes them as the A operand of the output products.  (At 64: see Plan.)
 //               The arithmetic of a tile is ONE basic block (tiles that need a mask run a second copy
 //               of the loop): measured with every MMA removed, the element-wise chain (TMEM load ->
 //               arithmetic -> shared-memory store -> hand-over), not the tensor pipe, sets the pace,
 //               and the independent column pairs of a thread must be free to interleave.
 //
-// TMEM columns: acc0 [0,128) (dQ | dK), acc1 [128,256) (dR | dV), S1 [256,320), S2 [320,384), A [384,448),
+// TMEM columns at head_dim 128: acc0 [0,128) (dQ | dK), acc1 [128,256) (dR | dV), S1 [256,320), S2 [320,384), A [384,448),
 // and at [448,512) the M-side tile that is the A operand of score products: k in DKV mode (S1^T, S2^T), dO in DQR mode (A).
+// At 64: acc0 [0,64), acc1 [64,128), the two score buffers at 128 and 320.
 #include <cuda.h>
 
 #include <climits>
@@ -50,9 +51,7 @@ using namespace sm100;
 namespace {
 
 constexpr int kModeDQR = 0, kModeDKV = 1;
-#ifndef PLX_BWD_EW_WARPS
-#define PLX_BWD_EW_WARPS 8    // element-wise warps per CTA (8 or 16)
-#endif
+constexpr int kEwWarps = 8;                    // element-wise warps per CTA: two per lane quarter of tensor memory
 constexpr int kBM = 128, kBN = 64;
 constexpr uint32_t kResPanel = kBM * 128;      // one 64-channel panel of a resident tile: [128][128 B]
 constexpr uint32_t kStrPanel = kBN * 128;      // one 64-channel panel of a streamed tile: [64][128 B]
@@ -73,38 +72,67 @@ struct Fmt<__half> {
 };
 
 constexpr uint32_t kStatBytes = kBN * 16;      // four planes of 64 floats: -mL, -(1 + bart), b, (b - t) * scale
-constexpr int kStatStages = 2;
-constexpr int kStatWriters = 64;               // one thread per row of the streamed tile
 
-// DQR keeps q, r, dO of its rows in shared memory.  DKV keeps only v there: its k tile is the A
-// operand of two of the three score products and lives in tensor memory (64 columns), which frees
-// the shared memory for a third stage of streamed tiles.
+// How a kernel is laid out, by head_dim.
+//
+// 128: the accumulators take half of the tensor memory, which leaves room for one score buffer {S1, S2, A} and for the
+// M-side tile that is the A operand of two (DKV: k) or one (DQR: dO) of the score products (kMTile); that frees the
+// shared memory for another stage of streamed tiles.  All element-wise warps work on every tile, 32 columns per thread,
+// and leave gl / gu / -W as 16-bit tiles in shared memory.
+//
+// 64 (kTwo): two score buffers, and two groups of four element-wise warps that take the streamed tiles in turn, so that
+// one group's arithmetic runs under the waits and the hand-overs of the other.  gl / gu / -W go IN PLACE over the scores they
+// came from (16-bit pairs, the first 32 of 64 columns), as A operands from tensor memory: a buffer is free for the
+// scores of tile g + 2 when the output products of tile g have completed.
+// Bound by the latency of the element-wise warps, two per scheduler.  B=8, H=16, L=4096, fp16, us: dk/dv 1330 -> 1066,
+// dq/dr 875 -> 755.  Two groups alone, with the tiles in shared memory: 1354 and 750, and 32768 tokens in sequences of 1 to
+// 256 dq/dr 205 against 191 (before 223).  Two groups at 128 (one score buffer, S1 and S2 of a whole tile read at once into
+// 224 registers a thread) changed nothing, 1498 -> 1494: a tile then lives 7700 clocks and the ring has three stages;
+// short sequences were slower (dk/dv 239 -> 260).
+template <int D, int MODE>
+struct Plan {
+    static constexpr bool kTwo = D == 64, kMTile = D == 128;
+    static constexpr int kGroups = kTwo ? 2 : 1;                            // of element-wise warps, = score buffers
+    static constexpr int kStatStages = kTwo ? 4 : 2;                        // tiles' row statistics (DKV): what is left at head_dim 128
+    // stages of streamed tiles: what the shared memory allows at 128; six at 64 (four: dq/dr 4 %, dk/dv 1 % slower, measured
+    // before the two groups)
+    static constexpr int NS = kTwo ? 6 : MODE == kModeDQR ? 4 : 3;
+};
+
 // D = head dim (64 or 128): tiles are D / 64 panels.
-template <int D, int MODE, int NS>
+template <int D, int MODE>
 struct Smem {
+    using P = Plan<D, MODE>;
+    static constexpr int NS = P::NS, kStatStages = P::kStatStages;
     static constexpr int kPanels = D / 64;
     static constexpr uint32_t kResBytes = kPanels * kResPanel;   // resident tile (128 rows)
     static constexpr uint32_t kStrBytes = kPanels * kStrPanel;   // streamed tile (64 rows)
-    static constexpr int kNRes = MODE == kModeDQR ? 2 : 1;   // DQR: q, r (its dO tile is in tensor memory); DKV: v
+    static constexpr int kNRes = (MODE == kModeDQR ? 2 : 1) + (P::kMTile ? 0 : 1);   // DQR: q, r (, dO); DKV: v (, k)
     static constexpr int kNStr = MODE == kModeDQR ? 2 : 3;
-    static constexpr int kNG = MODE == kModeDQR ? 2 : 3;
+    static constexpr int kNG = P::kTwo ? 0 : MODE == kModeDQR ? 2 : 3;
     static constexpr uint32_t kRes = 0;
     static constexpr uint32_t kStr = kNRes * kResBytes;
+    // A stage.  DQR: k, v.  DKV: the panels of q and r in turn (q0 r0 q1 r1: a panel pair is the B operand of ONE score
+    // product of 128 columns, 64 rows of q beside 64 of r), then dO.
     static constexpr uint32_t kStage = kNStr * kStrBytes;
     static constexpr uint32_t kG = kStr + NS * kStage;
     static constexpr uint32_t kStats = kG + kNG * kGBytes;
     static constexpr uint32_t kBars = kStats + (MODE == kModeDKV ? kStatStages * kStatBytes : 0);
-    // per streamed tile: NFull / NEmpty (ring), SFull / SFree (score columns), GFull / GFree (G tiles), StatFull;
-    // per work item: XFull / XEmpty (resident tiles), KReady (M-side tile in tensor memory), AccDone / AccFree
-    static constexpr int kXFull = 0, kXEmpty = 1, kNFull = 2, kNEmpty = 2 + NS, kSFull = 2 + 2 * NS, kSFree = kSFull + 1,
-                         kGFull = kSFull + 2, kGFree = kSFull + 3, kAccDone = kSFull + 4, kAccFree = kSFull + 5,
-                         kKReady = kSFull + 6, kStatFull = kSFull + 7, kItemFull = kStatFull + kStatStages,
-                         kItemEmpty = kItemFull + kItemSlots, kClcFull = kItemEmpty + kItemSlots, kNumBars = kClcFull + 1;
+    // per streamed tile: NFull / NEmpty (ring), SFull / SFree (score columns), GFull / GFree (G tiles), the latter four in
+    // pairs for even and odd tiles where two groups take them in turn (a group waits for every second tile, so a phase has to
+    // be as long as two), StatFull / StatEmpty (DKV); per work item: XFull / XEmpty (resident tiles), KReady (M-side tile in tensor memory),
+    // AccDone / AccFree
+    static constexpr int kXFull = 0, kXEmpty = 1, kNFull = 2, kNEmpty = 2 + NS, kSFull = 2 + 2 * NS, kSFree = kSFull + 2,
+                         kGFull = kSFull + 4, kGFree = kSFull + 6, kAccDone = kSFull + 8, kAccFree = kSFull + 9,
+                         kKReady = kSFull + 10, kStatFull = kSFull + 11, kStatEmpty = kStatFull + kStatStages,
+                         kItemFull = kStatEmpty + kStatStages, kItemEmpty = kItemFull + kItemSlots,
+                         kClcFull = kItemEmpty + kItemSlots, kNumBars = kClcFull + 1;
     static constexpr uint32_t kItems = (kBars + 8 * kNumBars + 15u) & ~15u;      // item ring, then the launch-control answer
     static constexpr uint32_t kClc = kItems + 4 * kItemWords * kItemSlots;
     static constexpr uint32_t kTmemSlot = kClc + 16;
     static constexpr uint32_t kAbort = kTmemSlot + 8;
     static constexpr uint32_t kBytes = kTmemSlot + 16;   // the dynamic shared memory must start 1024-byte aligned
+    static_assert(kBytes <= 227 * 1024, "more than a CTA may have");
     static constexpr uint32_t kStageTx = kStage;
 };
 
@@ -177,39 +205,45 @@ __device__ __forceinline__ int item_index(int n, int chunk_shift) {
 // accumulators, and the hand-overs for those are arranged so that the loads, the tensor-memory tile and
 // the first score products of the next item are under way while the element-wise warps write out the
 // accumulators of the current one.  TMEM allocation, barrier set-up and launch latency are paid once.
-template <typename T, int D, int MODE, int NS, int EW>
-__global__ void __launch_bounds__((4 + EW) * 32, 1)
+template <typename T, int D, int MODE>
+__global__ void __launch_bounds__((4 + kEwWarps) * 32, 1)
 bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorMap tm_q,
                  const __grid_constant__ CUtensorMap tm_r, const __grid_constant__ CUtensorMap tm_go,
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const ErrSink sink,
                  int n_mt, int n_items, int chunk_shift, int group) {
-    using L = Smem<D, MODE, NS>;
-    constexpr bool DQR = MODE == kModeDQR;
+    using P = Plan<D, MODE>;
+    using L = Smem<D, MODE>;
+    constexpr int NS = P::NS, kStatStages = P::kStatStages;
+    constexpr bool DQR = MODE == kModeDQR, kMTile = P::kMTile;
     constexpr uint32_t kResBytes = L::kResBytes, kStrBytes = L::kStrBytes;
-    constexpr int CG = EW / 4;        // element-wise warps per TMEM lane quarter = column groups of a streamed tile
-    constexpr int CPT = kBN / CG;     // columns of a streamed tile per element-wise thread
-    constexpr int kEwThreads = EW * 32;
-    static_assert(EW == 8 || EW == 16, "two or four element-wise warps per lane quarter");
+    constexpr int GR = P::kGroups, CH = 32;      // columns of a tile that a thread holds at once
     extern __shared__ __align__(1024) unsigned char smem_raw[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     const uint32_t base = smem_u32(smem_raw);
     auto res = [&](int i) -> uint32_t { return base + L::kRes + i * kResBytes; };
-    auto str = [&](int s, int i) -> uint32_t { return base + L::kStr + s * L::kStage + i * kStrBytes; };
+    // streamed tile i of stage s (see Smem)
+    auto str = [&](int s, int i) -> uint32_t { return base + L::kStr + s * L::kStage + (DQR || i == 2 ? i * kStrBytes : i * kStrPanel); };
+    auto str_panel = [](int i) -> uint32_t { return DQR || i == 2 ? kStrPanel : 2 * kStrPanel; };   // distance of its panels
     auto gt = [&](int i) -> uint32_t { return base + L::kG + i * kGBytes; };
     auto bar = [&](int i) -> uint32_t { return base + L::kBars + 8u * i; };
+    // barrier and phase of tile g where there is one per group
+    auto tile_bar = [&](int i, int g) -> uint32_t { return bar(i + (GR == 2 ? g & 1 : 0)); };
+    auto tile_phase = [](int g) -> uint32_t { return (GR == 2 ? g >> 1 : g) & 1; };
     const uint32_t tmem_slot = base + L::kTmemSlot;
     const WaitCtx err{sink, base + L::kAbort};
 
     if (threadIdx.x == 0) {
         asm volatile("st.shared.u32 [%0], %1;\n" ::"r"(err.abort_flag), "r"(0u) : "memory");
         for (int i = 0; i < L::kNumBars; ++i) {
-            // arrivals from all element-wise threads
-            const bool all_ew = i == L::kSFree || i == L::kGFull || i == L::kKReady || i == L::kAccFree;
-            const bool stat = i >= L::kStatFull && i < L::kStatFull + kStatStages;
-            // every role that reads the items: two MMA issuers and the element-wise warps
+            // arrivals from the element-wise threads: of the tile's group, or all
+            const bool group_ew = i == L::kSFree || i == L::kSFree + 1 || i == L::kGFull || i == L::kGFull + 1 ||
+                                  (i >= L::kStatEmpty && i < L::kStatEmpty + kStatStages);
+            const bool stat_full = i >= L::kStatFull && i < L::kStatFull + kStatStages;      // from the statistics warp
+            const bool all_ew = i == L::kKReady || i == L::kAccFree;
+            // every role that reads the items: two MMA issuers, the element-wise warps and (DKV) the statistics warp
             const bool item_empty = i >= L::kItemEmpty && i < L::kItemEmpty + kItemSlots;
-            mbar_init(bar(i), all_ew ? kEwThreads : stat ? kStatWriters : item_empty ? 2 + EW : 1);
+            mbar_init(bar(i), group_ew ? 32 * kEwWarps / GR : all_ew ? 32 * kEwWarps : stat_full ? 32 : item_empty ? 2 + kEwWarps + (DQR ? 0 : 1) : 1);
         }
         fence_barrier_init();
         prefetch_tensormap(&tm_q);
@@ -228,8 +262,9 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
     tc_fence_after();
     uint32_t tmem_base;
     asm volatile("ld.shared.u32 %0, [%1];\n" : "=r"(tmem_base) : "r"(tmem_slot));
-    const uint32_t tAcc0 = tmem_base, tAcc1 = tmem_base + 128, tS = tmem_base + 256;  // S1, S2, A at tS + 0 / 64 / 128
-    const uint32_t tK = tmem_base + 448;                                              // the M-side tile as an A operand
+    const uint32_t tAcc0 = tmem_base, tAcc1 = tmem_base + D;
+    auto tS = [&](int sb) -> uint32_t { return tmem_base + 2 * D + 192 * sb; };       // S1, S2, A at + 0 / 64 / 128
+    const uint32_t tK = tmem_base + 448;                                              // kMTile: the M-side tile as an A operand
     const bool misaligned = cta_aborted(err);
     // Set-up may run under the end of the kernel before.  dk/dv waits here for the row statistics, then lets dq/dr
     // start; dq/dr waits for dk/dv at its end, so that whatever follows on the stream follows both.
@@ -316,13 +351,15 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
                 mbar_expect_tx(bar(L::kXFull), L::kNRes * kResBytes);
                 ++x_issued;
                 if (DQR) {
-                    const CUtensorMap *maps[2] = {&tm_q, &tm_r};
-                    for (int j = 0; j < 2; ++j)
+                    const CUtensorMap *maps[3] = {&tm_q, &tm_r, &tm_go};
+                    for (int j = 0; j < L::kNRes; ++j)
                         for (int pn = 0; pn < L::kPanels; ++pn)
                             tma_load_4d(res(j) + pn * kResPanel, maps[j], bar(L::kXFull), 64 * pn, it.bos + it.m0, it.hy, it.b);
                 } else {
-                    for (int pn = 0; pn < L::kPanels; ++pn)
-                        tma_load_4d(res(0) + pn * kResPanel, &tm_v, bar(L::kXFull), 64 * pn, it.bos + it.m0, it.hk, it.b);
+                    const CUtensorMap *maps[2] = {&tm_v, &tm_k};
+                    for (int j = 0; j < L::kNRes; ++j)
+                        for (int pn = 0; pn < L::kPanels; ++pn)
+                            tma_load_4d(res(j) + pn * kResPanel, maps[j], bar(L::kXFull), 64 * pn, it.bos + it.m0, it.hk, it.b);
                 }
                 // streamed tile t of the item -> stage s (DQR: k, v of key tile t; DKV: q, r, dO of a 64-row tile of one q head)
                 int hq = it.hk * a.n_rep, tt = 0;
@@ -342,7 +379,7 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
                         const CUtensorMap *maps[3] = {&tm_q, &tm_r, &tm_go};
                         for (int j = 0; j < 3; ++j)
                             for (int pn = 0; pn < L::kPanels; ++pn)
-                                tma_load_4d(str(s, j) + pn * kStrPanel, maps[j], bar(L::kNFull + s), 64 * pn, row0, hq, it.b);
+                                tma_load_4d(str(s, j) + pn * str_panel(j), maps[j], bar(L::kNFull + s), 64 * pn, row0, hq, it.b);
                     }
                     if (++tt == it.n_t) {
                         tt = 0;
@@ -376,66 +413,66 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
         // This path is kept to a few instructions per MMA: descriptor low words are "base + immediate",
         // high words and flags are compile-time constants.
         constexpr uint32_t idesc_s = umma_idesc(Fmt<T>::kUmma, 0, 0, kBM, kBN);
+        constexpr uint32_t idesc_s2 = umma_idesc(Fmt<T>::kUmma, 0, 0, kBM, 2 * kBN);
         constexpr uint32_t idesc_o = umma_idesc(Fmt<T>::kUmma, 0, 1, kBM, D);
         constexpr uint32_t hi = umma_desc_hi(1024);
-        // DQR: q, r (dO comes from tensor memory).  DKV: only v (index 0) is in shared memory, k is in TMEM.
-        const uint32_t res_lo0 = umma_desc_lo(res(0), 16), res_lo1 = umma_desc_lo(res(DQR ? 1 : 0), 16);
+        // DQR: q, r and dO; DKV: v and k (the last of them in tensor memory where kMTile)
+        const uint32_t res_lo0 = umma_desc_lo(res(0), 16), res_lo1 = umma_desc_lo(res(kMTile && !DQR ? 0 : 1), 16),
+                       res_lo2 = umma_desc_lo(res(DQR && !kMTile ? 2 : 0), 16);
         const uint32_t g_lo0 = umma_desc_lo(gt(0), 16), g_lo1 = umma_desc_lo(gt(1), 16), g_lo2 = umma_desc_lo(gt(DQR ? 1 : 2), 16);
         const uint32_t strk_lo0 = umma_desc_lo(str(0, 0), 16);          // streamed tiles as K-major B (scores)
-        const uint32_t strm_lo0 = umma_desc_lo(str(0, 0), kStrPanel);   // streamed tiles as MN-major B (outputs)
+        const uint32_t strm_lo0 = umma_desc_lo(str(0, 0), str_panel(0));   // streamed tiles as MN-major B (outputs)
+        const uint32_t strm_lo2 = umma_desc_lo(str(0, DQR ? 0 : 2), kStrPanel);
         // scores: S1, S2, A into tS + 0 / 64 / 128
-        auto issue_scores = [&](int s) {
-            const uint32_t b0 = strk_lo0 + s * (L::kStage >> 4);
+        auto issue_scores = [&](int s, int sb) {
+            const uint32_t b0 = strk_lo0 + s * (L::kStage >> 4), d = tS(sb);
 #pragma unroll
             for (int ks = 0; ks < D / 16; ++ks) {
                 const uint32_t aoff = ((ks >> 2) * kResPanel + (ks & 3) * 32) >> 4;
-                const uint32_t boff = ((ks >> 2) * kStrPanel + (ks & 3) * 32) >> 4;
-                // DQR: (Q, K) (R, K) (dO, V);  DKV: (K, Q) (K, R) (V, dO)
-                const uint32_t a1 = res_lo0 + aoff, a2 = res_lo1 + aoff;
-                const uint32_t b1 = b0 + boff, b2 = b0 + (DQR ? 0 : (kStrBytes >> 4)) + boff,
-                               b3 = b0 + ((DQR ? 1 : 2) * (kStrBytes >> 4)) + boff;
-                if (DQR) {
-                    if (ks == 0) {
-                        umma_ss_lean<false>(tS, a1, hi, b1, hi, idesc_s);
-                        umma_ss_lean<false>(tS + 64, a2, hi, b2, hi, idesc_s);
-                        umma_ts_lean<false>(tS + 128, tK + ks * 8, b3, hi, idesc_s);   // dO from tensor memory
-                    } else {
-                        umma_ss_lean<true>(tS, a1, hi, b1, hi, idesc_s);
-                        umma_ss_lean<true>(tS + 64, a2, hi, b2, hi, idesc_s);
-                        umma_ts_lean<true>(tS + 128, tK + ks * 8, b3, hi, idesc_s);
+                const uint32_t boff = ((ks >> 2) * kStrPanel + (ks & 3) * 32) >> 4, qoff = ((ks >> 2) * str_panel(0) + (ks & 3) * 32) >> 4;
+                auto products = [&](auto acc) {
+                    constexpr bool kAcc = decltype(acc)::value;
+                    if (DQR) {     // (Q, K) (R, K) (dO, V)
+                        const uint32_t b3 = b0 + (kStrBytes >> 4) + boff;
+                        umma_ss_lean<kAcc>(d, res_lo0 + aoff, hi, b0 + boff, hi, idesc_s);
+                        umma_ss_lean<kAcc>(d + 64, res_lo1 + aoff, hi, b0 + boff, hi, idesc_s);
+                        if (kMTile) umma_ts_lean<kAcc>(d + 128, tK + ks * 8, b3, hi, idesc_s);    // 16 channels = 8 columns per step
+                        else umma_ss_lean<kAcc>(d + 128, res_lo2 + aoff, hi, b3, hi, idesc_s);
+                    } else {       // (K, Q | R) (V, dO)
+                        if (kMTile) umma_ts_lean<kAcc>(d, tK + ks * 8, b0 + qoff, hi, idesc_s2);
+                        else umma_ss_lean<kAcc>(d, res_lo1 + aoff, hi, b0 + qoff, hi, idesc_s2);
+                        umma_ss_lean<kAcc>(d + 128, res_lo0 + aoff, hi, b0 + 2 * (kStrBytes >> 4) + boff, hi, idesc_s);
                     }
-                } else {   // k from tensor memory: 16 channels = 8 columns per step
-                    if (ks == 0) {
-                        umma_ts_lean<false>(tS, tK + ks * 8, b1, hi, idesc_s);
-                        umma_ts_lean<false>(tS + 64, tK + ks * 8, b2, hi, idesc_s);
-                        umma_ss_lean<false>(tS + 128, a1, hi, b3, hi, idesc_s);
-                    } else {
-                        umma_ts_lean<true>(tS, tK + ks * 8, b1, hi, idesc_s);
-                        umma_ts_lean<true>(tS + 64, tK + ks * 8, b2, hi, idesc_s);
-                        umma_ss_lean<true>(tS + 128, a1, hi, b3, hi, idesc_s);
-                    }
-                }
+                };
+                if (ks == 0) products(std::false_type{});
+                else products(std::true_type{});
             }
         };
         // outputs: A = G tile (K-major, 64 wide), B = streamed tile as MN-major [64 rows][128 channels]
         //   DQR: acc0 += G0 K, acc1 += G1 K;   DKV: acc0 += G0 Q + G1 R, acc1 += G2 dO
-        auto issue_out = [&](int s, bool first) {
-            const uint32_t b0 = strm_lo0 + s * (L::kStage >> 4);
-            const uint32_t bq = b0, br = b0 + (DQR ? 0 : (kStrBytes >> 4)), bg = b0 + 2 * (kStrBytes >> 4);
+        auto issue_out = [&](int s, int g, bool first) {
+            const uint32_t bq = strm_lo0 + s * (L::kStage >> 4), br = bq + (DQR ? 0 : (kStrPanel >> 4)), bg = strm_lo2 + s * (L::kStage >> 4);
+            const uint32_t gtm = tS(g % GR);
+            auto product = [&](auto acc, uint32_t d, int i, int kk, uint32_t b) {     // G tile i, rows 16 kk .. 16 kk + 15 of b
+                constexpr bool kAcc = decltype(acc)::value;
+                if (P::kTwo) umma_ts_lean<kAcc>(d, gtm + 64 * i + 8 * kk, b + kk * (2048 >> 4), hi, idesc_o);
+                else umma_ss_lean<kAcc>(d, (i == 0 ? g_lo0 : i == 1 ? g_lo1 : g_lo2) + kk * (32 >> 4), hi, b + kk * (2048 >> 4), hi, idesc_o);
+            };
+            using yes = std::true_type;
+            using no = std::false_type;
             if (first) {
-                umma_ss_lean<false>(tAcc0, g_lo0, hi, bq, hi, idesc_o);
-                umma_ss_lean<false>(tAcc1, DQR ? g_lo1 : g_lo2, hi, DQR ? br : bg, hi, idesc_o);
+                product(no{}, tAcc0, 0, 0, bq);
+                product(no{}, tAcc1, DQR ? 1 : 2, 0, DQR ? br : bg);
             } else {
-                umma_ss_lean<true>(tAcc0, g_lo0, hi, bq, hi, idesc_o);
-                umma_ss_lean<true>(tAcc1, DQR ? g_lo1 : g_lo2, hi, DQR ? br : bg, hi, idesc_o);
+                product(yes{}, tAcc0, 0, 0, bq);
+                product(yes{}, tAcc1, DQR ? 1 : 2, 0, DQR ? br : bg);
             }
-            if (!DQR) umma_ss_lean<true>(tAcc0, g_lo1, hi, br, hi, idesc_o);
+            if (!DQR) product(yes{}, tAcc0, 1, 0, br);
 #pragma unroll
             for (int kk = 1; kk < kBN / 16; ++kk) {
-                const uint32_t ao = kk * (32 >> 4), bo = kk * (2048 >> 4);
-                umma_ss_lean<true>(tAcc0, g_lo0 + ao, hi, bq + bo, hi, idesc_o);
-                umma_ss_lean<true>(tAcc1, (DQR ? g_lo1 : g_lo2) + ao, hi, (DQR ? br : bg) + bo, hi, idesc_o);
-                if (!DQR) umma_ss_lean<true>(tAcc0, g_lo1 + ao, hi, br + bo, hi, idesc_o);
+                product(yes{}, tAcc0, 0, kk, bq);
+                product(yes{}, tAcc1, DQR ? 1 : 2, kk, DQR ? br : bg);
+                if (!DQR) product(yes{}, tAcc0, 1, kk, br);
             }
         };
         int g = 0, n = 0, s = 0;
@@ -447,18 +484,20 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
             if (!ok || !it.valid) break;
             if (it.n_iter == 0) continue;
             if (warp == 1) {
-                ok = mbar_wait(bar(L::kXFull), n & 1, err, 4) && mbar_wait(bar(L::kKReady), n & 1, err, 14);
+                ok = mbar_wait(bar(L::kXFull), n & 1, err, 4);
+                if (kMTile && ok) ok = mbar_wait(bar(L::kKReady), n & 1, err, 14);
                 ok = __all_sync(0xffffffffu, ok);
                 for (int t = 0; t < it.n_iter && ok; ++t, ++g) {
                     ok = mbar_wait(bar(L::kNFull + s), ph, err, 6);
-                    // the score columns are free once the element-wise warps have read the previous tile
-                    if (ok && g > 0) ok = mbar_wait(bar(L::kSFree), (g - 1) & 1, err, 7);
+                    // the score columns are free once the element-wise warps have read the tile before in them, or (G in
+                    // place) its output products have completed
+                    if (ok && g >= GR) ok = mbar_wait(tile_bar(P::kTwo ? L::kGFree : L::kSFree, g - GR), tile_phase(g - GR), err, 7);
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                     tc_fence_after();
                     if (elect_one_sync()) {
-                        issue_scores(s);
-                        umma_commit(bar(L::kSFull));
+                        issue_scores(s, g % GR);
+                        umma_commit(tile_bar(L::kSFull, g));
                         if (t == it.n_iter - 1) umma_commit(bar(L::kXEmpty));   // resident tiles and the TMEM tile may be replaced
                     }
                     __syncwarp();
@@ -469,15 +508,15 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
                 }
             } else {
                 for (int t = 0; t < it.n_iter && ok; ++t, ++g) {
-                    ok = mbar_wait(bar(L::kGFull), g & 1, err, 8);
+                    ok = mbar_wait(tile_bar(L::kGFull, g), tile_phase(g), err, 8);
                     // the first product of an item overwrites the accumulators: the previous item's epilogue must have read them
                     if (ok && t == 0 && n > 0) ok = mbar_wait(bar(L::kAccFree), (n - 1) & 1, err, 13);
                     ok = __all_sync(0xffffffffu, ok);
                     if (!ok) break;
                     tc_fence_after();
                     if (elect_one_sync()) {
-                        issue_out(s, t == 0);
-                        umma_commit(bar(L::kGFree));
+                        issue_out(s, g, t == 0);
+                        umma_commit(tile_bar(L::kGFree, g));
                         umma_commit(bar(L::kNEmpty + s));
                         if (t == it.n_iter - 1) umma_commit(bar(L::kAccDone));
                     }
@@ -487,47 +526,67 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
             }
             ++n;
         }
+    } else if (warp == 3) {
+        // ------------------------------------------------------------------ row statistics (DKV)
+        // The per-row statistics of a streamed tile are per-COLUMN constants of the element-wise warps.  This warp
+        // fetches them ({b, mL, 1 + bart, (b - t) * scale}, 16 bytes a row, two rows a lane, a tile ahead) and lays them
+        // out in shared memory as four planes of 64 floats (with mL and 1 + bart negated, the latter also times scale), so
+        // that a thread reads the constants of adjacent columns as aligned pairs for the packed two-wide arithmetic.
+        if constexpr (!DQR) {
+            bool ok = true;
+            int g = 0;
+            for (int i = 0; ok; ++i) {
+                Item it;
+                ok = ring.read(i, it, true, err, 22);
+                if (!ok || !it.valid) break;
+                int hq = it.hk * a.n_rep, tt = 0;
+                float4 x[2];
+                auto fetch = [&]() {
+                    const int row0 = it.bos + (it.t_lo + tt) * kBN;
+                    const float4 *src = reinterpret_cast<const float4 *>(a.cst) + (static_cast<int64_t>(it.b) * a.heads_q + hq) * n_tok + row0;
+                    // (rows past the sequence: those of the next one or of the next head, masked; the records end with 64 spare ones)
+                    x[0] = __ldcg(src + lane);
+                    x[1] = __ldcg(src + 32 + lane);
+                    if (++tt == it.n_t) {
+                        tt = 0;
+                        ++hq;
+                    }
+                };
+                if (it.n_iter > 0) fetch();
+                for (int t = 0; t < it.n_iter; ++t, ++g) {
+                    const int st = g % kStatStages;
+                    if (g >= kStatStages) {
+                        ok = __all_sync(0xffffffffu, mbar_wait(bar(L::kStatEmpty + st), (g / kStatStages - 1) & 1, err, 15));
+                        if (!ok) break;
+                    }
+                    float *dst = reinterpret_cast<float *>(smem_raw + L::kStats + st * kStatBytes) + lane;
+#pragma unroll
+                    for (int h = 0; h < 2; ++h) {
+                        dst[32 * h] = -x[h].y;
+                        dst[kBN + 32 * h] = -x[h].z * a.scale;
+                        dst[2 * kBN + 32 * h] = x[h].x;
+                        dst[3 * kBN + 32 * h] = x[h].w;
+                    }
+                    mbar_arrive(bar(L::kStatFull + st));
+                    if (t + 1 < it.n_iter) fetch();
+                }
+            }
+        }
     } else if (warp >= 4) {
         // ------------------------------------------------------------------ element-wise + epilogue
-        // warp 4 + w: TMEM lane quarter w % 4 (a warp may only touch the lanes of its own quarter), column
-        // group cg = w / 4 of the streamed tile (CPT columns), and for the accumulators one of the two
-        const int quarter = warp & 3, cg = (warp - 4) >> 2;
+        // warp 4 + w: TMEM lane quarter w % 4 (a warp may only touch the lanes of its own quarter); `sel` = w / 4 is its
+        // group (GR = 2: the tiles g with g % 2 = sel, GR = 1: columns 32 * sel .. of every tile) and its accumulator
+        const int quarter = warp & 3, sel = (warp - 4) >> 2;
         const int ml = quarter * 32 + lane;                 // lane of the M tile: query row (DQR) / key (DKV)
         const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
-        const int col0 = cg * CPT;
-        const int acc_sel = cg / (CG / 2), part = cg % (CG / 2);   // accumulator (0: dQ | dK, 1: dR | dV) and this warp's share of it
         const float2 c2v = make_float2(a.c2, a.c2), scale2 = make_float2(a.scale, a.scale);
-        const int wid = static_cast<int>(threadIdx.x) - 128;
-        const bool stat_writer = !DQR && wid < kStatWriters;
         bool ok = true;
-        int g = 0, n = 0, i_next = 0;
+        int g0 = 0, n = 0, i_next = 0;                      // streamed tiles before this item, items, items looked at
 
         // With mL = m + log2(d1), c1 = 1 + bart, ct = b - t:
         //   p = 2^(S1*c2 - mL), un = S2 - c1, dn = b - A   =>   W = -p un, gu = p dn, gl = (p un) dn + p ct
         // DQR: the constants of this thread's row
         float r_ml = INFINITY, r_c1 = 0.f, r_ct = 0.f, r_b = 0.f;
-        float4 stat_next = make_float4(0.f, 0.f, 0.f, 0.f);
-
-        // DKV: the per-row statistics of a streamed tile are per-COLUMN constants here.  The first 64
-        // element-wise threads fetch one row each ({b, mL, 1 + bart, (b - t) * scale}, 16 bytes) a tile
-        // ahead and lay them out in shared memory as four planes of 64 floats (with mL and 1 + bart
-        // negated, the latter also times scale), so that every thread reads the constants of adjacent
-        // columns as aligned pairs for the packed two-wide arithmetic.  Two buffers: tile g of the CTA
-        // uses buffer g & 1.
-        auto stat_fetch = [&](const Item &it, int t) -> float4 {
-            if (t >= it.n_iter) return make_float4(0.f, 0.f, 0.f, 0.f);
-            const int hq = it.hk * a.n_rep + t / it.n_t;
-            const int row0 = it.bos + (it.t_lo + t % it.n_t) * kBN;
-            return __ldcg(reinterpret_cast<const float4 *>(a.cst + ((static_cast<int64_t>(it.b) * a.heads_q + hq) * n_tok + row0 + wid) * 4));
-        };
-        auto stat_publish = [&](int gg, const float4 &v) {
-            float *dst = reinterpret_cast<float *>(smem_raw + L::kStats + (gg % kStatStages) * kStatBytes);
-            dst[wid] = -v.y;
-            dst[kBN + wid] = -v.z * a.scale;
-            dst[2 * kBN + wid] = v.x;
-            dst[3 * kBN + wid] = v.w;
-            mbar_arrive(bar(L::kStatFull + gg % kStatStages));
-        };
 
         Item cur;
         // next item of this CTA that has tiles to stream; items without any (no visible key / no row
@@ -539,28 +598,28 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
                 if (cur.n_iter > 0) return true;
                 const int row = cur.m0 + ml;
                 if (row < (DQR ? cur.nq : cur.nk)) {
-                    constexpr int kCh = D / (CG / 2);          // channels of the row written by this thread
-                    T *dst = DQR ? static_cast<T *>(acc_sel == 0 ? a.dq : a.dr) + cur.b * a.q_sb + cur.hy * a.q_sh + static_cast<int64_t>(cur.bos + row) * a.q_st
-                                 : static_cast<T *>(acc_sel == 0 ? a.dk : a.dv) + cur.b * a.kv_sb + cur.hy * a.kv_sh + static_cast<int64_t>(cur.bos + row) * a.kv_st;
+                    T *dst = DQR ? static_cast<T *>(sel == 0 ? a.dq : a.dr) + cur.b * a.q_sb + cur.hy * a.q_sh + static_cast<int64_t>(cur.bos + row) * a.q_st
+                                 : static_cast<T *>(sel == 0 ? a.dk : a.dv) + cur.b * a.kv_sb + cur.hy * a.kv_sh + static_cast<int64_t>(cur.bos + row) * a.kv_st;
 #pragma unroll
-                    for (int c = 0; c < kCh / 8; ++c) *reinterpret_cast<uint4 *>(dst + part * kCh + 8 * c) = make_uint4(0u, 0u, 0u, 0u);
+                    for (int c = 0; c < D / 8; ++c) *reinterpret_cast<uint4 *>(dst + 8 * c) = make_uint4(0u, 0u, 0u, 0u);
                 }
             }
         };
-        // Start of an item (n-th with tiles of this CTA): the tile of the M side that is the A operand of
-        // score products and fits the 64 spare TMEM columns -- DKV: k (S1^T, S2^T), DQR: dO (A) -- goes
-        // there instead of shared memory, where MMA operand reads are the scarce resource: this thread's
-        // share (D / CG channels) of row mg, two 16-bit channels per column.
+        // Start of an item (nn-th with tiles of this CTA): the row's constants (DQR), and where kMTile the tile of the M side
+        // that is the A operand of score products goes to the 64 spare TMEM columns instead of shared memory, where MMA
+        // operand reads are the scarce resource: this thread's half of row mg, two 16-bit channels per column.
         auto prologue = [&](int nn) -> bool {
             const int mg = cur.m0 + ml;
-            uint32_t kw[D / (2 * CG)];
-            const T *krow = DQR ? static_cast<const T *>(a.go) + cur.b * a.q_sb + cur.hy * a.q_sh + static_cast<int64_t>(cur.bos + mg) * a.q_st + cg * (D / CG)
-                                : static_cast<const T *>(a.k) + cur.b * a.kv_sb + cur.hk * a.kv_sh + static_cast<int64_t>(cur.bos + mg) * a.kv_st + cg * (D / CG);
+            uint32_t kw[D / 4];
+            if (kMTile) {
+                const T *krow = DQR ? static_cast<const T *>(a.go) + cur.b * a.q_sb + cur.hy * a.q_sh + static_cast<int64_t>(cur.bos + mg) * a.q_st + sel * (D / 2)
+                                    : static_cast<const T *>(a.k) + cur.b * a.kv_sb + cur.hk * a.kv_sh + static_cast<int64_t>(cur.bos + mg) * a.kv_st + sel * (D / 2);
 #pragma unroll
-            for (int c = 0; c < D / (8 * CG); ++c) {
-                uint4 x = make_uint4(0u, 0u, 0u, 0u);
-                if (mg < (DQR ? cur.nq : cur.nk)) x = *reinterpret_cast<const uint4 *>(krow + 8 * c);
-                kw[4 * c] = x.x; kw[4 * c + 1] = x.y; kw[4 * c + 2] = x.z; kw[4 * c + 3] = x.w;
+                for (int c = 0; c < D / 16; ++c) {
+                    uint4 x = make_uint4(0u, 0u, 0u, 0u);
+                    if (mg < (DQR ? cur.nq : cur.nk)) x = *reinterpret_cast<const uint4 *>(krow + 8 * c);
+                    kw[4 * c] = x.x; kw[4 * c + 1] = x.y; kw[4 * c + 2] = x.z; kw[4 * c + 3] = x.w;
+                }
             }
             if (DQR) {
                 r_ml = INFINITY;
@@ -574,21 +633,15 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
                     r_ct = hi4.w / a.scale;
                 }
             }
-            float4 st0 = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (stat_writer) {
-                st0 = stat_fetch(cur, 0);
-                stat_next = stat_fetch(cur, 1);
+            if (kMTile) {
+                // the previous item's score products (the readers of the TMEM tile) must have completed
+                if (nn > 0 && !__all_sync(0xffffffffu, mbar_wait(bar(L::kXEmpty), (nn - 1) & 1, err, 16))) return false;
+                tc_fence_after();
+                tmem_st_cols(tK + lane_base + sel * (D / 4), kw);
+                tmem_wait_st();
+                tc_fence_before();
+                mbar_arrive(bar(L::kKReady));
             }
-            // the previous item's score products (the readers of the TMEM tile) must have completed
-            if (nn > 0 && !__all_sync(0xffffffffu, mbar_wait(bar(L::kXEmpty), (nn - 1) & 1, err, 16))) return false;
-            tc_fence_after();
-            tmem_st_cols(tK + lane_base + cg * (D / (2 * CG)), kw);
-            tmem_wait_st();
-            tc_fence_before();
-            mbar_arrive(bar(L::kKReady));
-            // Every thread has handed over the tile before this item's first one (g - 1) and, through the
-            // G-buffer wait of that tile, seen tile g - 2 completed by all: the statistics buffer of tile g is free.
-            if (stat_writer) stat_publish(g, st0);
             return true;
         };
 
@@ -596,48 +649,33 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
         if (have && ok) ok = prologue(0);
         while (have && ok) {
             const int m0 = cur.m0, nq = cur.nq, nk = cur.nk, off = cur.off, mg = m0 + ml;
-            for (int it = 0; it < cur.n_iter; ++it, ++g) {
-                ok = __all_sync(0xffffffffu, mbar_wait(bar(L::kSFull), g & 1, err, 9));
+            for (int it = GR == 2 ? (g0 ^ sel) & 1 : 0; it < cur.n_iter; it += GR) {
+                const int g = g0 + it;
+                ok = __all_sync(0xffffffffu, mbar_wait(tile_bar(L::kSFull, g), tile_phase(g), err, 9));
                 if (!ok) break;
                 tc_fence_after();
-                uint32_t x1[CPT], x2[CPT], x3[CPT];
-                tmem_ld_cols(tS + lane_base + col0, x1);
-                tmem_ld_cols(tS + 64 + lane_base + col0, x2);
-                tmem_ld_cols(tS + 128 + lane_base + col0, x3);
-                tmem_wait_ld();
-                tc_fence_before();
-                mbar_arrive(bar(L::kSFree));
 
                 const int tile0 = (cur.t_lo + (DQR ? it : it % cur.n_t)) * kBN;   // first streamed index of the tile
-                const int n0 = tile0 + col0;                                      // ... of this thread's columns
-                // DQR: columns are keys n0 + c, visible iff n0 + c <= lim_hi.   DKV: columns are rows, visible iff lim_lo <= n0 + c <= lim_hi
                 const int win = a.window;
-                const int lim_lo = DQR ? (win < 0 ? INT_MIN : mg + off - win + 1) : max(mg - off, 0);
-                const int lim_hi = DQR ? (mg < nq ? min(mg + off, nk - 1) : -1)
-                                       : (mg < nk ? (win < 0 ? nq - 1 : min(nq - 1, mg - off + win - 1)) : -1);
                 // tile-uniform: every element of the tile is visible
                 const bool full = DQR ? (tile0 + kBN - 1 <= m0 + off && tile0 + kBN <= nk && m0 + kBM <= nq &&
                                          (win < 0 || tile0 >= m0 + kBM + off - win))
                                       : (tile0 >= m0 + kBM - 1 - off && tile0 + kBN <= nq && m0 + kBM <= nk &&
                                          (win < 0 || tile0 + kBN - 1 <= m0 - off + win - 1));
-                const int ss = g % kStatStages;
-                const float *stats = reinterpret_cast<const float *>(smem_raw + L::kStats + ss * kStatBytes);
-                if (!DQR) {
-                    ok = __all_sync(0xffffffffu, mbar_wait(bar(L::kStatFull + ss), (g / kStatStages) & 1, err, 15));
-                    if (!ok) break;
-                }
-                uint32_t g0[CPT / 2], g1[CPT / 2], g2[CPT / 2];
-                // One pair of adjacent columns: constants nml = -mL, nc1 = -(1 + bart), bb = b, ct = b - t (DKV:
-                // times scale; DKV: nc1 times scale too).  The third tile carries -W * scale = p un scale (DKV
+                const float *stats = reinterpret_cast<const float *>(smem_raw + L::kStats + (g % kStatStages) * kStatBytes);
+                // One pair of adjacent columns: constants nml = -mL, nc1 = -(1 + bart), bb = b, ct = b - t (DKV: times
+                // scale; DKV: nc1 times scale too).  The third tile carries -W * scale = p un scale (DKV
                 // only): the dV accumulator is multiplied by -1 / scale when it is written out, which saves a
                 // negation and a multiplication per element here.  `masked` is a compile-time tag:
                 // tiles that are visible as a whole (all but the ones on the diagonal or at a window edge) run
                 // the loop without any mask arithmetic AND as one basic block, so that the independent pairs
-                // interleave; a branch per pair would keep them apart.
-                auto pair = [&](auto masked, int c, const float2 &nml, const float2 &nc1, const float2 &bb, const float2 &ct) {
-                    const float2 s1 = make_float2(__uint_as_float(x1[c]), __uint_as_float(x1[c + 1]));
-                    const float2 s2 = make_float2(__uint_as_float(x2[c]), __uint_as_float(x2[c + 1]));
-                    const float2 av = make_float2(__uint_as_float(x3[c]), __uint_as_float(x3[c + 1]));
+                // interleave; a branch per pair would keep them apart.  Else columns lo .. hi are visible.
+                auto element_pair = [&](auto masked, int lo, int hi, int col, uint32_t s1a, uint32_t s1b, uint32_t s2a, uint32_t s2b, uint32_t aa,
+                                        uint32_t ab, const float2 &nml, const float2 &nc1, const float2 &bb, const float2 &ct, uint32_t &w0,
+                                        uint32_t &w1, uint32_t &w2) {
+                    const float2 s1 = make_float2(__uint_as_float(s1a), __uint_as_float(s1b));
+                    const float2 s2 = make_float2(__uint_as_float(s2a), __uint_as_float(s2b));
+                    const float2 av = make_float2(__uint_as_float(aa), __uint_as_float(ab));
                     const float2 arg = __ffma2_rn(s1, c2v, nml);
                     const float2 p = make_float2(fast_exp2(arg.x), fast_exp2(arg.y));
                     // DKV carries qk_scale on gl = (p un scale) dn + p ct scale: nc1 and ct come scaled from the
@@ -649,72 +687,150 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
                     float2 gu = __fmul2_rn(p, dn);
                     float2 gl = __ffma2_rn(wn, dn, pc);
                     if (decltype(masked)::value) {
-                        const bool v0 = n0 + c >= lim_lo && n0 + c <= lim_hi, v1 = n0 + c + 1 >= lim_lo && n0 + c + 1 <= lim_hi;
+                        const bool v0 = col >= lo && col <= hi, v1 = col + 1 >= lo && col + 1 <= hi;
                         gl = make_float2(v0 ? gl.x : 0.f, v1 ? gl.y : 0.f);
                         gu = make_float2(v0 ? gu.x : 0.f, v1 ? gu.y : 0.f);
                         wn = make_float2(v0 ? wn.x : 0.f, v1 ? wn.y : 0.f);
                     }
-                    g0[c >> 1] = Elem<T>::pack(gl.x, gl.y);
-                    g1[c >> 1] = Elem<T>::pack(gu.x, gu.y);
-                    if (!DQR) g2[c >> 1] = Elem<T>::pack(wn.x, wn.y);
+                    w0 = Elem<T>::pack(gl.x, gl.y);
+                    w1 = Elem<T>::pack(gu.x, gu.y);
+                    if (!DQR) w2 = Elem<T>::pack(wn.x, wn.y);
                 };
-                auto tile_math = [&](auto masked) {
-                    if (DQR) {
-                        const float2 nml = make_float2(-r_ml, -r_ml), nc1 = make_float2(-r_c1, -r_c1), bb = make_float2(r_b, r_b),
-                                     ct = make_float2(r_ct, r_ct);
+                auto stats_ready = [&]() -> bool {
+                    return __all_sync(0xffffffffu, mbar_wait(bar(L::kStatFull + g % kStatStages), (g / kStatStages) & 1, err, 15));
+                };
+                const uint32_t tsg = tS(g % GR) + lane_base;
+                if constexpr (P::kTwo && !DQR) {
+                    // The fragment arrangement: in each half h of the warp's 32 lanes (keys), this thread has the keys
+                    // 16 h + lane / 4 and + 8 and the columns 8 k + 2 (lane % 4), + 1 -- so it needs the constants of 16
+                    // columns for 32 elements.  (With one key and 32 columns a thread, every thread of a warp reads every constant.)
+                    const int gq = lane >> 2, t2 = 2 * (lane & 3);
+                    const float *st2 = stats + t2;
+                    auto constant = [&](int plane, int k) { return *reinterpret_cast<const float2 *>(st2 + plane * kBN + 8 * k); };
+#pragma unroll 1
+                    for (int h = 0; h < 2; ++h) {
+                        const uint32_t at = tsg + (16u * h << 16);
+                        uint32_t x1[32], x2[32], x3[32], w0[16], w1[16], w2[16];
+                        tmem_ld_16x256b_x8(at, x1);
+                        tmem_ld_16x256b_x8(at + 64, x2);
+                        tmem_ld_16x256b_x8(at + 128, x3);
+                        tmem_wait_ld();
+                        if (h == 0) {
+                            ok = stats_ready();
+                            if (!ok) break;
+                        }
+                        auto math = [&](auto masked) {
+                            int lo[2], hi[2];                  // visible rows of the two keys
 #pragma unroll
-                        for (int c = 0; c < CPT; c += 2) pair(masked, c, nml, nc1, bb, ct);
-                    } else {
-                        const float *pl = stats + col0;
+                            for (int j = 0; j < 2; ++j) {
+                                const int key = m0 + quarter * 32 + 16 * h + 8 * j + gq;
+                                lo[j] = max(key - off, 0);
+                                hi[j] = key < nk ? (win < 0 ? nq - 1 : min(nq - 1, key - off + win - 1)) : -1;
+                            }
 #pragma unroll
-                        for (int c = 0; c < CPT; c += 4) {
-                            const float4 nml = *reinterpret_cast<const float4 *>(pl + c);
-                            const float4 nc1 = *reinterpret_cast<const float4 *>(pl + kBN + c);
-                            const float4 bb = *reinterpret_cast<const float4 *>(pl + 2 * kBN + c);
-                            const float4 ct = *reinterpret_cast<const float4 *>(pl + 3 * kBN + c);
-                            pair(masked, c, make_float2(nml.x, nml.y), make_float2(nc1.x, nc1.y), make_float2(bb.x, bb.y), make_float2(ct.x, ct.y));
-                            pair(masked, c + 2, make_float2(nml.z, nml.w), make_float2(nc1.z, nc1.w), make_float2(bb.z, bb.w), make_float2(ct.z, ct.w));
+                            for (int k = 0; k < 8; ++k) {
+                                const float2 nml = constant(0, k), nc1 = constant(1, k), bb = constant(2, k), ct = constant(3, k);
+#pragma unroll
+                                for (int j = 0; j < 2; ++j) {
+                                    const int e = 4 * k + 2 * j;
+                                    element_pair(masked, lo[j], hi[j], tile0 + 8 * k + t2, x1[e], x1[e + 1], x2[e], x2[e + 1], x3[e], x3[e + 1], nml,
+                                                 nc1, bb, ct, w0[2 * k + j], w1[2 * k + j], w2[2 * k + j]);
+                                }
+                            }
+                        };
+                        if (full) math(std::false_type{});
+                        else math(std::true_type{});
+                        tmem_st_16x128b_x8(at, w0);
+                        tmem_st_16x128b_x8(at + 64, w1);
+                        tmem_st_16x128b_x8(at + 128, w2);
+                    }
+                    if (!ok) break;
+                    mbar_arrive(bar(L::kStatEmpty + g % kStatStages));
+                } else {
+                    // one row (DQR) or key (DKV) a thread, CH columns at a time
+                    const int lo = DQR ? (win < 0 ? INT_MIN : mg + off - win + 1) : max(mg - off, 0);      // visible columns
+                    const int hi = DQR ? (mg < nq ? min(mg + off, nk - 1) : -1)
+                                       : (mg < nk ? (win < 0 ? nq - 1 : min(nq - 1, mg - off + win - 1)) : -1);
+#pragma unroll 1
+                    for (int ch = 0; ch < GR; ++ch) {
+                        const int col0 = (GR == 2 ? ch : sel) * CH;
+                        uint32_t x1[CH], x2[CH], x3[CH], w0[CH / 2], w1[CH / 2], w2[CH / 2];
+                        tmem_ld_cols(tsg + col0, x1);
+                        tmem_ld_cols(tsg + 64 + col0, x2);
+                        tmem_ld_cols(tsg + 128 + col0, x3);
+                        tmem_wait_ld();
+                        if constexpr (!P::kTwo) {
+                            tc_fence_before();
+                            mbar_arrive(tile_bar(L::kSFree, g));
+                        }
+                        if constexpr (!DQR) {
+                            ok = stats_ready();
+                            if (!ok) break;
+                        }
+                        auto math = [&](auto masked) {
+#pragma unroll
+                            for (int c = 0; c < CH; c += 4) {
+                                float4 st[4];
+                                const float row[4] = {-r_ml, -r_c1, r_b, r_ct};
+#pragma unroll
+                                for (int i = 0; i < 4; ++i)
+                                    st[i] = DQR ? make_float4(row[i], row[i], row[i], row[i]) : *reinterpret_cast<const float4 *>(stats + i * kBN + col0 + c);
+#pragma unroll
+                                for (int e = c; e < c + 4; e += 2) {
+                                    auto half = [&](int i) { return e == c ? make_float2(st[i].x, st[i].y) : make_float2(st[i].z, st[i].w); };
+                                    element_pair(masked, lo, hi, tile0 + col0 + e, x1[e], x1[e + 1], x2[e], x2[e + 1], x3[e], x3[e + 1], half(0), half(1),
+                                                 half(2), half(3), w0[e / 2], w1[e / 2], w2[e / 2]);
+                                }
+                            }
+                        };
+                        if (full) math(std::false_type{});
+                        else math(std::true_type{});
+                        if constexpr (!DQR) mbar_arrive(bar(L::kStatEmpty + g % kStatStages));
+                        if constexpr (P::kTwo) {
+                            // (the second half of the columns is still to be read: the first half of G goes over the first)
+                            tmem_st_cols(tsg + col0 / 2, w0);
+                            tmem_st_cols(tsg + 64 + col0 / 2, w1);
+                        } else {
+                            // the G tiles are free once the output products of the tile before have completed
+                            if (g > 0) {
+                                ok = __all_sync(0xffffffffu, mbar_wait(tile_bar(L::kGFree, g - 1), tile_phase(g - 1), err, 10));
+                                if (!ok) break;
+                            }
+                            // row ml of each G tile: 128 bytes, 16-byte chunk i stored at position i ^ (ml & 7)
+#pragma unroll
+                            for (int c = 0; c < CH / 8; ++c) {
+                                const uint32_t o = static_cast<uint32_t>(ml) * 128u + static_cast<uint32_t>(((col0 / 8 + c) ^ (ml & 7)) * 16);
+                                st_shared_v4(gt(0) + o, w0[4 * c], w0[4 * c + 1], w0[4 * c + 2], w0[4 * c + 3]);
+                                st_shared_v4(gt(1) + o, w1[4 * c], w1[4 * c + 1], w1[4 * c + 2], w1[4 * c + 3]);
+                                if (!DQR) st_shared_v4(gt(2) + o, w2[4 * c], w2[4 * c + 1], w2[4 * c + 2], w2[4 * c + 3]);
+                            }
                         }
                     }
-                };
-                if (full) tile_math(std::false_type{});
-                else tile_math(std::true_type{});
-                // the G tiles are free once the output products of the previous tile have completed
-                if (g > 0) {
-                    ok = __all_sync(0xffffffffu, mbar_wait(bar(L::kGFree), (g - 1) & 1, err, 10));
                     if (!ok) break;
                 }
-                // Every thread has handed over tile g - 1 (the output products that just completed needed all
-                // of its G rows), so nobody reads the statistics buffer of tile g - 1 any more: refill it.
-                if (stat_writer && it + 1 < cur.n_iter) {
-                    stat_publish(g + 1, stat_next);
-                    stat_next = stat_fetch(cur, it + 2);
+                if constexpr (P::kTwo) {
+                    tmem_wait_st();
+                    tc_fence_before();
+                } else {
+                    fence_proxy_async();
                 }
-                // row ml of each G tile: 128 bytes, 16-byte chunk i stored at position i ^ (ml & 7)
-#pragma unroll
-                for (int c = 0; c < CPT / 8; ++c) {
-                    const uint32_t o = static_cast<uint32_t>(ml) * 128u + static_cast<uint32_t>(((cg * (CPT / 8) + c) ^ (ml & 7)) * 16);
-                    st_shared_v4(gt(0) + o, g0[4 * c], g0[4 * c + 1], g0[4 * c + 2], g0[4 * c + 3]);
-                    st_shared_v4(gt(1) + o, g1[4 * c], g1[4 * c + 1], g1[4 * c + 2], g1[4 * c + 3]);
-                    if (!DQR) st_shared_v4(gt(2) + o, g2[4 * c], g2[4 * c + 1], g2[4 * c + 2], g2[4 * c + 3]);
-                }
-                fence_proxy_async();
-                mbar_arrive(bar(L::kGFull));
+                mbar_arrive(tile_bar(L::kGFull, g));
             }
             if (!ok) break;
 
             // ---- what the epilogue of this item needs, then the start of the next item: its TMEM tile and
             // first score products are under way while the accumulators of this one are written out
             // dQ carries qk_scale; the dV accumulator holds -dV * qk_scale (the W tile is stored as -W * qk_scale)
-            const float mul = DQR ? (acc_sel == 0 ? a.scale : 1.f) : (acc_sel == 0 ? 1.f : -1.f / a.scale);
+            g0 += cur.n_iter;
+            const float mul = DQR ? (sel == 0 ? a.scale : 1.f) : (sel == 0 ? 1.f : -1.f / a.scale);
             const int rows_left = (DQR ? nq : nk) - m0;
             T *dst0;
             int64_t row_stride;
             if (DQR) {
-                dst0 = static_cast<T *>(acc_sel == 0 ? a.dq : a.dr) + cur.b * a.q_sb + cur.hy * a.q_sh + static_cast<int64_t>(cur.bos + m0) * a.q_st;
+                dst0 = static_cast<T *>(sel == 0 ? a.dq : a.dr) + cur.b * a.q_sb + cur.hy * a.q_sh + static_cast<int64_t>(cur.bos + m0) * a.q_st;
                 row_stride = a.q_st;
             } else {
-                dst0 = static_cast<T *>(acc_sel == 0 ? a.dk : a.dv) + cur.b * a.kv_sb + cur.hy * a.kv_sh + static_cast<int64_t>(cur.bos + m0) * a.kv_st;
+                dst0 = static_cast<T *>(sel == 0 ? a.dk : a.dv) + cur.b * a.kv_sb + cur.hy * a.kv_sh + static_cast<int64_t>(cur.bos + m0) * a.kv_st;
                 row_stride = a.kv_st;
             }
             have = next_item();
@@ -722,24 +838,23 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
             if (!ok) break;
 
             // epilogue: half of the element-wise warps write acc0 (dQ | dK), the other half acc1 (dR | dV); an
-            // accumulator is 2 x D / 64 units of 16 rows x 64 columns per lane quarter, dealt out to the CG / 2
-            // warps of the quarter.  The accumulators are read in the fragment arrangement (a row is spread
+            // accumulator is 2 x D / 64 units of 16 rows x 64 columns per lane quarter.  The accumulators are read in the fragment arrangement (a row is spread
             // over the four lanes of a quad); a 4 x 4 word transpose inside the quad gives every thread 16
             // contiguous bytes, so a warp store covers 64 contiguous bytes of 8 rows.
             ok = __all_sync(0xffffffffu, mbar_wait(bar(L::kAccDone), n & 1, err, 11));
             if (!ok) break;
             tc_fence_after();
             const int gq = lane >> 2, t = lane & 3;
-            const uint32_t acc = acc_sel == 0 ? tAcc0 : tAcc1;
-            constexpr int kUnits = 2 * (D / 64), kParts = CG / 2;
+            const uint32_t acc = sel == 0 ? tAcc0 : tAcc1;
+            constexpr int kUnits = 2 * (D / 64);
 #pragma unroll 1
-            for (int u = part; u < kUnits; u += kParts) {
+            for (int u = 0; u < kUnits; ++u) {
                 const int rh = u / (D / 64), cc = u % (D / 64);
                 const int rl = quarter * 32 + rh * 16 + gq;     // local rows of this thread: rl and rl + 8
                 uint32_t x[32];
                 tmem_ld_16x256b_x8(acc + (static_cast<uint32_t>(quarter * 32 + rh * 16) << 16) + 64 * cc, x);
                 tmem_wait_ld();
-                if (u + kParts >= kUnits) {
+                if (u == kUnits - 1) {
                     // this thread's share of the accumulators is in registers: the next item may overwrite them
                     tc_fence_before();
                     mbar_arrive(bar(L::kAccFree));
@@ -776,10 +891,7 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
 // ------------------------------------------------------------------------- //
 template <typename T, int D, int MODE>
 int launch_mode(const TrainArgs &a, int n_tok, const ErrSink &sink, bool overlap, cudaStream_t stream) {
-    // Ring depth: as many stages as the 227 KB of shared memory allow at head_dim 128 (dk/dv 3, dq/dr 4); six at
-    // head_dim 64 (measured against four: dq/dr 0.883 vs 0.919 ms, dk/dv 1.337 vs 1.352 ms; two stages cost 20 %).
-    constexpr int NS = D == 64 ? 6 : (MODE == kModeDKV ? 3 : 4);
-    using L = Smem<D, MODE, NS>;
+    using L = Smem<D, MODE>;
     constexpr bool DQR = MODE == kModeDQR;
     const int q_rows = DQR ? kBM : kBN, kv_rows = DQR ? kBN : kBM;
     CUtensorMap tq, tr, tg, tk, tv;
@@ -790,12 +902,7 @@ int launch_mode(const TrainArgs &a, int n_tok, const ErrSink &sink, bool overlap
         !tma::make_map(&tk, dt, a.k, D, a.len_k, a.heads_kv, a.batch, a.kv_st, a.kv_sh, a.kv_sb, kv_rows) ||
         !tma::make_map(&tv, dt, a.v, D, a.len_k, a.heads_kv, a.batch, a.kv_st, a.kv_sh, a.kv_sb, kv_rows))
         return PLX_ERR_LAUNCH;
-    // Eight element-wise warps (32 of the 64 streamed columns per thread).  Sixteen were faster while the
-    // tile arithmetic had a branch per column pair; as one basic block the longer per-thread chain
-    // interleaves well enough, and eight measured 1.150 / 1.530 ms (dq/dr, dk/dv) against 1.176 / 1.588 with
-    // sixteen at B=8, H=16, L=4096, head_dim 128 (head_dim 64: 0.923 / 1.353 against 0.926 / 1.50).
-    constexpr int EW = PLX_BWD_EW_WARPS;
-    auto kern = bwd_sm100_kernel<T, D, MODE, NS, EW>;
+    auto kern = bwd_sm100_kernel<T, D, MODE>;
     static std::mutex attr_mu;
     static bool attr_done[tma::kMaxDevices] = {};
     if (!tma::opt_in_smem(kern, static_cast<int>(L::kBytes), attr_done, attr_mu)) return PLX_ERR_LAUNCH;
@@ -810,7 +917,7 @@ int launch_mode(const TrainArgs &a, int n_tok, const ErrSink &sink, bool overlap
     const int group = !dynamic && n_items > sms ? 0 : dynamic && a.cu ? 1 : item_group(a.batch * (DQR ? a.heads_q : a.heads_kv), tiles, sms);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(dynamic || units < sms ? units : sms);
-    cfg.blockDim = dim3((4 + EW) * 32);
+    cfg.blockDim = dim3((4 + kEwWarps) * 32);
     cfg.dynamicSmemBytes = L::kBytes;
     cfg.stream = stream;
     cudaLaunchAttribute attr[1];

@@ -1,0 +1,27 @@
+"""The head_dim 64 backward, whose element-wise groups take the streamed tiles in turn: work items of every small
+tile count in a row on one CTA, so that items begin with either group and a group has no tile of some of them."""
+import pytest
+import torch
+
+from oracle import parallax_oracle as orc
+from tests._util import TRAIN_MAX_REL, TRAIN_REL_L2, assert_close
+from tests import test_varlen_gpu as tv
+
+pytestmark = pytest.mark.gpu
+
+
+# lengths either side of the 64-wide streamed tiles and the 128-wide resident ones: 1 to 5 streamed tiles an item.  160 heads
+# are more items than SMs, so a CTA walks several.
+@pytest.mark.parametrize("lens,hq,hkv,window,dtype", [
+    ([63, 64, 65, 129, 191, 257, 40, 320], 32, 32, -1, torch.bfloat16),
+    ([65, 128, 130, 193, 33, 127], 48, 16, -1, torch.float16),
+    ([200, 64, 310, 129], 64, 64, 70, torch.bfloat16),
+    ([96], 160, 160, -1, torch.bfloat16),
+])
+def test_items_begin_with_either_group(lens, hq, hkv, window, dtype):
+    q, r, k, v, go, cu = (x.to(dtype) if x.is_floating_point() else x for x in tv.make(lens, hq, hkv, 64, 77))
+    got = tv.run_gpu(q, r, k, v, go, cu, window)
+    ref_o = orc.varlen_forward(q, r, k, v, cu, None, window)["o"]
+    ref_g = orc.varlen_backward(q, r, k, v, go.float(), cu, None, window)
+    for name, g, e in zip(("o", "dq", "dr", "dk", "dv"), got, (ref_o, *ref_g)):
+        assert_close(g, e, TRAIN_REL_L2, TRAIN_MAX_REL, f"{lens} {hq}:{hkv} W={window} {dtype} {name}")
