@@ -19,7 +19,8 @@ pytestmark = pytest.mark.gpu
     ([96], 160, 160, -1, torch.bfloat16),
 ])
 def test_items_begin_with_either_group(lens, hq, hkv, window, dtype):
-    q, r, k, v, go, cu = (x.to(dtype) if x.is_floating_point() else x for x in tv.make(lens, hq, hkv, 64, 77))
+    *x, cu = tv.make(lens, hq, hkv, 64, 77)
+    q, r, k, v, go = (t.to(dtype) for t in x)
     got = tv.run_gpu(q, r, k, v, go, cu, window)
     ref_o = orc.varlen_forward(q, r, k, v, cu, None, window)["o"]
     ref_g = orc.varlen_backward(q, r, k, v, go.float(), cu, None, window)
