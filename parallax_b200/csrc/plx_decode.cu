@@ -26,7 +26,7 @@ namespace plx {
 
 __device__ __forceinline__ uint4 ld_stream16(const void *p) {
     uint4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n"
+    asm volatile("ld.global.L1::no_allocate.v4.u32 {%0,%1,%2,%3}, [%4];\n"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                  : "l"(p));
     return v;
@@ -88,10 +88,12 @@ __device__ __forceinline__ void cluster_sync() {
 
 // Paged cache: element offset of key kj of batch row b inside k / v (head and channel offsets not
 // included).  Dense caches are addressed by strides directly at the call sites.
-__device__ __forceinline__ int64_t paged_key_offset(const DecodeArgs &a, int b, int kj) {
+__device__ __forceinline__ uint32_t paged_key_page(const DecodeArgs &a, int b, int kj) {
     // page numbers are kept inside the pool: a row length that the caller is yet to find out of range may lead here
-    const uint32_t page = min(static_cast<uint32_t>(__ldg(a.page_table + static_cast<int64_t>(b) * a.pages_per_seq + (kj >> a.page_shift))), a.last_page);
-    return static_cast<int64_t>(page) * a.kv_sb + static_cast<int64_t>(kj & a.page_mask) * a.kv_st;
+    return min(static_cast<uint32_t>(a.page_table[static_cast<int64_t>(b) * a.pages_per_seq + (kj >> a.page_shift)]), a.last_page);
+}
+__device__ __forceinline__ int64_t paged_key_offset(const DecodeArgs &a, int b, int kj) {
+    return static_cast<int64_t>(paged_key_page(a, b, kj)) * a.kv_sb + static_cast<int64_t>(kj & a.page_mask) * a.kv_st;
 }
 
 __device__ __forceinline__ float finalize(float d1, float d2, float o1, float o2) {
@@ -112,13 +114,32 @@ __device__ __forceinline__ void store_elem<__half>(void *out, int64_t idx, float
 
 // Merge of n <= 32 partial records (stride REC floats) by one warp.  On return every lane holds the
 // maximum, the two sums, and the D / 32 channels lane * (D / 32) .. of O1 and O2, all relative to
-// the common maximum.
-template <int D>
+// the common maximum.  Bound by round trips to the L2: the channels of the first N records are requested together
+// with the headers of all.
+template <int D, int N = 8>
 __device__ __forceinline__ void warp_merge(const float *rec0, int n, int lane, float &big, float &D1, float &D2,
                                            float (&O1)[D / 32], float (&O2)[D / 32]) {
     constexpr int CH = D / 32, REC = 2 * D + 4;
     float4 h = make_float4(-INFINITY, 0.f, 0.f, 0.f);
     if (lane < n) h = __ldcg(reinterpret_cast<const float4 *>(rec0 + static_cast<int64_t>(lane) * REC));
+    const float *col = rec0 + 4 + lane * CH;
+    float x[N][CH], y[N][CH];
+    auto load = [&](int j0) {
+#pragma unroll
+        for (int j = 0; j < N; ++j) {
+            const float *pr = col + static_cast<int64_t>(min(j0 + j, n - 1)) * REC;   // weight 0 past the end
+            if (CH == 4) {
+                const float4 u = __ldcg(reinterpret_cast<const float4 *>(pr)), v = __ldcg(reinterpret_cast<const float4 *>(pr + D));
+                x[j][0] = u.x; x[j][1] = u.y; x[j][CH - 2] = u.z; x[j][CH - 1] = u.w;
+                y[j][0] = v.x; y[j][1] = v.y; y[j][CH - 2] = v.z; y[j][CH - 1] = v.w;
+            } else {
+                const float2 u = __ldcg(reinterpret_cast<const float2 *>(pr)), v = __ldcg(reinterpret_cast<const float2 *>(pr + D));
+                x[j][0] = u.x; x[j][1] = u.y;
+                y[j][0] = v.x; y[j][1] = v.y;
+            }
+        }
+    };
+    load(0);
     big = h.x;
 #pragma unroll
     for (int off = 16; off > 0; off >>= 1) big = fmaxf(big, __shfl_xor_sync(0xffffffffu, big, off));
@@ -133,32 +154,19 @@ __device__ __forceinline__ void warp_merge(const float *rec0, int n, int lane, f
     }
 #pragma unroll
     for (int e = 0; e < CH; ++e) O1[e] = O2[e] = 0.f;
-    const float *col = rec0 + 4 + lane * CH;
 #pragma unroll
-    for (int j0 = 0; j0 < 32; j0 += 8) {
+    for (int j0 = 0; j0 < 32; j0 += N) {
         if (j0 >= n) break;
-        float x[8][CH], y[8][CH], w[8];
+        if (j0 > 0) load(j0);
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            w[j] = __shfl_sync(0xffffffffu, wl, j0 + j);
-            const float *pr = col + static_cast<int64_t>(min(j0 + j, n - 1)) * REC;   // weight 0 past the end
-            if (CH == 4) {
-                const float4 u = __ldcg(reinterpret_cast<const float4 *>(pr)), v = __ldcg(reinterpret_cast<const float4 *>(pr + D));
-                x[j][0] = u.x; x[j][1] = u.y; x[j][CH - 2] = u.z; x[j][CH - 1] = u.w;
-                y[j][0] = v.x; y[j][1] = v.y; y[j][CH - 2] = v.z; y[j][CH - 1] = v.w;
-            } else {
-                const float2 u = __ldcg(reinterpret_cast<const float2 *>(pr)), v = __ldcg(reinterpret_cast<const float2 *>(pr + D));
-                x[j][0] = u.x; x[j][1] = u.y;
-                y[j][0] = v.x; y[j][1] = v.y;
-            }
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j)
+        for (int j = 0; j < N; ++j) {
+            const float w = __shfl_sync(0xffffffffu, wl, j0 + j);
 #pragma unroll
             for (int e = 0; e < CH; ++e) {
-                O1[e] = fmaf(w[j], x[j][e], O1[e]);
-                O2[e] = fmaf(w[j], y[j][e], O2[e]);
+                O1[e] = fmaf(w, x[j][e], O1[e]);
+                O2[e] = fmaf(w, y[j][e], O2[e]);
             }
+        }
     }
 }
 
@@ -252,8 +260,8 @@ __device__ __forceinline__ void exchange_merge_warp(const DecodeArgs &a, int64_t
 // Active key range [lo, hi) of a batch row, as indices into this buffer.
 __device__ __forceinline__ void row_range(const DecodeArgs &a, int b, int &lo, int &hi) {
     int hi_g = a.total_len;
-    if (a.seqused) hi_g = min(max(__ldg(a.seqused + b), 1), a.total_len);
-    int lo_g = a.cache_start ? max(__ldg(a.cache_start + b), 0) : 0;
+    if (a.seqused) hi_g = min(max(a.seqused[b], 1), a.total_len);
+    int lo_g = a.cache_start ? max(a.cache_start[b], 0) : 0;
     if (a.window >= 0) lo_g = max(lo_g, hi_g - a.window);
     lo = min(max(lo_g - a.kv_offset, 0), a.cache_len);
     hi = min(max(hi_g - a.kv_offset, 0), a.cache_len);
@@ -362,6 +370,28 @@ __device__ __forceinline__ SplitPlan plan_slot(const DecodeArgs &a, int slot, in
     return p;             // p.b < 0: a slot that no row needs
 }
 
+// Decode kernels are launched without waiting for the kernel before them to be over and done with (launch_overlapped): their
+// CTAs come as soon as its last one has left, and wait (grid_wait, before anything touches global memory) for its writes.
+// What they read may have been written while they were already resident, so no load takes the non-coherent path.
+// Calls one after the other, us: B = 1, 8192 keys, 32 : 8 heads 14.8 -> 13.1, 1000 keys 14.5 -> 12.1; 8 : 8 heads, B = 1, 4096
+// keys 12.2 -> 9.9, B = 32, 1024 keys 30.6 -> 28.5, B = 16, 8192 keys 92 -> 90.  Letting the next launch in earlier
+// (griddepcontrol.launch_dependents, at the start or after the sweep) was slower: its CTAs then go where SMs are free first
+// instead of evenly over the chip.  B = 64, 4096 keys, 32 : 8 heads, 128 CTAs: 164 us at the end, 180 after the sweep.
+template <typename... Params, typename... Args>
+static cudaError_t launch_overlapped(void (*kern)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t stream, const Args &...args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, args...);
+}
+
 // One WARP per (split, q head, batch row); a CTA is HG warps working on HG adjacent q
 // heads of the same key range, so that together they sweep contiguous memory (all heads
 // of a key are adjacent in the cache layout).  One q head per kv head.  Streams are merged by
@@ -378,6 +408,7 @@ __device__ __forceinline__ SplitPlan plan_slot(const DecodeArgs &a, int slot, in
 // launches without lengths were 0.3 to 0.6 us longer (32 rows of 300 down to 100 keys, 8 : 8 heads, 12.4 -> 13.0).
 template <typename T, int D, int HG, int U, bool SG, bool DEAL>
 __global__ void __launch_bounds__(HG * 32, U > 4 ? 1 : 512 / (HG * 32)) decode_kernel(const DecodeArgs a) {
+    grid_wait();
     constexpr int LPK = D / 8;      // lanes per key row
     constexpr int NS = 32 / LPK;    // streams per warp
     constexpr int REC = 2 * D + 4;  // floats per partial record
@@ -893,6 +924,7 @@ struct GqaSmem {
 // one kernel, with a register spilled: B = 64, 8192 keys, 32 q / 8 kv heads 348 us against 329, B = 8, 32768 keys 182 against 175.)
 template <typename T, int D, bool PAGED>
 __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const DecodeArgs a, int n_hgroups) {
+    grid_wait();
     constexpr int LD = D + 8;                       // padded row: ldmatrix without bank conflicts
     constexpr int REC = 2 * D + 4, CH = D / 32;
     constexpr int KS = D / 16;                      // k-steps of the score products
@@ -1223,21 +1255,19 @@ static int launch_decode_gqa(const DecodeArgs &a, cudaStream_t stream) {
         }
     }
     const int64_t ctas = (static_cast<int64_t>(a.batch) * a.n_splits + kGqaWarps - 1) / kGqaWarps * a.heads_kv * n_hgroups;
-    kern<<<static_cast<unsigned>(ctas), kGqaWarps * 32, kSmem, stream>>>(a, n_hgroups);
+    const cudaError_t st = launch_overlapped(kern, dim3(static_cast<unsigned>(ctas)), kGqaWarps * 32, kSmem, stream, a, n_hgroups);
     count_launch();
-    return cudaGetLastError() == cudaSuccess ? PLX_OK : PLX_ERR_LAUNCH;
+    return st == cudaSuccess && cudaGetLastError() == cudaSuccess ? PLX_OK : PLX_ERR_LAUNCH;
 }
 
 template <typename T, int D, int HG>
 static int launch_decode_hg(const DecodeArgs &a, cudaStream_t stream) {
     constexpr int U = 4;  // key rows per stream and register buffer (two buffers: 8 rows of K and of V in flight)
     dim3 grid(a.n_splits, a.heads_q / HG, a.batch);
-    if (a.balanced)
-        decode_kernel<T, D, HG, U, false, true><<<grid, HG * 32, 0, stream>>>(a);
-    else
-        decode_kernel<T, D, HG, U, false, false><<<grid, HG * 32, 0, stream>>>(a);
+    auto kern = a.balanced ? decode_kernel<T, D, HG, U, false, true> : decode_kernel<T, D, HG, U, false, false>;
+    const cudaError_t st = launch_overlapped(kern, grid, HG * 32, 0, stream, a);
     count_launch();
-    return cudaGetLastError() == cudaSuccess ? PLX_OK : PLX_ERR_LAUNCH;
+    return st == cudaSuccess && cudaGetLastError() == cudaSuccess ? PLX_OK : PLX_ERR_LAUNCH;
 }
 
 // number of SMs of the current device (cached per device; 0 on failure)
@@ -1278,11 +1308,13 @@ static int launch_decode_sg(const DecodeArgs &a, cudaStream_t stream) {
     cfg.blockDim = dim3(256);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = static_cast<unsigned>(n_cta);
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = static_cast<unsigned>(n_cta);
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
     cfg.attrs = attr;
     // When every CTA gets an SM of its own, a warp keeps 16 rows of K and of V in flight per buffer
     // (U = 8, more registers, one CTA per SM); otherwise 8 rows and two CTAs per SM.  The CTAs of a
@@ -1298,7 +1330,7 @@ static int launch_decode_sg(const DecodeArgs &a, cudaStream_t stream) {
         const int slot = n_cta == 2 ? 1 : n_cta == 4 ? 2 : 3;
         int n = resident[dev][slot].load(std::memory_order_acquire);
         if (n == 0) {
-            cfg.numAttrs = 1;
+            cfg.numAttrs = 2;
             if (cudaOccupancyMaxActiveClusters(&n, decode_kernel<T, D, 8, 8, true, false>, &cfg) != cudaSuccess || n < 1) {
                 (void)cudaGetLastError();
                 n = -1;
@@ -1308,7 +1340,7 @@ static int launch_decode_sg(const DecodeArgs &a, cudaStream_t stream) {
         roomy = roomy && units <= n;
     }
     auto kern = roomy ? decode_kernel<T, D, 8, 8, true, false> : decode_kernel<T, D, 8, 4, true, false>;
-    cfg.numAttrs = cluster ? 1 : 0;
+    cfg.numAttrs = cluster ? 2 : 1;
     cudaError_t st = cudaLaunchKernelEx(&cfg, kern, a);
     count_launch();
     return st == cudaSuccess && cudaGetLastError() == cudaSuccess ? PLX_OK : PLX_ERR_LAUNCH;
@@ -1378,6 +1410,7 @@ struct StageLens {
 };
 __global__ void __launch_bounds__(256) decode_stage_kernel(uint4 *q, const uint4 *q_src, uint4 *r, const uint4 *r_src, int64_t n16, int32_t *lens,
                                                            const __grid_constant__ StageLens src, int n) {
+    grid_wait();
     const int64_t i0 = static_cast<int64_t>(blockIdx.x) * 256 + threadIdx.x, step = static_cast<int64_t>(gridDim.x) * 256;
     for (int64_t i = i0; i < n16; i += step) {
         if (q_src) q[i] = q_src[i];
@@ -1394,10 +1427,11 @@ int launch_decode_stage(void *q, const void *q_src, void *r, const void *r_src, 
     const int64_t n16 = q_src || r_src ? static_cast<int64_t>(bytes / 16) : 0, items = n16 > n ? n16 : n;
     if (items == 0) return PLX_OK;
     const int64_t blocks = (items + 255) / 256;
-    decode_stage_kernel<<<static_cast<unsigned>(blocks < 1024 ? blocks : 1024), 256, 0, stream>>>(
-        static_cast<uint4 *>(q), static_cast<const uint4 *>(q_src), static_cast<uint4 *>(r), static_cast<const uint4 *>(r_src), n16, lens, src, n);
+    const cudaError_t st = launch_overlapped(decode_stage_kernel, dim3(static_cast<unsigned>(blocks < 1024 ? blocks : 1024)), 256, 0, stream,
+                                             static_cast<uint4 *>(q), static_cast<const uint4 *>(q_src), static_cast<uint4 *>(r),
+                                             static_cast<const uint4 *>(r_src), n16, lens, src, n);
     count_launch();
-    return cudaGetLastError() == cudaSuccess ? PLX_OK : PLX_ERR_LAUNCH;
+    return st == cudaSuccess && cudaGetLastError() == cudaSuccess ? PLX_OK : PLX_ERR_LAUNCH;
 }
 
 template <typename T, int D>
