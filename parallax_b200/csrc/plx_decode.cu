@@ -894,6 +894,11 @@ int launch_decode_exchange_merge(const ExchangeArgs &x, const float *part, int h
 // forms S1 = Q_g K^T and S2 = R_g K^T, runs the online softmax per row in the accumulator
 // fragments, and accumulates O1 += P1 V, O2 += P2 V with the P fragments as the A operand.  The eight
 // warps of a CTA are adjacent splits of one kv head; they meet in shared memory at the end.
+//
+// Short launches are bound by latency, long ones by HBM and by what the warps have in flight: three tiles each from the
+// start (q and r go straight to registers instead of through the last stage), the next one as soon as a stage is free.
+// 32 : 8 heads, us, with the transposed products below: B = 1, 8192 keys 15.4 -> 13.1, B = 1, 32768 keys 31.4 -> 28.4; B = 64,
+// 4096 keys 168 -> 164 (6.5 TB/s); 16 : 2 heads, B = 3, 3000 keys 15.0 -> 13.8.
 // ========================================================================= //
 // a lane's channels of a record, 16 or 8 bytes
 __device__ __forceinline__ void load_channels(const float *p, float (&x)[4]) {
@@ -911,6 +916,13 @@ __device__ __forceinline__ void store_channels(float *p, const float (&x)[2]) {
     __stcg(reinterpret_cast<float2 *>(p), make_float2(x[0], x[1]));
 }
 
+// transpose of an 8 x 8 block of 16-bit elements (lane 4 g + t holds elements 2 t, + 1 of row g)
+__device__ __forceinline__ uint32_t movmatrix_t(uint32_t x) {
+    uint32_t y;
+    asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;\n" : "=r"(y) : "r"(x));
+    return y;
+}
+
 constexpr int kGqaTile = 16;     // keys per staged tile
 constexpr int kGqaStages = 3;
 constexpr int kGqaWarps = kDecodeGqaWarps;   // warps (independent splits) per CTA
@@ -922,7 +934,12 @@ struct GqaSmem {
 
 // PAGED: a kernel of its own, so that the dense sweep carries neither the page numbers nor the choice in its loop.  (In
 // one kernel, with a register spilled: B = 64, 8192 keys, 32 q / 8 kv heads 348 us against 329, B = 8, 32768 keys 182 against 175.)
-template <typename T, int D, bool PAGED>
+//
+// FEW: at most 8 q heads per kv head, the usual case.  Then the products are transposed -- keys are the M dimension of the
+// scores (S^T = K Q_g^T), channels that of the outputs (O^T += V^T P^T), and the heads the 8 columns -- which takes half the
+// MMAs, with none of them on rows of zeros, and half the registers; a movmatrix per 8 x 8 block turns P^T around.
+// B = 16, 1024 keys, 32 : 8 heads 16.7 -> 16.0 us, B = 8, 4000 keys, rows of different lengths 40.8 -> 34.0.
+template <typename T, int D, bool PAGED, bool FEW>
 __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const DecodeArgs a, int n_hgroups) {
     grid_wait();
     constexpr int LD = D + 8;                       // padded row: ldmatrix without bank conflicts
@@ -951,33 +968,23 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
     auto sV = [&](int st) -> uint32_t { return sbase + st * 2 * kTileBytes + kTileBytes; };
     if (lane == 0) s_row[warp] = plan.b;
 
-    // ---- q and r of the group -> the buffers of the last stage; the first tiles follow at once
-    {
-        const T *qg = static_cast<const T *>(a.q) + (static_cast<int64_t>(b) * a.heads_q + hq0) * D;
-        const T *rg = static_cast<const T *>(a.r) + (static_cast<int64_t>(b) * a.heads_q + hq0) * D;
-#pragma unroll
-        for (int c = lane; c < 16 * CPR; c += 32) {
-            const int row = c / CPR, col = c % CPR;
-            const int bytes = row < n_rows ? 16 : 0;                      // rows past the group: zeros
-            const int64_t at = static_cast<int64_t>(row < n_rows ? row : 0) * D + col * 8;
-            cp_async16(sK(kGqaStages - 1) + (row * LD + col * 8) * 2, qg + at, bytes);
-            cp_async16(sV(kGqaStages - 1) + (row * LD + col * 8) * 2, rg + at, bytes);
-        }
-        cp_async_commit();
-    }
-
     // Tile i of this warp -> stage i % kGqaStages.  A lane copies the same 16-byte column of every
     // (32 / CPR)-th row, so its source and destination advance by constants; rows past my_hi (last tile
     // only) are zero-filled.  In a paged cache a tile lies in one page when pages hold at least a tile and the
     // range starts on a tile boundary (it does but for windows and cache_start): one page number per tile then,
-    // read a tile ahead.
+    // read three tiles ahead.
     constexpr int RPI = 32 / CPR;                                  // rows covered by one instruction of the warp
     const int my_row = lane / CPR, my_col = lane % CPR;
     const bool page_per_tile = PAGED && a.page_mask + 1 >= kGqaTile && my_lo % kGqaTile == 0;
     const T *kp = static_cast<const T *>(a.k) + (PAGED ? 0 : b * a.kv_sb) + hk * a.kv_sh + my_col * 8;
     const T *vp = static_cast<const T *>(a.v) + (PAGED ? 0 : b * a.kv_sb) + hk * a.kv_sh + my_col * 8;
     const uint32_t my_dst = (my_row * LD + my_col * 8) * 2;
-    int64_t next_tile = page_per_tile && n_tiles > 0 ? paged_key_offset(a, b, my_lo) : 0;   // of the next tile's first row
+    // pages of the next tiles to be loaded (as many as there are stages, so that no load waits for the page number of another)
+    uint32_t next_page[kGqaStages];
+    auto page_of_tile = [&](int i) -> uint32_t { return page_per_tile && i < n_tiles ? paged_key_page(a, b, my_lo + i * kGqaTile) : 0u; };
+    if (PAGED)
+#pragma unroll
+        for (int i = 0; i < kGqaStages; ++i) next_page[i] = page_of_tile(i);
     auto load_tile = [&](int i) {
         if (i < n_tiles) {
             const int st = i % kGqaStages, tile0 = my_lo + i * kGqaTile, key0 = tile0 + my_row;
@@ -985,8 +992,13 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
             const bool whole = tile0 + kGqaTile <= my_hi;
             if (!PAGED || page_per_tile) {
                 const int64_t step = static_cast<int64_t>(RPI) * a.kv_st;
-                const int64_t at = page_per_tile ? next_tile + my_row * a.kv_st : static_cast<int64_t>(key0) * a.kv_st;
-                if (page_per_tile && i + 1 < n_tiles) next_tile = paged_key_offset(a, b, tile0 + kGqaTile);
+                const int64_t at = page_per_tile ? static_cast<int64_t>(next_page[0]) * a.kv_sb + static_cast<int64_t>(key0 & a.page_mask) * a.kv_st
+                                                 : static_cast<int64_t>(key0) * a.kv_st;
+                if (PAGED) {
+#pragma unroll
+                    for (int n = 1; n < kGqaStages; ++n) next_page[n - 1] = next_page[n];
+                    next_page[kGqaStages - 1] = page_of_tile(i + kGqaStages);
+                }
                 if (whole) {
 #pragma unroll
                     for (int j = 0; j < kGqaTile / RPI; ++j) {
@@ -1013,32 +1025,102 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
         }
         cp_async_commit();             // always: keeps the group count uniform
     };
+    // q and r of the group as A fragments (rows past the group: zeros), straight from global memory, so that all stages
+    // are free for the first tiles; requested behind the first tile, with which they are needed.
+    // (FEW: as B fragments, of 8 rows.)
+    constexpr int QF = FEW ? 2 : 4;
+    uint32_t qa[KS][QF], ra[KS][QF];
+    load_tile(0);
+    {
+        const T *qg = static_cast<const T *>(a.q) + (static_cast<int64_t>(b) * a.heads_q + hq0) * D + 2 * t;
+        const T *rg = static_cast<const T *>(a.r) + (static_cast<int64_t>(b) * a.heads_q + hq0) * D + 2 * t;
 #pragma unroll
-    for (int i = 0; i < kGqaStages - 1; ++i) load_tile(i);
-
-    uint32_t qa[KS][4], ra[KS][4];     // q and r as A fragments
-    cp_async_wait<kGqaStages - 1>();
-    __syncwarp();
+        for (int ks = 0; ks < KS; ++ks)
 #pragma unroll
-    for (int ks = 0; ks < KS; ++ks) {
-        ldsm_x4(qa[ks], a_addr<LD>(sK(kGqaStages - 1), 0, ks * 16, lane));
-        ldsm_x4(ra[ks], a_addr<LD>(sV(kGqaStages - 1), 0, ks * 16, lane));
+            for (int e = 0; e < QF; ++e) {
+                const int row = FEW ? g : g + 8 * (e & 1), at = row * D + ks * 16 + 8 * (FEW ? e : e >> 1);
+                qa[ks][e] = row < n_rows ? *reinterpret_cast<const uint32_t *>(qg + at) : 0u;
+                ra[ks][e] = row < n_rows ? *reinterpret_cast<const uint32_t *>(rg + at) : 0u;
+            }
     }
-
-    // per-row state (rows g and g + 8 of the group); d1 / d2 are this thread's share until the end
-    float m[2] = {-INFINITY, -INFINITY}, d1[2] = {0.f, 0.f}, d2[2] = {0.f, 0.f};
-    float o1[D / 8][4], o2[D / 8][4];
 #pragma unroll
-    for (int i = 0; i < D / 8; ++i)
+    for (int i = 1; i < kGqaStages; ++i) load_tile(i);
+
+    // State of two rows of the group, g and g + 8 (FEW: 2 t and 2 t + 1); d1 / d2 are this thread's share until the end.
+    // Accumulators: channels 8 i + 2 t, + 1 of the two rows (FEW: channels 16 i + g and + 8).
+    constexpr int NO = FEW ? D / 16 : D / 8;
+    float m[2] = {-INFINITY, -INFINITY}, d1[2] = {0.f, 0.f}, d2[2] = {0.f, 0.f};
+    float o1[NO][4], o2[NO][4];
+#pragma unroll
+    for (int i = 0; i < NO; ++i)
 #pragma unroll
         for (int e = 0; e < 4; ++e) o1[i][e] = o2[i][e] = 0.f;
 
     for (int i = 0; i < n_tiles; ++i) {
         const int st = i % kGqaStages, key0 = my_lo + i * kGqaTile;
-        cp_async_wait<kGqaStages - 2>();
-        __syncwarp();                    // tile i has landed for every lane, and every lane has left tile i - 1 (i = 0: q and r)
-        load_tile(i + kGqaStages - 1);   // into the stage that tile i - 1 has just left
+        cp_async_wait<kGqaStages - 1>();
+        __syncwarp();                    // tile i has landed for every lane
 
+        if constexpr (FEW) {
+            // S1^T, S2^T: 16 keys x 8 rows; this thread has keys g and g + 8 of its two rows
+            float s1[4] = {0.f, 0.f, 0.f, 0.f}, s2[4] = {0.f, 0.f, 0.f, 0.f};
+#pragma unroll
+            for (int ks = 0; ks < KS; ++ks) {
+                uint32_t ka[4];
+                ldsm_x4(ka, a_addr<LD>(sK(st), 0, ks * 16, lane));
+                Elem<T>::mma(s1, ka, qa[ks][0], qa[ks][1]);
+                Elem<T>::mma(s2, ka, ra[ks][0], ra[ks][1]);
+            }
+            uint32_t pb1[2], pb2[2];
+            float alpha[2], m_safe[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+                s1[e] = key0 + g < my_hi ? s1[e] * a.c2 : -INFINITY;
+                s1[2 + e] = key0 + g + 8 < my_hi ? s1[2 + e] * a.c2 : -INFINITY;
+                float mx = fmaxf(s1[e], s1[2 + e]);
+#pragma unroll
+                for (int off = 4; off < 32; off <<= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, off));
+                const float m_new = fmaxf(m[e], mx);
+                m_safe[e] = m_new == -INFINITY ? 0.f : m_new;
+                alpha[e] = fast_exp2(m[e] - m_safe[e]);
+                m[e] = m_new;
+            }
+            if (alpha[0] != 1.f || alpha[1] != 1.f) {
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    d1[e] *= alpha[e];
+                    d2[e] *= alpha[e];
+                }
+#pragma unroll
+                for (int i2 = 0; i2 < NO; ++i2)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        o1[i2][e] *= alpha[e & 1];
+                        o2[i2][e] *= alpha[e & 1];
+                    }
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float p0 = fast_exp2(s1[2 * h] - m_safe[0]), p1 = fast_exp2(s1[2 * h + 1] - m_safe[1]);
+                const uint32_t u = Elem<T>::pack(p0, p1), w = Elem<T>::pack(p0 * s2[2 * h], p1 * s2[2 * h + 1]);
+                // (the sums are those of the ROUNDED weights, see below)
+                const float2 pr = Elem<T>::unpack(u), qr = Elem<T>::unpack(w);
+                d1[0] += pr.x;
+                d1[1] += pr.y;
+                d2[0] += qr.x;
+                d2[1] += qr.y;
+                pb1[h] = movmatrix_t(u);
+                pb2[h] = movmatrix_t(w);
+            }
+#pragma unroll
+            for (int cb = 0; cb < NO; ++cb) {
+                uint32_t vb[4];
+                ldsm_x4_t(vb, bt_addr<LD>(sV(st), 0, cb * 16, lane));
+                const uint32_t va[4] = {vb[0], vb[2], vb[1], vb[3]};
+                Elem<T>::mma(o1[cb], va, pb1[0], pb1[1]);
+                Elem<T>::mma(o2[cb], va, pb2[0], pb2[1]);
+            }
+        } else {
         // S1, S2: 16 rows x 16 keys (two 8-key blocks)
         float s1[2][4], s2[2][4];
 #pragma unroll
@@ -1108,34 +1190,45 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
             Elem<T>::mma(o2[2 * db], pa2, vb[0], vb[1]);
             Elem<T>::mma(o2[2 * db + 1], pa2, vb[2], vb[3]);
         }
+        }
+        __syncwarp();                    // every lane has left tile i
+        load_tile(i + kGqaStages);       // into its stage
     }
     cp_async_wait<0>();
 #pragma unroll
-    for (int hh = 0; hh < 2; ++hh) {
-        d1[hh] += __shfl_xor_sync(0xffffffffu, d1[hh], 1);
-        d1[hh] += __shfl_xor_sync(0xffffffffu, d1[hh], 2);
-        d2[hh] += __shfl_xor_sync(0xffffffffu, d2[hh], 1);
-        d2[hh] += __shfl_xor_sync(0xffffffffu, d2[hh], 2);
-    }
+    for (int hh = 0; hh < 2; ++hh)
+#pragma unroll
+        for (int off = FEW ? 4 : 1; off < (FEW ? 32 : 4); off <<= 1) {     // the lanes that share a row
+            d1[hh] += __shfl_xor_sync(0xffffffffu, d1[hh], off);
+            d2[hh] += __shfl_xor_sync(0xffffffffu, d2[hh], off);
+        }
 
     // ---- merge.  Every warp leaves its state in its own shared memory, where its tiles were: one record per row of
     // the group.  The warps of a batch row are neighbours (a segment).  The rows of all segments are dealt out to the
     // warps; a segment that is all of its (batch row, head) writes the result, any other one record per row to
     // global memory, and the CTA whose segment arrives last there merges those.
     // (Through global memory warp by warp, in two levels beyond 32 splits, the merge was most of a short launch, which is
-    // bound by latency: 29.5 us at B = 1, 8192 keys, 32 q / 8 kv heads, now 16.5.)
+    // bound by latency: B = 1, 8192 keys, 32 q / 8 kv heads 29.5 -> 16.5 us.)
     float *own = reinterpret_cast<float *>(gqa_smem + warp * GqaSmem<D>::kPerWarp);
-    __syncwarp();                        // every lane has left the last tile (and q, r, where there was none)
+    __syncwarp();                        // every lane has left the last tile
 #pragma unroll
     for (int hh = 0; hh < 2; ++hh) {
-        const int row = g + 8 * hh;
+        const int row = FEW ? 2 * t + hh : g + 8 * hh;
         if (row >= n_rows) continue;
-        float *rec = own + row * REC;    // this thread holds channels 8 i + 2 t, + 1
-        if (t == 0) *reinterpret_cast<float4 *>(rec) = make_float4(m[hh], d1[hh], d2[hh], 0.f);
+        float *rec = own + row * REC;
+        if ((FEW ? g : t) == 0) *reinterpret_cast<float4 *>(rec) = make_float4(m[hh], d1[hh], d2[hh], 0.f);
 #pragma unroll
-        for (int i = 0; i < D / 8; ++i) {
-            *reinterpret_cast<float2 *>(rec + 4 + 8 * i + 2 * t) = make_float2(o1[i][2 * hh], o1[i][2 * hh + 1]);
-            *reinterpret_cast<float2 *>(rec + 4 + D + 8 * i + 2 * t) = make_float2(o2[i][2 * hh], o2[i][2 * hh + 1]);
+        for (int i = 0; i < NO; ++i) {
+            if constexpr (FEW) {
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    rec[4 + 16 * i + 8 * c + g] = o1[i][2 * c + hh];
+                    rec[4 + D + 16 * i + 8 * c + g] = o2[i][2 * c + hh];
+                }
+            } else {
+                *reinterpret_cast<float2 *>(rec + 4 + 8 * i + 2 * t) = make_float2(o1[i][2 * hh], o1[i][2 * hh + 1]);
+                *reinterpret_cast<float2 *>(rec + 4 + D + 8 * i + 2 * t) = make_float2(o2[i][2 * hh], o2[i][2 * hh + 1]);
+            }
         }
     }
     // segment of this warp: warps w0 .. w0 + n_seg - 1; where its (batch row, head) begins among the slots
@@ -1214,10 +1307,10 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
     // last: merge the n_ctas records of every row, 32 at a time
     for (int row = warp - w0; row < n_rows; row += n_seg) {
         const float *recs = recs_of(row);
-        warp_merge<D>(recs, min(n_ctas, 32), lane, big, D1, D2, O1, O2);
+        warp_merge<D, 16>(recs, min(n_ctas, 32), lane, big, D1, D2, O1, O2);
         for (int j = 32; j < n_ctas; j += 32) {
             float big2, E1, E2, P1[CH], P2[CH];
-            warp_merge<D>(recs + static_cast<int64_t>(j) * REC, min(n_ctas - j, 32), lane, big2, E1, E2, P1, P2);
+            warp_merge<D, 16>(recs + static_cast<int64_t>(j) * REC, min(n_ctas - j, 32), lane, big2, E1, E2, P1, P2);
             const float top = fmaxf(big, big2), safe = top == -INFINITY ? 0.f : top;
             const float wa = fast_exp2(big - safe), wb = fast_exp2(big2 - safe);
             big = top;
@@ -1234,11 +1327,11 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
     if (warp == w0 && lane == 0) a.ws_counters[bh_of(0)] = 0;   // ready for the next launch on this workspace
 }
 
-template <typename T, int D, bool PAGED>
+template <typename T, int D, bool PAGED, bool FEW>
 static int launch_decode_gqa(const DecodeArgs &a, cudaStream_t stream) {
     const int n_hgroups = (a.n_rep + 15) / 16;
     constexpr int kSmem = kGqaWarps * GqaSmem<D>::kPerWarp;
-    auto kern = decode_gqa_kernel<T, D, PAGED>;
+    auto kern = decode_gqa_kernel<T, D, PAGED, FEW>;
     {   // the shared-memory opt-in is a per-device function attribute: set it once per device
         constexpr int kMaxDevices = 64;
         static std::mutex mu;
@@ -1348,8 +1441,10 @@ static int launch_decode_sg(const DecodeArgs &a, cudaStream_t stream) {
 
 template <typename T, int D>
 static int launch_decode_t(const DecodeArgs &a, cudaStream_t stream) {
-    if (a.n_rep >= 2)   // grouped heads: tensor-core kernel
-        return a.page_table ? launch_decode_gqa<T, D, true>(a, stream) : launch_decode_gqa<T, D, false>(a, stream);
+    if (a.n_rep > 8)    // grouped heads: tensor-core kernel
+        return a.page_table ? launch_decode_gqa<T, D, true, false>(a, stream) : launch_decode_gqa<T, D, false, false>(a, stream);
+    if (a.n_rep >= 2)
+        return a.page_table ? launch_decode_gqa<T, D, true, true>(a, stream) : launch_decode_gqa<T, D, false, true>(a, stream);
     if (decode_split_groups(a)) return launch_decode_sg<T, D>(a, stream);
     // adjacent q heads share a CTA (one warp each): the largest group that divides the head count
     if (a.heads_q % 8 == 0) return launch_decode_hg<T, D, 8>(a, stream);

@@ -1,9 +1,11 @@
-"""Decode launches that overlap the end of the kernel before them."""
+"""Decode launches that overlap the end of the kernel before them, and the grouped-head sweep at the edges of its tiles and
+stages."""
 import pytest
 import torch
 
 import parallax_b200 as plx
-from tests._util import seeded_bf16
+from oracle import parallax_oracle as orc
+from tests._util import DECODE_MAX_REL, DECODE_REL_L2, assert_close, seeded_bf16
 
 pytestmark = pytest.mark.gpu
 
@@ -43,3 +45,17 @@ def test_calls_that_feed_each_other(bsz, hq, hkv, t, page):
     want = chain(torch.cuda.synchronize)
     for x, y in zip(chain(lambda: None), want):
         assert torch.equal(x, y)
+
+
+@pytest.mark.parametrize("hq,hkv,d", [(4, 1, 128), (18, 1, 128), (32, 8, 64)])
+def test_grouped_heads_at_the_edges_of_tiles_and_stages(hq, hkv, d, monkeypatch):
+    """0 to 5 tiles of 16 keys per warp (three stages), the last one whole, of one key and one key short."""
+    monkeypatch.setenv("PLX_DECODE_SPLITS", "2")
+    for t in (1, 15, 16, 17, 33, 47, 48, 63, 64, 65, 95, 96, 97, 129, 160):
+        q, r, k, v = inputs(1, hq, hkv, t, d, seed=t)
+        o = plx.parallax_decode(q, r, k, v)
+        assert_close(o.float().cpu(), orc.decode(*[x.cpu() for x in (q, r, k, v)]), DECODE_REL_L2, DECODE_MAX_REL, f"{hq}:{hkv} {t}")
+        if t % 16 == 0:
+            table = torch.arange(t // 16, device="cuda", dtype=torch.int32).flip(0).view(1, -1)
+            kp, vp = (x.view(t // 16, 16, hkv, d).flip(0).contiguous() for x in (k, v))
+            assert torch.equal(plx.parallax_attn_with_kvcache(q, r, kp, vp, page_table=table), o)
