@@ -26,6 +26,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <list>
+#include <memory>
 #include <mutex>
 #include <optional>
 
@@ -324,16 +325,56 @@ Workspaces &workspaces() {
     return *w;
 }
 
-// The lengths of the rows on their way to the host.  The copy is queued BEFORE the launch they belong to and
-// waited for after it, so reading them does not leave the GPU idle.  Launching on lengths that turn out to be out
+// A stream of this library beside one of the caller's, for small copies that must not stand between two kernels there.
+// One per (device, stream), so that no copy waits for work of a stream that it has nothing to do with.  At most kMax are
+// kept; one that is dropped lives on until its last user has waited for its copy.
+class SideStreams {
+public:
+    using Handle = std::shared_ptr<CUstream_st>;
+    Handle get(const c10::cuda::CUDAStream &main) {
+        const Key key{main.device_index(), reinterpret_cast<uintptr_t>(main.stream())};
+        std::lock_guard<std::mutex> lock(mu_);
+        for (auto it = list_.begin(); it != list_.end(); ++it)
+            if (it->first == key) {
+                list_.splice(list_.begin(), list_, it);
+                return it->second;
+            }
+        cudaStream_t made = nullptr;
+        C10_CUDA_CHECK(cudaStreamCreateWithFlags(&made, cudaStreamNonBlocking));
+        list_.emplace_front(key, Handle(made, [](cudaStream_t st) { (void)cudaStreamDestroy(st); }));
+        if (list_.size() > kMax) list_.pop_back();
+        return list_.front().second;
+    }
+
+private:
+    using Key = std::pair<int64_t, uintptr_t>;
+    static constexpr size_t kMax = 32;
+    std::mutex mu_;
+    std::list<std::pair<Key, Handle>> list_;
+};
+SideStreams &side_streams() {
+    static SideStreams *s = new SideStreams;   // not destroyed at exit, when the CUDA context may be gone
+    return *s;
+}
+
+// The lengths of the rows on their way to the host.  The copy is queued before the launch they belong to and waited for
+// after it, so reading them does not leave the GPU idle; in a launch that lasts (`beside`) it runs beside the launch, behind
+// what the stream held before it, and is no gap between two launches either.  Launching on lengths that turn out to be out
 // of range is harmless: the kernels clamp them (and page numbers) to the buffers, and the result is dropped.
 class LengthCheck {
 public:
-    LengthCheck(const OptTensor &lens, const c10::cuda::CUDAStream &stream) {
+    LengthCheck(const OptTensor &lens, const c10::cuda::CUDAStream &stream, bool beside) {
         if (!lens) return;
         host_ = at::empty({lens->numel()}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
-        C10_CUDA_CHECK(cudaMemcpyAsync(host_.data_ptr(), lens->data_ptr(), sizeof(int32_t) * lens->numel(), cudaMemcpyDeviceToHost, stream.stream()));
-        copied_.record(stream);
+        c10::cuda::CUDAStream on = stream;
+        if (beside) {
+            side_ = side_streams().get(stream);
+            on = c10::cuda::getStreamFromExternal(side_.get(), stream.device_index());
+            ready_.record(stream);
+            ready_.block(on);
+        }
+        C10_CUDA_CHECK(cudaMemcpyAsync(host_.data_ptr(), lens->data_ptr(), sizeof(int32_t) * lens->numel(), cudaMemcpyDeviceToHost, on.stream()));
+        copied_.record(on);
     }
     ~LengthCheck() {
         if (host_.defined() && !waited_) cudaEventSynchronize(copied_.event());   // the copy still writes to host_
@@ -353,9 +394,20 @@ public:
 
 private:
     Tensor host_;
-    at::cuda::CUDAEvent copied_{cudaEventDisableTiming};
+    SideStreams::Handle side_;
+    at::cuda::CUDAEvent ready_{cudaEventDisableTiming}, copied_{cudaEventDisableTiming};
     bool waited_ = false;
 };
+
+// What lasts: by the keys and values of a decode launch at the cache ceiling, by the products of a prefill launch.  The
+// way over a second stream takes the host 1 to 2 us more per call, which short launches do not hide.  Before the launch
+// against beside it, us per call: 32 : 8 heads, 4 MB 18.9 / 19.0, 17 MB 22.5 / 20.2, 34 MB 26.6 / 18.4, 134 MB 40.6 / 30.7; 8 : 8
+// heads, 8 MB 15.2 / 16.8, 34 MB 16.7 / 17.1, 67 MB 27.5 / 21.3; prefill, 0.3 GFLOP 15.9 / 17.0, 1.1 GFLOP 23.4 / 17.5, 137 GFLOP
+// 107 / 101.
+bool decode_lasts(const Tensor &q, const Tensor &k, int64_t n_keys) {
+    return 4. * q.size(0) * n_keys * k.size(2) * q.size(3) >= (q.size(2) > k.size(2) ? 4e6 : 48e6);
+}
+bool prefill_lasts(const Tensor &q, int64_t ceiling) { return 8. * q.numel() * ceiling >= 1e9; }
 
 bool int32_vector(const OptTensor &t, int64_t n, const at::Device &device) {
     return !t || (plain_tensor(*t) && t->scalar_type() == at::kInt && t->dim() == 1 && t->size(0) == n && t->is_contiguous() && t->device() == device);
@@ -380,6 +432,30 @@ bool cache_call_ok(const Tensor &q, const Tensor &r, const Tensor &k, const Tens
     return int32_vector(lens, q.size(0), q.device()) && page_table_ok(table, q.size(0), k.size(1), q.device()) && !recorded({&q, &r, &k, &v});
 }
 
+plx_decode_problem decode_problem(const Tensor &q, const Tensor &k, int64_t ceiling, const OptTensor &table, double scale, int64_t window,
+                                  int32_t n_splits) {
+    plx_decode_problem p{};
+    p.dtype = dtype_code(q);
+    p.batch = static_cast<int32_t>(q.size(0));
+    p.heads_q = static_cast<int32_t>(q.size(2));
+    p.heads_kv = static_cast<int32_t>(k.size(2));
+    p.head_dim = static_cast<int32_t>(q.size(3));
+    p.cache_len = static_cast<int32_t>(ceiling);
+    p.window_left = static_cast<int32_t>(window);
+    p.qk_scale = static_cast<float>(scale);
+    p.n_splits = n_splits;
+    p.kv_stride_b = k.stride(0);
+    p.kv_stride_t = k.stride(1);
+    p.kv_stride_h = k.stride(2);
+    if (table) {
+        p.page_table = int_ptr(table);
+        p.page_size = static_cast<int32_t>(k.size(1));
+        p.pages_per_seq = static_cast<int32_t>(table->size(1));
+        p.n_pages = static_cast<int32_t>(k.size(0));
+    }
+    return p;
+}
+
 py::object decode(const py::object &q_, const py::object &r_, const py::object &k_, const py::object &v_, const py::object &scale_,
                   const py::object &window_, const py::object &lens_, const py::object &start_, const py::object &table_) {
     bool ok = true;
@@ -397,31 +473,14 @@ py::object decode(const py::object &q_, const py::object &r_, const py::object &
     if (capturing()) return py::none();
     RECORD_FUNCTION("plx::decode_out", Values({q, r, k, v}));
     const c10::cuda::CUDAStream stream = c10::cuda::getCurrentCUDAStream();
-    plx_decode_problem p{};
-    p.dtype = dtype_code(q);
-    p.batch = static_cast<int32_t>(q.size(0));
-    p.heads_q = static_cast<int32_t>(q.size(2));
-    p.heads_kv = static_cast<int32_t>(k.size(2));
-    p.head_dim = static_cast<int32_t>(q.size(3));
-    p.cache_len = static_cast<int32_t>(ceiling);
-    p.window_left = static_cast<int32_t>(window);
-    p.qk_scale = static_cast<float>(scale);
-    p.kv_stride_b = k.stride(0);
-    p.kv_stride_t = k.stride(1);
-    p.kv_stride_h = k.stride(2);
-    if (table) {
-        p.page_table = int_ptr(table);
-        p.page_size = static_cast<int32_t>(k.size(1));
-        p.pages_per_seq = static_cast<int32_t>(table->size(1));
-        p.n_pages = static_cast<int32_t>(k.size(0));
-    }
+    plx_decode_problem p = decode_problem(q, k, ceiling, table, scale, window, 1);
     const int32_t n_keys = window < 0 ? p.cache_len : std::max(1, std::min(p.cache_len, p.window_left));
     p.n_splits = api.decode_choose_splits_gqa(p.batch, p.heads_q, p.heads_kv, n_keys, at::cuda::getDeviceProperties(q.get_device())->multiProcessorCount);
     size_t need = 0;
     if (api.decode_workspace_bytes(&p, &need) != PLX_OK) return py::none();
     const Tensor ws = workspaces().get(stream, q, p.n_splits, static_cast<int64_t>(need / sizeof(float)));
     Tensor out = at::empty(q.sizes(), q.options());
-    LengthCheck check(lens, stream);
+    LengthCheck check(lens, stream, decode_lasts(q, k, n_keys));
     if (api.decode(&p, q.data_ptr(), r.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), int_ptr(lens), int_ptr(start), ws.data_ptr(), need,
                    stream.stream()) != PLX_OK ||
         !check.within(1, ceiling))
@@ -448,7 +507,7 @@ py::object extend(const py::object &q_, const py::object &r_, const py::object &
     plx_train_problem p = train_problem(q, k, Tensor(), scale, window, kBTHD, std::nullopt);
     p.len_k = static_cast<int32_t>(ceiling);
     Tensor out = at::empty(q.sizes(), q.options());
-    LengthCheck check(lens, stream);
+    LengthCheck check(lens, stream, prefill_lasts(q, ceiling));
     if (api.train_extend(&p, q.data_ptr(), r.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), int_ptr(lens), int_ptr(table),
                          table ? static_cast<int32_t>(k.size(1)) : 0, table ? static_cast<int32_t>(table->size(1)) : 0,
                          table ? static_cast<int32_t>(k.size(0)) : 0, stream.stream()) != PLX_OK ||

@@ -1,5 +1,5 @@
-"""Decode launches that overlap the end of the kernel before them, and the grouped-head sweep at the edges of its tiles and
-stages."""
+"""Decode launches that overlap the end of the kernel before them, the grouped-head sweep at the edges of its tiles and
+stages, and the lengths that reach the host beside a launch."""
 import pytest
 import torch
 
@@ -59,3 +59,27 @@ def test_grouped_heads_at_the_edges_of_tiles_and_stages(hq, hkv, d, monkeypatch)
             table = torch.arange(t // 16, device="cuda", dtype=torch.int32).flip(0).view(1, -1)
             kp, vp = (x.view(t // 16, 16, hkv, d).flip(0).contiguous() for x in (k, v))
             assert torch.equal(plx.parallax_attn_with_kvcache(q, r, kp, vp, page_table=table), o)
+
+
+@pytest.mark.parametrize("bsz,hq,hkv,t,lq", [(2, 32, 8, 4096, 1), (8, 16, 16, 2048, 1), (2, 32, 8, 700, 64)])
+def test_lengths_beside_a_long_launch(bsz, hq, hkv, t, lq):
+    """The lengths are checked as they are in stream order -- written by a kernel that is still to run when the call is made,
+    on any stream -- and a length out of range raises, whichever row it is in."""
+    _, _, k, v = inputs(bsz, hq, hkv, t)
+    q = seeded_bf16((bsz, lq, hq, 128), 9).cuda()
+    lens = torch.full((bsz,), t, dtype=torch.int32, device="cuda")
+    want = plx.parallax_attn_with_kvcache(q, q, k, v, seqused_k=lens)
+    big = torch.randn(4096, 4096, device="cuda")
+    for stream in (torch.cuda.current_stream(), torch.cuda.Stream(), torch.cuda.Stream()):
+        with torch.cuda.stream(stream):
+            for row in range(bsz):
+                lens.fill_(t)
+                for _ in range(8):
+                    big @ big
+                bad = lens.clone()
+                bad[row] = t + 1
+                with pytest.raises(ValueError):
+                    plx.parallax_attn_with_kvcache(q, q, k, v, seqused_k=bad)
+                bad[row] = t
+                assert torch.equal(plx.parallax_attn_with_kvcache(q, q, k, v, seqused_k=bad), want)
+        torch.cuda.synchronize()
