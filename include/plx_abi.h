@@ -220,6 +220,14 @@ int plx_decode_workspace_bytes(const plx_decode_problem *p, size_t *bytes);
 int plx_decode_stage(void *q, const void *q_src, void *r, const void *r_src, size_t bytes,
                      int32_t *seqused_k, const int32_t *seqused_src, int32_t n, plx_stream_t stream);
 
+/* plx_decode_stage and the plx_decode behind it (no cache_start) as ONE launch, for at most PLX_DECODE_STEP_ROWS batch rows
+ * (else PLX_ERR_UNSUPPORTED): the sweep reads q_src and r_src (null: q, r) and the HOST lengths seqused_src (null: the
+ * device array seqused_k, or none) and leaves copies in q, r and seqused_k. */
+#define PLX_DECODE_STEP_ROWS 64
+int plx_decode_step(const plx_decode_problem *p, void *q, const void *q_src, void *r, const void *r_src,
+                    const void *k, const void *v, void *out, int32_t *seqused_k, const int32_t *seqused_src,
+                    void *workspace, size_t workspace_bytes, plx_stream_t stream);
+
 /* out = Parallax decode.  seqused_k and cache_start are device int32 (batch,)
  * arrays or NULL.  Replaces parallax.triton.parallax_decode + its kernel
  * [parallax/triton/parallax_decode.py:100-148, 20-97] and the CuTeDSL path

@@ -23,7 +23,7 @@ ABI_VERSION = 3
 SYMBOLS = (
     "plx_abi_version", "plx_strerror", "plx_kernel_launch_count", "plx_device_error", "plx_device_error_peek",
     "plx_train_workspace_bytes", "plx_train_fwd", "plx_train_extend", "plx_train_bwd", "plx_train_bwd_stages",
-    "plx_decode_choose_splits", "plx_decode_choose_splits_gqa", "plx_decode_workspace_bytes", "plx_decode_stage", "plx_decode", "plx_decode_static", "plx_decode_partial",
+    "plx_decode_choose_splits", "plx_decode_choose_splits_gqa", "plx_decode_workspace_bytes", "plx_decode_stage", "plx_decode_step", "plx_decode", "plx_decode_static", "plx_decode_partial",
     "plx_decode_merge", "plx_decode_exchange_bytes", "plx_decode_exchange_merge", "plx_decode_partial_exchange",
 )
 EXCHANGE_MAX_RANKS = 16
@@ -101,6 +101,8 @@ def _declare(lib):
     lib.plx_decode_workspace_bytes.argtypes = [C.POINTER(DecodeProblem), C.POINTER(sz)]
     lib.plx_decode_stage.restype = C.c_int
     lib.plx_decode_stage.argtypes = [vp, vp, vp, vp, sz, vp, vp, i32, vp]
+    lib.plx_decode_step.restype = C.c_int
+    lib.plx_decode_step.argtypes = [C.POINTER(DecodeProblem)] + [vp] * 9 + [vp, sz, vp]
     lib.plx_decode.restype = C.c_int
     lib.plx_decode.argtypes = [C.POINTER(DecodeProblem)] + [vp] * 7 + [vp, sz, vp]
     lib.plx_decode_static.restype = C.c_int

@@ -129,9 +129,17 @@ static int make_exchange_args(const plx_exchange *x, ExchangeArgs &e) {
     return PLX_OK;
 }
 
+// where a step leaves copies of its inputs (null: nowhere)
+struct StepCopies {
+    void *q, *r;
+    int32_t *lens;
+    const int32_t *lens_src;   // host
+};
+
 static int run_decode(const plx_decode_problem *p, const void *q, const void *r, const void *k, const void *v, void *out,
                       float *part, const int32_t *seqused_k, const int32_t *cache_start, void *workspace,
-                      size_t workspace_bytes, cudaStream_t stream, const plx_exchange *xch = nullptr) {
+                      size_t workspace_bytes, cudaStream_t stream, const plx_exchange *xch = nullptr,
+                      const StepCopies *step = nullptr) {
     int st = check_decode_args(p, q, r, k, v, out, part);
     if (st != PLX_OK) return st;
     if (p->n_splits > 1 && (!workspace || workspace_bytes < decode_ws_bytes(p) || misaligned16(workspace)))
@@ -166,6 +174,13 @@ static int run_decode(const plx_decode_problem *p, const void *q, const void *r,
         if (!ew.word) return PLX_ERR_LAUNCH;
         a.xch.err_word = ew.word;
         a.xch.err_mirror = ew.mirror;
+    }
+    if (step) {
+        a.q_copy = step->q;
+        a.r_copy = step->r;
+        a.lens_copy = step->lens_src ? step->lens : nullptr;
+        a.n_lens = step->lens_src ? p->batch : 0;
+        for (int i = 0; i < a.n_lens; ++i) a.lens[i] = step->lens_src[i];
     }
     a.page_table = p->page_table;
     if (p->page_table) {
@@ -418,6 +433,15 @@ int plx_decode_stage(void *q, const void *q_src, void *r, const void *r_src, siz
     int st = check_device();
     if (st != PLX_OK) return st;
     return launch_decode_stage(q, q_src, r, r_src, bytes, seqused_k, seqused_src, n, reinterpret_cast<cudaStream_t>(stream));
+}
+
+int plx_decode_step(const plx_decode_problem *p, void *q, const void *q_src, void *r, const void *r_src, const void *k, const void *v, void *out,
+                    int32_t *seqused_k, const int32_t *seqused_src, void *workspace, size_t workspace_bytes, plx_stream_t stream) {
+    if (!p || !out || !q || !r || (seqused_src && !seqused_k) || misaligned16(q) || misaligned16(r)) return PLX_ERR_BAD_ARG;
+    if (p->batch > PLX_DECODE_STEP_ROWS) return PLX_ERR_UNSUPPORTED;
+    const StepCopies step{q_src ? q : nullptr, r_src ? r : nullptr, seqused_k, seqused_src};
+    return run_decode(p, q_src ? q_src : q, r_src ? r_src : r, k, v, out, nullptr, seqused_src ? nullptr : seqused_k, nullptr, workspace,
+                      workspace_bytes, reinterpret_cast<cudaStream_t>(stream), nullptr, &step);
 }
 
 int plx_decode(const plx_decode_problem *p, const void *q, const void *r, const void *k, const void *v, void *out,

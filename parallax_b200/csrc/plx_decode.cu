@@ -260,7 +260,8 @@ __device__ __forceinline__ void exchange_merge_warp(const DecodeArgs &a, int64_t
 // Active key range [lo, hi) of a batch row, as indices into this buffer.
 __device__ __forceinline__ void row_range(const DecodeArgs &a, int b, int &lo, int &hi) {
     int hi_g = a.total_len;
-    if (a.seqused) hi_g = min(max(a.seqused[b], 1), a.total_len);
+    if (a.n_lens) hi_g = min(max(a.lens[b], 1), a.total_len);
+    else if (a.seqused) hi_g = min(max(a.seqused[b], 1), a.total_len);
     int lo_g = a.cache_start ? max(a.cache_start[b], 0) : 0;
     if (a.window >= 0) lo_g = max(lo_g, hi_g - a.window);
     lo = min(max(lo_g - a.kv_offset, 0), a.cache_len);
@@ -440,8 +441,14 @@ __global__ void __launch_bounds__(HG * 32, U > 4 ? 1 : 512 / (HG * 32)) decode_k
     float qf[8], rf[8];
     {
         const int64_t qi = (static_cast<int64_t>(b) * a.heads_q + hq) * D + sl * 8;
-        unpack8<T>(*reinterpret_cast<const uint4 *>(static_cast<const T *>(a.q) + qi), qf);
-        unpack8<T>(*reinterpret_cast<const uint4 *>(static_cast<const T *>(a.r) + qi), rf);
+        const uint4 qv = *reinterpret_cast<const uint4 *>(static_cast<const T *>(a.q) + qi), rv = *reinterpret_cast<const uint4 *>(static_cast<const T *>(a.r) + qi);
+        unpack8<T>(qv, qf);
+        unpack8<T>(rv, rf);
+        if (plan.part == 0 && sid == 0) {
+            if (a.q_copy) *reinterpret_cast<uint4 *>(static_cast<T *>(a.q_copy) + qi) = qv;
+            if (a.r_copy) *reinterpret_cast<uint4 *>(static_cast<T *>(a.r_copy) + qi) = rv;
+            if (a.lens_copy && hq == 0 && sl == 0) a.lens_copy[b] = a.lens[b];
+        }
     }
     const bool paged = a.page_table != nullptr;      // uniform over the launch
     const int64_t row0 = (paged ? 0 : b * a.kv_sb) + hq * a.kv_sh + sl * 8;
@@ -1195,6 +1202,14 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
         load_tile(i + kGqaStages);       // into its stage
     }
     cp_async_wait<0>();
+    if (plan.b >= 0 && plan.part == 0) {
+        const int64_t at = (static_cast<int64_t>(b) * a.heads_q + hq0) * D;
+        for (int c = lane; c < n_rows * CPR; c += 32) {
+            if (a.q_copy) reinterpret_cast<uint4 *>(static_cast<T *>(a.q_copy) + at)[c] = reinterpret_cast<const uint4 *>(static_cast<const T *>(a.q) + at)[c];
+            if (a.r_copy) reinterpret_cast<uint4 *>(static_cast<T *>(a.r_copy) + at)[c] = reinterpret_cast<const uint4 *>(static_cast<const T *>(a.r) + at)[c];
+        }
+        if (a.lens_copy && hunit == 0 && lane == 0) a.lens_copy[b] = a.lens[b];
+    }
 #pragma unroll
     for (int hh = 0; hh < 2; ++hh)
 #pragma unroll
@@ -1471,7 +1486,7 @@ bool decode_fused_exchange_supported(const DecodeArgs &a) {
 // 14.7 us).  Also against an even cut of grouped heads: rows that end inside a CTA of another row (3 rows of 1000 keys in 15
 // parts, 16 : 2 heads, 20.0 us even, 15.0 dealt out).
 static int balance_from(const DecodeArgs &a, int head_dim) {
-    if ((!a.seqused && !a.cache_start) || a.batch < 2 || a.batch > kBalancedRows || a.n_splits < 2 || a.part_out || a.xch.world != 0 ||
+    if ((!a.seqused && !a.n_lens && !a.cache_start) || a.batch < 2 || a.batch > kBalancedRows || a.n_splits < 2 || a.part_out || a.xch.world != 0 ||
         decode_split_groups(a))
         return 0;
     const int64_t n_keys = a.window >= 0 && a.window < a.cache_len ? a.window : a.cache_len, part = n_keys / a.n_splits * head_dim;

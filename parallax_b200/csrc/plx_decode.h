@@ -36,6 +36,12 @@ struct DecodeArgs {
     const int32_t *page_table;
     int page_shift, page_mask, pages_per_seq;
     uint32_t last_page;   // page numbers above it are read as it
+    // Inputs of a step from elsewhere (plx_decode_step): q, r (where the pointers above are not the step's buffers) and the
+    // active lengths, which come in the launch parameters, are copied to the buffers by the first part of each row.
+    void *q_copy, *r_copy;
+    int32_t *lens_copy;
+    int n_lens;           // 0: lengths from `seqused`
+    int32_t lens[PLX_DECODE_STEP_ROWS];
     // Fused sweep + exchange (xch.world >= 1): the warp that holds the merged state of a (batch, head) does
     // not write a partial record but pushes it to every rank's inbox, waits for the peers' and merges.
     ExchangeArgs xch;

@@ -5,7 +5,7 @@
 // which stays the definition of the API: each function returns None, with nothing enqueued that shows, for any
 // call that is not plainly an eager one on well-formed CUDA tensors -- a tensor subclass, a torch function or
 // dispatch mode, functorch or forward-mode differentiation, tracing, shapes, strides or types that need a copy or an
-// error message -- and the caller then takes the Python path, which handles it or raises.  decode, extend and stage also
+// error message -- and the caller then takes the Python path, which handles it or raises.  decode, extend and step also
 // leave a stream that is being captured to it; train and extend a device error waiting to be reported (the ops
 // of a single-token step do not look at it either).  decode and extend find a length out of range after their launch,
 // whose result is then dropped.
@@ -52,6 +52,7 @@ struct Api {
     decltype(&plx_decode_workspace_bytes) decode_workspace_bytes;
     decltype(&plx_decode) decode;
     decltype(&plx_decode_stage) decode_stage;
+    decltype(&plx_decode_step) decode_step;
 };
 Api api;
 
@@ -69,6 +70,7 @@ void bind(const py::dict &addresses) {
     bind_one(api.decode_workspace_bytes, addresses, "plx_decode_workspace_bytes");
     bind_one(api.decode, addresses, "plx_decode");
     bind_one(api.decode_stage, addresses, "plx_decode_stage");
+    bind_one(api.decode_step, addresses, "plx_decode_step");
 }
 
 // ------------------------------------------------------------------------- //
@@ -523,40 +525,58 @@ py::object attend(const py::object &q, const py::object &r, const py::object &k,
     return t.dim() == 4 && t.size(1) == 1 ? decode(q, r, k, v, scale, window, lens, py::none(), table) : extend(q, r, k, v, scale, window, lens, table);
 }
 
-// q, r and the lengths of a GraphedDecode step into its buffers; False, having done nothing, for anything but
-// tensors like the buffers and lengths given as Python integers in [1, most].
-bool stage(const py::object &q_, const py::object &q_src_, const py::object &r_, const py::object &r_src_, const py::object &lens_,
-           const py::object &lens_src, int64_t most) {
+// A GraphedDecode step: q, r and the lengths into its buffers, and the launch that its graph holds, on the same buffers and
+// scratch, in one (up to PLX_DECODE_STEP_ROWS rows; else only the inputs are put in place).  kNothing, having done nothing, for
+// anything but tensors like the buffers and lengths given as Python integers in [1, most].
+// 4 rows of up to 4096 keys, 8 : 8 heads: 22.3 us for a launch that puts the inputs in place and the graph behind it.
+enum Step { kNothing = 0, kStaged = 1, kDone = 2 };
+int step(const py::object &q_, const py::object &q_src_, const py::object &r_, const py::object &r_src_, const py::object &lens_,
+         const py::object &lens_src, int64_t most, const py::object &k_, const py::object &v_, const py::object &out_, const py::object &ws_,
+         double scale, int64_t window, int64_t n_splits) {
     bool ok = true;
     const Tensor q = take(q_, ok), r = take(r_, ok);
     const OptTensor q_src = take_optional(q_src_, ok), r_src = take_optional(r_src_, ok), lens = take_optional(lens_, ok);
     if (!ok || !plain_thread() || !plain_tensor(q) || !plain_tensor(r) || !q.is_contiguous() || !r.is_contiguous() || q.numel() != r.numel() ||
         !aligned16(q) || !aligned16(r) || recorded({&q, &r}))
-        return false;
+        return kNothing;
     for (const OptTensor *src : {&q_src, &r_src})
         if (*src && (!plain_tensor(**src) || (*src)->sizes() != q.sizes() || (*src)->scalar_type() != q.scalar_type() ||
                      (*src)->device() != q.device() || !(*src)->is_contiguous() || !aligned16(**src) || recorded({&**src})))
-            return false;
+            return kNothing;
     int32_t values[PLX_DECODE_STAGE_LENS];
     int64_t n = 0;
     if (!lens_src.is_none()) {
-        if (!lens || !int32_vector(lens, q.size(0), q.device()) || lens->numel() > PLX_DECODE_STAGE_LENS) return false;
+        if (!lens || !int32_vector(lens, q.size(0), q.device()) || lens->numel() > PLX_DECODE_STAGE_LENS) return kNothing;
         n = lens->numel();
         const bool list = PyList_CheckExact(lens_src.ptr());
-        if (list ? PyList_GET_SIZE(lens_src.ptr()) != n : !PyLong_CheckExact(lens_src.ptr())) return false;
+        if (list ? PyList_GET_SIZE(lens_src.ptr()) != n : !PyLong_CheckExact(lens_src.ptr())) return kNothing;
         for (int64_t i = 0; i < n; ++i) {
             PyObject *x = list ? PyList_GET_ITEM(lens_src.ptr(), i) : lens_src.ptr();
             int overflow = 0;
             const long long len = PyLong_CheckExact(x) ? PyLong_AsLongLongAndOverflow(x, &overflow) : 0;
-            if (overflow || len < 1 || len > most) return false;
+            if (overflow || len < 1 || len > most) return kNothing;
             values[i] = static_cast<int32_t>(len);
         }
     }
     const c10::cuda::CUDAGuard device(q.device());
-    if (capturing()) return false;
-    return api.decode_stage(q.data_ptr(), q_src ? q_src->data_ptr() : nullptr, r.data_ptr(), r_src ? r_src->data_ptr() : nullptr, q.nbytes(),
-                            lens ? static_cast<int32_t *>(lens->data_ptr()) : nullptr, n ? values : nullptr, static_cast<int32_t>(n),
-                            c10::cuda::getCurrentCUDAStream().stream()) == PLX_OK;
+    if (capturing()) return kNothing;
+    const cudaStream_t stream = c10::cuda::getCurrentCUDAStream().stream();
+    const void *q_from = q_src ? q_src->data_ptr() : nullptr, *r_from = r_src ? r_src->data_ptr() : nullptr;
+    int32_t *lens_to = lens ? static_cast<int32_t *>(lens->data_ptr()) : nullptr;
+    const Tensor k = take(k_, ok), v = take(v_, ok), out = take(out_, ok), ws = take(ws_, ok);
+    // (a source that shares memory with the buffers or the output would be read and written by one launch)
+    const auto apart = [](const Tensor &x, const Tensor &y) { return !x.is_alias_of(y); };
+    const auto source_apart = [&](const OptTensor &src) { return !src || (apart(*src, q) && apart(*src, r) && apart(*src, out)); };
+    if (ok && q.dim() == 4 && q.size(0) <= PLX_DECODE_STEP_ROWS && cache_call_ok(q, r, k, v, lens, std::nullopt) && plain_tensor(out) && plain_tensor(ws) &&
+        out.sizes() == q.sizes() && out.scalar_type() == q.scalar_type() && out.device() == q.device() && out.is_contiguous() &&
+        source_apart(q_src) && source_apart(r_src)) {
+        const plx_decode_problem p = decode_problem(q, k, k.size(1), std::nullopt, scale, window, static_cast<int32_t>(n_splits));
+        if (api.decode_step(&p, q.data_ptr(), q_from, r.data_ptr(), r_from, k.data_ptr(), v.data_ptr(), out.data_ptr(), lens_to, n ? values : nullptr,
+                            ws.data_ptr(), ws.nbytes(), stream) == PLX_OK)
+            return kDone;
+    }
+    return api.decode_stage(q.data_ptr(), q_from, r.data_ptr(), r_from, q.nbytes(), lens_to, n ? values : nullptr, static_cast<int32_t>(n), stream) == PLX_OK
+               ? kStaged : kNothing;
 }
 
 }  // namespace
@@ -568,5 +588,5 @@ PYBIND11_MODULE(_plx_host, m) {
     m.def("train", &train);
     m.def("decode", &decode);
     m.def("attend", &attend);
-    m.def("stage", &stage);
+    m.def("step", &step);
 }

@@ -352,7 +352,11 @@ class GraphedDecode:
         # this object's own split-KV workspace, allocated and zeroed BEFORE the capture: the captured
         # launch of one GraphedDecode never shares scratch with another, whatever stream replays it
         window_left = _window_size_to_left(self._window)
-        self._workspace = new_workspace(self.q, split_count(self.q, self.k, window_left))
+        self._n_splits = split_count(self.q, self.k, window_left)
+        self._workspace = new_workspace(self.q, self._n_splits)
+        self._window_left = window_left
+        # what the captured launch reads and writes, whatever the attributes are rebound to later
+        self._captured = (self.q, self.r, self.k, self.v, self.out, self.cache_seqlens)
 
         def call():
             if self.cache_seqlens is not None:
@@ -376,10 +380,19 @@ class GraphedDecode:
 
     def __call__(self, *, q=None, r=None, k=None, v=None, cache_seqlens=None) -> torch.Tensor:
         host = ops.eager_host()
-        lens = cache_seqlens if self.cache_seqlens is not None else None
-        if host is not None and host.stage(self.q, q, self.r, r, self.cache_seqlens, lens, self.max_kv_len):
-            q = r = cache_seqlens = None                   # done, in one launch
-        for dst, src in ((self.q, q), (self.r, r), (self.k, k), (self.v, v)):
+        for dst, src in ((self.k, k), (self.v, v)):
+            if src is not None:
+                dst.copy_(src)
+        if host is not None and all(x is y for x, y in zip(
+                (self.q, self.r, self.k, self.v, self.out, self.cache_seqlens), self._captured)):
+            lens = cache_seqlens if self.cache_seqlens is not None else None
+            done = host.step(self.q, q, self.r, r, self.cache_seqlens, lens, self.max_kv_len, self.k, self.v, self.out, self._workspace,
+                             float(self._scale), self._window_left, self._n_splits)
+            if done == 2:                                  # staged and launched
+                return self.out
+            if done == 1:                                  # staged
+                q = r = cache_seqlens = None
+        for dst, src in ((self.q, q), (self.r, r)):
             if src is not None:
                 dst.copy_(src)
         if cache_seqlens is not None and self.cache_seqlens is not None:

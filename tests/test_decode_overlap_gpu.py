@@ -5,6 +5,7 @@ import torch
 
 import parallax_b200 as plx
 from oracle import parallax_oracle as orc
+from parallax_b200 import _cabi
 from tests._util import DECODE_MAX_REL, DECODE_REL_L2, assert_close, seeded_bf16
 
 pytestmark = pytest.mark.gpu
@@ -59,6 +60,31 @@ def test_grouped_heads_at_the_edges_of_tiles_and_stages(hq, hkv, d, monkeypatch)
             table = torch.arange(t // 16, device="cuda", dtype=torch.int32).flip(0).view(1, -1)
             kp, vp = (x.view(t // 16, 16, hkv, d).flip(0).contiguous() for x in (k, v))
             assert torch.equal(plx.parallax_attn_with_kvcache(q, r, kp, vp, page_table=table), o)
+
+
+@pytest.mark.parametrize("bsz,hq,hkv", [(1, 8, 8), (64, 8, 8), (64, 8, 2), (65, 8, 8)])
+def test_a_graphed_step_in_one_launch(bsz, hq, hkv):
+    """Up to 64 rows the inputs and the sweep are one launch; its buffers and answer are those of the copies and the replay."""
+    t = 400
+    gd = plx.GraphedDecode(bsz, hq, max_kv_len=t, H_kv=hkv)
+    q, r, k, v = inputs(bsz, hq, hkv, t)
+    lens = [t - (i * 37) % (t - 1) for i in range(bsz)]
+    want = gd(q=q, r=r, k=k, v=v, cache_seqlens=torch.tensor(lens)).clone()
+    assert torch.equal(gd.replay(), want)
+    for t_ in (gd.q, gd.r, gd.out, gd.cache_seqlens):
+        t_.zero_()
+    gd.cache_seqlens += 1
+    before = _cabi.launch_count()
+    assert torch.equal(gd(q=q, r=r, cache_seqlens=lens), want)
+    assert _cabi.launch_count() == before + 1
+    assert torch.equal(gd.q, q) and torch.equal(gd.r, r) and gd.cache_seqlens.tolist() == lens
+    gd.out.zero_()
+    assert torch.equal(gd.replay(), want)
+    assert torch.equal(gd(), want)
+    # an input that shares memory with the output or the buffers
+    two = gd(q=gd.out).clone()
+    assert torch.equal(gd.q, want) and torch.equal(gd.replay(), two)
+    assert torch.equal(gd(q=gd.r, r=gd.q), gd.replay())
 
 
 @pytest.mark.parametrize("bsz,hq,hkv,t,lq", [(2, 32, 8, 4096, 1), (8, 16, 16, 2048, 1), (2, 32, 8, 700, 64)])
