@@ -89,20 +89,24 @@ constexpr uint32_t kStatBytes = kBN * 16;      // four planes of 64 floats: -mL,
 // 256 dq/dr 205 against 191 (before 223).  Two groups at 128 (one score buffer, S1 and S2 of a whole tile read at once into
 // 224 registers a thread) changed nothing, 1498 -> 1494: a tile then lives 7700 clocks and the ring has three stages;
 // short sequences were slower (dk/dv 239 -> 260).
-template <int D, int MODE>
+//
+// SHORT (dq/dr at 128): dO is a resident tile in shared memory like q and r, which costs a stage of the ring.  On the way into
+// tensor memory it passes through the registers of the element-wise warps at the start of an item, 2500 of the 11300 clocks
+// that an item of 2.3 streamed tiles takes.  See short_items.
+template <int D, int MODE, bool SHORT>
 struct Plan {
-    static constexpr bool kTwo = D == 64, kMTile = D == 128;
+    static constexpr bool kTwo = D == 64, kMTile = D == 128 && !SHORT;
     static constexpr int kGroups = kTwo ? 2 : 1;                            // of element-wise warps, = score buffers
     static constexpr int kStatStages = kTwo ? 4 : 2;                        // tiles' row statistics (DKV): what is left at head_dim 128
     // stages of streamed tiles: what the shared memory allows at 128; six at 64 (four: dq/dr 4 %, dk/dv 1 % slower, measured
     // before the two groups)
-    static constexpr int NS = kTwo ? 6 : MODE == kModeDQR ? 4 : 3;
+    static constexpr int NS = kTwo ? 6 : MODE == kModeDQR && !SHORT ? 4 : 3;
 };
 
 // D = head dim (64 or 128): tiles are D / 64 panels.
-template <int D, int MODE>
+template <int D, int MODE, bool SHORT>
 struct Smem {
-    using P = Plan<D, MODE>;
+    using P = Plan<D, MODE, SHORT>;
     static constexpr int NS = P::NS, kStatStages = P::kStatStages;
     static constexpr int kPanels = D / 64;
     static constexpr uint32_t kResBytes = kPanels * kResPanel;   // resident tile (128 rows)
@@ -205,14 +209,14 @@ __device__ __forceinline__ int item_index(int n, int chunk_shift) {
 // accumulators, and the hand-overs for those are arranged so that the loads, the tensor-memory tile and
 // the first score products of the next item are under way while the element-wise warps write out the
 // accumulators of the current one.  TMEM allocation, barrier set-up and launch latency are paid once.
-template <typename T, int D, int MODE>
+template <typename T, int D, int MODE, bool SHORT>
 __global__ void __launch_bounds__((4 + kEwWarps) * 32, 1)
 bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorMap tm_q,
                  const __grid_constant__ CUtensorMap tm_r, const __grid_constant__ CUtensorMap tm_go,
                  const __grid_constant__ CUtensorMap tm_k, const __grid_constant__ CUtensorMap tm_v, const ErrSink sink,
                  int n_mt, int n_items, int chunk_shift, int group) {
-    using P = Plan<D, MODE>;
-    using L = Smem<D, MODE>;
+    using P = Plan<D, MODE, SHORT>;
+    using L = Smem<D, MODE, SHORT>;
     constexpr int NS = P::NS, kStatStages = P::kStatStages;
     constexpr bool DQR = MODE == kModeDQR, kMTile = P::kMTile;
     constexpr uint32_t kResBytes = L::kResBytes, kStrBytes = L::kStrBytes;
@@ -889,9 +893,9 @@ bwd_sm100_kernel(const TrainArgs a, int n_tok, const __grid_constant__ CUtensorM
 // ------------------------------------------------------------------------- //
 // host side
 // ------------------------------------------------------------------------- //
-template <typename T, int D, int MODE>
+template <typename T, int D, int MODE, bool SHORT>
 int launch_mode(const TrainArgs &a, int n_tok, const ErrSink &sink, bool overlap, cudaStream_t stream) {
-    using L = Smem<D, MODE>;
+    using L = Smem<D, MODE, SHORT>;
     constexpr bool DQR = MODE == kModeDQR;
     const int q_rows = DQR ? kBM : kBN, kv_rows = DQR ? kBN : kBM;
     CUtensorMap tq, tr, tg, tk, tv;
@@ -902,7 +906,7 @@ int launch_mode(const TrainArgs &a, int n_tok, const ErrSink &sink, bool overlap
         !tma::make_map(&tk, dt, a.k, D, a.len_k, a.heads_kv, a.batch, a.kv_st, a.kv_sh, a.kv_sb, kv_rows) ||
         !tma::make_map(&tv, dt, a.v, D, a.len_k, a.heads_kv, a.batch, a.kv_st, a.kv_sh, a.kv_sb, kv_rows))
         return PLX_ERR_LAUNCH;
-    auto kern = bwd_sm100_kernel<T, D, MODE>;
+    auto kern = bwd_sm100_kernel<T, D, MODE, SHORT>;
     static std::mutex attr_mu;
     static bool attr_done[tma::kMaxDevices] = {};
     if (!tma::opt_in_smem(kern, static_cast<int>(L::kBytes), attr_done, attr_mu)) return PLX_ERR_LAUNCH;
@@ -930,6 +934,11 @@ int launch_mode(const TrainArgs &a, int n_tok, const ErrSink &sink, bool overlap
     return st == cudaSuccess && cudaGetLastError() == cudaSuccess ? PLX_OK : PLX_ERR_LAUNCH;
 }
 
+// SHORT pays where items are short and costs a stage of the ring where they are long.  dq/dr, us, tile in tensor memory against
+// shared memory: dense, 100 tokens 53.0 / 48.8, 512 85.0 / 77.0, 1024 109 / 107, 2048 170 / 171.5, 4096 1148 / 1148; packed, 16 : 4
+// heads, sequences of 1 to 256 290 / 268, 256 to 1024 376 / 366, 1000 to 3000 786 / 788, 64 to 8192 (65536 tokens) 3296 / 3370.
+bool short_items(const TrainArgs &a) { return (a.cu ? a.len_q / a.n_seqs : a.len_q) <= 1024; }
+
 }  // namespace
 
 bool train_bwd_sm100_supported(const TrainArgs &a, int head_dim) {
@@ -947,17 +956,19 @@ int launch_train_bwd_sm100(const TrainArgs &a, int dtype, int head_dim, int stag
     const bool dqr = stage == PLX_BWD_DQR;
     if (dtype == PLX_BF16) {
         if (head_dim == 64)
-            return dqr ? launch_mode<__nv_bfloat16, 64, kModeDQR>(a, n_tok, err, overlap, stream)
-                       : launch_mode<__nv_bfloat16, 64, kModeDKV>(a, n_tok, err, overlap, stream);
-        return dqr ? launch_mode<__nv_bfloat16, 128, kModeDQR>(a, n_tok, err, overlap, stream)
-                   : launch_mode<__nv_bfloat16, 128, kModeDKV>(a, n_tok, err, overlap, stream);
+            return dqr ? launch_mode<__nv_bfloat16, 64, kModeDQR, false>(a, n_tok, err, overlap, stream)
+                       : launch_mode<__nv_bfloat16, 64, kModeDKV, false>(a, n_tok, err, overlap, stream);
+        return dqr ? (short_items(a) ? launch_mode<__nv_bfloat16, 128, kModeDQR, true>(a, n_tok, err, overlap, stream)
+                                     : launch_mode<__nv_bfloat16, 128, kModeDQR, false>(a, n_tok, err, overlap, stream))
+                   : launch_mode<__nv_bfloat16, 128, kModeDKV, false>(a, n_tok, err, overlap, stream);
     }
     if (dtype == PLX_FP16) {
         if (head_dim == 64)
-            return dqr ? launch_mode<__half, 64, kModeDQR>(a, n_tok, err, overlap, stream)
-                       : launch_mode<__half, 64, kModeDKV>(a, n_tok, err, overlap, stream);
-        return dqr ? launch_mode<__half, 128, kModeDQR>(a, n_tok, err, overlap, stream)
-                   : launch_mode<__half, 128, kModeDKV>(a, n_tok, err, overlap, stream);
+            return dqr ? launch_mode<__half, 64, kModeDQR, false>(a, n_tok, err, overlap, stream)
+                       : launch_mode<__half, 64, kModeDKV, false>(a, n_tok, err, overlap, stream);
+        return dqr ? (short_items(a) ? launch_mode<__half, 128, kModeDQR, true>(a, n_tok, err, overlap, stream)
+                                     : launch_mode<__half, 128, kModeDQR, false>(a, n_tok, err, overlap, stream))
+                   : launch_mode<__half, 128, kModeDKV, false>(a, n_tok, err, overlap, stream);
     }
     return PLX_ERR_UNSUPPORTED;
 }
