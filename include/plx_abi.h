@@ -214,7 +214,8 @@ int plx_decode_workspace_bytes(const plx_decode_problem *p, size_t *bytes);
 
 /* The inputs of one step into the stable buffers that a captured decode launch reads, in one launch: `bytes`
  * (a multiple of 16) of q and of r, and n (at most PLX_DECODE_STAGE_LENS) active lengths from HOST memory.  A null
- * source leaves its buffer alone.  Plays the role of the copies of GraphedDecode.__call__
+ * source leaves its buffer alone; one that overlaps a buffer that is written (other than being q or r itself) is
+ * PLX_ERR_UNSUPPORTED.  Plays the role of the copies of GraphedDecode.__call__
  * [parallax/cute/parallax_decode.py:1665-1815]. */
 #define PLX_DECODE_STAGE_LENS 512
 int plx_decode_stage(void *q, const void *q_src, void *r, const void *r_src, size_t bytes,
@@ -222,7 +223,8 @@ int plx_decode_stage(void *q, const void *q_src, void *r, const void *r_src, siz
 
 /* plx_decode_stage and the plx_decode behind it (no cache_start) as ONE launch, for at most PLX_DECODE_STEP_ROWS batch rows
  * (else PLX_ERR_UNSUPPORTED): the sweep reads q_src and r_src (null: q, r) and the HOST lengths seqused_src (null: the
- * device array seqused_k, or none) and leaves copies in q, r and seqused_k. */
+ * device array seqused_k, or none) and leaves copies in q, r and seqused_k.  A source that overlaps what the launch writes (the
+ * buffers of the copies, out, the workspace) is PLX_ERR_UNSUPPORTED: stage it, then decode. */
 #define PLX_DECODE_STEP_ROWS 64
 int plx_decode_step(const plx_decode_problem *p, void *q, const void *q_src, void *r, const void *r_src,
                     const void *k, const void *v, void *out, int32_t *seqused_k, const int32_t *seqused_src,

@@ -47,6 +47,12 @@ static int check_train(const plx_train_problem *p) {
 
 static bool misaligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) != 0; }
 
+// n bytes from x and m bytes from y have one in common (null: none)
+static bool overlap(const void *x, size_t n, const void *y, size_t m) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(x), b = reinterpret_cast<uintptr_t>(y);
+    return x && y && a < b + m && b < a + n;
+}
+
 static TrainArgs make_train_args(const plx_train_problem *p) {
     TrainArgs a{};
     a.cu = p->cu_seqlens;
@@ -430,6 +436,12 @@ int plx_decode_stage(void *q, const void *q_src, void *r, const void *r_src, siz
     if ((q_src && !q) || (r_src && !r) || (seqused_src && !seqused_k) || n < 0 || n > PLX_DECODE_STAGE_LENS || (bytes & 15u) != 0)
         return PLX_ERR_BAD_ARG;
     if (misaligned16(q) || misaligned16(q_src) || misaligned16(r) || misaligned16(r_src)) return PLX_ERR_BAD_ARG;
+    // An element is copied to q, then to r, by one thread: a source may be the other buffer, but not a shifted part of one.
+    for (const void *src : {q_src, r_src}) {
+        if (q_src && src != q && overlap(src, bytes, q, bytes)) return PLX_ERR_UNSUPPORTED;
+        if (r_src && src != r && overlap(src, bytes, r, bytes)) return PLX_ERR_UNSUPPORTED;
+        if (seqused_src && overlap(src, bytes, seqused_k, n * sizeof(int32_t))) return PLX_ERR_UNSUPPORTED;
+    }
     int st = check_device();
     if (st != PLX_OK) return st;
     return launch_decode_stage(q, q_src, r, r_src, bytes, seqused_k, seqused_src, n, reinterpret_cast<cudaStream_t>(stream));
@@ -439,6 +451,16 @@ int plx_decode_step(const plx_decode_problem *p, void *q, const void *q_src, voi
                     int32_t *seqused_k, const int32_t *seqused_src, void *workspace, size_t workspace_bytes, plx_stream_t stream) {
     if (!p || !out || !q || !r || (seqused_src && !seqused_k) || misaligned16(q) || misaligned16(r)) return PLX_ERR_BAD_ARG;
     if (p->batch > PLX_DECODE_STEP_ROWS) return PLX_ERR_UNSUPPORTED;
+    const int st = check_decode(p);
+    if (st != PLX_OK) return st;
+    // The parts of a row read the sources while the first of them writes the copies: nothing that is written may lie in a source.
+    const size_t bytes = static_cast<size_t>(p->batch) * p->heads_q * p->head_dim * 2;
+    for (const void *src : {q_src, r_src}) {
+        if ((q_src && overlap(src, bytes, q, bytes)) || (r_src && overlap(src, bytes, r, bytes)) || overlap(src, bytes, out, bytes) ||
+            (seqused_src && overlap(src, bytes, seqused_k, p->batch * sizeof(int32_t))) ||
+            (p->n_splits > 1 && overlap(src, bytes, workspace, decode_ws_bytes(p))))
+            return PLX_ERR_UNSUPPORTED;
+    }
     const StepCopies step{q_src ? q : nullptr, r_src ? r : nullptr, seqused_k, seqused_src};
     return run_decode(p, q_src ? q_src : q, r_src ? r_src : r, k, v, out, nullptr, seqused_src ? nullptr : seqused_k, nullptr, workspace,
                       workspace_bytes, reinterpret_cast<cudaStream_t>(stream), nullptr, &step);

@@ -101,6 +101,56 @@ def test_decode_split_heuristic_and_workspace():
     assert lib.plx_decode_merge(None, 1, 1, 128, 0, None, None) == -1
 
 
+def _address(base, offset=0):
+    return C.c_void_p(base + offset)
+
+
+def test_a_step_refuses_sources_that_it_would_overwrite():
+    """One launch reads the sources and writes the copies, the output and its scratch: ranges of addresses are compared, whatever
+    objects own them.  (No call here can launch: the workspace is too small for every one.)"""
+    lib = _cabi.lib()
+    p = _cabi.DecodeProblem()
+    p.dtype, p.batch, p.heads_q, p.heads_kv, p.cache_len, p.head_dim = 0, 4, 8, 8, 4096, 128
+    p.window_left, p.n_splits, p.qk_scale = -1, 5, 0.088
+    p.kv_stride_b, p.kv_stride_t, p.kv_stride_h = 4096 * 8 * 128, 8 * 128, 128
+    n = 4 * 8 * 128 * 2
+    need = C.c_size_t(0)
+    assert lib.plx_decode_workspace_bytes(C.byref(p), C.byref(need)) == 0
+    q, r, out, lens, kv, ws = (i << 24 for i in range(1, 7))
+    far = 9 << 24
+    host_lens = (C.c_int32 * 4)(1, 2, 3, 4)
+
+    def step(q_src, r_src, with_lens=True, rows=4):
+        p.batch = rows
+        return lib.plx_decode_step(C.byref(p), _address(q), q_src, _address(r), r_src, _address(kv), _address(kv), _address(out),
+                                   _address(lens), host_lens if with_lens else None, _address(ws), 0, None)
+
+    unsupported = -2
+    for buffer, size in ((q, n), (r, n), (out, n), (lens, 16), (ws, need.value)):
+        for at in (buffer, buffer + (size - 16), buffer - (n - 16)):
+            assert step(_address(at), _address(far)) == unsupported
+            assert step(_address(far), _address(at)) == unsupported
+        for at in (buffer + size, buffer - n):
+            assert step(_address(at), _address(far)) != unsupported
+            assert step(_address(far), _address(at)) != unsupported
+    # what is not written may be read twice
+    assert step(None, _address(q)) != unsupported and step(_address(r), None) != unsupported
+    assert step(_address(lens), None, with_lens=False) != unsupported
+    assert step(None, None) != unsupported and step(_address(far), _address(far)) != unsupported
+    assert step(None, None, rows=65) == unsupported
+
+
+def test_staging_refuses_shifted_parts_of_its_buffers():
+    lib = _cabi.lib()
+    n, q, r, lens, far = 4096, 1 << 24, 2 << 24, 3 << 24, 9 << 24
+    host_lens = (C.c_int32 * 4)(1, 2, 3, 4)
+    for buffer in (q, r):
+        for at in (buffer + 16, buffer - 16, buffer + n - 16):
+            for src in ((at, far), (far, at)):
+                assert lib.plx_decode_stage(_address(q), _address(src[0]), _address(r), _address(src[1]), n, None, None, 0, None) == -2
+    assert lib.plx_decode_stage(_address(q), _address(lens), _address(r), None, n, _address(lens), host_lens, 4, None) == -2
+
+
 def test_exchange_sizes_and_argument_checks():
     lib = _cabi.lib()
     rec = 2 * 128 + 4

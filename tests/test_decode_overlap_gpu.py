@@ -87,6 +87,30 @@ def test_a_graphed_step_in_one_launch(bsz, hq, hkv):
     assert torch.equal(gd(q=gd.r, r=gd.q), gd.replay())
 
 
+def test_inputs_that_share_memory_but_not_a_storage():
+    """The buffers of a step behind a zero-copy import have storages of their own: the answers are still those of copies to q,
+    then to r, then the sweep."""
+    gd = plx.GraphedDecode(4, 8, max_kv_len=400)
+    q, r, k, v = inputs(4, 8, 8, 400)
+    gd(k=k, v=v)
+
+    def foreign(x):
+        y = torch.from_dlpack(x)
+        assert y.data_ptr() == x.data_ptr() and not torch._C._is_alias_of(x, y)
+        return y
+
+    def same(got, q, r):
+        assert torch.equal(gd.q, q) and torch.equal(gd.r, r)
+        assert torch.equal(got, plx.parallax_decode(q, r, k, v))
+
+    same(gd(q=q, r=foreign(gd.q)), q, q)
+    gd(q=q, r=r)
+    same(gd(q=foreign(gd.r), r=q), r, q)
+    want = gd(q=q, r=r).clone()
+    same(gd(q=foreign(gd.out)), want, r)
+    same(gd(q=foreign(gd.k[:, 5:6]).contiguous()), k[:, 5:6], r)
+
+
 @pytest.mark.parametrize("bsz,hq,hkv,t,lq", [(2, 32, 8, 4096, 1), (8, 16, 16, 2048, 1), (2, 32, 8, 700, 64)])
 def test_lengths_beside_a_long_launch(bsz, hq, hkv, t, lq):
     """The lengths are checked as they are in stream order -- written by a kernel that is still to run when the call is made,
