@@ -525,6 +525,31 @@ py::object attend(const py::object &q, const py::object &r, const py::object &k,
     return t.dim() == 4 && t.size(1) == 1 ? decode(q, r, k, v, scale, window, lens, py::none(), table) : extend(q, r, k, v, scale, window, lens, table);
 }
 
+// No address of the sources (tensors or None) lies in one of the buffers; false where that cannot be told.
+bool apart(const py::tuple &sources, const py::tuple &buffers) {
+    const auto span = [](const Tensor &t) {
+        int64_t last = t.numel() > 0 ? 1 : 0;
+        for (int64_t i = 0; i < t.dim() && last > 0; ++i) last += (t.size(i) - 1) * t.stride(i);
+        const auto at = reinterpret_cast<uintptr_t>(t.data_ptr());
+        return std::pair<uintptr_t, uintptr_t>(at, at + last * t.element_size());
+    };
+    bool ok = true;
+    for (const py::handle &s : sources) {
+        const OptTensor src = take_optional(py::reinterpret_borrow<py::object>(s), ok);
+        if (!ok) return false;
+        if (!src || src->is_cpu()) continue;
+        if (!plain_tensor(*src)) return false;
+        const auto x = span(*src);
+        for (const py::handle &b : buffers) {
+            const Tensor buffer = take(py::reinterpret_borrow<py::object>(b), ok);
+            if (!ok || !plain_tensor(buffer)) return false;
+            const auto y = span(buffer);
+            if (x.first < y.second && y.first < x.second) return false;
+        }
+    }
+    return true;
+}
+
 // A GraphedDecode step: q, r and the lengths into its buffers, and the launch that its graph holds, on the same buffers and
 // scratch, in one (up to PLX_DECODE_STEP_ROWS rows, inputs that lie apart from what it writes; else only the inputs are put in place).  kNothing, having done nothing, for
 // anything but tensors like the buffers and lengths given as Python integers in [1, most].
@@ -584,5 +609,6 @@ PYBIND11_MODULE(_plx_host, m) {
     m.def("train", &train);
     m.def("decode", &decode);
     m.def("attend", &attend);
+    m.def("apart", &apart);
     m.def("step", &step);
 }

@@ -380,11 +380,18 @@ class GraphedDecode:
 
     def __call__(self, *, q=None, r=None, k=None, v=None, cache_seqlens=None) -> torch.Tensor:
         host = ops.eager_host()
-        for dst, src in ((self.k, k), (self.v, v)):
-            if src is not None:
-                dst.copy_(src)
-        if host is not None and all(x is y for x, y in zip(
-                (self.q, self.r, self.k, self.v, self.out, self.cache_seqlens), self._captured)):
+        direct = host is not None and all(x is y for x, y in zip(
+            (self.q, self.r, self.k, self.v, self.out, self.cache_seqlens), self._captured))
+        if direct and (k is not None or v is not None):
+            # the caches come first, then one launch does the rest -- unless that could show: q, r, k, v are copied in this
+            # order where one of them may lie in a buffer that another is copied to
+            direct = host.apart((q, r, k, v), (self.q, self.r, self.k, self.v))
+            if direct:
+                for dst, src in ((self.k, k), (self.v, v)):
+                    if src is not None:
+                        dst.copy_(src)
+                k = v = None
+        if direct:
             lens = cache_seqlens if self.cache_seqlens is not None else None
             done = host.step(self.q, q, self.r, r, self.cache_seqlens, lens, self.max_kv_len, self.k, self.v, self.out, self._workspace,
                              float(self._scale), self._window_left, self._n_splits)
@@ -392,7 +399,7 @@ class GraphedDecode:
                 return self.out
             if done == 1:                                  # staged
                 q = r = cache_seqlens = None
-        for dst, src in ((self.q, q), (self.r, r)):
+        for dst, src in ((self.q, q), (self.r, r), (self.k, k), (self.v, v)):
             if src is not None:
                 dst.copy_(src)
         if cache_seqlens is not None and self.cache_seqlens is not None:

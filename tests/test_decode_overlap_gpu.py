@@ -111,6 +111,31 @@ def test_inputs_that_share_memory_but_not_a_storage():
     same(gd(q=foreign(gd.k[:, 5:6]).contiguous()), k[:, 5:6], r)
 
 
+@pytest.mark.parametrize("through", [lambda x: x, torch.from_dlpack])
+def test_inputs_are_copied_in_the_order_of_the_arguments(through):
+    """q, r, k, v: a q or an r that is part of the object's own caches is read before new caches arrive, and a k or a v that is
+    the object's q after the new q has."""
+    t = 400
+    (q, r, k, v), (q2, _, k2, v2) = inputs(4, 8, 8, t), inputs(4, 8, 8, t, seed=50)
+
+    def step(**given):
+        gd = plx.GraphedDecode(4, 8, max_kv_len=t)
+        gd(q=q, r=r, k=k, v=v)
+        out = gd(**{n: through(x(gd)) if callable(x) else x for n, x in given.items()})
+        return gd, out
+
+    def holds(got, q, r, k, v):
+        gd, out = got
+        for x, y in ((gd.q, q), (gd.r, r), (gd.k, k), (gd.v, v), (out, plx.parallax_decode(q, r, k, v))):
+            assert torch.equal(x, y)
+
+    holds(step(q=lambda gd: gd.k[:, 7:8], k=k2), k[:, 7:8], r, k2, v)
+    holds(step(r=lambda gd: gd.v[:, :1], k=k2, v=v2, cache_seqlens=t), q, v[:, :1], k2, v2)
+    holds(step(q=q2, k=lambda gd: gd.q.expand(4, t, 8, 128)), q2, r, q2.expand(4, t, 8, 128), v)
+    holds(step(q=q2, r=lambda gd: gd.q, k=k2, v=lambda gd: gd.k), q2, q2, k2, k2)
+    holds(step(q=q2, k=k2, v=v2), q2, r, k2, v2)          # nothing shared: one launch behind the copies
+
+
 @pytest.mark.parametrize("bsz,hq,hkv,t,lq", [(2, 32, 8, 4096, 1), (8, 16, 16, 2048, 1), (2, 32, 8, 700, 64)])
 def test_lengths_beside_a_long_launch(bsz, hq, hkv, t, lq):
     """The lengths are checked as they are in stream order -- written by a kernel that is still to run when the call is made,
