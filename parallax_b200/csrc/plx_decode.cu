@@ -115,7 +115,8 @@ __device__ __forceinline__ void store_elem<__half>(void *out, int64_t idx, float
 // Merge of n <= 32 partial records (stride REC floats) by one warp.  On return every lane holds the
 // maximum, the two sums, and the D / 32 channels lane * (D / 32) .. of O1 and O2, all relative to
 // the common maximum.  Bound by round trips to the L2: the channels of the first N records are requested together
-// with the headers of all.
+// with the headers of all (of those that there are: a warp may be the only one of its CTA to merge all rows of a kv head, and with N
+// records read for each whatever n, calls of 4 rows of 1000 keys went from 27 to 35 us at 16 : 1 heads, from 16.5 to 20.4 at 64 : 8).
 template <int D, int N = 8>
 __device__ __forceinline__ void warp_merge(const float *rec0, int n, int lane, float &big, float &D1, float &D2,
                                            float (&O1)[D / 32], float (&O2)[D / 32]) {
@@ -127,7 +128,12 @@ __device__ __forceinline__ void warp_merge(const float *rec0, int n, int lane, f
     auto load = [&](int j0) {
 #pragma unroll
         for (int j = 0; j < N; ++j) {
-            const float *pr = col + static_cast<int64_t>(min(j0 + j, n - 1)) * REC;   // weight 0 past the end
+            if (j0 + j >= n) {
+#pragma unroll
+                for (int e = 0; e < CH; ++e) x[j][e] = y[j][e] = 0.f;
+                continue;
+            }
+            const float *pr = col + static_cast<int64_t>(j0 + j) * REC;
             if (CH == 4) {
                 const float4 u = __ldcg(reinterpret_cast<const float4 *>(pr)), v = __ldcg(reinterpret_cast<const float4 *>(pr + D));
                 x[j][0] = u.x; x[j][1] = u.y; x[j][CH - 2] = u.z; x[j][CH - 1] = u.w;
@@ -944,7 +950,8 @@ struct GqaSmem {
 //
 // FEW: at most 8 q heads per kv head, the usual case.  Then the products are transposed -- keys are the M dimension of the
 // scores (S^T = K Q_g^T), channels that of the outputs (O^T += V^T P^T), and the heads the 8 columns -- which takes half the
-// MMAs, with none of them on rows of zeros, and half the registers; a movmatrix per 8 x 8 block turns P^T around.
+// MMAs, with none of them on rows of zeros, and half the registers for accumulators and fragments (in all 207 at head_dim 128,
+// where the other form fills 255); a movmatrix per 8 x 8 block turns P^T around.
 // B = 16, 1024 keys, 32 : 8 heads 16.7 -> 16.0 us, B = 8, 4000 keys, rows of different lengths 40.8 -> 34.0.
 template <typename T, int D, bool PAGED, bool FEW>
 __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const DecodeArgs a, int n_hgroups) {
@@ -979,19 +986,21 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
     // (32 / CPR)-th row, so its source and destination advance by constants; rows past my_hi (last tile
     // only) are zero-filled.  In a paged cache a tile lies in one page when pages hold at least a tile and the
     // range starts on a tile boundary (it does but for windows and cache_start): one page number per tile then,
-    // read three tiles ahead.
+    // read ahead.
     constexpr int RPI = 32 / CPR;                                  // rows covered by one instruction of the warp
     const int my_row = lane / CPR, my_col = lane % CPR;
     const bool page_per_tile = PAGED && a.page_mask + 1 >= kGqaTile && my_lo % kGqaTile == 0;
     const T *kp = static_cast<const T *>(a.k) + (PAGED ? 0 : b * a.kv_sb) + hk * a.kv_sh + my_col * 8;
     const T *vp = static_cast<const T *>(a.v) + (PAGED ? 0 : b * a.kv_sb) + hk * a.kv_sh + my_col * 8;
     const uint32_t my_dst = (my_row * LD + my_col * 8) * 2;
-    // pages of the next tiles to be loaded (as many as there are stages, so that no load waits for the page number of another)
-    uint32_t next_page[kGqaStages];
+    // Pages of the next tiles to be loaded: as many as there are stages, so that no load waits for the page number of another;
+    // two where registers are short (B = 64, 4096 keys, 16 : 1 heads, pages, 34.0 us, three 35.8).
+    constexpr int kPages = FEW ? kGqaStages : 2;
+    uint32_t next_page[kPages];
     auto page_of_tile = [&](int i) -> uint32_t { return page_per_tile && i < n_tiles ? paged_key_page(a, b, my_lo + i * kGqaTile) : 0u; };
     if (PAGED)
 #pragma unroll
-        for (int i = 0; i < kGqaStages; ++i) next_page[i] = page_of_tile(i);
+        for (int i = 0; i < kPages; ++i) next_page[i] = page_of_tile(i);
     auto load_tile = [&](int i) {
         if (i < n_tiles) {
             const int st = i % kGqaStages, tile0 = my_lo + i * kGqaTile, key0 = tile0 + my_row;
@@ -1003,8 +1012,8 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
                                                  : static_cast<int64_t>(key0) * a.kv_st;
                 if (PAGED) {
 #pragma unroll
-                    for (int n = 1; n < kGqaStages; ++n) next_page[n - 1] = next_page[n];
-                    next_page[kGqaStages - 1] = page_of_tile(i + kGqaStages);
+                    for (int n = 1; n < kPages; ++n) next_page[n - 1] = next_page[n];
+                    next_page[kPages - 1] = page_of_tile(i + kPages);
                 }
                 if (whole) {
 #pragma unroll
@@ -1032,26 +1041,44 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
         }
         cp_async_commit();             // always: keeps the group count uniform
     };
-    // q and r of the group as A fragments (rows past the group: zeros), straight from global memory, so that all stages
-    // are free for the first tiles; requested behind the first tile, with which they are needed.
-    // (FEW: as B fragments, of 8 rows.)
-    constexpr int QF = FEW ? 2 : 4;
+    // q and r of the group as A fragments (FEW: as B fragments, of 8 rows), rows past the group as zeros, straight from global
+    // memory, so that all stages are free for the first tiles; requested behind the first tile, with which they are needed.
+    // A lane takes 16 bytes of every fourth chunk of its rows and the quad trades words.  (A word of the fragment per
+    // load is eight lines for 128 bytes each time: 4 rows of 1000 keys, 16 : 1 heads 24.8 us against 28.7, 32 : 2 17.4 against 29.5.)
+    constexpr int QF = FEW ? 2 : 4, QC = D / 32;
     uint32_t qa[KS][QF], ra[KS][QF];
+    uint4 qx[QF / 2][QC], rx[QF / 2][QC];
     load_tile(0);
     {
-        const T *qg = static_cast<const T *>(a.q) + (static_cast<int64_t>(b) * a.heads_q + hq0) * D + 2 * t;
-        const T *rg = static_cast<const T *>(a.r) + (static_cast<int64_t>(b) * a.heads_q + hq0) * D + 2 * t;
+        const int64_t at = (static_cast<int64_t>(b) * a.heads_q + hq0) * D + 8 * t;
+        const T *qg = static_cast<const T *>(a.q) + at, *rg = static_cast<const T *>(a.r) + at;
 #pragma unroll
-        for (int ks = 0; ks < KS; ++ks)
+        for (int h = 0; h < QF / 2; ++h)
 #pragma unroll
-            for (int e = 0; e < QF; ++e) {
-                const int row = FEW ? g : g + 8 * (e & 1), at = row * D + ks * 16 + 8 * (FEW ? e : e >> 1);
-                qa[ks][e] = row < n_rows ? *reinterpret_cast<const uint32_t *>(qg + at) : 0u;
-                ra[ks][e] = row < n_rows ? *reinterpret_cast<const uint32_t *>(rg + at) : 0u;
+            for (int j = 0; j < QC; ++j) {
+                const int row = g + 8 * h;
+                qx[h][j] = rx[h][j] = make_uint4(0u, 0u, 0u, 0u);
+                if (row < n_rows) {
+                    qx[h][j] = *reinterpret_cast<const uint4 *>(qg + row * D + 32 * j);
+                    rx[h][j] = *reinterpret_cast<const uint4 *>(rg + row * D + 32 * j);
+                }
             }
     }
 #pragma unroll
     for (int i = 1; i < kGqaStages; ++i) load_tile(i);
+#pragma unroll
+    for (int h = 0; h < QF / 2; ++h)
+#pragma unroll
+        for (int j = 0; j < QC; ++j) {
+            auto trade = [&](const uint4 &x, uint32_t (&f)[KS][QF]) {
+                uint32_t w[4] = {x.x, x.y, x.z, x.w};
+                sm100::quad_transpose(w, t);                   // w[i]: channels 2 t, + 1 of chunk 4 j + i
+#pragma unroll
+                for (int i = 0; i < 4; ++i) f[2 * j + (i >> 1)][FEW ? i & 1 : h + 2 * (i & 1)] = w[i];
+            };
+            trade(qx[h][j], qa);
+            trade(rx[h][j], ra);
+        }
 
     // State of two rows of the group, g and g + 8 (FEW: 2 t and 2 t + 1); d1 / d2 are this thread's share until the end.
     // Accumulators: channels 8 i + 2 t, + 1 of the two rows (FEW: channels 16 i + g and + 8).
@@ -1320,12 +1347,13 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
     if (plan.b < 0 || alone || s_arrived[w0] != n_ctas - 1) return;
     __threadfence();
     // last: merge the n_ctas records of every row, 32 at a time
+    constexpr int kAhead = FEW ? 16 : 8;
     for (int row = warp - w0; row < n_rows; row += n_seg) {
         const float *recs = recs_of(row);
-        warp_merge<D, 16>(recs, min(n_ctas, 32), lane, big, D1, D2, O1, O2);
+        warp_merge<D, kAhead>(recs, min(n_ctas, 32), lane, big, D1, D2, O1, O2);
         for (int j = 32; j < n_ctas; j += 32) {
             float big2, E1, E2, P1[CH], P2[CH];
-            warp_merge<D, 16>(recs + static_cast<int64_t>(j) * REC, min(n_ctas - j, 32), lane, big2, E1, E2, P1, P2);
+            warp_merge<D, kAhead>(recs + static_cast<int64_t>(j) * REC, min(n_ctas - j, 32), lane, big2, E1, E2, P1, P2);
             const float top = fmaxf(big, big2), safe = top == -INFINITY ? 0.f : top;
             const float wa = fast_exp2(big - safe), wb = fast_exp2(big2 - safe);
             big = top;

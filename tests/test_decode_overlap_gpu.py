@@ -62,6 +62,17 @@ def test_grouped_heads_at_the_edges_of_tiles_and_stages(hq, hkv, d, monkeypatch)
             assert torch.equal(plx.parallax_attn_with_kvcache(q, r, kp, vp, page_table=table), o)
 
 
+# 9, 12, 16 and 18 q heads per kv head: rows of the second half of a tile, all or some of them; 2 and 8: half a tile
+@pytest.mark.parametrize("hq,hkv,d", [(9, 1, 128), (12, 1, 64), (16, 1, 128), (36, 2, 64), (64, 8, 128), (4, 2, 64)])
+def test_grouped_heads_whose_records_meet_in_memory(hq, hkv, d, monkeypatch):
+    """Splits that leave one warp of a row in a CTA, and 1 to 32 records a row to merge there: either side of 8 and 16."""
+    for bsz, t, splits in ((4, 1000, 15), (3, 400, 9), (2, 1100, 17), (1, 4100, 63), (1, 4100, 65), (1, 2100, 128), (1, 2100, 130), (1, 4100, 256)):
+        monkeypatch.setenv("PLX_DECODE_SPLITS", str(splits))
+        q, r, k, v = inputs(bsz, hq, hkv, t, d, seed=splits)
+        o = plx.parallax_decode(q, r, k, v)
+        assert_close(o.float().cpu(), orc.decode(*[x.cpu() for x in (q, r, k, v)]), DECODE_REL_L2, DECODE_MAX_REL, f"{hq}:{hkv} {bsz} {t} {splits}")
+
+
 @pytest.mark.parametrize("bsz,hq,hkv", [(1, 8, 8), (64, 8, 8), (64, 8, 2), (65, 8, 8)])
 def test_a_graphed_step_in_one_launch(bsz, hq, hkv):
     """Up to 64 rows the inputs and the sweep are one launch; its buffers and answer are those of the copies and the replay."""
