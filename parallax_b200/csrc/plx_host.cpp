@@ -26,6 +26,7 @@
 #include <cmath>
 #include <cstdlib>
 #include <list>
+#include <map>
 #include <memory>
 #include <mutex>
 #include <optional>
@@ -328,31 +329,68 @@ Workspaces &workspaces() {
 }
 
 // A stream of this library beside one of the caller's, for small copies that must not stand between two kernels there.
-// One per (device, stream), so that no copy waits for work of a stream that it has nothing to do with.  At most kMax are
-// kept; one that is dropped lives on until its last user has waited for its copy.
+struct SideStream {
+    cudaStream_t stream = nullptr;
+    SideStream() = default;
+    SideStream(const SideStream &) = delete;
+    bool make() { return cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) == cudaSuccess; }
+    ~SideStream() {
+        if (stream) (void)cudaStreamDestroy(stream);
+    }
+};
+
+// One per stream, so that no copy waits for work of a stream that it has nothing to do with; at most kMax per device, which is
+// as many as PyTorch hands out at a priority.  A stream beyond them takes the place of one that none of the last kStale
+// calls on the device was for, if there is one; else there is none to spare.  (Calls that went round 40 streams, with the least
+// recently used one dropped each time: 150 us each, 37 with the copies on their own streams.)  One that is dropped lives
+// on until its last user has waited for its copy.
 class SideStreams {
 public:
-    using Handle = std::shared_ptr<CUstream_st>;
+    using Handle = std::shared_ptr<SideStream>;
+    // null: none to spare
     Handle get(const c10::cuda::CUDAStream &main) {
-        const Key key{main.device_index(), reinterpret_cast<uintptr_t>(main.stream())};
         std::lock_guard<std::mutex> lock(mu_);
-        for (auto it = list_.begin(); it != list_.end(); ++it)
-            if (it->first == key) {
-                list_.splice(list_.begin(), list_, it);
-                return it->second;
+        PerDevice &d = devices_[main.device_index()];
+        const int64_t now = ++d.calls;
+        for (auto it = d.list.begin(); it != d.list.end(); ++it)
+            if (it->main == main.stream()) {
+                it->used = now;
+                d.list.splice(d.list.begin(), d.list, it);
+                return it->side;
             }
-        cudaStream_t made = nullptr;
-        C10_CUDA_CHECK(cudaStreamCreateWithFlags(&made, cudaStreamNonBlocking));
-        list_.emplace_front(key, Handle(made, [](cudaStream_t st) { (void)cudaStreamDestroy(st); }));
-        if (list_.size() > kMax) list_.pop_back();
-        return list_.front().second;
+        if (d.list.size() >= kMax) {
+            if (now - d.list.back().used < kStale) return nullptr;
+            d.list.pop_back();
+        }
+        Handle side = std::make_shared<SideStream>();
+        if (!side->make()) {
+            (void)cudaGetLastError();
+            return nullptr;
+        }
+        ++made_;
+        d.list.push_front(Entry{main.stream(), side, now});
+        return side;
+    }
+    int64_t made() {
+        std::lock_guard<std::mutex> lock(mu_);
+        return made_;
     }
 
 private:
-    using Key = std::pair<int64_t, uintptr_t>;
+    struct Entry {
+        cudaStream_t main;
+        Handle side;
+        int64_t used;
+    };
+    struct PerDevice {
+        std::list<Entry> list;     // the last used one first
+        int64_t calls = 0;
+    };
     static constexpr size_t kMax = 32;
+    static constexpr int64_t kStale = 1024;
     std::mutex mu_;
-    std::list<std::pair<Key, Handle>> list_;
+    std::map<int64_t, PerDevice> devices_;
+    int64_t made_ = 0;
 };
 SideStreams &side_streams() {
     static SideStreams *s = new SideStreams;   // not destroyed at exit, when the CUDA context may be gone
@@ -369,9 +407,9 @@ public:
         if (!lens) return;
         host_ = at::empty({lens->numel()}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
         c10::cuda::CUDAStream on = stream;
-        if (beside) {
-            side_ = side_streams().get(stream);
-            on = c10::cuda::getStreamFromExternal(side_.get(), stream.device_index());
+        if (beside) side_ = side_streams().get(stream);
+        if (side_) {
+            on = c10::cuda::getStreamFromExternal(side_->stream, stream.device_index());
             ready_.record(stream);
             ready_.block(on);
         }
@@ -611,4 +649,5 @@ PYBIND11_MODULE(_plx_host, m) {
     m.def("attend", &attend);
     m.def("apart", &apart);
     m.def("step", &step);
+    m.def("side_streams_made", [] { return side_streams().made(); });
 }

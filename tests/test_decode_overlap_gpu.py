@@ -169,3 +169,26 @@ def test_lengths_beside_a_long_launch(bsz, hq, hkv, t, lq):
                 bad[row] = t
                 assert torch.equal(plx.parallax_attn_with_kvcache(q, q, k, v, seqused_k=bad), want)
         torch.cuda.synchronize()
+
+
+def test_lengths_beside_launches_on_many_streams():
+    """More streams than the library keeps one beside: the answers and the errors are the same, and none is made anew each time."""
+    q, r, k, v = inputs(2, 32, 8, 4096)
+    streams = [torch.cuda.Stream(priority=p) for p in (0, -1) for _ in range(24)]
+    assert len({s.cuda_stream for s in streams}) > 40
+    lens = torch.tensor([4096, 3000], dtype=torch.int32, device="cuda")
+    bad = torch.tensor([4096, 4097], dtype=torch.int32, device="cuda")
+    want = plx.parallax_attn_with_kvcache(q, r, k, v, seqused_k=lens)
+    torch.cuda.synchronize()
+    made = None
+    for _ in range(3):
+        for s in streams:
+            with torch.cuda.stream(s):
+                got = plx.parallax_attn_with_kvcache(q, r, k, v, seqused_k=lens)
+                with pytest.raises(ValueError):
+                    plx.parallax_attn_with_kvcache(q, r, k, v, seqused_k=bad)
+            s.synchronize()
+            assert torch.equal(got, want)
+        if made is not None:
+            assert _cabi.host().side_streams_made() == made
+        made = _cabi.host().side_streams_made()
