@@ -328,13 +328,22 @@ Workspaces &workspaces() {
     return *w;
 }
 
-// A stream of this library beside one of the caller's, for small copies that must not stand between two kernels there.
+// A stream of this library beside one of the caller's, for small copies that must not stand between two kernels there, and
+// the two events of the way there and back (to make and drop two per call was 1 us of it).  Threads that share the caller's stream
+// share these: an event that another thread has recorded again is one that comes later on the same stream.
 struct SideStream {
     cudaStream_t stream = nullptr;
+    cudaEvent_t ready = nullptr, copied = nullptr;
     SideStream() = default;
     SideStream(const SideStream &) = delete;
-    bool make() { return cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) == cudaSuccess; }
+    bool make() {
+        return cudaStreamCreateWithFlags(&stream, cudaStreamNonBlocking) == cudaSuccess &&
+               cudaEventCreateWithFlags(&ready, cudaEventDisableTiming) == cudaSuccess &&
+               cudaEventCreateWithFlags(&copied, cudaEventDisableTiming) == cudaSuccess;
+    }
     ~SideStream() {
+        if (copied) (void)cudaEventDestroy(copied);
+        if (ready) (void)cudaEventDestroy(ready);
         if (stream) (void)cudaStreamDestroy(stream);
     }
 };
@@ -406,24 +415,25 @@ public:
     LengthCheck(const OptTensor &lens, const c10::cuda::CUDAStream &stream, bool beside) {
         if (!lens) return;
         host_ = at::empty({lens->numel()}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
-        c10::cuda::CUDAStream on = stream;
+        cudaStream_t on = stream.stream();
         if (beside) side_ = side_streams().get(stream);
         if (side_) {
-            on = c10::cuda::getStreamFromExternal(side_->stream, stream.device_index());
-            ready_.record(stream);
-            ready_.block(on);
+            C10_CUDA_CHECK(cudaEventRecord(side_->ready, on));
+            on = side_->stream;
+            C10_CUDA_CHECK(cudaStreamWaitEvent(on, side_->ready, 0));
         }
-        C10_CUDA_CHECK(cudaMemcpyAsync(host_.data_ptr(), lens->data_ptr(), sizeof(int32_t) * lens->numel(), cudaMemcpyDeviceToHost, on.stream()));
-        copied_.record(on);
+        C10_CUDA_CHECK(cudaMemcpyAsync(host_.data_ptr(), lens->data_ptr(), sizeof(int32_t) * lens->numel(), cudaMemcpyDeviceToHost, on));
+        if (side_) C10_CUDA_CHECK(cudaEventRecord(side_->copied, on));
+        else copied_.record(stream);
     }
     ~LengthCheck() {
-        if (host_.defined() && !waited_) cudaEventSynchronize(copied_.event());   // the copy still writes to host_
+        if (host_.defined() && !waited_) (void)cudaEventSynchronize(copied());   // the copy still writes to host_
     }
     bool within(int64_t lo, int64_t hi) {
         if (!host_.defined()) return true;
         {
             py::gil_scoped_release nogil;
-            copied_.synchronize();
+            C10_CUDA_CHECK(cudaEventSynchronize(copied()));
         }
         waited_ = true;
         const int32_t *n = host_.data_ptr<int32_t>();
@@ -433,21 +443,23 @@ public:
     }
 
 private:
+    cudaEvent_t copied() const { return side_ ? side_->copied : copied_.event(); }
     Tensor host_;
     SideStreams::Handle side_;
-    at::cuda::CUDAEvent ready_{cudaEventDisableTiming}, copied_{cudaEventDisableTiming};
+    at::cuda::CUDAEvent copied_{cudaEventDisableTiming};
     bool waited_ = false;
 };
 
-// What lasts: by the keys and values of a decode launch at the cache ceiling, by the products of a prefill launch.  The
-// way over a second stream takes the host 1 to 2 us more per call, which short launches do not hide.  Before the launch
-// against beside it, us per call: 32 : 8 heads, 4 MB 18.9 / 19.0, 17 MB 22.5 / 20.2, 34 MB 26.6 / 18.4, 134 MB 40.6 / 30.7; 8 : 8
-// heads, 8 MB 15.2 / 16.8, 34 MB 16.7 / 17.1, 67 MB 27.5 / 21.3; prefill, 0.3 GFLOP 15.9 / 17.0, 1.1 GFLOP 23.4 / 17.5, 137 GFLOP
-// 107 / 101.
+// What lasts: by the bytes of keys and values of a decode launch, by the products of a prefill launch, both at the cache ceiling
+// (the lengths themselves are on the device).  Where the launch does not last after all, as with short rows in a large cache,
+// the way over a second stream takes the host 0.2 to 0.3 us more per call (16 rows of 50 in 8192 keys in pages, 32 : 8 heads, 14.9 us
+// either way).  Copy before the launch against beside it, us per call: 32 : 8 heads, 1 MB 15.2 / 15.5, 2 MB 15.7 / 15.6,
+// 4 MB 20.7 / 15.8, 17 MB 22.1 / 16.6, 67 MB 29.0 / 22.8; 8 : 8 heads, 8 MB 15.3 / 15.4, 17 MB 16.5 / 15.8 and 15.3 / 15.5, 34 MB 26.8 / 17.3,
+// 67 MB 27.8 / 22.1; prefill, 32 : 8 heads, 0.1 GFLOP 15.5 / 15.7, 0.3 GFLOP 25.1 / 17.0 and 15.4 / 15.6, 1.1 GFLOP 42.0 / 36.7 and 17.3 / 15.7.
 bool decode_lasts(const Tensor &q, const Tensor &k, int64_t n_keys) {
-    return 4. * q.size(0) * n_keys * k.size(2) * q.size(3) >= (q.size(2) > k.size(2) ? 4e6 : 48e6);
+    return 4. * q.size(0) * n_keys * k.size(2) * q.size(3) >= (q.size(2) > k.size(2) ? 2e6 : 16e6);
 }
-bool prefill_lasts(const Tensor &q, int64_t ceiling) { return 8. * q.numel() * ceiling >= 1e9; }
+bool prefill_lasts(const Tensor &q, int64_t ceiling) { return 8. * q.numel() * ceiling >= 2.5e8; }
 
 bool int32_vector(const OptTensor &t, int64_t n, const at::Device &device) {
     return !t || (plain_tensor(*t) && t->scalar_type() == at::kInt && t->dim() == 1 && t->size(0) == n && t->is_contiguous() && t->device() == device);
