@@ -34,6 +34,7 @@
 // At 64: acc0 [0,64), acc1 [64,128), the two score buffers at 128 and 320.
 #include <cuda.h>
 
+#include <algorithm>
 #include <climits>
 #include <cstdlib>
 #include <mutex>
@@ -92,7 +93,7 @@ constexpr uint32_t kStatBytes = kBN * 16;      // four planes of 64 floats: -mL,
 //
 // SHORT (dq/dr at 128): dO is a resident tile in shared memory like q and r, which costs a stage of the ring.  On the way into
 // tensor memory it passes through the registers of the element-wise warps at the start of an item, 2500 of the 11300 clocks
-// that an item of 2.3 streamed tiles takes.  See short_items.
+// that an item of 2.3 streamed tiles took.  See short_items.
 template <int D, int MODE, bool SHORT>
 struct Plan {
     static constexpr bool kTwo = D == 64, kMTile = D == 128 && !SHORT;
@@ -934,10 +935,22 @@ int launch_mode(const TrainArgs &a, int n_tok, const ErrSink &sink, bool overlap
     return st == cudaSuccess && cudaGetLastError() == cudaSuccess ? PLX_OK : PLX_ERR_LAUNCH;
 }
 
-// SHORT pays where items are short and costs a stage of the ring where they are long.  dq/dr, us, tile in tensor memory against
-// shared memory: dense, 100 tokens 53.0 / 48.8, 512 85.0 / 77.0, 1024 109 / 107, 2048 170 / 171.5, 4096 1148 / 1148; packed, 16 : 4
-// heads, sequences of 1 to 256 290 / 268, 256 to 1024 376 / 366, 1000 to 3000 786 / 788, 64 to 8192 (65536 tokens) 3296 / 3370.
-bool short_items(const TrainArgs &a) { return (a.cu ? a.len_q / a.n_seqs : a.len_q) <= 1024; }
+// SHORT pays where an item streams few tiles and costs a stage of the ring where it streams many: what counts is the keys that
+// the mean item of 128 rows sees, len_k - len_q / 2 + 64 in a dense problem (rows are the last ones of the keys) and at
+// most the window and the item's own rows.  Lengths of packed sequences are on the device; for lengths spread evenly from 1 up
+// to twice their mean the mean item sees 2 / 3 of the mean and 64.
+// dq/dr alone, us, tile in tensor memory against shared memory.  By keys: dense, B=16, H=16, 128 tokens (128 keys) 20.5 / 16.5, 512
+// (320) 80.9 / 73.9, 1024 (576) 203 / 193; B=8, 1536 (832) 198.7 / 196.2, 2048 (1088) 325 / 317 to 334; B=4, 2048 165.6 / 166.6;
+// 128 rows against 512 keys (512) 43 / 40, 1024 (1024) 58.1 / 57.5, 2048 (2048) 87.9 / 94.4, 4096 (4096) 75.8 / 82.9; 512 against
+// 1024 (832) 80.4 / 78.8, 1536 (1344) 114.6 / 116.6, 2048 (1856) 151 / 156; 4096 tokens, window 64 (192) 138 / 111, 256 (384) 167 / 149, 512
+// (640) 216 / 211, 768 (896) 274 / 262, 1024 (1152) 326 / 317, 2048 506 / 505.  Packed, 1 to 256 tokens, 16 : 4 heads (149) 324 / 298,
+// 256 to 1024 (490) 378 / 374, 256 to 1700 (704) 463 / 463, 15 of 2048 625 / 623, 64 to 8192 2770 / 2786.  A few long sequences among very many
+// short ones are on the wrong side of it: one of 16384 and 256 of 64 2445 / 2568, two of 8192 and 200 of 64 1257 / 1272.
+bool short_items(const TrainArgs &a) {
+    int64_t keys = a.cu ? 2ll * a.len_q / (3ll * a.n_seqs) + kBM / 2 : a.len_k - a.len_q / 2 + std::min(a.len_q, kBM) / 2;
+    if (a.window > 0) keys = std::min<int64_t>(keys, a.window + kBM);
+    return keys <= 14 * kBN;
+}
 
 }  // namespace
 
