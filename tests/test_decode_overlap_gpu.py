@@ -48,6 +48,35 @@ def test_calls_that_feed_each_other(bsz, hq, hkv, t, page):
         assert torch.equal(x, y)
 
 
+@pytest.mark.parametrize("bsz,n,h,d,hkv", [(1, 1500, 8, 128, 8), (2, 900, 16, 64, 4), (1, 2600, 8, 128, 2)])
+def test_a_decode_call_right_behind_a_backward(bsz, n, h, d, hkv):
+    """dk/dv lets dq/dr in early and dq/dr waits for it at its end: a decode launch behind them, which comes early too, reads dk and
+    dv as its caches and a row of dq and of dr as its query, with no synchronisation in between."""
+    gen = torch.Generator(device="cuda").manual_seed(3)
+
+    def randn(*shape):
+        return torch.randn(*shape, generator=gen, device="cuda").bfloat16()
+
+    leaves = [randn(bsz, n, heads, d).requires_grad_(True) for heads in (h, h, hkv, hkv)]
+    o = plx.parallax_varlen_func(*leaves)
+    grads = [randn(bsz, n, h, d) for _ in range(6)]
+
+    def chain(wait):
+        got = []
+        for go in grads:
+            dq, dr, dk, dv = torch.autograd.grad(o, leaves, go, retain_graph=True)
+            wait()
+            got.append(plx.parallax_decode(dq[:, -1:], dr[:, -1:], dk, dv))
+            wait()
+            got.append(plx.parallax_decode(got[-1], dr[:, :1], dv, dk))
+        return got
+
+    want = chain(torch.cuda.synchronize)
+    torch.cuda.synchronize()
+    for x, y in zip(chain(lambda: None), want):
+        assert torch.equal(x, y)
+
+
 @pytest.mark.parametrize("hq,hkv,d", [(4, 1, 128), (18, 1, 128), (32, 8, 64)])
 def test_grouped_heads_at_the_edges_of_tiles_and_stages(hq, hkv, d, monkeypatch):
     """0 to 5 tiles of 16 keys per warp (three stages), the last one whole, of one key and one key short."""
@@ -96,6 +125,50 @@ def test_a_graphed_step_in_one_launch(bsz, hq, hkv):
     two = gd(q=gd.out).clone()
     assert torch.equal(gd.q, want) and torch.equal(gd.replay(), two)
     assert torch.equal(gd(q=gd.r, r=gd.q), gd.replay())
+
+
+@pytest.mark.parametrize("bsz,hq,hkv,d,dtype,window,static", [
+    (4, 8, 8, 128, torch.bfloat16, None, False), (64, 8, 8, 64, torch.float16, 50, False), (3, 36, 2, 128, torch.bfloat16, None, False),
+    (16, 12, 1, 64, torch.bfloat16, 70, False), (20, 32, 8, 128, torch.float16, None, False), (2, 16, 16, 128, torch.bfloat16, None, True),
+    (5, 8, 2, 128, torch.bfloat16, 33, True), (65, 8, 8, 128, torch.bfloat16, None, False)])
+def test_which_way_a_step_goes(bsz, hq, hkv, d, dtype, window, static):
+    """Up to 64 rows a step leaves its graph alone, beyond them it replays it once; either way its buffers and answer are those of
+    copies and a replay, with q, r and lengths given or only some of them, with lengths that are dealt out (far apart), windows,
+    two groups of heads per kv head, and at a static length."""
+    t = 900
+    gd = plx.GraphedDecode(bsz, hq, **({"kv_len": t} if static else {"max_kv_len": t}), head_dim=d, H_kv=hkv, dtype=dtype, window_size=window)
+    ref = plx.GraphedDecode(bsz, hq, **({"kv_len": t} if static else {"max_kv_len": t}), head_dim=d, H_kv=hkv, dtype=dtype, window_size=window)
+    q, r, k, v = (x.to(dtype) for x in inputs(bsz, hq, hkv, t, d))
+    for g in (gd, ref):
+        g.k.copy_(k)
+        g.v.copy_(v)
+    graph, replays = gd.graph, []
+
+    class Counted:
+        def replay(self):
+            replays.append(1)
+            graph.replay()
+
+    gd.graph = Counted()
+    lens = [t if i % 5 == 0 else 1 + (i * 37) % 200 for i in range(bsz)]
+    steps = [dict(q=q, r=r), dict(r=q), dict(q=r), dict()]
+    if not static:
+        steps += [dict(q=q, r=r, cache_seqlens=lens), dict(r=q), dict(cache_seqlens=lens[::-1]), dict(q=r, cache_seqlens=t)]
+    for i, given in enumerate(steps):
+        for name in ("q", "r"):
+            if name in given:
+                getattr(ref, name).copy_(given[name])
+        if "cache_seqlens" in given:
+            n = given["cache_seqlens"]
+            ref.cache_seqlens.copy_(torch.tensor(n if isinstance(n, list) else [n] * bsz, dtype=torch.int32))
+        want = ref.replay()
+        replays.clear()
+        gd.out.zero_()
+        got = gd(**given)
+        assert len(replays) == (0 if bsz <= 64 else 1), i
+        assert torch.equal(got, want), i
+        for x, y in ((gd.q, ref.q), (gd.r, ref.r), (gd.cache_seqlens, ref.cache_seqlens)):
+            assert (x is None and y is None) or torch.equal(x, y), i
 
 
 def test_inputs_that_share_memory_but_not_a_storage():
