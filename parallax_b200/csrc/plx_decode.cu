@@ -380,8 +380,7 @@ __device__ __forceinline__ SplitPlan plan_slot(const DecodeArgs &a, int slot, in
 // Decode kernels are launched without waiting for the kernel before them to be over and done with (launch_overlapped): their
 // CTAs come as soon as its last one has left, and wait (grid_wait, before anything touches global memory) for its writes.
 // What they read may have been written while they were already resident, so no load takes the non-coherent path.
-// Calls one after the other, us: B = 1, 8192 keys, 32 : 8 heads 14.8 -> 13.1, 1000 keys 14.5 -> 12.1; 8 : 8 heads, B = 1, 4096
-// keys 12.2 -> 9.9, B = 32, 1024 keys 30.6 -> 28.5, B = 16, 8192 keys 92 -> 90.  Letting the next launch in earlier
+// Calls one after the other, us: 8 : 8 heads, B = 1, 4096 keys 12.2 -> 9.9, B = 32, 1024 keys 30.6 -> 28.5, B = 16, 8192 keys 92 -> 90.  Letting the next launch in earlier
 // (griddepcontrol.launch_dependents, at the start or after the sweep) was slower: its CTAs then go where SMs are free first
 // instead of evenly over the chip.  B = 64, 4096 keys, 32 : 8 heads, 128 CTAs: 164 us at the end, 180 after the sweep.
 template <typename... Params, typename... Args>
@@ -910,8 +909,9 @@ int launch_decode_exchange_merge(const ExchangeArgs &x, const float *part, int h
 //
 // Short launches are bound by latency, long ones by HBM and by what the warps have in flight: three tiles each from the
 // start (q and r go straight to registers instead of through the last stage), the next one as soon as a stage is free.
-// 32 : 8 heads, us, with the transposed products below: B = 1, 8192 keys 15.4 -> 13.1, B = 1, 32768 keys 31.4 -> 28.4; B = 64,
-// 4096 keys 168 -> 164 (6.5 TB/s); 16 : 2 heads, B = 3, 3000 keys 15.0 -> 13.8.
+// Calls one after the other, us, this, the overlapped launches (above) and the transposed products (below) together: 32 : 8 heads, B = 1,
+// 1000 keys 16.5 -> 12.2, 8192 keys 16.4 -> 12.2, 32768 keys 31.7 -> 28.1, B = 64, 4096 keys 163.6 -> 157.2 (6.8 TB/s); 16 : 2 heads, B = 3,
+// 3000 keys 18.6 -> 13.8; 16 : 1 heads, B = 8, 8192 keys 22.8 -> 19.0.
 // ========================================================================= //
 // a lane's channels of a record, 16 or 8 bytes
 __device__ __forceinline__ void load_channels(const float *p, float (&x)[4]) {
@@ -950,8 +950,8 @@ struct GqaSmem {
 //
 // FEW: at most 8 q heads per kv head, the usual case.  Then the products are transposed -- keys are the M dimension of the
 // scores (S^T = K Q_g^T), channels that of the outputs (O^T += V^T P^T), and the heads the 8 columns -- which takes half the
-// MMAs, with none of them on rows of zeros, and half the registers for accumulators and fragments (in all 207 at head_dim 128,
-// where the other form fills 255); a movmatrix per 8 x 8 block turns P^T around.
+// MMAs, with none of them on rows of zeros, and half the registers for accumulators and fragments (in all 190 to 201 at
+// head_dim 128, where the other form fills 255); a movmatrix per 8 x 8 block turns P^T around.
 // B = 16, 1024 keys, 32 : 8 heads 16.7 -> 16.0 us, B = 8, 4000 keys, rows of different lengths 40.8 -> 34.0.
 template <typename T, int D, bool PAGED, bool FEW>
 __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const DecodeArgs a, int n_hgroups) {

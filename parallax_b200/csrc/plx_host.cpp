@@ -603,7 +603,9 @@ bool apart(const py::tuple &sources, const py::tuple &buffers) {
 // A GraphedDecode step: q, r and the lengths into its buffers, and the launch that its graph holds, on the same buffers and
 // scratch, in one (up to PLX_DECODE_STEP_ROWS rows, inputs that lie apart from what it writes; else only the inputs are put in place).  kNothing, having done nothing, for
 // anything but tensors like the buffers and lengths given as Python integers in [1, most].
-// 4 rows of up to 4096 keys, 8 : 8 heads: 22.3 us for a launch that puts the inputs in place and the graph behind it.
+// 8 : 8 heads, a launch that puts the inputs in place and the graph behind it against one launch, us: 4 rows of up to 4096 keys
+// 20.5 / 14.1, 64 rows of up to 512 34.9 / 28.1.  (64: the lengths are launch parameters of every decode kernel, 4 bytes a row; more
+// rows were not measured.)
 enum Step { kNothing = 0, kStaged = 1, kDone = 2 };
 int step(const py::object &q_, const py::object &q_src_, const py::object &r_, const py::object &r_src_, const py::object &lens_,
          const py::object &lens_src, int64_t most, const py::object &k_, const py::object &v_, const py::object &out_, const py::object &ws_,

@@ -1,6 +1,6 @@
 """The two plans of the backward that depend on the problem.  head_dim 64, whose element-wise groups take the streamed tiles in
 turn: work items of every small tile count in a row on one CTA, so that items begin with either group and a group has no
-tile of some of them.  head_dim 128, whose dq/dr keeps dO in shared memory up to 1024 tokens and in tensor memory above."""
+tile of some of them.  head_dim 128, whose dq/dr keeps dO in shared memory where items see few keys and in tensor memory else."""
 import pytest
 import torch
 
@@ -84,7 +84,7 @@ def test_dq_dr_of_few_and_many_keys(lq, lk, window):
 
 
 @pytest.mark.parametrize("lens,lk,window,short", [
-    ([1024], 1024, -1, True), ([1600], 1600, -1, True), ([1700], 1700, -1, False), ([128], 4096, -1, False), ([512], 2048, -1, False),
+    ([1024], 1024, -1, True), ([1664], 1664, -1, True), ([1665], 1665, -1, False), ([3000], 3000, 768, True), ([3000], 3000, 769, False), ([128], 4096, -1, False), ([512], 2048, -1, False),
     ([128], 512, -1, True), ([3000], 3000, 100, True), ([3000], 3000, 1100, False), ([100] * 20, 0, -1, True), ([3000, 2000], 0, -1, False),
     ([3000, 2000], 0, 64, True)])
 def test_which_dq_dr_runs(lens, lk, window, short):
