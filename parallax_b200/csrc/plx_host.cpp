@@ -450,16 +450,17 @@ private:
     bool waited_ = false;
 };
 
-// What lasts: by the bytes of keys and values of a decode launch, by the products of a prefill launch, both at the cache ceiling
-// (the lengths themselves are on the device).  Where the launch does not last after all, as with short rows in a large cache,
-// the way over a second stream takes the host 0.2 to 0.3 us more per call (16 rows of 50 in 8192 keys in pages, 32 : 8 heads, 14.9 us
-// either way).  Copy before the launch against beside it, us per call: 32 : 8 heads, 1 MB 15.2 / 15.5, 2 MB 15.7 / 15.6,
-// 4 MB 20.7 / 15.8, 17 MB 22.1 / 16.6, 67 MB 29.0 / 22.8; 8 : 8 heads, 8 MB 15.3 / 15.4, 17 MB 16.5 / 15.8 and 15.3 / 15.5, 34 MB 26.8 / 17.3,
-// 67 MB 27.8 / 22.1; prefill, 32 : 8 heads, 0.1 GFLOP 15.5 / 15.7, 0.3 GFLOP 25.1 / 17.0 and 15.4 / 15.6, 1.1 GFLOP 42.0 / 36.7 and 17.3 / 15.7.
+// What lasts: a decode launch by the bytes of its keys and values, a prefill launch by the keys that an item goes through or by its
+// products, all at the cache ceiling (the lengths themselves are on the device).  Where the launch does not last after all, as with
+// short rows in a large cache, the way over a second stream takes the host 0.2 to 0.3 us more per call (16 rows of 50 in 8192 keys in
+// pages, 32 : 8 heads, 14.9 us either way).  Copy before the launch against beside it, us per call: 32 : 8 heads, 1 MB 15.2 / 15.5, 2 MB
+// 15.7 / 15.6, 4 MB 20.7 / 15.8, 17 MB 22.1 / 16.6, 67 MB 29.0 / 22.8; 8 : 8 heads, 8 MB 15.3 / 15.4, 17 MB 16.5 / 15.8 and 15.3 / 15.5,
+// 34 MB 26.8 / 17.3, 67 MB 27.8 / 22.1; prefill, 32 : 8 heads, 1 row of 8 or 46 tokens, 190 keys 15.3 / 15.4, 256 15.5 / 15.6, 320 16.1 / 15.7,
+// 512 22.6 / 16.4, 1000 27.6 / 22.5; 4 of 32, 190 keys (0.8 GFLOP) 15.3 / 15.6, 320 16.8 / 15.7; 8 of 64, 64 keys (1.1 GFLOP) 16.7 / 15.6, 190 27.2 / 17.7.
 bool decode_lasts(const Tensor &q, const Tensor &k, int64_t n_keys) {
     return 4. * q.size(0) * n_keys * k.size(2) * q.size(3) >= (q.size(2) > k.size(2) ? 2e6 : 16e6);
 }
-bool prefill_lasts(const Tensor &q, int64_t ceiling) { return 8. * q.numel() * ceiling >= 2.5e8; }
+bool prefill_lasts(const Tensor &q, int64_t ceiling) { return ceiling > 256 || 8. * q.numel() * ceiling >= 1e9; }
 
 bool int32_vector(const OptTensor &t, int64_t n, const at::Device &device) {
     return !t || (plain_tensor(*t) && t->scalar_type() == at::kInt && t->dim() == 1 && t->size(0) == n && t->is_contiguous() && t->device() == device);
