@@ -115,9 +115,11 @@ __device__ __forceinline__ void store_elem<__half>(void *out, int64_t idx, float
 // Merge of n <= 32 partial records (stride REC floats) by one warp.  On return every lane holds the
 // maximum, the two sums, and the D / 32 channels lane * (D / 32) .. of O1 and O2, all relative to
 // the common maximum.  Bound by round trips to the L2: the channels of the first N records are requested together
-// with the headers of all (of those that there are: a warp may be the only one of its CTA to merge all rows of a kv head, and with N
-// records read for each whatever n, calls of 4 rows of 1000 keys went from 27 to 35 us at 16 : 1 heads, from 16.5 to 20.4 at 64 : 8).
-template <int D, int N = 8>
+// with the headers of all.  SKIP: of those that there are (grouped heads: a warp may be the only one of its CTA to merge all rows of
+// a kv head, and with N records read for each whatever n, calls of 4 rows of 1000 keys went from 27 to 35 us at 16 : 1 heads, from
+// 16.5 to 20.4 at 64 : 8).  Without it where a warp merges one row: there the condition costs more than the reads (25 rows of 14518
+// down to 5000 keys, 8 : 8 heads, 166.9 us against 165.7).
+template <int D, int N = 8, bool SKIP = false>
 __device__ __forceinline__ void warp_merge(const float *rec0, int n, int lane, float &big, float &D1, float &D2,
                                            float (&O1)[D / 32], float (&O2)[D / 32]) {
     constexpr int CH = D / 32, REC = 2 * D + 4;
@@ -128,12 +130,12 @@ __device__ __forceinline__ void warp_merge(const float *rec0, int n, int lane, f
     auto load = [&](int j0) {
 #pragma unroll
         for (int j = 0; j < N; ++j) {
-            if (j0 + j >= n) {
+            if (SKIP && j0 + j >= n) {
 #pragma unroll
                 for (int e = 0; e < CH; ++e) x[j][e] = y[j][e] = 0.f;
                 continue;
             }
-            const float *pr = col + static_cast<int64_t>(j0 + j) * REC;
+            const float *pr = col + static_cast<int64_t>(SKIP ? j0 + j : min(j0 + j, n - 1)) * REC;   // weight 0 past the end
             if (CH == 4) {
                 const float4 u = __ldcg(reinterpret_cast<const float4 *>(pr)), v = __ldcg(reinterpret_cast<const float4 *>(pr + D));
                 x[j][0] = u.x; x[j][1] = u.y; x[j][CH - 2] = u.z; x[j][CH - 1] = u.w;
@@ -910,7 +912,7 @@ int launch_decode_exchange_merge(const ExchangeArgs &x, const float *part, int h
 // Short launches are bound by latency, long ones by HBM and by what the warps have in flight: three tiles each from the
 // start (q and r go straight to registers instead of through the last stage), the next one as soon as a stage is free.
 // Calls one after the other, us, this, the overlapped launches (above) and the transposed products (below) together: 32 : 8 heads, B = 1,
-// 1000 keys 16.5 -> 12.2, 8192 keys 16.4 -> 12.2, 32768 keys 31.7 -> 28.1, B = 64, 4096 keys 163.6 -> 157.2 (6.8 TB/s); 16 : 2 heads, B = 3,
+// 1000 keys 16.5 -> 12.2, 8192 keys 16.4 -> 11.8, 32768 keys 31.7 -> 28.1, B = 64, 4096 keys 163.6 -> 157.2 (6.8 TB/s); 16 : 2 heads, B = 3,
 // 3000 keys 18.6 -> 13.8; 16 : 1 heads, B = 8, 8192 keys 22.8 -> 19.0.
 // ========================================================================= //
 // a lane's channels of a record, 16 or 8 bytes
@@ -1043,42 +1045,54 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
     };
     // q and r of the group as A fragments (FEW: as B fragments, of 8 rows), rows past the group as zeros, straight from global
     // memory, so that all stages are free for the first tiles; requested behind the first tile, with which they are needed.
-    // A lane takes 16 bytes of every fourth chunk of its rows and the quad trades words.  (A word of the fragment per
-    // load is eight lines for 128 bytes each time: 4 rows of 1000 keys, 16 : 1 heads 24.8 us against 28.7, 32 : 2 17.4 against 29.5.)
+    // Beyond 4 rows a lane takes 16 bytes of every fourth chunk of its rows and the quad trades words, else a word of the fragment
+    // per load, which is a line per row each time.  (Words against 16 bytes: 4 rows of 1000 keys, 16 : 1 heads 28.7 / 24.8 us, 64 : 8
+    // 16.8 / 13.1; one row of 400 keys, 32 : 8 heads 8.75 / 8.9.)
     constexpr int QF = FEW ? 2 : 4, QC = D / 32;
+    const bool words = FEW && n_rows <= 4;
     uint32_t qa[KS][QF], ra[KS][QF];
     uint4 qx[QF / 2][QC], rx[QF / 2][QC];
     load_tile(0);
     {
-        const int64_t at = (static_cast<int64_t>(b) * a.heads_q + hq0) * D + 8 * t;
+        const int64_t at = (static_cast<int64_t>(b) * a.heads_q + hq0) * D;
         const T *qg = static_cast<const T *>(a.q) + at, *rg = static_cast<const T *>(a.r) + at;
+        if (words) {
+#pragma unroll
+            for (int ks = 0; ks < KS; ++ks)
+#pragma unroll
+                for (int e = 0; e < 2; ++e) {
+                    const int x = g * D + ks * 16 + 8 * e + 2 * t;
+                    qa[ks][e] = g < n_rows ? *reinterpret_cast<const uint32_t *>(qg + x) : 0u;
+                    ra[ks][e] = g < n_rows ? *reinterpret_cast<const uint32_t *>(rg + x) : 0u;
+                }
+        } else {
+#pragma unroll
+            for (int h = 0; h < QF / 2; ++h)
+#pragma unroll
+                for (int j = 0; j < QC; ++j) {
+                    const int row = g + 8 * h, x = row * D + 32 * j + 8 * t;
+                    qx[h][j] = row < n_rows ? *reinterpret_cast<const uint4 *>(qg + x) : make_uint4(0u, 0u, 0u, 0u);
+                    rx[h][j] = row < n_rows ? *reinterpret_cast<const uint4 *>(rg + x) : make_uint4(0u, 0u, 0u, 0u);
+                }
+        }
+    }
+#pragma unroll
+    for (int i = 1; i < kGqaStages; ++i) load_tile(i);
+    if (!words) {
 #pragma unroll
         for (int h = 0; h < QF / 2; ++h)
 #pragma unroll
             for (int j = 0; j < QC; ++j) {
-                const int row = g + 8 * h;
-                qx[h][j] = rx[h][j] = make_uint4(0u, 0u, 0u, 0u);
-                if (row < n_rows) {
-                    qx[h][j] = *reinterpret_cast<const uint4 *>(qg + row * D + 32 * j);
-                    rx[h][j] = *reinterpret_cast<const uint4 *>(rg + row * D + 32 * j);
-                }
+                auto trade = [&](const uint4 &x, uint32_t (&f)[KS][QF]) {
+                    uint32_t w[4] = {x.x, x.y, x.z, x.w};
+                    sm100::quad_transpose(w, t);               // w[i]: channels 2 t, + 1 of chunk 4 j + i
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) f[2 * j + (i >> 1)][FEW ? i & 1 : h + 2 * (i & 1)] = w[i];
+                };
+                trade(qx[h][j], qa);
+                trade(rx[h][j], ra);
             }
     }
-#pragma unroll
-    for (int i = 1; i < kGqaStages; ++i) load_tile(i);
-#pragma unroll
-    for (int h = 0; h < QF / 2; ++h)
-#pragma unroll
-        for (int j = 0; j < QC; ++j) {
-            auto trade = [&](const uint4 &x, uint32_t (&f)[KS][QF]) {
-                uint32_t w[4] = {x.x, x.y, x.z, x.w};
-                sm100::quad_transpose(w, t);                   // w[i]: channels 2 t, + 1 of chunk 4 j + i
-#pragma unroll
-                for (int i = 0; i < 4; ++i) f[2 * j + (i >> 1)][FEW ? i & 1 : h + 2 * (i & 1)] = w[i];
-            };
-            trade(qx[h][j], qa);
-            trade(rx[h][j], ra);
-        }
 
     // State of two rows of the group, g and g + 8 (FEW: 2 t and 2 t + 1); d1 / d2 are this thread's share until the end.
     // Accumulators: channels 8 i + 2 t, + 1 of the two rows (FEW: channels 16 i + g and + 8).
@@ -1350,10 +1364,10 @@ __global__ void __launch_bounds__(kGqaWarps * 32, 1) decode_gqa_kernel(const Dec
     constexpr int kAhead = FEW ? 16 : 8;
     for (int row = warp - w0; row < n_rows; row += n_seg) {
         const float *recs = recs_of(row);
-        warp_merge<D, kAhead>(recs, min(n_ctas, 32), lane, big, D1, D2, O1, O2);
+        warp_merge<D, kAhead, true>(recs, min(n_ctas, 32), lane, big, D1, D2, O1, O2);
         for (int j = 32; j < n_ctas; j += 32) {
             float big2, E1, E2, P1[CH], P2[CH];
-            warp_merge<D, kAhead>(recs + static_cast<int64_t>(j) * REC, min(n_ctas - j, 32), lane, big2, E1, E2, P1, P2);
+            warp_merge<D, kAhead, true>(recs + static_cast<int64_t>(j) * REC, min(n_ctas - j, 32), lane, big2, E1, E2, P1, P2);
             const float top = fmaxf(big, big2), safe = top == -INFINITY ? 0.f : top;
             const float wa = fast_exp2(big - safe), wb = fast_exp2(big2 - safe);
             big = top;
